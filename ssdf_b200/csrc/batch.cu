@@ -41,7 +41,7 @@ struct ssdf_batch {
     BatchHeader *h_hdr = nullptr;  // [2]
     QueryArgs *h_jobs = nullptr, *h_jobs64 = nullptr;
     long long *h_first = nullptr, *h_first64 = nullptr;
-    // captured graphs, one per (warp, wide, budget, FP64 table) key: a run reuses the graph of its key
+    // captured graphs, one per (warp, wide, FP64 table) key: a run reuses the graph of its key
     cudaGraphExec_t exec[16] = {};
     int sms = 0;
     long long last_total = 0;
@@ -68,9 +68,8 @@ static void batch_free(ssdf_batch *b) {
 // The launch sequence of one run with the given traversal and arity: counters reset, then the
 // persistent kernel and the window stage, then (f64) the persistent FP64 kernel over the second
 // table. It reads the job tables from device memory only.
-static int enqueue_run(ssdf_batch *b, bool warp, bool wide, bool budget, bool f64, cudaStream_t s) {
+static int enqueue_run(ssdf_batch *b, bool warp, bool wide, bool f64, cudaStream_t s) {
     BatchLaunch L;
-    L.budget = budget;
     L.hdr = b->d_hdr;
     L.jobs = b->d_jobs;
     L.first_block = b->d_first;
@@ -85,7 +84,6 @@ static int enqueue_run(ssdf_batch *b, bool warp, bool wide, bool budget, bool f6
     SSDF_CHECK(launch_batch(L, b->precision, s));
     if (!f64) return SSDF_OK;
     BatchLaunch D = L;
-    D.budget = false;
     D.hdr = b->d_hdr + 1;
     D.jobs = b->d_jobs64;
     D.first_block = b->d_first64;
@@ -94,20 +92,14 @@ static int enqueue_run(ssdf_batch *b, bool warp, bool wide, bool budget, bool f6
     return launch_batch(D, SSDF_PREC_F64, s);
 }
 
-// The packet budget exists for the fix-up kernel's packet walks (binary and 4-wide).
-static bool budget_applies(const ssdf_batch *b, bool warp, bool wide) {
-    (void)wide;
-    return b->precision == SSDF_PREC_F32_FIXUP && warp;
+static int graph_key(bool warp, bool wide, bool f64) {
+    return (warp ? 1 : 0) | (wide ? 2 : 0) | (f64 ? 4 : 0);
 }
 
-static int graph_key(bool warp, bool wide, bool budget, bool f64) {
-    return (warp ? 1 : 0) | (wide ? 2 : 0) | (budget ? 4 : 0) | (f64 ? 8 : 0);
-}
-
-// Captures (once) the graph of a (traversal, arity, budget, FP64 table) key on a private stream,
+// Captures (once) the graph of a (traversal, arity, FP64 table) key on a private stream,
 // thread-local mode.
-static int capture_key(ssdf_batch *b, bool warp, bool wide, bool budget, bool f64) {
-    const int key = graph_key(warp, wide, budget, f64);
+static int capture_key(ssdf_batch *b, bool warp, bool wide, bool f64) {
+    const int key = graph_key(warp, wide, f64);
     if (b->exec[key]) return SSDF_OK;
     cudaStream_t cap;
     SSDF_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
@@ -115,7 +107,7 @@ static int capture_key(ssdf_batch *b, bool warp, bool wide, bool budget, bool f6
     cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
     int st = SSDF_OK;
     if (e == cudaSuccess) {
-        st = enqueue_run(b, warp, wide, budget, f64, cap);
+        st = enqueue_run(b, warp, wide, f64, cap);
         e = cudaStreamEndCapture(cap, &g);
     }
     if (e == cudaSuccess && st == SSDF_OK) e = cudaGraphInstantiate(&b->exec[key], g, 0);
@@ -135,11 +127,8 @@ int batch_capture_graphs(ssdf_batch *b) {
         for (int wide = 0; wide < 2; wide++) {
             if ((b->traversal == 1 && !warp) || (b->traversal == 2 && warp)) continue;
             if ((b->arity == 2 && wide) || (b->arity == 4 && !wide)) continue;
-            for (int f64 = 0; f64 < (b->precision == SSDF_PREC_F32_FIXUP ? 2 : 1); f64++) {
-                SSDF_CHECK(capture_key(b, warp != 0, wide != 0, false, f64 != 0));
-                if (budget_applies(b, warp != 0, wide != 0))
-                    SSDF_CHECK(capture_key(b, warp != 0, wide != 0, true, f64 != 0));
-            }
+            for (int f64 = 0; f64 < (b->precision == SSDF_PREC_F32_FIXUP ? 2 : 1); f64++)
+                SSDF_CHECK(capture_key(b, warp != 0, wide != 0, f64 != 0));
         }
     return SSDF_OK;
 }
@@ -202,9 +191,9 @@ static int batch_add(ssdf_batch *b, const QueryArgs &a, const ssdf_query_opts *o
     if (opts->precision != b->precision)
         return fail(SSDF_ERR_INVALID_ARGUMENT, "a batch runs one arithmetic: job precision differs from the batch's");
     if (int(b->jobs.size()) >= b->max_jobs) return fail(SSDF_ERR_INVALID_ARGUMENT, "batch is full");
-    if (b->precision == SSDF_PREC_F64 && !a.m.nodes64)
+    if (b->precision == SSDF_PREC_F64 && !a.m.tris64)
         return fail(SSDF_ERR_INVALID_ARGUMENT, "mesh built without double data (keep_fp64=0)");
-    if (b->precision == SSDF_PREC_F32_FIXUP && (!a.m.tris64 || !a.m.nodes64 || !a.m.filt32))
+    if (b->precision == SSDF_PREC_F32_FIXUP && (!a.m.tris64 || !a.m.filt32))
         return fail(SSDF_ERR_INVALID_ARGUMENT, "fix-up queries need the double triangles and BVH (keep_fp64=1)");
     if (a.output == SSDF_OUT_SDF && (!a.m.face_n || !a.m.tris64))
         return fail(SSDF_ERR_INVALID_ARGUMENT, "signed queries need a mesh built with normals=1 and keep_fp64=1");
@@ -314,7 +303,7 @@ int ssdf_batch_run(ssdf_batch *b, int use_graph, void *stream_) {
     int k = 0, k64 = 0;
     for (int r = 0; r < njobs; r++) {
         QueryArgs a = b->jobs[order[r]];
-        a.warp_budget = resolve_warp_budget(a.warp_budget, nq, a.m.nt);
+        a.warp_budget = resolve_warp_budget(a.warp_budget, nq, a.m.nt, a.is_grid != 0);
         if (a.is_grid) a.grid_steps = steps;
         if (sort_points && !a.is_grid && a.npoints >= kSortMinPoints) {
             int *ord = nullptr;
@@ -361,13 +350,10 @@ int ssdf_batch_run(ssdf_batch *b, int use_graph, void *stream_) {
         SSDF_CUDA(
             cudaMemcpyAsync(b->d_first64, b->h_first64, sizeof(long long) * k64, cudaMemcpyHostToDevice, stream));
     }
-    bool budget = false;
-    for (int j = 0; j < k; j++) budget |= b->h_jobs[j].warp_budget > 0;
-    budget = budget && budget_applies(b, warp, wide);
     const bool f64 = k64 > 0;
-    if (!use_graph) return enqueue_run(b, warp, wide, budget, f64, stream);
-    SSDF_CHECK(capture_key(b, warp, wide, budget, f64));
-    SSDF_CUDA(cudaGraphLaunch(b->exec[graph_key(warp, wide, budget, f64)], stream));
+    if (!use_graph) return enqueue_run(b, warp, wide, f64, stream);
+    SSDF_CHECK(capture_key(b, warp, wide, f64));
+    SSDF_CUDA(cudaGraphLaunch(b->exec[graph_key(warp, wide, f64)], stream));
     return SSDF_OK;
 }
 

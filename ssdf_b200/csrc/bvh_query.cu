@@ -2,9 +2,9 @@
 //
 // Stands in for the reference's device query (serial/bvh/bvh.cu:60-76 + cuBQL CPAT) and its CPU
 // grid samplers (serial/bvh/bvh.cpp:1574-1798). Three arithmetics (SSDF_PREC_*):
-//   F64   double nodes and triangles, the reference's exact double expression; lexicographic
+//   F64   the reference's exact double expression per triangle; lexicographic
 //         (d^2, triangle index) minimum: bitwise the reference's double value;
-//   F32   the same over float nodes/triangles with the reference's float expression (its
+//   F32   the same over float triangles with the reference's float expression (its
 //         edf<float> value);
 //   F32X  float traversal with fused multiply-adds keeps the K smallest float d^2 inside a
 //         window (sqrt(best) + tau)^2; the window's members are re-evaluated in double and the
@@ -14,7 +14,10 @@
 //         warp per query).
 //         Result: bitwise the F64 result.
 // Traversal: nearest child first, the farther one pushed with its box distance on a per-lane stack
-// and culled on pop against the current thresholds. Each lane answers kQ queries (a build option;
+// and culled on pop against the current thresholds. All three walk the same float tree of oriented boxes
+// (DeviceMesh::obb), whose distances are lower bounds in every arithmetic: on the torus-knot 256^3 grid
+// a 32-query packet visits 86 nodes and 59 triangles where it met 140 and 197 with axis-aligned boxes
+// (16.6 -> 10.1 ms; plain double 31.1 -> 11.4 ms). Each lane answers kQ queries (a build option;
 // 1 by default, 2 measured no faster: it shares each node and triangle load between two chains of
 // arithmetic but costs the registers of the second). Grid queries map a
 // warp to a 4 x 4 x 2kQ brick of nodes, so the warp's traversals stay coherent; by default a grid
@@ -47,13 +50,13 @@ constexpr int kThreads = 128;
 #endif
 constexpr int kCand = SSDF_B200_WINDOW_SLOTS;
 
-// Minimum resident blocks per SM the float query kernels are compiled for: 10 blocks of 128 cap
-// them at 48 registers (the fix-up window lives in shared memory). The traversal is issue-latency
-// bound, so the occupancy this buys outweighs the spills (measured on the torus-knot grid with the
-// packed box test: 16.79 ms against 17.22 ms for 9 blocks at 56 registers, 17.72 ms for 8 at 64 and
-// 16.77 ms for 11 at 40); the double kernel keeps its registers.
+// Minimum resident blocks per SM the float query kernels are compiled for: 7 blocks of 128 (72
+// registers). A node visit loads 128 bytes into registers, so the kernels want more of them than with
+// 64-byte axis-aligned nodes (whose best was 10 blocks at 48). Torus-knot 256^3 grid, fix-up: 10.15 ms
+// at 7, 10.33 at 8, 10.68 at 9, 11.47 at 10; 4M points on the beam lattice, float: 5.34 / 5.45 / 5.38 /
+// 5.63 ms.
 #ifndef SSDF_B200_QUERY_MIN_BLOCKS
-#define SSDF_B200_QUERY_MIN_BLOCKS 10
+#define SSDF_B200_QUERY_MIN_BLOCKS 7
 #endif
 
 // The double kernel keeps 5 resident blocks per SM (at most 102 registers), its occupancy before the
@@ -81,13 +84,16 @@ __device__ __forceinline__ bool map_query(const QueryArgs &a, long long b, int s
         q = a.order ? (long long)__ldg(a.order + slot) : slot;
         return true;
     }
-    const long long bxn = grid_blocks_x(a.nx), byn = grid_blocks_y(a.ny);
-    const long long bx = b % bxn, r = b / bxn;
-    const long long by = r % byn, bz = r / byn;
+    // fewer than 2^31 blocks: 32-bit divisions
+    const unsigned bxn = unsigned(grid_blocks_x(a.nx)), byn = unsigned(grid_blocks_y(a.ny));
+    const unsigned r = unsigned(b) / bxn;
+    const long long bx = unsigned(b) - r * bxn;
+    const unsigned bz = r / byn;
+    const long long by = r - bz * byn;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     i = bx * 8 + (warp & 1) * 4 + (lane & 3);
     j = by * 4 + ((lane >> 2) & 3);
-    k = (((bz * a.grid_steps + step) * 4 + (warp >> 1) * 2) + (lane >> 4)) * kQ + s;
+    k = ((((long long)bz * a.grid_steps + step) * 4 + (warp >> 1) * 2) + (lane >> 4)) * kQ + s;
     q = i + a.nx * (j + a.ny * k);
     return i < a.nx && j < a.ny && k < a.nz;
 }
@@ -134,40 +140,6 @@ __device__ __forceinline__ void store_out(const QueryArgs &a, long long q, doubl
 
 // ---- node and triangle loads ----------------------------------------------------------------------
 
-struct Node32 {
-    float4 a, b, c;
-    int r0, r1;
-};
-__device__ __forceinline__ Node32 load_node32(const float4 *__restrict__ nodes, int n) {
-    Node32 o;
-    o.a = __ldg(nodes + 4 * n);
-    o.b = __ldg(nodes + 4 * n + 1);
-    o.c = __ldg(nodes + 4 * n + 2);
-    const float4 d = __ldg(nodes + 4 * n + 3);
-    o.r0 = __float_as_int(d.x);
-    o.r1 = __float_as_int(d.y);
-    return o;
-}
-
-struct Node64 {
-    double2 x0, y0, z0, x1, y1, z1;
-    int r0, r1;
-};
-__device__ __forceinline__ Node64 load_node64(const double2 *__restrict__ nodes, int n) {
-    Node64 o;
-    const double2 *p = nodes + 8 * n;
-    o.x0 = __ldg(p);
-    o.y0 = __ldg(p + 1);
-    o.z0 = __ldg(p + 2);
-    o.x1 = __ldg(p + 3);
-    o.y1 = __ldg(p + 4);
-    o.z1 = __ldg(p + 5);
-    const double2 r = __ldg(p + 6);
-    o.r0 = int((unsigned)__double_as_longlong(r.x));
-    o.r1 = int((unsigned)__double_as_longlong(r.y));
-    return o;
-}
-
 // 4-wide node: per child c, box (lox, hix, loy, hiy, loz, hiz)[c] and reference r[c].
 template <typename T>
 __device__ __forceinline__ void boxes4_exact(const DeviceMesh &m, int node, T px, T py, T pz, T (&d)[4], int (&r)[4]);
@@ -204,22 +176,8 @@ __device__ __forceinline__ void boxes4_exact<double>(const DeviceMesh &m, int no
     r[0] = int(unsigned(a)), r[1] = int(unsigned(a >> 32)), r[2] = int(unsigned(b)), r[3] = int(unsigned(b >> 32));
 }
 
-// box_dist_sq_fast of both children of a node at once, bit for bit: the clamps per child, the
-// differences and the squared norms as packed FP32 pairs (child 0, child 1) of sm_100's
-// two-wide FP32 instructions (__fadd2_rn, __fmul2_rn and __ffma2_rn round each half as the scalar
-// operation does). One node visit issues 18 instructions for the two boxes instead of 24.
-__device__ __forceinline__ float2 box_dist_sq_pair(const float px, const float py, const float pz, const Node32 &n) {
-    const float2 dx = __fadd2_rn(make_float2(px, px), make_float2(-fminf(fmaxf(px, n.a.x), n.a.y),
-                                                                  -fminf(fmaxf(px, n.b.x), n.b.y)));
-    const float2 dy = __fadd2_rn(make_float2(py, py), make_float2(-fminf(fmaxf(py, n.a.z), n.a.w),
-                                                                  -fminf(fmaxf(py, n.b.z), n.b.w)));
-    const float2 dz = __fadd2_rn(make_float2(pz, pz), make_float2(-fminf(fmaxf(pz, n.c.x), n.c.y),
-                                                                  -fminf(fmaxf(pz, n.c.z), n.c.w)));
-    return __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-}
-
-// The 4-wide node's child-box distances (box_dist_sq_fast's, bit for bit), children (0, 1) and (2, 3)
-// as packed FP32 pairs.
+// The 4-wide node's child-box distances (p - clamp(p, lo, hi) per axis, fused squared norm), children
+// (0, 1) and (2, 3) as packed FP32 pairs.
 __device__ __forceinline__ void boxes4_pair(const DeviceMesh &m, int node, float px, float py, float pz,
                                             float (&d)[4], int (&r)[4]) {
     const float4 *p = m.nodes4_32 + 8 * node;
@@ -278,57 +236,77 @@ struct ExactData;
 template <>
 struct ExactData<double> {
     using Tri = Tri64;
-    static constexpr double rel = 1.0 + 1.0 / 65536.0;
-    static __device__ __forceinline__ double abs_margin(float scale) {
-        const double s = double(scale) * 0x1p-40;
+    // squared margin added to the prune threshold
+    static __device__ __forceinline__ double margin(const DeviceMesh &m) {
+        const double s = double(m.coord_scale) * 0x1p-40;
         return s * s;
     }
-    static __device__ __forceinline__ Node64 node(const DeviceMesh &m, int n) { return load_node64(m.nodes64, n); }
-    static __device__ __forceinline__ void boxes(const Node64 &n, double px, double py, double pz, double &d0,
-                                                 double &d1) {
-        d0 = box_dist_sq<double>(px, py, pz, n.x0.x, n.x0.y, n.y0.x, n.y0.y, n.z0.x, n.z0.y);
-        d1 = box_dist_sq<double>(px, py, pz, n.x1.x, n.x1.y, n.y1.x, n.y1.y, n.z1.x, n.z1.y);
+    // the float threshold of the boxes (in the box frame's scale), rounded up
+    static __device__ __forceinline__ float box_thr(double best, double margin, const DeviceMesh &m) {
+        const double t = (best * (1.0 + 1.0 / 65536.0) + margin) * (double(m.box_scale) * double(m.box_scale));
+        return fmaxf(__double2float_ru(t), FLT_MIN);  // a box at distance 0 is always wanted
     }
+    static __device__ __forceinline__ float box_coord(double p, int d, const DeviceMesh &m) {
+        return float((p - double(m.box_c[d])) * double(m.box_scale));
+    }
+    // a threshold beyond float's range is +inf: a box distance that overflowed still counts as inside
+    static __device__ __forceinline__ float box_key(float d) { return fminf(d, FLT_MAX); }
+    static __device__ __forceinline__ float key_of(double d) { return fminf(__double2float_rd(d), FLT_MAX); }
     static __device__ __forceinline__ Tri tri(const DeviceMesh &m, int pos) { return load_tri64(m.tris64, pos); }
 };
 template <>
 struct ExactData<float> {
     using Tri = Tri32;
-    static constexpr float rel = 1.0f + 1.0f / 65536.0f;
-    static __device__ __forceinline__ float abs_margin(float scale) {
-        const float s = scale * 0x1p-16f;
-        return s * s;
+    // distance margin of the prune threshold: the float vertices against the (perhaps double) ones the
+    // boxes hold, and the float squared distances' absolute error
+    static __device__ __forceinline__ float margin(const DeviceMesh &m) { return m.coord_scale * 0x1p-16f; }
+    static __device__ __forceinline__ float box_thr(float best, float margin, const DeviceMesh &m) {
+        const float d = sqrtf(best) + 0x1p-7f * margin;  // 2^-23 of the coordinates' magnitude
+        const float t = fmaxf(d * d, best + margin * margin) * (1.0f + 1.0f / 65536.0f);
+        return fmaxf(t * m.box_scale * m.box_scale, FLT_MIN);
     }
-    static __device__ __forceinline__ Node32 node(const DeviceMesh &m, int n) { return load_node32(m.nodes32, n); }
-    static __device__ __forceinline__ void boxes(const Node32 &n, float px, float py, float pz, float &d0, float &d1) {
-        d0 = box_dist_sq<float>(px, py, pz, n.a.x, n.a.y, n.a.z, n.a.w, n.c.x, n.c.y);
-        d1 = box_dist_sq<float>(px, py, pz, n.b.x, n.b.y, n.b.z, n.b.w, n.c.z, n.c.w);
+    static __device__ __forceinline__ float box_coord(float p, int d, const DeviceMesh &m) {
+        return (p - m.box_c[d]) * m.box_scale;
     }
+    static __device__ __forceinline__ float box_key(float d) { return d; }
+    static __device__ __forceinline__ float key_of(float d) { return d; }
     static __device__ __forceinline__ Tri tri(const DeviceMesh &m, int pos) { return load_tri32(m.tris32, pos); }
 };
 
+__device__ __forceinline__ float2 twice(float v) { return make_float2(v, v); }
+// Box coordinate of a lane without a query: farther from every box than any query's.
+constexpr float kNowhere = 0x1p62f;
+
 // Lexicographic (d^2, id) minimum over all triangles, starting from (best, -1): a triangle replaces
 // the incumbent if strictly closer, or equally close with a lower index (never the initial bound on
-// a tie). Boxes are kept while their distance is below best * (1 + 2^-16) + margin, so rounding in
-// box distances never drops a tie.
+// a tie). The walk is float in either arithmetic: oriented boxes whose float distance is a lower bound
+// of their triangles' are kept while it is below best * (1 + 2^-16) + margin, so neither rounding in box
+// distances nor the conversion drops a tie. (Walking float boxes instead of double ones took the
+// plain double kernel's nodes off its FP64 pipe, which was 52 % busy.) A point with a NaN or infinite
+// coordinate has no finite distance to anything: it keeps its incoming bound without a walk.
 template <typename T, int Q>
 struct ExactPolicy {
-    using R = T;
+    using R = float;
     static constexpr int kQn = Q;
     const DeviceMesh &m;
-    T px[Q], py[Q], pz[Q], best[Q], thr[Q];
+    T px[Q], py[Q], pz[Q], best[Q];
+    float2 bx[Q], by[Q], bz[Q];  // the point in the box frame, each coordinate twice (two-wide FP32)
+    float thr[Q];
     int bid[Q], bpos[Q];
     T margin;
-    __device__ explicit ExactPolicy(const DeviceMesh &mesh) : m(mesh) {
-        margin = ExactData<T>::abs_margin(m.coord_scale);
-    }
+    __device__ explicit ExactPolicy(const DeviceMesh &mesh) : m(mesh) { margin = ExactData<T>::margin(m); }
     __device__ __forceinline__ void set(int q, T x, T y, T z, T init) {
         px[q] = x, py[q] = y, pz[q] = z, best[q] = init, bid[q] = -1, bpos[q] = -1;
-        thr[q] = init * ExactData<T>::rel + margin;
+        bx[q] = twice(ExactData<T>::box_coord(x, 0, m));
+        by[q] = twice(ExactData<T>::box_coord(y, 1, m));
+        bz[q] = twice(ExactData<T>::box_coord(z, 2, m));
+        const bool finite = isfinite(x) && isfinite(y) && isfinite(z);
+        thr[q] = finite ? ExactData<T>::box_thr(init, margin, m) : -1.f;
     }
     __device__ __forceinline__ void disable(int q) {
         px[q] = py[q] = pz[q] = T(0), best[q] = T(0), bid[q] = -1, bpos[q] = -1;
-        thr[q] = T(-1);
+        bx[q] = by[q] = bz[q] = twice(kNowhere);
+        thr[q] = -1.f;
     }
     // Starts query q from the triangle at leaf position pos, as if the walk had tested it first (it
     // replaces the incoming bound only when strictly closer; the walk meets it again without effect).
@@ -339,27 +317,28 @@ struct ExactPolicy {
             best[q] = d2;
             bid[q] = t.id;
             bpos[q] = pos;
-            thr[q] = best[q] * ExactData<T>::rel + margin;
+            thr[q] = ExactData<T>::box_thr(best[q], margin, m);
         }
     }
-    __device__ __forceinline__ void boxes(int node, T (&d0)[Q], T (&d1)[Q], int &r0, int &r1) const {
-        const auto n = ExactData<T>::node(m, node);
+    __device__ __forceinline__ void boxes(int node, float (&d0)[Q], float (&d1)[Q], int &r0, int &r1) const {
 #pragma unroll
-        for (int q = 0; q < Q; q++) ExactData<T>::boxes(n, px[q], py[q], pz[q], d0[q], d1[q]);
-        r0 = n.r0;
-        r1 = n.r1;
+        for (int q = 0; q < Q; q++) {
+            const float2 d = obb_dist_sq_pair(bx[q], by[q], bz[q], m.obb + 8 * node, r0, r1);
+            d0[q] = ExactData<T>::box_key(d.x);
+            d1[q] = ExactData<T>::box_key(d.y);
+        }
     }
-    __device__ __forceinline__ void boxes4(int node, T (&d)[4][Q], int (&r)[4]) const {
+    __device__ __forceinline__ void boxes4(int node, float (&d)[4][Q], int (&r)[4]) const {
 #pragma unroll
         for (int q = 0; q < Q; q++) {
             T dq[4];
             boxes4_exact<T>(m, node, px[q], py[q], pz[q], dq, r);
 #pragma unroll
-            for (int c = 0; c < 4; c++) d[c][q] = dq[c];
+            for (int c = 0; c < 4; c++) d[c][q] = ExactData<T>::key_of(dq[c] * T(m.box_scale) * T(m.box_scale));
         }
     }
-    __device__ __forceinline__ T max_thr() const {
-        T t = thr[0];
+    __device__ __forceinline__ float max_thr() const {
+        float t = thr[0];
 #pragma unroll
         for (int q = 1; q < Q; q++) t = t > thr[q] ? t : thr[q];
         return t;
@@ -378,7 +357,7 @@ struct ExactPolicy {
                     best[q] = d2;
                     bid[q] = t.id;
                     bpos[q] = first + k;
-                    thr[q] = best[q] * ExactData<T>::rel + margin;
+                    thr[q] = ExactData<T>::box_thr(best[q], margin, m);
                 }
             }
         }
@@ -408,13 +387,19 @@ __device__ __forceinline__ float window_thr(float best, float tau_rel, float sca
     return w * w * (1.0f + 1.0f / 65536.0f);
 }
 
+// A query coordinate as the filter and its boxes take it: less the mesh's middle, rounded once.
+__device__ __forceinline__ float filter_coord(double p, int d, const DeviceMesh &m) {
+    return float(p - double(m.box_c[d]));
+}
+
 template <int Q>
 struct FastPolicy {
     using R = float;
     static constexpr int kQn = Q;
     static constexpr bool kBudgeted = true;
     const DeviceMesh &m;
-    float px[Q], py[Q], pz[Q], best[Q], thr[Q], evicted[Q];
+    float2 bx[Q], by[Q], bz[Q];  // the point in the box frame (the filter records' too), each coordinate twice
+    float best[Q], thr[Q], evicted[Q];
     int used[Q];  // window slots in use
     float tau_rel;
     float *wd;
@@ -423,11 +408,13 @@ struct FastPolicy {
         : m(mesh), tau_rel(tau), wd(sd + threadIdx.x), wp(sp + threadIdx.x) {}
     __device__ __forceinline__ int slot(int q, int s) const { return (q * kCand + s) * kThreads; }
     __device__ __forceinline__ void set(int q, float x, float y, float z, float init) {
-        px[q] = x, py[q] = y, pz[q] = z, best[q] = init, evicted[q] = finf(), used[q] = 0;
-        thr[q] = window_thr(init, tau_rel, m.coord_scale);
+        bx[q] = twice(x), by[q] = twice(y), bz[q] = twice(z), best[q] = init, evicted[q] = finf(), used[q] = 0;
+        // a NaN or infinite coordinate: no finite distance, nothing to walk for
+        const bool finite = isfinite(x) && isfinite(y) && isfinite(z);
+        thr[q] = finite ? window_thr(init, tau_rel, m.coord_scale) : -1.f;
     }
     __device__ __forceinline__ void disable(int q) {
-        set(q, 0.f, 0.f, 0.f, finf());
+        set(q, kNowhere, kNowhere, kNowhere, finf());
         thr[q] = -1.f;
     }
     // Starts query q's window from the key of the triangle at leaf position pos (not a proxy), as the
@@ -435,7 +422,7 @@ struct FastPolicy {
     // the triangle when it meets it.
     __device__ __forceinline__ void seed(int q, int pos) {
         const FiltRec t = load_filt(m.filt32, pos);
-        const float d2 = tri_dist_sq_filter(px[q], py[q], pz[q], t);
+        const float d2 = tri_dist_sq_filter(bx[q].x, by[q].x, bz[q].x, t);
         if (t.pen == 0.f && d2 < best[q]) {
             best[q] = d2;
             thr[q] = window_thr(best[q], tau_rel, m.coord_scale);
@@ -448,21 +435,18 @@ struct FastPolicy {
             if (thr[q] > 0.f) evicted[q] = 0.f;
     }
     __device__ __forceinline__ void boxes(int node, float (&d0)[Q], float (&d1)[Q], int &r0, int &r1) const {
-        const Node32 n = load_node32(m.nodes32, node);
 #pragma unroll
         for (int q = 0; q < Q; q++) {
-            const float2 d = box_dist_sq_pair(px[q], py[q], pz[q], n);
+            const float2 d = obb_dist_sq_pair(bx[q], by[q], bz[q], m.obb + 8 * node, r0, r1);
             d0[q] = d.x;
             d1[q] = d.y;
         }
-        r0 = n.r0;
-        r1 = n.r1;
     }
     __device__ __forceinline__ void boxes4(int node, float (&d)[4][Q], int (&r)[4]) const {
 #pragma unroll
         for (int q = 0; q < Q; q++) {
             float dq[4];
-            boxes4_pair(m, node, px[q], py[q], pz[q], dq, r);
+            boxes4_pair(m, node, bx[q].x + m.box_c[0], by[q].x + m.box_c[1], bz[q].x + m.box_c[2], dq, r);
 #pragma unroll
             for (int c = 0; c < 4; c++) d[c][q] = dq[c];
         }
@@ -513,7 +497,7 @@ struct FastPolicy {
 #pragma unroll
             for (int q = 0; q < Q; q++) {
                 if (!((mask >> q) & 1u)) continue;
-                const float d2 = tri_dist_sq_filter(px[q], py[q], pz[q], t);
+                const float d2 = tri_dist_sq_filter(bx[q].x, by[q].x, bz[q].x, t);
                 if (COUNT) cnt.tri++;
                 if (d2 < thr[q]) {
                     insert(q, d2, first + k);
@@ -543,13 +527,6 @@ __device__ __forceinline__ R min_of(const R (&d)[Q]) {
     return v;
 }
 
-// Stack entries of a packet walk hold a float: distances round down and thresholds up, so the
-// float comparison never culls what the exact one would keep.
-__device__ __forceinline__ float stack_key_lo(float d) { return d; }
-__device__ __forceinline__ float stack_key_lo(double d) { return __double2float_rd(d); }
-__device__ __forceinline__ float stack_key_hi(float t) { return t; }
-__device__ __forceinline__ float stack_key_hi(double t) { return __double2float_ru(t); }
-
 // Policies that can hand their queries to a second stage (P::kBudgeted) stop a packet's walk after a
 // work budget; the others always finish it.
 template <class P, class = void>
@@ -563,76 +540,90 @@ constexpr bool budgeted() {
 
 constexpr int kRepLane = 21;  // (1, 1, 1) of the 4 x 4 x 2 brick
 
+// Warp minimum / maximum of a float (sm_100's redux on floats).
+__device__ __forceinline__ float warp_min(float v) {
+    float r;
+    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 // Packet walk (a grid warp as one packet): the node ids on the stack are the same in every lane, so
 // the warp keeps one stack in shared memory instead of 32 copies in local memory. An entry keeps
-// the smallest box distance over the warp's lanes (one redux.sync on the float bits, which order
-// like the values for non-negative floats) and is entered on pop while that is below the largest
-// lane threshold: a superset of "some lane's distance below its own threshold", so never a miss.
-template <bool COUNT, bool BUDGET, class P>
+// the smallest box distance over the warp's lanes and is entered on pop while that is below the
+// largest lane threshold: a superset of "some lane's distance below its own threshold", so never a
+// miss. Lanes without a query sit far from the mesh (P::disable), so they take no part in the keys.
+// Of two wanted children the one the brick's centre lane ranks first is the nearer; a wanted leaf is
+// tested at once, and when it was the nearer one the other child is asked for again, its lanes'
+// thresholds having shrunk.
+template <bool COUNT, class P>
 __device__ __forceinline__ void traverse_packet(P &p, Counters &cnt, int budget) {
-    using R = typename P::R;
     constexpr int Q = P::kQn;
     constexpr unsigned kAll = 0xffffffffu;
-    int work = 0;  // triangle records the packet has tested (the same in every lane; BUDGET only)
+    int work = 0;  // triangle records the packet has tested (the same in every lane)
     if (budget <= 0) budget = 0x7fffffff;
-    __shared__ int s_node[kThreads / 32][kStackSize];
-    __shared__ float s_dist[kThreads / 32][kStackSize];
-    int *snode = s_node[threadIdx.x >> 5];
-    float *sdist = s_dist[threadIdx.x >> 5];
-    const bool live = p.max_thr() >= R(0);  // lanes without a query take no part in the keys
+    __shared__ int2 s_entry[kThreads / 32][kStackSize];  // node, key bits
+    int2 *const entry = s_entry[threadIdx.x >> 5];
     int sp = 0;
     int node = 0;
+    auto test_leaf = [&](int ref, unsigned m) {
+        p.template leaf<COUNT>(leaf_first(ref), leaf_count(ref), m, cnt);
+        if constexpr (budgeted<P>()) work += leaf_count(ref);
+    };
     while (true) {
-        R d0[Q], d1[Q];
+        float d0[Q], d1[Q];
         int r0, r1;
         p.boxes(node, d0, d1, r0, r1);
         if (COUNT) cnt.box += 2 * Q;
-        R k0 = min_of<R, Q>(d0), k1 = min_of<R, Q>(d1);
-        if (__shfl_sync(kAll, k1 < k0, kRepLane)) {  // the nearer child for the brick's centre lane
-#pragma unroll
-            for (int q = 0; q < Q; q++) {
-                const R t = d0[q];
-                d0[q] = d1[q];
-                d1[q] = t;
-            }
-            const R tk = k0;
-            k0 = k1;
-            k1 = tk;
-            const int tr = r0;
-            r0 = r1;
-            r1 = tr;
-        }
+        const unsigned m0 = want_mask(p, d0), m1 = r1 == kEmptyRef ? 0u : want_mask(p, d1);
+        const bool any0 = __any_sync(kAll, m0 != 0u), any1 = __any_sync(kAll, m1 != 0u);
         int next = -1;
+        if (any0 && any1) {
+            const float k0 = min_of<float, Q>(d0), k1 = min_of<float, Q>(d1);
+            const bool swap = (__ballot_sync(kAll, k1 < k0) >> kRepLane) & 1u;
+            const int rn = swap ? r1 : r0, rf = swap ? r0 : r1;
+            if (rf >= 0 && rn >= 0) {
+                if (sp < kStackSize) {
+                    entry[sp] = make_int2(rf, __float_as_int(warp_min(swap ? k0 : k1)));  // every lane stores the same
+                    sp++;
+                }
+                next = rn;
+            } else if (rn >= 0) {
+                test_leaf(rf, swap ? m0 : m1);
+                next = rn;
+            } else {
+                test_leaf(rn, swap ? m1 : m0);
+                float df[Q];
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int rc = h ? r1 : r0;
-            const unsigned m = rc == kEmptyRef ? 0u : (h ? want_mask(p, d1) : want_mask(p, d0));
-            if (!__any_sync(kAll, m != 0u)) continue;
-            if (rc < 0) {
-                p.template leaf<COUNT>(leaf_first(rc), leaf_count(rc), m, cnt);
-                if constexpr (BUDGET && budgeted<P>()) work += leaf_count(rc);
-            } else if (next < 0) {
-                next = rc;
-            } else if (sp < kStackSize) {
-                const float key = live ? stack_key_lo(h ? k1 : k0) : finf();
-                snode[sp] = rc;  // every lane stores the same values
-                sdist[sp] = __uint_as_float(__reduce_min_sync(kAll, __float_as_uint(key)));
-                sp++;
+                for (int q = 0; q < Q; q++) df[q] = swap ? d0[q] : d1[q];
+                const unsigned mf = want_mask(p, df);
+                if (__any_sync(kAll, mf != 0u)) {
+                    if (rf < 0) test_leaf(rf, mf);
+                    else next = rf;
+                }
             }
+        } else if (any0 || any1) {
+            const int r = any0 ? r0 : r1;
+            if (r < 0) test_leaf(r, any0 ? m0 : m1);
+            else next = r;
         }
         if (next < 0) {
-            if constexpr (BUDGET && budgeted<P>()) {
+            if constexpr (budgeted<P>()) {
                 if (work > budget) {  // warp-uniform; checked where a path ends
                     p.abandon();
                     break;
                 }
             }
-            const float tl = live ? stack_key_hi(p.max_thr()) : 0.f;
-            const float tmax = __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(tl)));
+            const float tmax = warp_max(p.max_thr());
             while (sp > 0) {
                 sp--;
-                if (sdist[sp] < tmax) {
-                    next = snode[sp];
+                const int2 e = entry[sp];
+                if (__int_as_float(e.y) < tmax) {
+                    next = e.x;
                     break;
                 }
             }
@@ -648,10 +639,10 @@ __device__ __forceinline__ void traverse_packet(P &p, Counters &cnt, int budget)
 // one the brick's centre lane ranks first (traverse_packet) -- so node and triangle loads are
 // warp-uniform (broadcast) and leaf work does not diverge. Every lane must call it
 // (warp-synchronous when WARP).
-template <bool WARP, bool COUNT, bool BUDGET, class P>
+template <bool WARP, bool COUNT, class P>
 __device__ __forceinline__ void traverse(P &p, Counters &cnt, int budget) {
     if constexpr (WARP) {
-        traverse_packet<COUNT, BUDGET>(p, cnt, budget);
+        traverse_packet<COUNT>(p, cnt, budget);
         return;
     }
     using R = typename P::R;
@@ -803,7 +794,7 @@ __device__ __forceinline__ void traverse4(P &p, Counters &cnt) {
 // the one nearest the brick's centre lane is entered and the others go on the warp's shared stack
 // with the warp's smallest box distance, entered on pop while that is below the largest lane
 // threshold. At most 3 entries a level: the build keeps 3 x (4-wide depth) below kStackSize.
-template <bool COUNT, bool BUDGET, class P>
+template <bool COUNT, class P>
 __device__ __forceinline__ void traverse4_packet(P &p, Counters &cnt, int budget) {
     using R = typename P::R;
     constexpr int Q = P::kQn;
@@ -831,12 +822,12 @@ __device__ __forceinline__ void traverse4_packet(P &p, Counters &cnt, int budget
             if (!__any_sync(kAll, m != 0u)) continue;
             if (rc < 0) {
                 p.template leaf<COUNT>(leaf_first(rc), leaf_count(rc), m, cnt);
-                if constexpr (BUDGET && budgeted<P>()) work += leaf_count(rc);
+                if constexpr (budgeted<P>()) work += leaf_count(rc);
                 continue;
             }
             const R own = min_of<R, Q>(d[c]);
             const float key =
-                __uint_as_float(__reduce_min_sync(kAll, __float_as_uint(live ? stack_key_lo(own) : finf())));
+                __uint_as_float(__reduce_min_sync(kAll, __float_as_uint(live ? own : finf())));
             const float rank = __shfl_sync(kAll, float(own), kRepLane);
             int push = rc;
             float push_key = key;
@@ -854,13 +845,13 @@ __device__ __forceinline__ void traverse4_packet(P &p, Counters &cnt, int budget
             }
         }
         if (next < 0) {
-            if constexpr (BUDGET && budgeted<P>()) {
+            if constexpr (budgeted<P>()) {
                 if (work > budget) {
                     p.abandon();
                     break;
                 }
             }
-            const float tl = live ? stack_key_hi(p.max_thr()) : 0.f;
+            const float tl = live ? p.max_thr() : 0.f;
             const float tmax = __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(tl)));
             while (sp > 0) {
                 sp--;
@@ -875,14 +866,14 @@ __device__ __forceinline__ void traverse4_packet(P &p, Counters &cnt, int budget
     }
 }
 
-template <bool WARP, bool WIDE, bool COUNT, bool BUDGET = false, class P>
+template <bool WARP, bool WIDE, bool COUNT, class P>
 __device__ __forceinline__ void walk(P &p, Counters &cnt, int budget = 0) {
     if constexpr (WIDE && WARP)
-        traverse4_packet<COUNT, BUDGET>(p, cnt, budget);
+        traverse4_packet<COUNT>(p, cnt, budget);
     else if constexpr (WIDE)
         traverse4<WARP, COUNT>(p, cnt);
     else
-        traverse<WARP, COUNT, BUDGET>(p, cnt, budget);
+        traverse<WARP, COUNT>(p, cnt, budget);
 }
 
 // ---- outputs ----------------------------------------------------------------------------------------
@@ -1028,7 +1019,7 @@ __device__ __forceinline__ void signal_chunk(const QueryArgs &a) {
 // Lanes without a query (the edge of a grid brick, the tail of a point list) take part in warp-mode
 // traversal with a negative threshold, so they never ask for a node. seed[s] is the leaf position of
 // the closest triangle the lane's query s found one step below (-1: none); it is updated here.
-template <int PREC, bool WARP, bool WIDE, bool COUNT, bool BUDGET>
+template <int PREC, bool WARP, bool WIDE, bool COUNT>
 __device__ __forceinline__ void query_step(const QueryArgs &a, int step, const bool (&valid)[kQ],
                                            const long long (&qid)[kQ], const long long (&gi)[kQ],
                                            const long long (&gj)[kQ], const long long (&gk)[kQ], bool any,
@@ -1103,14 +1094,15 @@ __device__ __forceinline__ void query_step(const QueryArgs &a, int step, const b
                 if (exact[s]) {
                     p.disable(s);
                 } else {
-                    p.set(s, float(x), float(y), float(z), init < dinf() ? __double2float_ru(init) : finf());
+                    p.set(s, filter_coord(x, 0, a.m), filter_coord(y, 1, a.m), filter_coord(z, 2, a.m),
+                          init < dinf() ? __double2float_ru(init) : finf());
                     if (seeded && seed[s] >= 0) p.seed(s, seed[s]);
                 }
             } else {
                 p.disable(s);
             }
         }
-        if (WARP || any) walk<WARP, WIDE, COUNT, BUDGET>(p, cnt, a.warp_budget);
+        if (WARP || any) walk<WARP, WIDE, COUNT>(p, cnt, a.warp_budget);
 #pragma unroll
         for (int s = 0; s < Q; s++) {
             if (!valid[s]) continue;
@@ -1148,7 +1140,7 @@ __device__ __forceinline__ void query_step(const QueryArgs &a, int step, const b
 }
 
 // A point-list block, or a grid block's column step by step (each step seeded from the one below).
-template <int PREC, bool WARP, bool WIDE, bool COUNT, bool BUDGET>
+template <int PREC, bool WARP, bool WIDE, bool COUNT>
 __device__ __forceinline__ void query_block(const QueryArgs &a, long long block, Counters &cnt) {
     constexpr int Q = kQ;
     int seed[Q];
@@ -1169,20 +1161,18 @@ __device__ __forceinline__ void query_block(const QueryArgs &a, long long block,
         // decision, not a block one: the warps share nothing, and a block barrier per step made every
         // warp wait for the block's slowest (17 % on the torus knot)
         if (step > 0 && !__any_sync(0xffffffffu, any)) break;
-        query_step<PREC, WARP, WIDE, COUNT, BUDGET>(a, step, valid, qid, gi, gj, gk, any, seed, cnt);
+        query_step<PREC, WARP, WIDE, COUNT>(a, step, valid, qid, gi, gj, gk, any, seed, cnt);
     }
 }
 
-// BUDGET: the fix-up kernel's packets stop after QueryArgs::warp_budget triangle records (a separate
-// instantiation, so the kernels without it compile as if it did not exist).
 // SIGNAL: the streamed grid download's instantiation, whose blocks count themselves done per chunk
 // (a separate instantiation: the dormant signal code cost the fix-up kernel 3 % where it was merely
 // compiled in).
-template <int PREC, bool WARP, bool WIDE, bool COUNT, bool BUDGET = false, bool SIGNAL = false>
+template <int PREC, bool WARP, bool WIDE, bool COUNT, bool SIGNAL = false>
 __global__ void __launch_bounds__(kThreads, PREC == SSDF_PREC_F64 ? kF64MinBlocks : SSDF_B200_QUERY_MIN_BLOCKS)
     k_query(const QueryArgs a) {
     Counters cnt;
-    query_block<PREC, WARP, WIDE, COUNT, BUDGET>(a, blockIdx.x, cnt);
+    query_block<PREC, WARP, WIDE, COUNT>(a, blockIdx.x, cnt);
     if (COUNT) flush_counters(a, cnt);
     if constexpr (SIGNAL) signal_chunk(a);
 }
@@ -1253,14 +1243,13 @@ __device__ __noinline__ void window_subtree(const DeviceMesh &m, int root, float
     int sp = 0;
     st[sp++] = root;
     while (sp > 0) {
-        const Node32 n = load_node32(m.nodes32, st[--sp]);
-        const float d0 = box_dist_sq_fast(px, py, pz, n.a.x, n.a.y, n.a.z, n.a.w, n.c.x, n.c.y);
-        const float d1 = box_dist_sq_fast(px, py, pz, n.b.x, n.b.y, n.b.z, n.b.w, n.c.z, n.c.w);
+        int r0, r1;
+        const float2 d = obb_dist_sq_pair(twice(px), twice(py), twice(pz), m.obb + 8 * st[--sp], r0, r1);
         if (count) cnt.box += 2;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            const int c = h ? n.r1 : n.r0;
-            if (c == kEmptyRef || !in_window(h ? d1 : d0, thr)) continue;
+            const int c = h ? r1 : r0;
+            if (c == kEmptyRef || !in_window(h ? d.y : d.x, thr)) continue;
             if (c < 0)
                 window_leaf(m, c, px, py, pz, thr, qx, qy, qz, b, cnt, count, kbest);
             else if (sp < kStackSize)
@@ -1279,7 +1268,7 @@ __device__ void window_warp(const QueryArgs &a, int idx, int *__restrict__ stack
     if (a.is_grid) grid_ijk(a, q, i, j, k);
     double qx, qy, qz;
     query_point(a, q, i, j, k, qx, qy, qz);
-    const float px = float(qx), py = float(qy), pz = float(qz);
+    const float px = filter_coord(qx, 0, a.m), py = filter_coord(qy, 1, a.m), pz = filter_coord(qz, 2, a.m);
     float thr = a.fallback_thr[idx];
     const bool shrink = thr < finf();  // an infinite window (a point beyond the float range) stays
     float kbest = finf();
@@ -1296,13 +1285,10 @@ __device__ void window_warp(const QueryArgs &a, int idx, int *__restrict__ stack
         int c0 = kEmptyRef, c1 = kEmptyRef;
         bool w0 = false, w1 = false;
         if (node >= 0) {
-            const Node32 n = load_node32(m.nodes32, node);
-            const float d0 = box_dist_sq_fast(px, py, pz, n.a.x, n.a.y, n.a.z, n.a.w, n.c.x, n.c.y);
-            const float d1 = box_dist_sq_fast(px, py, pz, n.b.x, n.b.y, n.b.z, n.b.w, n.c.z, n.c.w);
+            const float2 d = obb_dist_sq_pair(twice(px), twice(py), twice(pz), m.obb + 8 * node, c0, c1);
             if (COUNT) cnt.box += 2;
-            c0 = n.r0, c1 = n.r1;
-            w0 = c0 != kEmptyRef && in_window(d0, thr);
-            w1 = c1 != kEmptyRef && in_window(d1, thr);
+            w0 = c0 != kEmptyRef && in_window(d.x, thr);
+            w1 = c1 != kEmptyRef && in_window(d.y, thr);
             if (w0 && c0 < 0) {
                 window_leaf(m, c0, px, py, pz, thr, qx, qy, qz, b, cnt, COUNT, kbest);
                 w0 = false;
@@ -1357,7 +1343,7 @@ __global__ void __launch_bounds__(kThreads) k_window(const QueryArgs a, int cap)
 // re-instantiated: only the table is rewritten before each replay. Blocks pull work items (one
 // 128-query block of one job) from an atomic counter, largest jobs first (the host orders them).
 
-template <int PREC, bool WARP, bool WIDE, bool COUNT, bool BUDGET = false>
+template <int PREC, bool WARP, bool WIDE, bool COUNT>
 __global__ void __launch_bounds__(kThreads, PREC == SSDF_PREC_F64 ? kF64MinBlocks : SSDF_B200_QUERY_MIN_BLOCKS)
     k_query_batch(const BatchHeader *__restrict__ hdr, const QueryArgs *__restrict__ jobs,
                   const long long *__restrict__ first_block, unsigned long long *__restrict__ next_item) {
@@ -1376,7 +1362,7 @@ __global__ void __launch_bounds__(kThreads, PREC == SSDF_PREC_F64 ? kF64MinBlock
             const int mid = (lo + hi + 1) >> 1;
             if (__ldg(first_block + mid) <= it) lo = mid; else hi = mid - 1;
         }
-        query_block<PREC, WARP, WIDE, COUNT, BUDGET>(jobs[lo], it - __ldg(first_block + lo), cnt);
+        query_block<PREC, WARP, WIDE, COUNT>(jobs[lo], it - __ldg(first_block + lo), cnt);
     }
     if (COUNT && njobs > 0) flush_counters(jobs[0], cnt);
 }
@@ -1411,23 +1397,10 @@ int window_stack_cap() {
 
 template <int PREC, bool WARP, bool WIDE>
 cudaError_t launch_batch_main(const BatchLaunch &b, bool count, cudaStream_t stream) {
-    constexpr bool kCanBudget = PREC == SSDF_PREC_F32_FIXUP && WARP;
-    if constexpr (kCanBudget) {
-        if (b.budget) {
-            if (count)
-                k_query_batch<PREC, WARP, WIDE, true, true><<<b.grid, kThreads, 0, stream>>>(b.hdr, b.jobs, b.first_block,
-                                                                                            b.next_item);
-            else
-                k_query_batch<PREC, WARP, WIDE, false, true><<<b.grid, kThreads, 0, stream>>>(b.hdr, b.jobs, b.first_block,
-                                                                                             b.next_item);
-        }
-    }
-    if (!kCanBudget || !b.budget) {
-        if (count)
-            k_query_batch<PREC, WARP, WIDE, true><<<b.grid, kThreads, 0, stream>>>(b.hdr, b.jobs, b.first_block, b.next_item);
-        else
-            k_query_batch<PREC, WARP, WIDE, false><<<b.grid, kThreads, 0, stream>>>(b.hdr, b.jobs, b.first_block, b.next_item);
-    }
+    if (count)
+        k_query_batch<PREC, WARP, WIDE, true><<<b.grid, kThreads, 0, stream>>>(b.hdr, b.jobs, b.first_block, b.next_item);
+    else
+        k_query_batch<PREC, WARP, WIDE, false><<<b.grid, kThreads, 0, stream>>>(b.hdr, b.jobs, b.first_block, b.next_item);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || PREC != SSDF_PREC_F32_FIXUP) return e;
     if (count)
@@ -1457,21 +1430,12 @@ thread_local unsigned long long t_last_counts[4] = {0, 0, 0, 0};
 
 template <int PREC, bool WARP, bool WIDE>
 cudaError_t launch_main(const QueryArgs &a, bool count, unsigned nblocks, cudaStream_t stream) {
-    if constexpr (PREC == SSDF_PREC_F32_FIXUP && WARP) {
-        if (a.warp_budget > 0) {
-            if (count)
-                k_query<PREC, WARP, WIDE, true, true><<<nblocks, kThreads, 0, stream>>>(a);
-            else
-                k_query<PREC, WARP, WIDE, false, true><<<nblocks, kThreads, 0, stream>>>(a);
-            return cudaGetLastError();
-        }
-    }
-    // a counting or budgeted launch raises no chunk flags: its streamed download copies every chunk
-    // once the launch has ended
+    // a counting launch raises no chunk flags: its streamed download copies every chunk once the launch
+    // has ended
     if (count)
         k_query<PREC, WARP, WIDE, true><<<nblocks, kThreads, 0, stream>>>(a);
     else if (a.chunk_flags)
-        k_query<PREC, WARP, WIDE, false, false, true><<<nblocks, kThreads, 0, stream>>>(a);
+        k_query<PREC, WARP, WIDE, false, true><<<nblocks, kThreads, 0, stream>>>(a);
     else
         k_query<PREC, WARP, WIDE, false><<<nblocks, kThreads, 0, stream>>>(a);
     return cudaGetLastError();
@@ -1637,9 +1601,9 @@ int launch_query_keep(const QueryArgs &args_in, int precision, cudaStream_t stre
     QueryArgs a = args_in;
     const long long n = a.is_grid ? a.nx * a.ny * a.nz : a.npoints;
     if (n <= 0) return SSDF_OK;
-    if (precision == SSDF_PREC_F64 && !a.m.nodes64)
+    if (precision == SSDF_PREC_F64 && !a.m.tris64)
         return fail(SSDF_ERR_INVALID_ARGUMENT, "mesh built without double data (keep_fp64=0)");
-    if (precision == SSDF_PREC_F32_FIXUP && (!a.m.tris64 || !a.m.nodes64 || !a.m.filt32))
+    if (precision == SSDF_PREC_F32_FIXUP && (!a.m.tris64 || !a.m.filt32))
         return fail(SSDF_ERR_INVALID_ARGUMENT, "fix-up queries need the double triangles and BVH (keep_fp64=1)");
     if (a.output == SSDF_OUT_SDF && !a.m.face_n)
         return fail(SSDF_ERR_INVALID_ARGUMENT, "signed queries need a mesh built with normals=1");
@@ -1649,7 +1613,7 @@ int launch_query_keep(const QueryArgs &args_in, int precision, cudaStream_t stre
     // plain FP64 kernel: the fix-up filter sees each such triangle through a wide proxy, whose keys
     // crowd the window. Both give the same bits.
     if (precision == SSDF_PREC_F32_FIXUP && fixup_runs_f64(a.m)) precision = SSDF_PREC_F64;
-    a.warp_budget = resolve_warp_budget(a.warp_budget, n, a.m.nt);
+    a.warp_budget = resolve_warp_budget(a.warp_budget, n, a.m.nt, a.is_grid != 0);
     if (a.output == SSDF_OUT_CLOSEST && (!a.m.tris64 || !a.outx || !a.outy || !a.outz || !a.outtri))
         return fail(SSDF_ERR_INVALID_ARGUMENT, "closest-point queries need outx/outy/outz/outtri and double data");
     if (precision == SSDF_PREC_F32 && (a.output == SSDF_OUT_SDF || a.output == SSDF_OUT_CLOSEST))
@@ -1811,7 +1775,7 @@ int launch_query_noalloc(const QueryArgs &args_in, cudaStream_t stream) {
         return fail(SSDF_ERR_NOT_SUPPORTED, "the allocation-free query takes at most " +
                                                 std::to_string(kNoAllocMaxQueries) + " queries per call, got " +
                                                 std::to_string(n) + ": split the grid into slabs");
-    if (!a.m.tris64 || !a.m.nodes64 || !a.m.filt32)
+    if (!a.m.tris64 || !a.m.filt32)
         return fail(SSDF_ERR_INVALID_ARGUMENT, "fix-up queries need the double triangles and BVH (keep_fp64=1)");
     if (a.output == SSDF_OUT_SDF && !a.m.face_n)
         return fail(SSDF_ERR_INVALID_ARGUMENT, "signed queries need a mesh built with normals=1");
@@ -1823,7 +1787,7 @@ int launch_query_noalloc(const QueryArgs &args_in, cudaStream_t stream) {
         if (e != cudaSuccess) return cuda_fail(e, "allocation-free query launch", __FILE__, __LINE__);
         return SSDF_OK;
     }
-    a.warp_budget = resolve_warp_budget(a.warp_budget, n, a.m.nt);
+    a.warp_budget = resolve_warp_budget(a.warp_budget, n, a.m.nt, a.is_grid != 0);
     int *scratch = nullptr;
     SSDF_CHECK(noalloc_scratch(&scratch));
     a.fallback_count = scratch;

@@ -384,6 +384,24 @@ struct MeshHold {
     }
 };
 
+// A mesh for the contact walks: the axis-aligned tree and the float records alone.
+int contact_mesh(MeshHold *mh, ptrdiff_t nt, const int *s0, const int *s1, const int *s2, ptrdiff_t nv, const void *sx,
+                 const void *sy, const void *sz, int coord_f64, int device_ptrs, long long nqueries) {
+    ssdf_build_opts bo;
+    bo.leaf_size = env_int("SSDF_B200_LEAF", 0), bo.keep_fp64 = 0, bo.normals = 0;
+    bo.treelet_opt = call_treelet_rounds(nqueries);
+    ssdf_mesh *h = new ssdf_mesh();
+    cudaGetDevice(&h->device);
+    const int st = mesh_build(&h->storage, &h->m, nt, s0, s1, s2, nv, sx, sy, sz, coord_f64, device_ptrs, bo, mh->stream,
+                              /*query_boxes=*/false);
+    if (st != SSDF_OK) {
+        delete h;
+        return st;
+    }
+    mh->mesh = h;
+    return SSDF_OK;
+}
+
 // The four reference functions over host arrays: validate, build the BVH (a quad as two halves),
 // upload, query, download. Blocking, like the reference.
 template <typename G, typename T, bool QUAD, bool LOCAL>
@@ -421,22 +439,18 @@ int within_radius_host(ptrdiff_t npoints, const G *x, const G *y, const G *z, pt
     MeshHold mh;
     mh.stream = stream;
     Buffers buf(stream);
-    const int cf = sizeof(G) == 8 ? SSDF_F64 : SSDF_F32;
+    const int g64 = sizeof(G) == 8;
     const bool have_mesh = ne > 0 && nv > 0;
     if (have_mesh) {
-        ssdf_build_opts bo;
-        bo.leaf_size = env_int("SSDF_B200_LEAF", 0), bo.keep_fp64 = 0, bo.normals = 0;
-        bo.treelet_opt = call_treelet_rounds(npoints);
         if (QUAD) {  // halves (0, 1, 2) and (0, 2, 3): record 2e + h belongs to quad e
             std::vector<int> h0(size_t(2 * ne)), h1(size_t(2 * ne)), h2(size_t(2 * ne));
             for (ptrdiff_t e = 0; e < ne; e++) {
                 h0[2 * e] = s0[e], h1[2 * e] = s1[e], h2[2 * e] = s2[e];
                 h0[2 * e + 1] = s0[e], h1[2 * e + 1] = s2[e], h2[2 * e + 1] = s3[e];
             }
-            SSDF_CHECK(ssdf_mesh_create(&mh.mesh, 2 * ne, h0.data(), h1.data(), h2.data(), nv, sx, sy, sz, cf, 0, &bo,
-                                        stream));
+            SSDF_CHECK(contact_mesh(&mh, 2 * ne, h0.data(), h1.data(), h2.data(), nv, sx, sy, sz, g64, 0, npoints));
         } else {
-            SSDF_CHECK(ssdf_mesh_create(&mh.mesh, ne, s0, s1, s2, nv, sx, sy, sz, cf, 0, &bo, stream));
+            SSDF_CHECK(contact_mesh(&mh, ne, s0, s1, s2, nv, sx, sy, sz, g64, 0, npoints));
         }
         a.nodes = mh.mesh->m.nodes32;
         a.tris = mh.mesh->m.tris32;
@@ -703,11 +717,7 @@ int potential_contact_host(ptrdiff_t ne, const int *s0, const int *s1, const int
     k_box_vertices<<<blocks, 128, 0, stream>>>(int(ne), nk, (const float4 *)prims, (float *)bx, (float *)by,
                                                (float *)bz, (int *)t0, (int *)t1);
     SSDF_CUDA(cudaGetLastError());
-    ssdf_build_opts bo;
-    bo.leaf_size = env_int("SSDF_B200_LEAF", 0), bo.keep_fp64 = 0, bo.normals = 0;
-    bo.treelet_opt = call_treelet_rounds(ne);
-    SSDF_CHECK(ssdf_mesh_create(&mh.mesh, ne, (const int *)t0, (const int *)t1, (const int *)t1, 2 * ne, bx, by, bz,
-                                SSDF_F32, 1, &bo, stream));
+    SSDF_CHECK(contact_mesh(&mh, ne, (const int *)t0, (const int *)t1, (const int *)t1, 2 * ne, bx, by, bz, 0, 1, ne));
     a.prims = (const float4 *)prims;
     a.nodes = mh.mesh->m.nodes32;
     a.boxes = mh.mesh->m.tris32;

@@ -200,7 +200,7 @@ int launch_query_streamed(const QueryArgs &args, int precision, void *host_out, 
     SSDF_CHECK(launch_query_keep(a, precision, stream, &cl.fb));
     SSDF_CUDA(cudaEventRecord(cl.done, stream));
 
-    // copy each chunk once its flag is up, or once the launch has ended (a counting or budgeted launch
+    // copy each chunk once its flag is up, or once the launch has ended (a counting launch
     // raises no flags)
     const volatile int *flags = r->flags;
     std::vector<char> sent(size_t(plan.nchunks), 0);

@@ -37,8 +37,10 @@ int cuda_fail(cudaError_t err, const char *what, const char *file, int line);
 // so one visit tests two boxes from one 64-byte (FP32) or 128-byte (FP64) record:
 //   FP32 node (4 x float4): (c0.lox, c0.hix, c0.loy, c0.hiy), (c1.lox, c1.hix, c1.loy, c1.hiy),
 //                           (c0.loz, c0.hiz, c1.loz, c1.hiz), (ref0, ref1, -, -) as int bits
-//   FP64 node (8 x double2): c0 x, c0 y, c0 z, c1 x, c1 y, c1 z as (lo, hi), (ref0, ref1) as
-//                            int bits, padding
+//   oriented node (8 x float4): the same children's oriented boxes in the mesh's box frame (see
+//                           DeviceMesh::obb); per axis k = u, v, n of both children: (kx of c0, kx of
+//                           c1, ky, ky), (kz, kz, -k.centre, -k.centre), then the half extents (hu, hu,
+//                           hv, hv), (hn, hn, ref0, ref1): pairs (c0, c1) throughout, for two-wide FP32
 //   4-wide FP32 node (8 x float4): lo x / hi x / lo y / hi y / lo z / hi z of children 0..3, then
 //                           the 4 references as int bits, padding
 //   4-wide FP64 node (14 x double2): the same six rows as pairs of double2, the 4 references as
@@ -67,7 +69,13 @@ struct DeviceMesh {
     int leaf_size = 4;
     int nleaves = 0;
     const float4 *nodes32 = nullptr;   // [4 * nnodes]
-    const double2 *nodes64 = nullptr;  // [8 * nnodes] or null
+    // Oriented boxes of the same tree's children, [8 * nnodes]: what the query kernels walk. Axes
+    // and extents are for points (p - box_c) * box_scale, with margins that make the float distance a
+    // lower bound of any contained triangle's distance, exact or as the float arithmetic evaluates it
+    // (mesh_build.cu, k_obb).
+    const float4 *obb = nullptr;
+    float box_c[3] = {0.f, 0.f, 0.f};
+    float box_scale = 1.f;
     // 4-wide BVH over the same leaves (collapsed from the binary one)
     int nnodes4 = 0;
     int depth4 = 0;
@@ -171,14 +179,15 @@ struct BatchLaunch {
     int grid;   // persistent blocks (SMs x resident blocks per SM)
     int sms;
     bool warp, wide;
-    bool budget;  // the fix-up packets stop after the jobs' warp_budget (k_query_batch<..., BUDGET>)
 };
 
 // ---- mesh build (mesh_build.cu) ------------------------------------------------------------------
 struct MeshStorage;  // owns the device allocations behind a DeviceMesh
 int mesh_build(MeshStorage **storage, DeviceMesh *mesh, ptrdiff_t nt, const int *s0, const int *s1, const int *s2,
                ptrdiff_t nv, const void *sx, const void *sy, const void *sz, int coord_f64, int device_ptrs,
-               const ssdf_build_opts &opts, cudaStream_t stream);
+               const ssdf_build_opts &opts, cudaStream_t stream, bool query_boxes = true);
+// query_boxes false: without the oriented boxes (DeviceMesh::obb null), for walks of the axis-aligned nodes
+// only (contact.cu).
 void mesh_free(MeshStorage *storage);                            // after the work using it completed
 void mesh_free_async(MeshStorage *storage, cudaStream_t stream);  // in stream order
 size_t mesh_bytes(const MeshStorage *storage);
@@ -313,28 +322,28 @@ constexpr int kResidentTreeletRounds = 3;
 
 // ---- small helpers -------------------------------------------------------------------------------
 inline int grid_blocks(long long n, int threads) { return int((n + threads - 1) / threads); }
-// Default of QueryArgs::warp_budget, for launches (single, or a whole batch) of at most
-// kBudgetMaxQueries queries; larger launches run without one. SSDF_B200_WARP_BUDGET sets it for every
-// launch (0 = no limit). Measured on B200: with 2048 the 64^3 icosphere grid runs 1.83 -> 1.31 ms and a
-// 110^3 grid on an 81,920-triangle sphere 22.2 -> 8.5 ms (packets near the centre, where every
-// triangle is almost equidistant, hand their queries to the warp-per-query stage: the launch's tail
-// shortens). A launch that fills the GPU many times over gains nothing from a shorter tail and pays
-// for the repeated work (the 256-mesh batch: 257 -> 275 ms).
-constexpr int kWarpBudget = 2048;
-constexpr long long kBudgetMaxQueries = 1ll << 21;
-// QueryArgs::warp_budget for a launch of n queries when it was left to the default (< 0): 5.6 sqrt(T)
-// records for a mesh of T triangles, within [128, kWarpBudget] -- a packet that has tested that many
-// is in a near-equidistant region. Measured on B200 (sphere grids, the best budget of each sweep in
-// brackets): 1,280 triangles 48^3 [200]: 0.20 ms against 0.28 ms at 400; 5,120 triangles 64^3 [400]:
-// 0.49 ms against 0.58 at 640 and 0.53 at 480; 20,480 triangles 96^3 [600 .. 1,280]: 1.64 ms against
-// 1.89 at 2048; the serving leg's 110^3 grid on 81,920 triangles [1,536 .. 2,048]: 8.2 ms against 8.7
-// at 1024 and 10.1 at 512.
-constexpr int kWarpBudgetMin = 128;
-inline int resolve_warp_budget(int b, long long n, int ntri) {
+// QueryArgs::warp_budget of a launch (or of a batch's jobs) that left it to the default (< 0): a launch or
+// batch of n queries, a mesh of T triangles. A packet in a region where every triangle is almost
+// equidistant (near a sphere's centre), or of scattered points, sets the launch's tail; handing its
+// queries to the warp-per-query stage cuts it. The best budget grows with T, faster on grids, whose packets
+// start close together, than on point lists; a launch that fills the GPU several times over repays less of
+// a shorter tail and takes a larger one. Measured on B200, us
+// without a budget and at 64 / 128 / 256 / 450 / 700 records: 64^3 grid on 5,120 triangles 373: 349 / 247 /
+// 284 / 348 / 377; 96^3 on 20,480 1,264: 2,740 / 1,098 / 778 / 754 / 887; 110^3 on 81,920 13,872: 11,175 /
+// 4,373 / 2,720 / 2,145 / 2,262; 64^3 around the 131,072-triangle knot 1,021: 3,010 / 2,364 / 1,279 / 876 /
+// 807; 500,003 points near it 1,467: 2,579 / 1,360 / 978 / 987 / 1,130; 50,000 1,707: 754 / 712 / 546 / 624 /
+// 748; 1,000,000 in its box 2,653: 10,229 / 6,473 / 2,882 / 2,102 / 2,054. Above 2^21 queries: 200^3 on 81,920
+// triangles 12,950 without, 7,040 / 6,518 / 6,641 / 7,572 at 500 / 700 / 1,000 / 1,500; 48 uneven meshes,
+// 42M queries in one batch, 44.2 ms without, 26.4 at 700; the knot's 256^3 unchanged.
+// SSDF_B200_WARP_BUDGET sets it for every launch (0 = no limit).
+constexpr int kWarpBudgetMin = 64, kWarpBudgetMax = 700;
+constexpr long long kBudgetSmallLaunch = 1ll << 21;
+inline int resolve_warp_budget(int b, long long n, int ntri, bool grid) {
     if (b >= 0) return b;
-    if (n > kBudgetMaxQueries) return 0;
-    const int v = int(5.6 * std::sqrt(double(ntri > 0 ? ntri : 0)));
-    return v < kWarpBudgetMin ? kWarpBudgetMin : (v > kWarpBudget ? kWarpBudget : v);
+    const double t = ntri > 0 ? ntri : 0;
+    auto within = [](double v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : int(v)); };
+    if (n > kBudgetSmallLaunch) return within(3.0 * std::sqrt(t), 2 * kWarpBudgetMin, 1000);
+    return within(grid ? t / 40 : 1.2 * std::sqrt(t), kWarpBudgetMin, kWarpBudgetMax);
 }
 // Point lists of at least this many queries are visited in Morton order (SSDF_B200_SORT_POINTS=0
 // keeps input order).

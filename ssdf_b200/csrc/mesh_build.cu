@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <cfloat>
+#include <cstring>
 #include <vector>
 
 #include "internal.h"
@@ -245,65 +246,39 @@ __global__ void k_counts(int n, const int *__restrict__ child_l, const int *__re
 __global__ void k_write_nodes(int n, int L, const int *__restrict__ child_l, const int *__restrict__ child_r,
                               const int *__restrict__ first_of, const int *__restrict__ count,
                               const int *__restrict__ sorted_ids, const float *__restrict__ pbox32,
-                              const double *__restrict__ pbox64, const float *__restrict__ nbox32,
-                              const double *__restrict__ nbox64, float4 *__restrict__ nodes32,
-                              double2 *__restrict__ nodes64) {
+                              const float *__restrict__ nbox32, float4 *__restrict__ nodes32) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n - 1) return;
     int ref[2];
     const float *b32[2];
-    const double *b64[2];
     const int c[2] = {child_l[i], child_r[i]};
     for (int h = 0; h < 2; h++) {
         if (c[h] < 0) {
             const int pos = -c[h] - 1;
             ref[h] = leaf_ref(pos, 1);
             b32[h] = pbox32 + 6 * sorted_ids[pos];
-            b64[h] = pbox64 + 6 * sorted_ids[pos];
         } else {
             ref[h] = count[c[h]] <= L ? leaf_ref(first_of[c[h]], count[c[h]]) : c[h];
             b32[h] = nbox32 + 6 * c[h];
-            b64[h] = nbox64 + 6 * c[h];
         }
     }
     nodes32[4 * i + 0] = make_float4(b32[0][0], b32[0][1], b32[0][2], b32[0][3]);
     nodes32[4 * i + 1] = make_float4(b32[1][0], b32[1][1], b32[1][2], b32[1][3]);
     nodes32[4 * i + 2] = make_float4(b32[0][4], b32[0][5], b32[1][4], b32[1][5]);
     nodes32[4 * i + 3] = make_float4(__int_as_float(ref[0]), __int_as_float(ref[1]), 0.f, 0.f);
-    if (nodes64) {
-        for (int h = 0; h < 2; h++)
-            for (int d = 0; d < 3; d++) nodes64[8 * i + 3 * h + d] = make_double2(b64[h][2 * d], b64[h][2 * d + 1]);
-        nodes64[8 * i + 6] = make_double2(__longlong_as_double((long long)(unsigned)ref[0]),
-                                          __longlong_as_double((long long)(unsigned)ref[1]));
-        nodes64[8 * i + 7] = make_double2(0.0, 0.0);
-    }
 }
 
 // A single root holding one leaf over all n <= L triangles (child 1 empty, inverted box).
-__global__ void k_write_small_root(int n, const float *__restrict__ box32, const double *__restrict__ box64,
-                                   float4 *__restrict__ nodes32, double2 *__restrict__ nodes64) {
+__global__ void k_write_small_root(int n, const float *__restrict__ box32, float4 *__restrict__ nodes32) {
     float b[6] = {FLT_MAX, -FLT_MAX, FLT_MAX, -FLT_MAX, FLT_MAX, -FLT_MAX};
-    double e[6] = {DBL_MAX, -DBL_MAX, DBL_MAX, -DBL_MAX, DBL_MAX, -DBL_MAX};
     for (int t = 0; t < n; t++)
-        for (int k = 0; k < 6; k += 2) {
+        for (int k = 0; k < 6; k += 2)
             b[k] = fminf(b[k], box32[6 * t + k]), b[k + 1] = fmaxf(b[k + 1], box32[6 * t + k + 1]);
-            e[k] = fmin(e[k], box64[6 * t + k]), e[k + 1] = fmax(e[k + 1], box64[6 * t + k + 1]);
-        }
     const float inf = __int_as_float(0x7f800000);
     nodes32[0] = make_float4(b[0], b[1], b[2], b[3]);
     nodes32[1] = make_float4(inf, -inf, inf, -inf);
     nodes32[2] = make_float4(b[4], b[5], inf, -inf);
     nodes32[3] = make_float4(__int_as_float(leaf_ref(0, n)), __int_as_float(kEmptyRef), 0.f, 0.f);
-    if (nodes64) {
-        const double dinf = __longlong_as_double(0x7ff0000000000000ll);
-        for (int d = 0; d < 3; d++) {
-            nodes64[d] = make_double2(e[2 * d], e[2 * d + 1]);
-            nodes64[3 + d] = make_double2(dinf, -dinf);
-        }
-        nodes64[6] = make_double2(__longlong_as_double((long long)(unsigned)leaf_ref(0, n)),
-                                  __longlong_as_double((long long)(unsigned)kEmptyRef));
-        nodes64[7] = make_double2(0.0, 0.0);
-    }
 }
 
 // 4-wide nodes, top-down: a node starts from its binary node's two children and repeatedly opens
@@ -454,6 +429,18 @@ __global__ void k_depth(int n, int L, const int *__restrict__ count, const int *
     atomicAdd(&stats[1], leaves);
 }
 
+// Whether the float filter sees a triangle through a proxy: height below 1/8 of the longest edge.
+__device__ bool ill_conditioned(double ax, double ay, double az, double bx, double by, double bz, double cx, double cy,
+                                double cz) {
+    const double abx = bx - ax, aby = by - ay, abz = bz - az, acx = cx - ax, acy = cy - ay, acz = cz - az;
+    const double bcx = cx - bx, bcy = cy - by, bcz = cz - bz;
+    const double lab = abx * abx + aby * aby + abz * abz, lac = acx * acx + acy * acy + acz * acz;
+    const double lbc = bcx * bcx + bcy * bcy + bcz * bcz;
+    const double l2 = fmax(fmax(lab, lac), lbc);
+    const double nx = aby * acz - abz * acy, ny = abz * acx - abx * acz, nz = abx * acy - aby * acx;
+    return l2 > 0.0 && !(64.0 * (nx * nx + ny * ny + nz * nz) >= l2 * l2);
+}
+
 // The fix-up path's FP32 filter record of one triangle: the triangle itself, or, when it is
 // ill-conditioned (height below 1/8 of its longest edge PQ, third corner R), a proxy triangle that
 // contains it: PQ widened by L/4 at both ends (L = |PQ|) and an apex L/2 off its middle, towards R in
@@ -461,15 +448,13 @@ __global__ void k_depth(int n, int L, const int *__restrict__ count, const int *
 // proxy is at least L/6 high over all of PQ, so it contains P, Q and R; its distance is a lower
 // bound of the triangle's, and its height (1/3 of its base) keeps the float test accurate. A proxy's
 // record has the sign bit of its ab.ab set: its key may enter the window but never moves its centre.
-__device__ bool filter_record(double ax, double ay, double az, double bx, double by, double bz, double cx,
-                              double cy, double cz, int t, float4 *__restrict__ out) {
+__device__ void filter_record(double ax, double ay, double az, double bx, double by, double bz, double cx,
+                              double cy, double cz, bool ill, float4 *__restrict__ out) {
     const double abx = bx - ax, aby = by - ay, abz = bz - az, acx = cx - ax, acy = cy - ay, acz = cz - az;
     const double bcx = cx - bx, bcy = cy - by, bcz = cz - bz;
     const double lab = abx * abx + aby * aby + abz * abz, lac = acx * acx + acy * acy + acz * acz;
     const double lbc = bcx * bcx + bcy * bcy + bcz * bcz;
     const double l2 = fmax(fmax(lab, lac), lbc);
-    const double nx = aby * acz - abz * acy, ny = abz * acx - abx * acz, nz = abx * acy - aby * acx;
-    const bool ill = l2 > 0.0 && !(64.0 * (nx * nx + ny * ny + nz * nz) >= l2 * l2);
     double v[3][3] = {{ax, ay, az}, {bx, by, bz}, {cx, cy, cz}};
     if (ill) {
         // P, Q: the longest edge; R: the third corner
@@ -515,8 +500,6 @@ __device__ bool filter_record(double ax, double ay, double az, double bx, double
     out[0] = make_float4(f[0][0], f[0][1], f[0][2], ill ? __int_as_float(__float_as_int(fbb) | 0x80000000) : fbb);
     out[1] = make_float4(float(eb[0]), float(eb[1]), float(eb[2]), float(cc));
     out[2] = make_float4(float(ec[0]), float(ec[1]), float(ec[2]), float(bc));
-    (void)t;
-    return ill;
 }
 
 // The fix-up window's bound term of one filter record (the triangle the float corners describe, or its
@@ -576,10 +559,37 @@ void set_filter_window(DeviceMesh *m, float largest_term, bool records_safe) {
 
 namespace {
 
+// Middle and scale of the mesh's box (the union of the root's children), and M in that frame: w[0..2],
+// w[3], w[4] as floats. A mesh outside [2^-60, 2^100], or with a coordinate that is not finite, gets M < 0:
+// its boxes cull nothing.
+__global__ void k_box_frame(const float4 *__restrict__ nodes, int *__restrict__ w) {
+    const float4 a = nodes[0], b = nodes[1], c = nodes[2];
+    const float lo[3] = {fminf(a.x, b.x), fminf(a.z, b.z), fminf(c.x, c.z)};
+    const float hi[3] = {fmaxf(a.y, b.y), fmaxf(a.w, b.w), fmaxf(c.y, c.w)};
+    float mid[3], m = 0.f;
+    for (int d = 0; d < 3; d++) {
+        mid[d] = 0.5f * lo[d] + 0.5f * hi[d];
+        m = fmaxf(m, fmaxf(hi[d] - mid[d], mid[d] - lo[d]));
+    }
+    float scale = 1.f;
+    if (!(m >= 0x1p-60f && m <= 0x1p100f)) {
+        m = -1.f;
+        for (int d = 0; d < 3; d++) mid[d] = 0.f;
+    } else if (m > 0x1p60f) {
+        int e;
+        m = frexpf(m, &e);  // M in [0.5, 1)
+        scale = ldexpf(1.f, -e);
+    }
+    for (int d = 0; d < 3; d++) w[d] = __float_as_int(mid[d]);
+    w[3] = __float_as_int(scale);
+    w[4] = __float_as_int(m);
+}
+
 __global__ void k_tri_records(int nt, const int *__restrict__ sorted_ids, const int *__restrict__ s0,
                               const int *__restrict__ s1, const int *__restrict__ s2, const double *__restrict__ vx,
                               const double *__restrict__ vy, const double *__restrict__ vz, float4 *__restrict__ t32,
-                              double2 *__restrict__ t64, float4 *__restrict__ filt, int *__restrict__ nill) {
+                              double2 *__restrict__ t64, float4 *__restrict__ filt, const int *__restrict__ frame,
+                              int *__restrict__ nill) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= nt) return;
     const int t = sorted_ids[p];
@@ -590,10 +600,20 @@ __global__ void k_tri_records(int nt, const int *__restrict__ sorted_ids, const 
     t32[3 * p + 1] = make_float4(float(by), float(bz), float(cx), float(cy));
     t32[3 * p + 2] = make_float4(float(cz), __int_as_float(t), 0.f, 0.f);
     if (filt) {
-        if (filter_record(ax, ay, az, bx, by, bz, cx, cy, cz, t, filt + 3 * size_t(p))) atomicAdd(nill, 1);
-        float term;
-        if (filter_bound(filt + 3 * size_t(p), &term))
-            atomicMax(nill + 1, __float_as_int(term));  // non-negative floats order like their bits
+        // the record is taken relative to the mesh's middle, where its corners round least; whether the
+        // filter serves the mesh, and its window's width, are judged at the mesh's place too (the larger
+        // bound term, both records safe)
+        const bool ill = ill_conditioned(ax, ay, az, bx, by, bz, cx, cy, cz);
+        if (ill) atomicAdd(nill, 1);
+        float4 placed[3];
+        float term, term_mid;
+        filter_record(ax, ay, az, bx, by, bz, cx, cy, cz, ill, placed);
+        const double mx = __int_as_float(frame[0]), my = __int_as_float(frame[1]), mz = __int_as_float(frame[2]);
+        filter_record(ax - mx, ay - my, az - mz, bx - mx, by - my, bz - mz, cx - mx, cy - my, cz - mz, ill,
+                      filt + 3 * size_t(p));
+        const bool safe = filter_bound(placed, &term) && filter_bound(filt + 3 * size_t(p), &term_mid);
+        if (safe)
+            atomicMax(nill + 1, __float_as_int(fmaxf(term, term_mid)));  // non-negative floats order like their bits
         else
             atomicAdd(nill + 2, 1);
     }
@@ -604,6 +624,215 @@ __global__ void k_tri_records(int nt, const int *__restrict__ sorted_ids, const 
         t64[5 * p + 3] = make_double2(cx, cy);
         t64[5 * p + 4] = make_double2(cz, double(t));
     }
+}
+
+// ---- oriented boxes --------------------------------------------------------------------------------
+//
+// The boxes the query kernels walk (DeviceMesh::obb). On a curved surface an axis-aligned box sticks out
+// of the surface by its triangles' tilt, and a query far from small triangles then wants every leaf of a
+// wide patch; a box along the patch does not. Per 32-query packet of the torus-knot 256^3 grid
+// (131,072 triangles) the walk meets 52 triangle iterations and 79 nodes instead of 187 and 133, on the
+// lattice of thin beams 23 and 164 instead of 166 and 225.
+//
+// Box frame: points are taken as (p - box_c) * box_scale, box_c the middle of the mesh's box (a float,
+// so p - box_c has one rounding) and box_scale 1 unless the mesh is larger than 2^60. M below is the
+// largest coordinate in that frame, u = 2^-24, d the distance from a query to a point q of the child.
+// Why the float box distance is a lower bound of d:
+// - With R the matrix of the three float axes, each axis' excess |axis.(p - centre)| - h is at most
+//   |axis.(p - q)|, so the box distance is at most |R (p - q)| <= (1 + 20 u) d (axes unit and orthogonal within 2^-20).
+// - Roundings of a coordinate along an axis: the vertices (float records against double ones, 1.8 u M),
+//   their offsets from the first vertex (3.5 u M), the dot products (10.4 u M), middle and half extent
+//   (7 u M), the centre's coordinate (10.4 u M), the query's (10.4 u M + 3 u d), its point (1.8 u M + u d):
+//   45 u M + 4 u d. Half extents are stored 64 u M = 2^-18 M larger, and everything scaled by 1 - 64 u, which
+//   covers the relative terms (at most 62 u of the squared distance).
+// - The float arithmetic (SSDF_PREC_F32) compares distances that may lie below the true ones: its
+//   region tests, on dot products within 11 u of their lengths, put the closest point at most D = 90 u
+//   alpha R off the triangle (alpha = longest edge / smallest altitude, R <= d + L the distance to the
+//   farthest corner, L the longest edge), in its plane. So half extents are also stored 128 u alpha L
+//   larger and everything scaled by 1 / (1 + 128 u alpha), alpha and L over the child's triangles. A child
+//   with alpha above kObbMaxAlpha keeps its axis-aligned box, as does one of more than kObbMaxTris
+//   triangles (its patch is no longer flat; building it would read every triangle at every level).
+constexpr int kObbMaxTris = 64;
+constexpr float kObbMaxAlpha = 2048.f;
+
+struct Vec3 {
+    float x, y, z;
+};
+__device__ __forceinline__ Vec3 vsub(Vec3 a, Vec3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
+__device__ __forceinline__ float vdot(Vec3 a, Vec3 b) { return fmaf(a.x, b.x, fmaf(a.y, b.y, a.z * b.z)); }
+__device__ __forceinline__ Vec3 vcross(Vec3 a, Vec3 b) {
+    return {fmaf(a.y, b.z, -a.z * b.y), fmaf(a.z, b.x, -a.x * b.z), fmaf(a.x, b.y, -a.y * b.x)};
+}
+
+// Corners of the triangle at leaf position p in the box frame.
+__device__ __forceinline__ void frame_corners(const float4 *__restrict__ t32, const double2 *__restrict__ t64, int p,
+                                              const float (&mid)[3], float scale, Vec3 (&v)[3]) {
+    if (t64) {
+        const double2 *r = t64 + 5 * size_t(p);
+        const double2 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2), d = __ldg(r + 3);
+        const double e = __ldg(&r[4].x), mx = mid[0], my = mid[1], mz = mid[2], s = scale;
+        v[0] = {float((a.x - mx) * s), float((a.y - my) * s), float((b.x - mz) * s)};
+        v[1] = {float((b.y - mx) * s), float((c.x - my) * s), float((c.y - mz) * s)};
+        v[2] = {float((d.x - mx) * s), float((d.y - my) * s), float((e - mz) * s)};
+    } else {
+        const float4 a = __ldg(t32 + 3 * p), b = __ldg(t32 + 3 * p + 1);
+        const float e = __ldg(&t32[3 * p + 2].x);
+        v[0] = {(a.x - mid[0]) * scale, (a.y - mid[1]) * scale, (a.z - mid[2]) * scale};
+        v[1] = {(a.w - mid[0]) * scale, (b.x - mid[1]) * scale, (b.y - mid[2]) * scale};
+        v[2] = {(b.z - mid[0]) * scale, (b.w - mid[1]) * scale, (e - mid[2]) * scale};
+    }
+}
+
+// A warp per child of a node: each lane takes a candidate frame -- the box frame's axes, a normal of one of
+// up to seven of the child's triangles with one of its edges, or the sum of the triangles' normals with an
+// edge -- and projects every corner on it; the frame of least half surface area wins (the summed normal
+// often does: with triangle normals alone the torus knot keeps 75 triangle iterations a packet, not 52).
+// Bound by the triangle records' loads, read once per level of up to kObbMaxTris triangles.
+__global__ void __launch_bounds__(128) k_obb(int nnodes, int L, const int *__restrict__ count,
+                                             const int *__restrict__ first_of, const double *__restrict__ pbox64,
+                                             const double *__restrict__ nbox64, const int *__restrict__ sorted_ids,
+                                             const float4 *__restrict__ nodes, const float4 *__restrict__ t32,
+                                             const double2 *__restrict__ t64, const int *__restrict__ frame,
+                                             float *__restrict__ obb) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const long long w = (blockIdx.x * 128ll + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    const int i = int(w >> 1), h = int(w & 1);
+    if (i >= nnodes) return;
+    if (i != 0 && (!count || count[i] <= L)) return;  // not a node of the walked tree (one leaf: the root alone is)
+    const float4 r4 = nodes[4 * size_t(i) + 3];
+    const int ref = __float_as_int(h ? r4.y : r4.x);
+    const float mid[3] = {__int_as_float(frame[0]), __int_as_float(frame[1]), __int_as_float(frame[2])};
+    const float scale = __int_as_float(frame[3]), M = __int_as_float(frame[4]);
+    // child's axes, -centre coordinates and half extents (a box that culls nothing)
+    Vec3 ax[3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+    float off[3] = {0.f, 0.f, 0.f}, half[3] = {0.f, 0.f, 0.f};
+    int writer = 0;
+    if (ref != kEmptyRef && M >= 0.f) {
+        const bool leaf = ref < 0;
+        const int n = leaf ? leaf_count(ref) : count[ref], first = leaf ? leaf_first(ref) : first_of[ref];
+        const float margin = 0x1p-18f * M;
+        // normals' sum, and the float arithmetic's terms over the child's triangles
+        float grow = 0.f, alpha = 0.f;
+        Vec3 ns{0.f, 0.f, 0.f};
+        const bool small = n <= kObbMaxTris;
+        if (small) {
+            for (int t = lane; t < n; t += 32) {
+                Vec3 v[3];
+                frame_corners(t32, t64, first + t, mid, scale, v);
+                const Vec3 e1 = vsub(v[1], v[0]), e2 = vsub(v[2], v[0]), e3 = vsub(v[2], v[1]);
+                const Vec3 c = vcross(e1, e2);
+                const float l2 = fmaxf(vdot(e1, e1), fmaxf(vdot(e2, e2), vdot(e3, e3)));
+                // all corners equal: no region test can err
+                const float al = l2 > 0.f ? l2 / sqrtf(vdot(c, c)) : 0.f;
+                alpha = al <= kObbMaxAlpha ? fmaxf(alpha, al) : FLT_MAX;  // a NaN or an overflow: too thin
+                grow = fmaxf(grow, al * sqrtf(l2));
+                ns = {ns.x + c.x, ns.y + c.y, ns.z + c.z};
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                alpha = fmaxf(alpha, __shfl_xor_sync(kAll, alpha, o));
+                grow = fmaxf(grow, __shfl_xor_sync(kAll, grow, o));
+                ns.x += __shfl_xor_sync(kAll, ns.x, o);
+                ns.y += __shfl_xor_sync(kAll, ns.y, o);
+                ns.z += __shfl_xor_sync(kAll, ns.z, o);
+            }
+        }
+        if (small && alpha <= kObbMaxAlpha) {
+            // this lane's frame
+            const int nsample = n < 7 ? n : 7;
+            const bool summed = lane >= 22 && lane < 31;
+            const int j = summed ? (lane - 22) / 3 : (lane - 1) / 3, e = summed ? (lane - 22) % 3 : (lane + 2) % 3;
+            bool ok = lane == 0;
+            ax[0] = {1.f, 0.f, 0.f}, ax[1] = {0.f, 1.f, 0.f}, ax[2] = {0.f, 0.f, 1.f};
+            if (lane > 0 && lane < 31 && j < nsample) {
+                Vec3 v[3];
+                frame_corners(t32, t64, first + (j * n) / nsample, mid, scale, v);
+                const Vec3 edge = e == 0 ? vsub(v[1], v[0]) : (e == 1 ? vsub(v[2], v[0]) : vsub(v[2], v[1]));
+                Vec3 c = summed ? ns : vcross(vsub(v[1], v[0]), vsub(v[2], v[0]));
+                const float rc = rsqrtf(vdot(c, c));
+                c = {c.x * rc, c.y * rc, c.z * rc};
+                const float along = vdot(edge, c);
+                Vec3 d{fmaf(-along, c.x, edge.x), fmaf(-along, c.y, edge.y), fmaf(-along, c.z, edge.z)};
+                float rd = rsqrtf(vdot(d, d));
+                d = {d.x * rd, d.y * rd, d.z * rd};
+                const float again = vdot(d, c);  // orthogonal to rounding
+                d = {fmaf(-again, c.x, d.x), fmaf(-again, c.y, d.y), fmaf(-again, c.z, d.z)};
+                rd = rsqrtf(vdot(d, d));
+                d = {d.x * rd, d.y * rd, d.z * rd};
+                const Vec3 f = vcross(c, d);
+                // unit and orthogonal within 2^-20 (a NaN is not)
+                ok = fabsf(vdot(c, c) - 1.f) < 0x1p-20f && fabsf(vdot(d, d) - 1.f) < 0x1p-20f &&
+                     fabsf(vdot(c, d)) < 0x1p-20f && fabsf(vdot(f, f) - 1.f) < 0x1p-20f;
+                if (ok) ax[0] = d, ax[1] = f, ax[2] = c;
+            }
+            Vec3 o[3];
+            frame_corners(t32, t64, first, mid, scale, o);
+            float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+            for (int t = 0; t < n; t++) {
+                Vec3 v[3];
+                frame_corners(t32, t64, first + t, mid, scale, v);
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    const Vec3 q = vsub(v[k], o[0]);
+#pragma unroll
+                    for (int a = 0; a < 3; a++) {
+                        const float x = vdot(ax[a], q);
+                        lo[a] = fminf(lo[a], x), hi[a] = fmaxf(hi[a], x);
+                    }
+                }
+            }
+            const float pad = margin + 128.f * 0x1p-24f * grow * 1.001f;
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                half[a] = 0.5f * (hi[a] - lo[a]) + pad;
+                off[a] = -(vdot(ax[a], o[0]) + 0.5f * (lo[a] + hi[a]));
+            }
+            const float area = half[0] * half[1] + half[1] * half[2] + half[2] * half[0];
+            const unsigned key = ok && area < FLT_MAX ? __float_as_uint(area) : 0x7f800000u;
+            const unsigned least = __reduce_min_sync(kAll, key);
+            writer = __ffs(__ballot_sync(kAll, key == least)) - 1;
+            // lane 0's frame is always a candidate; all keys infinite (an overflow): keep its box
+            const float s = (1.f - 0x1p-18f) / (1.f + 128.f * 0x1p-24f * alpha);
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                ax[a] = {ax[a].x * s, ax[a].y * s, ax[a].z * s};
+                off[a] *= s;
+                // an extent the margins cannot bound (an overflow) culls nothing
+                half[a] = half[a] < FLT_MAX ? half[a] * s : __int_as_float(0x7f800000);
+            }
+        } else {
+            // the axis-aligned box of the double corners
+            const double *b = leaf && n == 1 ? pbox64 + 6 * size_t(sorted_ids[first])
+                                             : (leaf ? nullptr : nbox64 + 6 * size_t(ref));
+            double e[6];
+            if (b) {
+                for (int k = 0; k < 6; k++) e[k] = b[k];
+            } else {  // a leaf of several triangles: the union of their boxes
+                for (int k = 0; k < 6; k++) e[k] = (k & 1) ? -DBL_MAX : DBL_MAX;
+                for (int t = 0; t < n; t++) {
+                    const double *q = pbox64 + 6 * size_t(sorted_ids[first + t]);
+                    for (int k = 0; k < 6; k += 2) e[k] = fmin(e[k], q[k]), e[k + 1] = fmax(e[k + 1], q[k + 1]);
+                }
+            }
+            const float s = 1.f - 0x1p-18f;
+            ax[0] = {s, 0.f, 0.f}, ax[1] = {0.f, s, 0.f}, ax[2] = {0.f, 0.f, s};
+            for (int a = 0; a < 3; a++) {
+                const float lo = float((e[2 * a] - double(mid[a])) * double(scale));
+                const float hi = float((e[2 * a + 1] - double(mid[a])) * double(scale));
+                half[a] = (0.5f * (hi - lo) + margin) * s;
+                off[a] = -0.5f * (lo + hi) * s;
+            }
+        }
+    }
+    if (ref == kEmptyRef) off[0] = 0x1p60f;  // never entered, and the farther child
+    if (lane != writer) return;
+    float *o = obb + 32 * size_t(i) + h;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        o[8 * a] = ax[a].x, o[8 * a + 2] = ax[a].y, o[8 * a + 4] = ax[a].z, o[8 * a + 6] = off[a];
+        o[24 + 2 * a] = half[a];
+    }
+    o[30] = __int_as_float(ref);
 }
 
 // ---- pseudo-normals --------------------------------------------------------------------------------
@@ -769,7 +998,8 @@ static int readback_words(int **out) {
 
 static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int nt, const int *s0_in,
                            const int *s1_in, const int *s2_in, int nv, const void *sx, const void *sy, const void *sz,
-                           int coord_f64, int device_ptrs, const ssdf_build_opts &opts, cudaStream_t stream) {
+                           int coord_f64, int device_ptrs, const ssdf_build_opts &opts, bool query_boxes,
+                           cudaStream_t stream) {
     const int L = opts.leaf_size > 0 ? opts.leaf_size : 4;
     m->nt = nt;
     m->nv = nv;
@@ -810,9 +1040,9 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
     LAUNCH_CHECK("k_widen");
     // validation + per-triangle boxes
     // [0] first bad triangle, [1..6] scene, [7] scale, [8..9] depth / leaves, [10] ill, [11] largest
-    // filter bound term (float bits), [12] records unsafe for the float filter
+    // filter bound term (float bits), [12] records unsafe for the float filter, [16..20] the box frame
     int *flags;
-    SSDF_CHECK(dalloc(tmp, &flags, 16, stream));
+    SSDF_CHECK(dalloc(tmp, &flags, 24, stream));
     k_init_flags<<<1, 32, 0, stream>>>(flags);
     LAUNCH_CHECK("k_init_flags");
     if (device_ptrs) {
@@ -848,26 +1078,29 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
     const int nint = nt > 1 ? nt - 1 : 0;
     m->nnodes = nint > 0 ? nint : 1;
     float4 *nodes32;
-    double2 *nodes64 = nullptr;
+    float4 *obb = nullptr;
     SSDF_CHECK(dalloc(s, &nodes32, 4 * size_t(m->nnodes), stream));
-    if (keep64) SSDF_CHECK(dalloc(s, &nodes64, 8 * size_t(m->nnodes), stream));
+    if (query_boxes) SSDF_CHECK(dalloc(s, &obb, 8 * size_t(m->nnodes), stream));
     float4 *nodes4_32;
     double2 *nodes4_64 = nullptr;
     SSDF_CHECK(dalloc(s, &nodes4_32, 8 * size_t(m->nnodes), stream));
     if (keep64) SSDF_CHECK(dalloc(s, &nodes4_64, 14 * size_t(m->nnodes), stream));
     // read-backs: [0..1] depth and leaves, [2..2 + kMaxLevels4] 4-wide level sizes, then the slots
-    // used, then the coordinate scale and the three filter words
-    static_assert(2 + kMaxLevels4 + 2 + 4 <= kReadbackWords, "read-back words");
+    // used, then the coordinate scale, the three filter words and the four of the box frame
+    static_assert(2 + kMaxLevels4 + 2 + 8 <= kReadbackWords, "read-back words");
     int *rb = nullptr;
     SSDF_CHECK(readback_words(&rb));
     int *const depth_leaves = rb, *const level_hist = rb + 2;
     int *const scale_word = rb + 2 + kMaxLevels4 + 2, *const filt_info = scale_word + 1;
+    int *const frame_words = filt_info + 3;
     depth_leaves[0] = depth_leaves[1] = 1;
     int nnodes4 = 1, depth4 = 1;
     bool collapsed = false;
+    const int *obb_first = nullptr, *obb_count = nullptr;  // subtree ranges (null: the small root)
+    const double *obb_nbox = nullptr;
     if (nt <= L) {
         // one leaf over everything (its triangle order is the Morton order)
-        k_write_small_root<<<1, 1, 0, stream>>>(nt, box32, box64, nodes32, nodes64);
+        k_write_small_root<<<1, 1, 0, stream>>>(nt, box32, nodes32);
         LAUNCH_CHECK("k_write_small_root");
         k_write_small_root4<<<1, 1, 0, stream>>>(nt, box32, box64, nodes4_32, nodes4_64);
         LAUNCH_CHECK("k_write_small_root4");
@@ -901,7 +1134,7 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
                                                            arrivals);
         LAUNCH_CHECK("k_counts");
         k_write_nodes<<<grid_blocks(nint, 256), 256, 0, stream>>>(nt, L, child_l, child_r, first_of, count, ids,
-                                                                  box32, box64, nbox32, nbox64, nodes32, nodes64);
+                                                                  box32, nbox32, nodes32);
         LAUNCH_CHECK("k_write_nodes");
         k_depth<<<grid_blocks(nint, 256), 256, 0, stream>>>(nt, L, count, parent_int, child_l, child_r, flags + 8);
         LAUNCH_CHECK("k_depth");
@@ -934,6 +1167,7 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
         SSDF_CUDA(cudaMemcpyAsync(level_hist, level_sizes, sizeof(int) * (kMaxLevels4 + 2), cudaMemcpyDeviceToHost,
                                   stream));  // page-locked: no wait here
         collapsed = true;
+        obb_first = first_of, obb_count = count, obb_nbox = nbox64;
     }
     // triangle records in leaf order
     float4 *t32, *filt = nullptr;
@@ -941,9 +1175,18 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
     SSDF_CHECK(dalloc(s, &t32, 3 * size_t(nt), stream));
     if (keep64) SSDF_CHECK(dalloc(s, &t64, 5 * size_t(nt), stream));
     if (keep64) SSDF_CHECK(dalloc(s, &filt, 3 * size_t(nt), stream));  // the fix-up path's filter records
+    k_box_frame<<<1, 1, 0, stream>>>(nodes32, flags + 16);
+    LAUNCH_CHECK("k_box_frame");
     k_tri_records<<<grid_blocks(nt, 256), 256, 0, stream>>>(nt, ids, s0, s1, s2, vx, vy, vz, t32, t64, filt,
-                                                            flags + 10);
+                                                            flags + 16, flags + 10);
     LAUNCH_CHECK("k_tri_records");
+    // oriented boxes of the tree's children, from the triangle records
+    if (query_boxes) {
+        k_obb<<<grid_blocks(2ll * m->nnodes * 32, 128), 128, 0, stream>>>(
+            m->nnodes, L, obb_count, obb_first, box64, obb_nbox, ids, nodes32, t32, t64, flags + 16, (float *)obb);
+        LAUNCH_CHECK("k_obb");
+    }
+    SSDF_CUDA(cudaMemcpyAsync(frame_words, flags + 16, 4 * sizeof(int), cudaMemcpyDeviceToHost, stream));
     SSDF_CUDA(cudaMemcpyAsync(scale_word, flags + 7, sizeof(int), cudaMemcpyDeviceToHost, stream));
     SSDF_CUDA(cudaMemcpyAsync(filt_info, flags + 10, 3 * sizeof(int), cudaMemcpyDeviceToHost, stream));
     if (opts.normals) SSDF_CHECK(build_normals(s, m, s0, s1, s2, vx, vy, vz, stream));
@@ -951,6 +1194,8 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
     float scale;
     memcpy(&scale, scale_word, sizeof(float));
     m->coord_scale = scale;
+    memcpy(m->box_c, frame_words, 3 * sizeof(float));
+    memcpy(&m->box_scale, frame_words + 3, sizeof(float));
     m->nill = filt_info[0];
     if (keep64) {
         float term;
@@ -965,7 +1210,7 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
     m->depth = depth_leaves[0];
     m->nleaves = depth_leaves[1];
     m->nodes32 = nodes32;
-    m->nodes64 = nodes64;
+    m->obb = obb;
     m->nodes4_32 = nodes4_32;
     m->nodes4_64 = nodes4_64;
     m->nnodes4 = nnodes4;
@@ -982,7 +1227,7 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
 
 int mesh_build(MeshStorage **storage, DeviceMesh *mesh, ptrdiff_t nt, const int *s0, const int *s1, const int *s2,
                ptrdiff_t nv, const void *sx, const void *sy, const void *sz, int coord_f64, int device_ptrs,
-               const ssdf_build_opts &opts, cudaStream_t stream) {
+               const ssdf_build_opts &opts, cudaStream_t stream, bool query_boxes) {
     if (nt <= 0 || nv <= 0) return fail(SSDF_ERR_INVALID_ARGUMENT, "empty mesh");
     if (nt >= kMaxTriangles) return fail(SSDF_ERR_NOT_SUPPORTED, "more than 2^26 triangles in one mesh");
     if (nv >= (1ll << 31)) return fail(SSDF_ERR_NOT_SUPPORTED, "more than 2^31 vertices");
@@ -994,7 +1239,7 @@ int mesh_build(MeshStorage **storage, DeviceMesh *mesh, ptrdiff_t nt, const int 
     MeshStorage tmp;
     *mesh = DeviceMesh();
     int st = mesh_build_impl(s, &tmp, mesh, int(nt), s0, s1, s2, int(nv), sx, sy, sz, coord_f64, device_ptrs, opts,
-                             stream);
+                             query_boxes, stream);
     for (void *p : tmp.blocks) cudaFreeAsync(p, stream);
     if (st == SSDF_OK) {
         cudaError_t e = cudaStreamSynchronize(stream);
