@@ -451,7 +451,7 @@ int ssdf_points_aabb_signed_distance(ptrdiff_t npoints, const void *x, const voi
 typedef struct ssdf_batch ssdf_batch;
 
 /* traversal: 0 automatic (warp packets for grids), 1 warp packets, 2 thread per query;
- * arity: 0 automatic (binary), 2, 4. One arithmetic (precision) per batch. */
+ * arity: 0, 2 or 4; all walk the same (binary) tree. One arithmetic (precision) per batch. */
 int ssdf_batch_create(ssdf_batch **batch, int max_jobs, int precision, int traversal, int arity);
 int ssdf_batch_destroy(ssdf_batch *batch);
 /* Pre-sizes the batch's fix-up overflow lists for runs of up to max_queries queries in total, so
@@ -486,11 +486,11 @@ long long ssdf_batch_last_blocks(const ssdf_batch *batch);
 typedef struct {
     int leaf_size; /* BVH leaf size: 2, 4 or 8                                               */
     int traversal; /* 1 warp packets, 2 thread per query                                      */
-    int arity;     /* 2 binary, 4 four-wide                                                   */
+    int arity;     /* 2 (binary)                                                              */
     double ms;     /* measured time of the winner on the sample grid                         */
 } ssdf_tuning;
 
-/* Times leaf sizes {2, 4, 8} x traversal {warp, thread} x arity {2, 4} for this mesh (host double
+/* Times leaf sizes {2, 4, 8} x traversal {warp, thread} for this mesh (host double
  * arrays) on a sample of the grid -- the same box at up to 2^21 nodes -- in the given arithmetic,
  * and returns the fastest. With cache_path (a JSON file) the winner is stored per size class
  * (log2 triangles, log2 nodes, arithmetic) and later calls of that class return it untimed. */

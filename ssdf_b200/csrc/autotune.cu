@@ -1,7 +1,7 @@
-// autotune.cu -- picks the BVH leaf size, traversal mode and BVH arity for a mesh and a query grid.
+// autotune.cu -- picks the BVH leaf size and traversal mode for a mesh and a query grid.
 //
 // No reference counterpart. The candidates are leaf sizes {2, 4, 8} x {warp packets, thread per
-// query} x {binary, 4-wide}. Each is timed (CUDA events, best of two after a warm-up) on a sample of
+// query}. Each is timed (CUDA events, best of two after a warm-up) on a sample of
 // the grid: the same box at a resolution scaled down to at most 2^21 nodes, so the distances -- and
 // the traversal cost per query -- stay those of the full grid. The winner is cached per size class
 // (log2 of the triangle count, log2 of the node count, arithmetic) in a small JSON file, one entry
@@ -119,29 +119,25 @@ int ssdf_autotune_grid(ptrdiff_t nselements, const int *s0, const int *s1, const
         qo.coord_type = SSDF_F64;
         qo.out_type = SSDF_F64;
         for (int trav = 1; trav <= 2 && st == SSDF_OK; trav++) {
-            for (int ar = 2; ar <= 4 && st == SSDF_OK; ar += 2) {
-                QueryArgs a;
-                st = fill_grid_args(m, sn[0], sn[1], sn[2], lo, hi, out, nullptr, &qo, &a);
-                if (st != SSDF_OK) break;
-                a.force_traversal = trav;
-                a.force_arity = ar;
-                float bestms = 1e30f;
-                for (int rep = 0; rep < 3 && st == SSDF_OK; rep++) {
-                    if (precision == SSDF_PREC_F32) cudaMemsetAsync(out, 0x7f, sizeof(double) * size_t(ns), stream);
-                    cudaEventRecord(e0, stream);
-                    st = launch_query(a, precision, stream);
-                    cudaEventRecord(e1, stream);
-                    if (cudaEventSynchronize(e1) != cudaSuccess) st = fail(SSDF_ERR_CUDA, "autotune timing");
-                    float ms = 0.f;
-                    cudaEventElapsedTime(&ms, e0, e1);
-                    if (rep > 0) bestms = std::min(bestms, ms);
-                }
-                if (st == SSDF_OK && bestms < win.ms) {
-                    win.ms = bestms;
-                    win.leaf_size = leaves[li];
-                    win.traversal = trav;
-                    win.arity = ar;
-                }
+            QueryArgs a;
+            st = fill_grid_args(m, sn[0], sn[1], sn[2], lo, hi, out, nullptr, &qo, &a);
+            if (st != SSDF_OK) break;
+            a.force_traversal = trav;
+            float bestms = 1e30f;
+            for (int rep = 0; rep < 3 && st == SSDF_OK; rep++) {
+                if (precision == SSDF_PREC_F32) cudaMemsetAsync(out, 0x7f, sizeof(double) * size_t(ns), stream);
+                cudaEventRecord(e0, stream);
+                st = launch_query(a, precision, stream);
+                cudaEventRecord(e1, stream);
+                if (cudaEventSynchronize(e1) != cudaSuccess) st = fail(SSDF_ERR_CUDA, "autotune timing");
+                float ms = 0.f;
+                cudaEventElapsedTime(&ms, e0, e1);
+                if (rep > 0) bestms = std::min(bestms, ms);
+            }
+            if (st == SSDF_OK && bestms < win.ms) {
+                win.ms = bestms;
+                win.leaf_size = leaves[li];
+                win.traversal = trav;
             }
         }
         ssdf_mesh_destroy(m);

@@ -27,7 +27,6 @@ struct ssdf_batch {
     int max_jobs = 0;
     int precision = SSDF_PREC_F32_FIXUP;
     int traversal = 0;  // 0 auto, 1 warp, 2 thread
-    int arity = 0;      // 0 auto, 2, 4
     std::vector<QueryArgs> jobs;
     // device tables: [0] the batch's own arithmetic, [1] the FP64 jobs of a fix-up batch
     BatchHeader *d_hdr = nullptr;  // [2]
@@ -41,8 +40,8 @@ struct ssdf_batch {
     BatchHeader *h_hdr = nullptr;  // [2]
     QueryArgs *h_jobs = nullptr, *h_jobs64 = nullptr;
     long long *h_first = nullptr, *h_first64 = nullptr;
-    // captured graphs, one per (warp, wide, FP64 table) key: a run reuses the graph of its key
-    cudaGraphExec_t exec[16] = {};
+    // captured graphs, one per (warp, FP64 table) key: a run reuses the graph of its key
+    cudaGraphExec_t exec[4] = {};
     int sms = 0;
     long long last_total = 0;
 };
@@ -65,10 +64,10 @@ static void batch_free(ssdf_batch *b) {
     cudaFreeHost(b->h_first64);
 }
 
-// The launch sequence of one run with the given traversal and arity: counters reset, then the
+// The launch sequence of one run with the given traversal: counters reset, then the
 // persistent kernel and the window stage, then (f64) the persistent FP64 kernel over the second
 // table. It reads the job tables from device memory only.
-static int enqueue_run(ssdf_batch *b, bool warp, bool wide, bool f64, cudaStream_t s) {
+static int enqueue_run(ssdf_batch *b, bool warp, bool f64, cudaStream_t s) {
     BatchLaunch L;
     L.hdr = b->d_hdr;
     L.jobs = b->d_jobs;
@@ -76,8 +75,7 @@ static int enqueue_run(ssdf_batch *b, bool warp, bool wide, bool f64, cudaStream
     L.next_item = b->d_next;
     L.sms = b->sms;
     L.warp = warp;
-    L.wide = wide;
-    L.grid = b->sms * batch_blocks_per_sm(b->precision, warp, wide);
+    L.grid = b->sms * batch_blocks_per_sm(b->precision, warp);
     cudaError_t e = cudaMemsetAsync(b->d_next, 0, 2 * sizeof(unsigned long long), s);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->d_fbcount, 0, sizeof(int) * b->max_jobs, s);
     if (e != cudaSuccess) return cuda_fail(e, "batch reset", __FILE__, __LINE__);
@@ -88,18 +86,18 @@ static int enqueue_run(ssdf_batch *b, bool warp, bool wide, bool f64, cudaStream
     D.jobs = b->d_jobs64;
     D.first_block = b->d_first64;
     D.next_item = b->d_next + 1;
-    D.grid = b->sms * batch_blocks_per_sm(SSDF_PREC_F64, warp, wide);
+    D.grid = b->sms * batch_blocks_per_sm(SSDF_PREC_F64, warp);
     return launch_batch(D, SSDF_PREC_F64, s);
 }
 
-static int graph_key(bool warp, bool wide, bool f64) {
-    return (warp ? 1 : 0) | (wide ? 2 : 0) | (f64 ? 4 : 0);
+static int graph_key(bool warp, bool f64) {
+    return (warp ? 1 : 0) | (f64 ? 2 : 0);
 }
 
-// Captures (once) the graph of a (traversal, arity, FP64 table) key on a private stream,
+// Captures (once) the graph of a (traversal, FP64 table) key on a private stream,
 // thread-local mode.
-static int capture_key(ssdf_batch *b, bool warp, bool wide, bool f64) {
-    const int key = graph_key(warp, wide, f64);
+static int capture_key(ssdf_batch *b, bool warp, bool f64) {
+    const int key = graph_key(warp, f64);
     if (b->exec[key]) return SSDF_OK;
     cudaStream_t cap;
     SSDF_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
@@ -107,7 +105,7 @@ static int capture_key(ssdf_batch *b, bool warp, bool wide, bool f64) {
     cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
     int st = SSDF_OK;
     if (e == cudaSuccess) {
-        st = enqueue_run(b, warp, wide, f64, cap);
+        st = enqueue_run(b, warp, f64, cap);
         e = cudaStreamEndCapture(cap, &g);
     }
     if (e == cudaSuccess && st == SSDF_OK) e = cudaGraphInstantiate(&b->exec[key], g, 0);
@@ -123,13 +121,11 @@ namespace ssdf_b200 {
 // running in one thread while another thread synchronises the device fails; the server calls this
 // before its threads start.
 int batch_capture_graphs(ssdf_batch *b) {
-    for (int warp = 0; warp < 2; warp++)
-        for (int wide = 0; wide < 2; wide++) {
-            if ((b->traversal == 1 && !warp) || (b->traversal == 2 && warp)) continue;
-            if ((b->arity == 2 && wide) || (b->arity == 4 && !wide)) continue;
-            for (int f64 = 0; f64 < (b->precision == SSDF_PREC_F32_FIXUP ? 2 : 1); f64++)
-                SSDF_CHECK(capture_key(b, warp != 0, wide != 0, f64 != 0));
-        }
+    for (int warp = 0; warp < 2; warp++) {
+        if ((b->traversal == 1 && !warp) || (b->traversal == 2 && warp)) continue;
+        for (int f64 = 0; f64 < (b->precision == SSDF_PREC_F32_FIXUP ? 2 : 1); f64++)
+            SSDF_CHECK(capture_key(b, warp != 0, f64 != 0));
+    }
     return SSDF_OK;
 }
 }  // namespace ssdf_b200
@@ -145,7 +141,7 @@ int ssdf_batch_create(ssdf_batch **out, int max_jobs, int precision, int travers
     b->max_jobs = max_jobs;
     b->precision = precision;
     b->traversal = traversal;
-    b->arity = arity;
+    (void)arity;  // 2 and 4 walk the same tree
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev);
@@ -251,7 +247,7 @@ int ssdf_batch_reserve(ssdf_batch *b, long long max_queries, void *stream_) {
 }
 
 // One persistent launch over every job (+ the fix-up window stage). use_graph: capture the launch
-// sequence once (per traversal mode and arity) and replay it afterwards.
+// sequence once (per traversal mode) and replay it afterwards.
 int ssdf_batch_run(ssdf_batch *b, int use_graph, void *stream_) {
     if (!b) return fail(SSDF_ERR_INVALID_ARGUMENT, "null batch");
     cudaStream_t stream = (cudaStream_t)stream_;
@@ -266,7 +262,6 @@ int ssdf_batch_run(ssdf_batch *b, int use_graph, void *stream_) {
         any_sorted |= sort_points && !j.is_grid && j.npoints >= kSortMinPoints;
     }
     const bool warp = b->traversal == 1 ? true : b->traversal == 2 ? false : default_warp(any_grid || any_sorted);
-    const bool wide = b->arity == 4 ? true : b->arity == 2 ? false : default_wide();
     // the FP64 table of a fix-up batch: jobs whose meshes the FP64 kernel answers (fixup_runs_f64)
     const bool fixup = b->precision == SSDF_PREC_F32_FIXUP;
     auto to_f64 = [&](const QueryArgs &a) { return fixup && fixup_runs_f64(a.m); };
@@ -351,9 +346,9 @@ int ssdf_batch_run(ssdf_batch *b, int use_graph, void *stream_) {
             cudaMemcpyAsync(b->d_first64, b->h_first64, sizeof(long long) * k64, cudaMemcpyHostToDevice, stream));
     }
     const bool f64 = k64 > 0;
-    if (!use_graph) return enqueue_run(b, warp, wide, f64, stream);
-    SSDF_CHECK(capture_key(b, warp, wide, f64));
-    SSDF_CUDA(cudaGraphLaunch(b->exec[graph_key(warp, wide, f64)], stream));
+    if (!use_graph) return enqueue_run(b, warp, f64, stream);
+    SSDF_CHECK(capture_key(b, warp, f64));
+    SSDF_CUDA(cudaGraphLaunch(b->exec[graph_key(warp, f64)], stream));
     return SSDF_OK;
 }
 

@@ -140,62 +140,6 @@ __device__ __forceinline__ void store_out(const QueryArgs &a, long long q, doubl
 
 // ---- node and triangle loads ----------------------------------------------------------------------
 
-// 4-wide node: per child c, box (lox, hix, loy, hiy, loz, hiz)[c] and reference r[c].
-template <typename T>
-__device__ __forceinline__ void boxes4_exact(const DeviceMesh &m, int node, T px, T py, T pz, T (&d)[4], int (&r)[4]);
-
-template <>
-__device__ __forceinline__ void boxes4_exact<float>(const DeviceMesh &m, int node, float px, float py, float pz,
-                                                    float (&d)[4], int (&r)[4]) {
-    const float4 *p = m.nodes4_32 + 8 * node;
-    const float4 lx = __ldg(p), hx = __ldg(p + 1), ly = __ldg(p + 2), hy = __ldg(p + 3), lz = __ldg(p + 4),
-                 hz = __ldg(p + 5), rr = __ldg(p + 6);
-    d[0] = box_dist_sq<float>(px, py, pz, lx.x, hx.x, ly.x, hy.x, lz.x, hz.x);
-    d[1] = box_dist_sq<float>(px, py, pz, lx.y, hx.y, ly.y, hy.y, lz.y, hz.y);
-    d[2] = box_dist_sq<float>(px, py, pz, lx.z, hx.z, ly.z, hy.z, lz.z, hz.z);
-    d[3] = box_dist_sq<float>(px, py, pz, lx.w, hx.w, ly.w, hy.w, lz.w, hz.w);
-    r[0] = __float_as_int(rr.x), r[1] = __float_as_int(rr.y), r[2] = __float_as_int(rr.z), r[3] = __float_as_int(rr.w);
-}
-
-template <>
-__device__ __forceinline__ void boxes4_exact<double>(const DeviceMesh &m, int node, double px, double py, double pz,
-                                                     double (&d)[4], int (&r)[4]) {
-    const double2 *p = m.nodes4_64 + 14 * node;
-    double2 row[12];
-#pragma unroll
-    for (int k = 0; k < 12; k++) row[k] = __ldg(p + k);
-    const double2 rr = __ldg(p + 12);
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        const int h = c >> 1;
-        auto pick = [&](int rw) { return (c & 1) ? row[2 * rw + h].y : row[2 * rw + h].x; };
-        d[c] = box_dist_sq<double>(px, py, pz, pick(0), pick(1), pick(2), pick(3), pick(4), pick(5));
-    }
-    const unsigned long long a = (unsigned long long)__double_as_longlong(rr.x);
-    const unsigned long long b = (unsigned long long)__double_as_longlong(rr.y);
-    r[0] = int(unsigned(a)), r[1] = int(unsigned(a >> 32)), r[2] = int(unsigned(b)), r[3] = int(unsigned(b >> 32));
-}
-
-// The 4-wide node's child-box distances (p - clamp(p, lo, hi) per axis, fused squared norm), children
-// (0, 1) and (2, 3) as packed FP32 pairs.
-__device__ __forceinline__ void boxes4_pair(const DeviceMesh &m, int node, float px, float py, float pz,
-                                            float (&d)[4], int (&r)[4]) {
-    const float4 *p = m.nodes4_32 + 8 * node;
-    const float4 lx = __ldg(p), hx = __ldg(p + 1), ly = __ldg(p + 2), hy = __ldg(p + 3), lz = __ldg(p + 4),
-                 hz = __ldg(p + 5), rr = __ldg(p + 6);
-    const float2 x2 = make_float2(px, px), y2 = make_float2(py, py), z2 = make_float2(pz, pz);
-    const float2 dx01 = __fadd2_rn(x2, make_float2(-fminf(fmaxf(px, lx.x), hx.x), -fminf(fmaxf(px, lx.y), hx.y)));
-    const float2 dy01 = __fadd2_rn(y2, make_float2(-fminf(fmaxf(py, ly.x), hy.x), -fminf(fmaxf(py, ly.y), hy.y)));
-    const float2 dz01 = __fadd2_rn(z2, make_float2(-fminf(fmaxf(pz, lz.x), hz.x), -fminf(fmaxf(pz, lz.y), hz.y)));
-    const float2 dx23 = __fadd2_rn(x2, make_float2(-fminf(fmaxf(px, lx.z), hx.z), -fminf(fmaxf(px, lx.w), hx.w)));
-    const float2 dy23 = __fadd2_rn(y2, make_float2(-fminf(fmaxf(py, ly.z), hy.z), -fminf(fmaxf(py, ly.w), hy.w)));
-    const float2 dz23 = __fadd2_rn(z2, make_float2(-fminf(fmaxf(pz, lz.z), hz.z), -fminf(fmaxf(pz, lz.w), hz.w)));
-    const float2 s01 = __ffma2_rn(dx01, dx01, __ffma2_rn(dy01, dy01, __fmul2_rn(dz01, dz01)));
-    const float2 s23 = __ffma2_rn(dx23, dx23, __ffma2_rn(dy23, dy23, __fmul2_rn(dz23, dz23)));
-    d[0] = s01.x, d[1] = s01.y, d[2] = s23.x, d[3] = s23.y;
-    r[0] = __float_as_int(rr.x), r[1] = __float_as_int(rr.y), r[2] = __float_as_int(rr.z), r[3] = __float_as_int(rr.w);
-}
-
 struct Tri32 {
     float ax, ay, az, bx, by, bz, cx, cy, cz;
     int id;
@@ -251,7 +195,6 @@ struct ExactData<double> {
     }
     // a threshold beyond float's range is +inf: a box distance that overflowed still counts as inside
     static __device__ __forceinline__ float box_key(float d) { return fminf(d, FLT_MAX); }
-    static __device__ __forceinline__ float key_of(double d) { return fminf(__double2float_rd(d), FLT_MAX); }
     static __device__ __forceinline__ Tri tri(const DeviceMesh &m, int pos) { return load_tri64(m.tris64, pos); }
 };
 template <>
@@ -269,7 +212,6 @@ struct ExactData<float> {
         return (p - m.box_c[d]) * m.box_scale;
     }
     static __device__ __forceinline__ float box_key(float d) { return d; }
-    static __device__ __forceinline__ float key_of(float d) { return d; }
     static __device__ __forceinline__ Tri tri(const DeviceMesh &m, int pos) { return load_tri32(m.tris32, pos); }
 };
 
@@ -326,15 +268,6 @@ struct ExactPolicy {
             const float2 d = obb_dist_sq_pair(bx[q], by[q], bz[q], m.obb + 8 * node, r0, r1);
             d0[q] = ExactData<T>::box_key(d.x);
             d1[q] = ExactData<T>::box_key(d.y);
-        }
-    }
-    __device__ __forceinline__ void boxes4(int node, float (&d)[4][Q], int (&r)[4]) const {
-#pragma unroll
-        for (int q = 0; q < Q; q++) {
-            T dq[4];
-            boxes4_exact<T>(m, node, px[q], py[q], pz[q], dq, r);
-#pragma unroll
-            for (int c = 0; c < 4; c++) d[c][q] = ExactData<T>::key_of(dq[c] * T(m.box_scale) * T(m.box_scale));
         }
     }
     __device__ __forceinline__ float max_thr() const {
@@ -440,15 +373,6 @@ struct FastPolicy {
             const float2 d = obb_dist_sq_pair(bx[q], by[q], bz[q], m.obb + 8 * node, r0, r1);
             d0[q] = d.x;
             d1[q] = d.y;
-        }
-    }
-    __device__ __forceinline__ void boxes4(int node, float (&d)[4][Q], int (&r)[4]) const {
-#pragma unroll
-        for (int q = 0; q < Q; q++) {
-            float dq[4];
-            boxes4_pair(m, node, bx[q].x + m.box_c[0], by[q].x + m.box_c[1], bz[q].x + m.box_c[2], dq, r);
-#pragma unroll
-            for (int c = 0; c < 4; c++) d[c][q] = dq[c];
         }
     }
     __device__ __forceinline__ float max_thr() const {
@@ -704,178 +628,6 @@ __device__ __forceinline__ void traverse(P &p, Counters &cnt, int budget) {
     }
 }
 
-// The same over the 4-wide BVH. Children are visited in ascending box distance -- the lane's own
-// smallest in thread mode, a representative lane's (the brick centre) in warp mode -- leaves first
-// in that order, then the nearest wanted internal child is entered and the others pushed
-// farthest-first.
-
-template <typename R, int Q>
-__device__ __forceinline__ void cswap4(float (&k)[4], R (&d)[4][Q], int (&r)[4], int i, int j) {
-    if (k[j] < k[i]) {
-        const float tk = k[i];
-        k[i] = k[j];
-        k[j] = tk;
-#pragma unroll
-        for (int q = 0; q < Q; q++) {
-            const R td = d[i][q];
-            d[i][q] = d[j][q];
-            d[j][q] = td;
-        }
-        const int tr = r[i];
-        r[i] = r[j];
-        r[j] = tr;
-    }
-}
-
-template <bool WARP, bool COUNT, class P>
-__device__ __forceinline__ void traverse4(P &p, Counters &cnt) {
-    using R = typename P::R;
-    constexpr int Q = P::kQn;
-    int snode[kStackSize];
-    R sdist[kStackSize];
-    int sp = 0;
-    int node = 0;
-    while (true) {
-        R d[4][Q];
-        int r[4];
-        p.boxes4(node, d, r);
-        if (COUNT) cnt.box += 4 * Q;
-        float key[4];
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const float own = float(min_of<R, Q>(d[c]));
-            key[c] = WARP ? __shfl_sync(0xffffffffu, own, kRepLane) : own;
-        }
-        cswap4<R, Q>(key, d, r, 0, 1);
-        cswap4<R, Q>(key, d, r, 2, 3);
-        cswap4<R, Q>(key, d, r, 0, 2);
-        cswap4<R, Q>(key, d, r, 1, 3);
-        cswap4<R, Q>(key, d, r, 1, 2);
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            if (r[c] >= 0 || r[c] == kEmptyRef) continue;
-            const unsigned m = want_mask(p, d[c]);
-            if (WARP ? !__any_sync(0xffffffffu, m != 0u) : m == 0u) continue;
-            p.template leaf<COUNT>(leaf_first(r[c]), leaf_count(r[c]), m, cnt);
-        }
-        int next = -1;
-        R next_d = R(0);
-#pragma unroll
-        for (int c = 3; c >= 0; c--) {
-            if (r[c] < 0) continue;
-            const unsigned m = want_mask(p, d[c]);
-            if (WARP ? !__any_sync(0xffffffffu, m != 0u) : m == 0u) continue;
-            if (next >= 0 && sp < kStackSize) {
-                snode[sp] = next;
-                sdist[sp] = next_d;
-                sp++;
-            }
-            next = r[c];
-            next_d = min_of<R, Q>(d[c]);
-        }
-        if (next < 0) {
-            const R tmax = p.max_thr();
-            while (sp > 0) {
-                sp--;
-                const bool w = sdist[sp] < tmax;
-                if (WARP ? __any_sync(0xffffffffu, w) : w) {
-                    next = snode[sp];
-                    break;
-                }
-            }
-            if (next < 0) break;
-        }
-        node = next;
-    }
-}
-
-// Packet walk of the 4-wide BVH, the binary packet walk's rules over four children: a child is
-// wanted when any lane wants it; wanted leaves are tested at once; of the wanted internal children
-// the one nearest the brick's centre lane is entered and the others go on the warp's shared stack
-// with the warp's smallest box distance, entered on pop while that is below the largest lane
-// threshold. At most 3 entries a level: the build keeps 3 x (4-wide depth) below kStackSize.
-template <bool COUNT, class P>
-__device__ __forceinline__ void traverse4_packet(P &p, Counters &cnt, int budget) {
-    using R = typename P::R;
-    constexpr int Q = P::kQn;
-    constexpr unsigned kAll = 0xffffffffu;
-    int work = 0;
-    if (budget <= 0) budget = 0x7fffffff;
-    __shared__ int s_node[kThreads / 32][kStackSize];
-    __shared__ float s_dist[kThreads / 32][kStackSize];
-    int *snode = s_node[threadIdx.x >> 5];
-    float *sdist = s_dist[threadIdx.x >> 5];
-    const bool live = p.max_thr() >= R(0);
-    int sp = 0;
-    int node = 0;
-    while (true) {
-        R d[4][Q];
-        int r[4];
-        p.boxes4(node, d, r);
-        if (COUNT) cnt.box += 4 * Q;
-        int next = -1;
-        float next_rank = 0.f, next_key = 0.f;
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const int rc = r[c];
-            const unsigned m = rc == kEmptyRef ? 0u : want_mask(p, d[c]);
-            if (!__any_sync(kAll, m != 0u)) continue;
-            if (rc < 0) {
-                p.template leaf<COUNT>(leaf_first(rc), leaf_count(rc), m, cnt);
-                if constexpr (budgeted<P>()) work += leaf_count(rc);
-                continue;
-            }
-            const R own = min_of<R, Q>(d[c]);
-            const float key =
-                __uint_as_float(__reduce_min_sync(kAll, __float_as_uint(live ? own : finf())));
-            const float rank = __shfl_sync(kAll, float(own), kRepLane);
-            int push = rc;
-            float push_key = key;
-            if (next < 0 || rank < next_rank) {
-                push = next;
-                push_key = next_key;
-                next = rc;
-                next_rank = rank;
-                next_key = key;
-            }
-            if (push >= 0 && sp < kStackSize) {
-                snode[sp] = push;  // every lane stores the same values
-                sdist[sp] = push_key;
-                sp++;
-            }
-        }
-        if (next < 0) {
-            if constexpr (budgeted<P>()) {
-                if (work > budget) {
-                    p.abandon();
-                    break;
-                }
-            }
-            const float tl = live ? p.max_thr() : 0.f;
-            const float tmax = __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(tl)));
-            while (sp > 0) {
-                sp--;
-                if (sdist[sp] < tmax) {
-                    next = snode[sp];
-                    break;
-                }
-            }
-            if (next < 0) break;
-        }
-        node = next;
-    }
-}
-
-template <bool WARP, bool WIDE, bool COUNT, class P>
-__device__ __forceinline__ void walk(P &p, Counters &cnt, int budget = 0) {
-    if constexpr (WIDE && WARP)
-        traverse4_packet<COUNT>(p, cnt, budget);
-    else if constexpr (WIDE)
-        traverse4<WARP, COUNT>(p, cnt);
-    else
-        traverse<WARP, COUNT>(p, cnt, budget);
-}
-
 // ---- outputs ----------------------------------------------------------------------------------------
 
 // Signed distance from the closest triangle (caller's index t, leaf position pos) and d^2, in
@@ -1019,7 +771,7 @@ __device__ __forceinline__ void signal_chunk(const QueryArgs &a) {
 // Lanes without a query (the edge of a grid brick, the tail of a point list) take part in warp-mode
 // traversal with a negative threshold, so they never ask for a node. seed[s] is the leaf position of
 // the closest triangle the lane's query s found one step below (-1: none); it is updated here.
-template <int PREC, bool WARP, bool WIDE, bool COUNT>
+template <int PREC, bool WARP, bool COUNT>
 __device__ __forceinline__ void query_step(const QueryArgs &a, int step, const bool (&valid)[kQ],
                                            const long long (&qid)[kQ], const long long (&gi)[kQ],
                                            const long long (&gj)[kQ], const long long (&gk)[kQ], bool any,
@@ -1039,7 +791,7 @@ __device__ __forceinline__ void query_step(const QueryArgs &a, int step, const b
                 p.disable(s);
             }
         }
-        if (WARP || any) walk<WARP, WIDE, COUNT>(p, cnt);
+        if (WARP || any) traverse<WARP, COUNT>(p, cnt, 0);
 #pragma unroll
         for (int s = 0; s < Q; s++) {
             if (!valid[s]) continue;
@@ -1062,7 +814,7 @@ __device__ __forceinline__ void query_step(const QueryArgs &a, int step, const b
                 p.disable(s);
             }
         }
-        if (WARP || any) walk<WARP, WIDE, COUNT>(p, cnt);
+        if (WARP || any) traverse<WARP, COUNT>(p, cnt, 0);
 #pragma unroll
         for (int s = 0; s < Q; s++) {
             if (!valid[s]) continue;
@@ -1102,7 +854,7 @@ __device__ __forceinline__ void query_step(const QueryArgs &a, int step, const b
                 p.disable(s);
             }
         }
-        if (WARP || any) walk<WARP, WIDE, COUNT>(p, cnt, a.warp_budget);
+        if (WARP || any) traverse<WARP, COUNT>(p, cnt, a.warp_budget);
 #pragma unroll
         for (int s = 0; s < Q; s++) {
             if (!valid[s]) continue;
@@ -1140,7 +892,7 @@ __device__ __forceinline__ void query_step(const QueryArgs &a, int step, const b
 }
 
 // A point-list block, or a grid block's column step by step (each step seeded from the one below).
-template <int PREC, bool WARP, bool WIDE, bool COUNT>
+template <int PREC, bool WARP, bool COUNT>
 __device__ __forceinline__ void query_block(const QueryArgs &a, long long block, Counters &cnt) {
     constexpr int Q = kQ;
     int seed[Q];
@@ -1161,18 +913,18 @@ __device__ __forceinline__ void query_block(const QueryArgs &a, long long block,
         // decision, not a block one: the warps share nothing, and a block barrier per step made every
         // warp wait for the block's slowest (17 % on the torus knot)
         if (step > 0 && !__any_sync(0xffffffffu, any)) break;
-        query_step<PREC, WARP, WIDE, COUNT>(a, step, valid, qid, gi, gj, gk, any, seed, cnt);
+        query_step<PREC, WARP, COUNT>(a, step, valid, qid, gi, gj, gk, any, seed, cnt);
     }
 }
 
 // SIGNAL: the streamed grid download's instantiation, whose blocks count themselves done per chunk
 // (a separate instantiation: the dormant signal code cost the fix-up kernel 3 % where it was merely
 // compiled in).
-template <int PREC, bool WARP, bool WIDE, bool COUNT, bool SIGNAL = false>
+template <int PREC, bool WARP, bool COUNT, bool SIGNAL = false>
 __global__ void __launch_bounds__(kThreads, PREC == SSDF_PREC_F64 ? kF64MinBlocks : SSDF_B200_QUERY_MIN_BLOCKS)
     k_query(const QueryArgs a) {
     Counters cnt;
-    query_block<PREC, WARP, WIDE, COUNT>(a, blockIdx.x, cnt);
+    query_block<PREC, WARP, COUNT>(a, blockIdx.x, cnt);
     if (COUNT) flush_counters(a, cnt);
     if constexpr (SIGNAL) signal_chunk(a);
 }
@@ -1189,8 +941,8 @@ __global__ void __launch_bounds__(kThreads, PREC == SSDF_PREC_F64 ? kF64MinBlock
 // lexicographic (d^2, index) minimum of the triangles it evaluated (the incoming bound ranks -1, so
 // it wins ties, as in the sequential rule) and a warp reduction takes the minimum of those: the
 // same value as the sequential walk, since each triangle's double distance does not depend on the
-// order. The boxes and the float test are the first stage's, on the binary tree: the double winner
-// lies inside the window by the margin tau, so its boxes pass under either arity.
+// order. The boxes and the float test are the first stage's: the double winner
+// lies inside the window by the margin tau, so its boxes pass.
 constexpr int kWinStack = 1024;  // node slots of a warp's shared stack
 // Blocks per SM of the second stage's grid. Its kernel keeps its registers (116: capping them at 64 or
 // 40 spilled the double evaluation and lost 10-100 %), so 4 blocks are resident per SM; a grid of 12
@@ -1343,7 +1095,7 @@ __global__ void __launch_bounds__(kThreads) k_window(const QueryArgs a, int cap)
 // re-instantiated: only the table is rewritten before each replay. Blocks pull work items (one
 // 128-query block of one job) from an atomic counter, largest jobs first (the host orders them).
 
-template <int PREC, bool WARP, bool WIDE, bool COUNT>
+template <int PREC, bool WARP, bool COUNT>
 __global__ void __launch_bounds__(kThreads, PREC == SSDF_PREC_F64 ? kF64MinBlocks : SSDF_B200_QUERY_MIN_BLOCKS)
     k_query_batch(const BatchHeader *__restrict__ hdr, const QueryArgs *__restrict__ jobs,
                   const long long *__restrict__ first_block, unsigned long long *__restrict__ next_item) {
@@ -1362,7 +1114,7 @@ __global__ void __launch_bounds__(kThreads, PREC == SSDF_PREC_F64 ? kF64MinBlock
             const int mid = (lo + hi + 1) >> 1;
             if (__ldg(first_block + mid) <= it) lo = mid; else hi = mid - 1;
         }
-        query_block<PREC, WARP, WIDE, COUNT>(jobs[lo], it - __ldg(first_block + lo), cnt);
+        query_block<PREC, WARP, COUNT>(jobs[lo], it - __ldg(first_block + lo), cnt);
     }
     if (COUNT && njobs > 0) flush_counters(jobs[0], cnt);
 }
@@ -1395,12 +1147,12 @@ int window_stack_cap() {
     return v < 1 ? 1 : (v > kWinStack ? kWinStack : v);
 }
 
-template <int PREC, bool WARP, bool WIDE>
+template <int PREC, bool WARP>
 cudaError_t launch_batch_main(const BatchLaunch &b, bool count, cudaStream_t stream) {
     if (count)
-        k_query_batch<PREC, WARP, WIDE, true><<<b.grid, kThreads, 0, stream>>>(b.hdr, b.jobs, b.first_block, b.next_item);
+        k_query_batch<PREC, WARP, true><<<b.grid, kThreads, 0, stream>>>(b.hdr, b.jobs, b.first_block, b.next_item);
     else
-        k_query_batch<PREC, WARP, WIDE, false><<<b.grid, kThreads, 0, stream>>>(b.hdr, b.jobs, b.first_block, b.next_item);
+        k_query_batch<PREC, WARP, false><<<b.grid, kThreads, 0, stream>>>(b.hdr, b.jobs, b.first_block, b.next_item);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || PREC != SSDF_PREC_F32_FIXUP) return e;
     if (count)
@@ -1412,42 +1164,34 @@ cudaError_t launch_batch_main(const BatchLaunch &b, bool count, cudaStream_t str
 
 template <int PREC>
 cudaError_t launch_batch_prec(const BatchLaunch &b, bool count, cudaStream_t stream) {
-    if (b.wide)
-        return b.warp ? launch_batch_main<PREC, true, true>(b, count, stream)
-                      : launch_batch_main<PREC, false, true>(b, count, stream);
-    return b.warp ? launch_batch_main<PREC, true, false>(b, count, stream)
-                  : launch_batch_main<PREC, false, false>(b, count, stream);
+    return b.warp ? launch_batch_main<PREC, true>(b, count, stream) : launch_batch_main<PREC, false>(b, count, stream);
 }
 
-template <int PREC, bool WARP, bool WIDE>
+template <int PREC, bool WARP>
 int batch_occupancy() {
     int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_query_batch<PREC, WARP, WIDE, false>, kThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_query_batch<PREC, WARP, false>, kThreads, 0);
     return nb > 0 ? nb : 1;
 }
 
 thread_local unsigned long long t_last_counts[4] = {0, 0, 0, 0};
 
-template <int PREC, bool WARP, bool WIDE>
+template <int PREC, bool WARP>
 cudaError_t launch_main(const QueryArgs &a, bool count, unsigned nblocks, cudaStream_t stream) {
     // a counting launch raises no chunk flags: its streamed download copies every chunk once the launch
     // has ended
     if (count)
-        k_query<PREC, WARP, WIDE, true><<<nblocks, kThreads, 0, stream>>>(a);
+        k_query<PREC, WARP, true><<<nblocks, kThreads, 0, stream>>>(a);
     else if (a.chunk_flags)
-        k_query<PREC, WARP, WIDE, false, true><<<nblocks, kThreads, 0, stream>>>(a);
+        k_query<PREC, WARP, false, true><<<nblocks, kThreads, 0, stream>>>(a);
     else
-        k_query<PREC, WARP, WIDE, false><<<nblocks, kThreads, 0, stream>>>(a);
+        k_query<PREC, WARP, false><<<nblocks, kThreads, 0, stream>>>(a);
     return cudaGetLastError();
 }
 
 template <int PREC>
-cudaError_t launch_prec(const QueryArgs &a, bool warp, bool wide, bool count, unsigned nblocks, cudaStream_t stream) {
-    if (wide)
-        return warp ? launch_main<PREC, true, true>(a, count, nblocks, stream)
-                    : launch_main<PREC, false, true>(a, count, nblocks, stream);
-    return warp ? launch_main<PREC, true, false>(a, count, nblocks, stream)
-                : launch_main<PREC, false, false>(a, count, nblocks, stream);
+cudaError_t launch_prec(const QueryArgs &a, bool warp, bool count, unsigned nblocks, cudaStream_t stream) {
+    return warp ? launch_main<PREC, true>(a, count, nblocks, stream) : launch_main<PREC, false>(a, count, nblocks, stream);
 }
 
 }  // namespace
@@ -1467,12 +1211,6 @@ int query_counts(int64_t *tri, int64_t *box, int64_t *fix, int64_t *fallback) {
 
 // Traversal mode: SSDF_B200_TRAVERSAL=warp|thread overrides; by default grids (coherent bricks) walk
 // in warp packets and point lists thread by thread.
-// BVH arity: SSDF_B200_ARITY=2|4; binary by default (measured as fast as 4-wide on the torus knot).
-static bool use_wide(const QueryArgs &a) {
-    if (a.force_arity) return a.force_arity == 4;
-    return env_int("SSDF_B200_ARITY", 2) == 4;
-}
-
 static bool use_warp(const QueryArgs &a) {
     if (a.force_traversal) return a.force_traversal == 1;
     const char *v = env_str("SSDF_B200_TRAVERSAL");
@@ -1634,7 +1372,6 @@ int launch_query_keep(const QueryArgs &args_in, int precision, cudaStream_t stre
         a.order = sorted.p;
     }
     const bool warp = use_warp(a);
-    const bool wide = use_wide(a);
     const long long nblocks = query_blocks(a);
     if (nblocks > 0x7fffffffll) return fail(SSDF_ERR_NOT_SUPPORTED, "too many queries in one launch");
     unsigned long long *counters = nullptr;
@@ -1656,7 +1393,7 @@ int launch_query_keep(const QueryArgs &args_in, int precision, cudaStream_t stre
             a.fallback_ids = fb + 1;
             a.fallback_thr = reinterpret_cast<float *>(fb + 1 + n);
             e = cudaMemsetAsync(fb, 0, sizeof(int), stream);
-            if (e == cudaSuccess) e = launch_prec<SSDF_PREC_F32_FIXUP>(a, warp, wide, count, unsigned(nblocks), stream);
+            if (e == cudaSuccess) e = launch_prec<SSDF_PREC_F32_FIXUP>(a, warp, count, unsigned(nblocks), stream);
             if (e == cudaSuccess) {
                 const unsigned wg = window_grid();
                 const int cap = window_stack_cap();
@@ -1666,9 +1403,9 @@ int launch_query_keep(const QueryArgs &args_in, int precision, cudaStream_t stre
             }
         }
     } else if (precision == SSDF_PREC_F64) {
-        e = launch_prec<SSDF_PREC_F64>(a, warp, wide, count, unsigned(nblocks), stream);
+        e = launch_prec<SSDF_PREC_F64>(a, warp, count, unsigned(nblocks), stream);
     } else {
-        e = launch_prec<SSDF_PREC_F32>(a, warp, wide, count, unsigned(nblocks), stream);
+        e = launch_prec<SSDF_PREC_F32>(a, warp, count, unsigned(nblocks), stream);
     }
     if (e != cudaSuccess && st == SSDF_OK) st = cuda_fail(e, "query launch", __FILE__, __LINE__);
     if (count && st == SSDF_OK) {
@@ -1690,17 +1427,12 @@ int launch_query_keep(const QueryArgs &args_in, int precision, cudaStream_t stre
 }
 
 // Resident blocks per SM of the batch kernel for this arithmetic / traversal.
-int batch_blocks_per_sm(int precision, bool warp, bool wide) {
+int batch_blocks_per_sm(int precision, bool warp) {
     if (precision == SSDF_PREC_F64)
-        return warp ? (wide ? batch_occupancy<SSDF_PREC_F64, true, true>() : batch_occupancy<SSDF_PREC_F64, true, false>())
-                    : (wide ? batch_occupancy<SSDF_PREC_F64, false, true>() : batch_occupancy<SSDF_PREC_F64, false, false>());
+        return warp ? batch_occupancy<SSDF_PREC_F64, true>() : batch_occupancy<SSDF_PREC_F64, false>();
     if (precision == SSDF_PREC_F32)
-        return warp ? (wide ? batch_occupancy<SSDF_PREC_F32, true, true>() : batch_occupancy<SSDF_PREC_F32, true, false>())
-                    : (wide ? batch_occupancy<SSDF_PREC_F32, false, true>() : batch_occupancy<SSDF_PREC_F32, false, false>());
-    return warp ? (wide ? batch_occupancy<SSDF_PREC_F32_FIXUP, true, true>()
-                        : batch_occupancy<SSDF_PREC_F32_FIXUP, true, false>())
-                : (wide ? batch_occupancy<SSDF_PREC_F32_FIXUP, false, true>()
-                        : batch_occupancy<SSDF_PREC_F32_FIXUP, false, false>());
+        return warp ? batch_occupancy<SSDF_PREC_F32, true>() : batch_occupancy<SSDF_PREC_F32, false>();
+    return warp ? batch_occupancy<SSDF_PREC_F32_FIXUP, true>() : batch_occupancy<SSDF_PREC_F32_FIXUP, false>();
 }
 
 // Enqueues the persistent batch kernel (and the fix-up window stage) on `stream`; the job table and
@@ -1726,8 +1458,6 @@ bool default_warp(int is_grid) {
     if (v && !strcmp(v, "thread")) return false;
     return is_grid != 0;
 }
-
-bool default_wide() { return env_int("SSDF_B200_ARITY", 2) == 4; }
 
 // ---- allocation-free variant of the fix-up grid query ------------------------------------------------
 //
@@ -1780,10 +1510,10 @@ int launch_query_noalloc(const QueryArgs &args_in, cudaStream_t stream) {
     if (a.output == SSDF_OUT_SDF && !a.m.face_n)
         return fail(SSDF_ERR_INVALID_ARGUMENT, "signed queries need a mesh built with normals=1");
     a.counters = nullptr;
-    const bool warp = use_warp(a), wide = use_wide(a);
+    const bool warp = use_warp(a);
     const long long nblocks = query_blocks(a);
     if (fixup_runs_f64(a.m)) {  // the same bits from the FP64 kernel, which has no overflow list
-        const cudaError_t e = launch_prec<SSDF_PREC_F64>(a, warp, wide, false, unsigned(nblocks), stream);
+        const cudaError_t e = launch_prec<SSDF_PREC_F64>(a, warp, false, unsigned(nblocks), stream);
         if (e != cudaSuccess) return cuda_fail(e, "allocation-free query launch", __FILE__, __LINE__);
         return SSDF_OK;
     }
@@ -1794,7 +1524,7 @@ int launch_query_noalloc(const QueryArgs &args_in, cudaStream_t stream) {
     a.fallback_ids = scratch + 1;
     a.fallback_thr = reinterpret_cast<float *>(scratch + 1 + n);
     cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(int), stream);  // the count starts at zero
-    if (e == cudaSuccess) e = launch_prec<SSDF_PREC_F32_FIXUP>(a, warp, wide, false, unsigned(nblocks), stream);
+    if (e == cudaSuccess) e = launch_prec<SSDF_PREC_F32_FIXUP>(a, warp, false, unsigned(nblocks), stream);
     if (e == cudaSuccess) {
         k_window<false><<<window_grid(), kThreads, 0, stream>>>(a, kWinStack);
         e = cudaGetLastError();

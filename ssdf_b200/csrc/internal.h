@@ -41,10 +41,6 @@ int cuda_fail(cudaError_t err, const char *what, const char *file, int line);
 //                           DeviceMesh::obb); per axis k = u, v, n of both children: (kx of c0, kx of
 //                           c1, ky, ky), (kz, kz, -k.centre, -k.centre), then the half extents (hu, hu,
 //                           hv, hv), (hn, hn, ref0, ref1): pairs (c0, c1) throughout, for two-wide FP32
-//   4-wide FP32 node (8 x float4): lo x / hi x / lo y / hi y / lo z / hi z of children 0..3, then
-//                           the 4 references as int bits, padding
-//   4-wide FP64 node (14 x double2): the same six rows as pairs of double2, the 4 references as
-//                            int bits in one double2, padding
 // A reference >= 0 is an internal node; < 0 is a leaf ~((first << 5) | (count - 1)) over the
 // triangle records in leaf order; kEmptyRef is an empty slot (its box is inverted).
 // Triangles in leaf order:
@@ -76,11 +72,6 @@ struct DeviceMesh {
     const float4 *obb = nullptr;
     float box_c[3] = {0.f, 0.f, 0.f};
     float box_scale = 1.f;
-    // 4-wide BVH over the same leaves (collapsed from the binary one)
-    int nnodes4 = 0;
-    int depth4 = 0;
-    const float4 *nodes4_32 = nullptr;   // [8 * nnodes4]
-    const double2 *nodes4_64 = nullptr;  // [14 * nnodes4] or null
     const float4 *tris32 = nullptr;    // [3 * nt], leaf order
     const double2 *tris64 = nullptr;   // [5 * nt], leaf order, or null
     // the fix-up path's FP32 filter records, [3 * nt], leaf order, with the double data or null:
@@ -143,9 +134,8 @@ struct QueryArgs {
     int *fallback_count;
     // optional counters [4]: triangle tests, box tests, fix-up evaluations, fallbacks
     unsigned long long *counters;
-    // 0: environment / default; traversal 1 warp packets, 2 thread per query; arity 2 or 4
+    // 0: environment / default; 1 warp packets, 2 thread per query
     int force_traversal;
-    int force_arity;
     // point lists: the visiting order (query index per slot, Morton-sorted), or null (input order)
     const int *order;
     // streamed download of a grid (launch_query_streamed): the blocks of chunk c (blockIdx.x /
@@ -178,7 +168,7 @@ struct BatchLaunch {
     unsigned long long *next_item;
     int grid;   // persistent blocks (SMs x resident blocks per SM)
     int sms;
-    bool warp, wide;
+    bool warp;
 };
 
 // ---- mesh build (mesh_build.cu) ------------------------------------------------------------------
@@ -222,9 +212,8 @@ int launch_batch(const BatchLaunch &b, int precision, cudaStream_t stream);
 // Whether a fix-up request on this mesh runs the FP64 kernel instead (bvh_query.cu).
 bool fixup_runs_f64(const DeviceMesh &m);
 int batch_capture_graphs(ssdf_batch *b);  // batch.cu
-int batch_blocks_per_sm(int precision, bool warp, bool wide);
+int batch_blocks_per_sm(int precision, bool warp);
 bool default_warp(int is_grid);
-bool default_wide();
 // Queries each lane of the query kernels answers (two independent arithmetic chains per node visit).
 #ifndef SSDF_B200_QUERIES_PER_LANE
 #define SSDF_B200_QUERIES_PER_LANE 1

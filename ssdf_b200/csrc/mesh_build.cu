@@ -281,97 +281,6 @@ __global__ void k_write_small_root(int n, const float *__restrict__ box32, float
     nodes32[3] = make_float4(__int_as_float(leaf_ref(0, n)), __int_as_float(kEmptyRef), 0.f, 0.f);
 }
 
-// 4-wide nodes, top-down: a node starts from its binary node's two children and repeatedly opens
-// the expandable child (internal, > L triangles) of largest surface area until it has four.
-// Internal children become the next level's nodes (slots taken from an atomic counter).
-__device__ __forceinline__ float box_area(const float *b) {
-    const float dx = b[1] - b[0], dy = b[3] - b[2], dz = b[5] - b[4];
-    return dx * dy + dy * dz + dz * dx;
-}
-
-__global__ void k_collapse4(const int *__restrict__ n_in_ptr, const int2 *__restrict__ qin, int2 *__restrict__ qout,
-                            int *__restrict__ n_out,
-                            int *__restrict__ slots, int L, const int *__restrict__ child_l,
-                            const int *__restrict__ child_r, const int *__restrict__ first_of,
-                            const int *__restrict__ count, const int *__restrict__ sorted_ids,
-                            const float *__restrict__ pbox32, const double *__restrict__ pbox64,
-                            const float *__restrict__ nbox32, const double *__restrict__ nbox64,
-                            float4 *__restrict__ n32, double2 *__restrict__ n64) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= *n_in_ptr) return;  // the level's size, written by the level above
-    const int b = qin[i].x, slot = qin[i].y;
-    int c[4] = {child_l[b], child_r[b], 0, 0};
-    int nc = 2;
-    while (nc < 4) {
-        int pick = -1;
-        float area = -1.f;
-        for (int k = 0; k < nc; k++) {
-            if (c[k] >= 0 && count[c[k]] > L) {
-                const float a = box_area(nbox32 + 6 * c[k]);
-                if (a > area) area = a, pick = k;
-            }
-        }
-        if (pick < 0) break;
-        const int x = c[pick];
-        c[pick] = child_l[x];
-        c[nc++] = child_r[x];
-    }
-    const float inf = __int_as_float(0x7f800000);
-    const double dinf = __longlong_as_double(0x7ff0000000000000ll);
-    float b32[6][4];
-    double b64[6][4];
-    int ref[4];
-    for (int k = 0; k < 4; k++) {
-        const float *f = nullptr;
-        const double *d = nullptr;
-        if (k >= nc) {
-            ref[k] = kEmptyRef;
-        } else if (c[k] < 0) {
-            const int pos = -c[k] - 1;
-            ref[k] = leaf_ref(pos, 1);
-            f = pbox32 + 6 * sorted_ids[pos];
-            d = pbox64 + 6 * sorted_ids[pos];
-        } else {
-            f = nbox32 + 6 * c[k];
-            d = nbox64 + 6 * c[k];
-            if (count[c[k]] <= L) {
-                ref[k] = leaf_ref(first_of[c[k]], count[c[k]]);
-            } else {
-                ref[k] = atomicAdd(slots, 1);
-                qout[atomicAdd(n_out, 1)] = make_int2(c[k], ref[k]);
-            }
-        }
-        for (int r = 0; r < 6; r++) {
-            b32[r][k] = f ? f[r] : ((r & 1) ? -inf : inf);
-            b64[r][k] = d ? d[r] : ((r & 1) ? -dinf : dinf);
-        }
-    }
-    // rows: lo x, hi x, lo y, hi y, lo z, hi z (box arrays are lo/hi interleaved per axis)
-    for (int r = 0; r < 6; r++) {
-        n32[8 * slot + r] = make_float4(b32[r][0], b32[r][1], b32[r][2], b32[r][3]);
-        if (n64) {
-            n64[14 * slot + 2 * r] = make_double2(b64[r][0], b64[r][1]);
-            n64[14 * slot + 2 * r + 1] = make_double2(b64[r][2], b64[r][3]);
-        }
-    }
-    n32[8 * slot + 6] =
-        make_float4(__int_as_float(ref[0]), __int_as_float(ref[1]), __int_as_float(ref[2]), __int_as_float(ref[3]));
-    n32[8 * slot + 7] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (n64) {
-        n64[14 * slot + 12] =
-            make_double2(__longlong_as_double((long long)(unsigned(ref[0])) | ((long long)(unsigned(ref[1])) << 32)),
-                         __longlong_as_double((long long)(unsigned(ref[2])) | ((long long)(unsigned(ref[3])) << 32)));
-        n64[14 * slot + 13] = make_double2(0.0, 0.0);
-    }
-}
-
-// Start of the 4-wide collapse: level 0 is the root (binary node 0 into slot 0), one slot used.
-__global__ void k_collapse4_init(int2 *__restrict__ q0, int *__restrict__ level_sizes, int *__restrict__ slots) {
-    q0[0] = make_int2(0, 0);
-    level_sizes[0] = 1;
-    *slots = 1;
-}
-
 // The flag words of the build: [0] the first bad triangle (none: INT_MAX), [1..6] the scene's box as
 // ordered ints (min seeded with +FLT_MAX, max with -FLT_MAX), the rest zero.
 __global__ void k_init_flags(int *__restrict__ flags) {
@@ -382,35 +291,6 @@ __global__ void k_init_flags(int *__restrict__ flags) {
     if (k >= 1 && k <= 3) v = 0x7f7fffff;
     if (k >= 4 && k <= 6) v = int(0xff7fffffu ^ 0x7fffffffu);
     flags[k] = v;
-}
-
-// The 4-wide root of a mesh of <= L triangles: one leaf, three empty slots.
-__global__ void k_write_small_root4(int n, const float *__restrict__ box32, const double *__restrict__ box64,
-                                    float4 *__restrict__ n32, double2 *__restrict__ n64) {
-    float b[6] = {FLT_MAX, -FLT_MAX, FLT_MAX, -FLT_MAX, FLT_MAX, -FLT_MAX};
-    double e[6] = {DBL_MAX, -DBL_MAX, DBL_MAX, -DBL_MAX, DBL_MAX, -DBL_MAX};
-    for (int t = 0; t < n; t++)
-        for (int k = 0; k < 6; k += 2) {
-            b[k] = fminf(b[k], box32[6 * t + k]), b[k + 1] = fmaxf(b[k + 1], box32[6 * t + k + 1]);
-            e[k] = fmin(e[k], box64[6 * t + k]), e[k + 1] = fmax(e[k + 1], box64[6 * t + k + 1]);
-        }
-    const float inf = __int_as_float(0x7f800000);
-    const double dinf = __longlong_as_double(0x7ff0000000000000ll);
-    for (int r = 0; r < 6; r++) {
-        const float pad = (r & 1) ? -inf : inf;
-        const double dpad = (r & 1) ? -dinf : dinf;
-        n32[r] = make_float4(b[r], pad, pad, pad);
-        if (n64) n64[2 * r] = make_double2(e[r], dpad), n64[2 * r + 1] = make_double2(dpad, dpad);
-    }
-    const int e0 = kEmptyRef;
-    n32[6] = make_float4(__int_as_float(leaf_ref(0, n)), __int_as_float(e0), __int_as_float(e0), __int_as_float(e0));
-    n32[7] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (n64) {
-        n64[12] = make_double2(
-            __longlong_as_double((long long)(unsigned(leaf_ref(0, n))) | ((long long)(unsigned(e0)) << 32)),
-            __longlong_as_double((long long)(unsigned(e0)) | ((long long)(unsigned(e0)) << 32)));
-        n64[13] = make_double2(0.0, 0.0);
-    }
 }
 
 // Depth and leaf count of the collapsed tree: a node is kept iff its subtree has > L triangles
@@ -982,10 +862,6 @@ void mesh_free_async(MeshStorage *storage, cudaStream_t stream) {
 
 size_t mesh_bytes(const MeshStorage *storage) { return storage ? storage->bytes : 0; }
 
-// Deepest 4-wide level the collapse writes: a tree that reaches it is refused (3 x depth4 must stay
-// below kStackSize), so one more level than an accepted tree can have.
-constexpr int kMaxLevels4 = kStackSize / 3 + 1;
-
 // Page-locked words for the build's read-backs (one set per calling thread, kept until exit), so the
 // copies stay asynchronous and the build waits once, at its end.
 constexpr int kReadbackWords = 64;
@@ -1081,29 +957,20 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
     float4 *obb = nullptr;
     SSDF_CHECK(dalloc(s, &nodes32, 4 * size_t(m->nnodes), stream));
     if (query_boxes) SSDF_CHECK(dalloc(s, &obb, 8 * size_t(m->nnodes), stream));
-    float4 *nodes4_32;
-    double2 *nodes4_64 = nullptr;
-    SSDF_CHECK(dalloc(s, &nodes4_32, 8 * size_t(m->nnodes), stream));
-    if (keep64) SSDF_CHECK(dalloc(s, &nodes4_64, 14 * size_t(m->nnodes), stream));
-    // read-backs: [0..1] depth and leaves, [2..2 + kMaxLevels4] 4-wide level sizes, then the slots
-    // used, then the coordinate scale, the three filter words and the four of the box frame
-    static_assert(2 + kMaxLevels4 + 2 + 8 <= kReadbackWords, "read-back words");
+    // read-backs: depth and leaves, the coordinate scale, the three filter words and the box frame's four
+    static_assert(10 <= kReadbackWords, "read-back words");
     int *rb = nullptr;
     SSDF_CHECK(readback_words(&rb));
-    int *const depth_leaves = rb, *const level_hist = rb + 2;
-    int *const scale_word = rb + 2 + kMaxLevels4 + 2, *const filt_info = scale_word + 1;
+    int *const depth_leaves = rb;
+    int *const scale_word = rb + 2, *const filt_info = scale_word + 1;
     int *const frame_words = filt_info + 3;
     depth_leaves[0] = depth_leaves[1] = 1;
-    int nnodes4 = 1, depth4 = 1;
-    bool collapsed = false;
     const int *obb_first = nullptr, *obb_count = nullptr;  // subtree ranges (null: the small root)
     const double *obb_nbox = nullptr;
     if (nt <= L) {
         // one leaf over everything (its triangle order is the Morton order)
         k_write_small_root<<<1, 1, 0, stream>>>(nt, box32, nodes32);
         LAUNCH_CHECK("k_write_small_root");
-        k_write_small_root4<<<1, 1, 0, stream>>>(nt, box32, box64, nodes4_32, nodes4_64);
-        LAUNCH_CHECK("k_write_small_root4");
     } else {
         int *child_l, *child_r, *first_of, *last_of, *parent_int, *parent_leaf, *arrivals, *count;
         float *nbox32;
@@ -1139,34 +1006,6 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
         k_depth<<<grid_blocks(nint, 256), 256, 0, stream>>>(nt, L, count, parent_int, child_l, child_r, flags + 8);
         LAUNCH_CHECK("k_depth");
         SSDF_CUDA(cudaMemcpyAsync(depth_leaves, flags + 8, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream));
-        // 4-wide collapse, one level per launch. Each level's kernel reads its size from the level
-        // above, so the host launches kMaxLevels4 levels without waiting between them (a grid of at
-        // most min(4^k, nint) threads at level k); the sizes come back with the build's last sync.
-        // A tree with a level at kMaxLevels4 is too deep for the traversal stack (3 x depth4 <
-        // kStackSize) and is refused below.
-        int2 *qa, *qb;
-        int *level_sizes;  // [kMaxLevels4 + 1] queue sizes per level, then the slots used
-        SSDF_CHECK(dalloc(tmp, &qa, nint, stream));
-        SSDF_CHECK(dalloc(tmp, &qb, nint, stream));
-        SSDF_CHECK(dalloc(tmp, &level_sizes, kMaxLevels4 + 2, stream));
-        SSDF_CUDA(cudaMemsetAsync(level_sizes, 0, sizeof(int) * (kMaxLevels4 + 2), stream));
-        k_collapse4_init<<<1, 1, 0, stream>>>(qa, level_sizes, level_sizes + kMaxLevels4 + 1);
-        LAUNCH_CHECK("k_collapse4_init");
-        long long bound = 1;
-        for (int k = 0; k < kMaxLevels4; k++) {
-            const int n_k = int(std::min<long long>(bound, nint));
-            k_collapse4<<<grid_blocks(n_k, 128), 128, 0, stream>>>(
-                level_sizes + k, qa, qb, level_sizes + k + 1, level_sizes + kMaxLevels4 + 1, L, child_l, child_r,
-                first_of, count, ids, box32, box64, nbox32, nbox64, nodes4_32, nodes4_64);
-            LAUNCH_CHECK("k_collapse4");
-            bound *= 4;
-            int2 *t = qa;
-            qa = qb;
-            qb = t;
-        }
-        SSDF_CUDA(cudaMemcpyAsync(level_hist, level_sizes, sizeof(int) * (kMaxLevels4 + 2), cudaMemcpyDeviceToHost,
-                                  stream));  // page-locked: no wait here
-        collapsed = true;
         obb_first = first_of, obb_count = count, obb_nbox = nbox64;
     }
     // triangle records in leaf order
@@ -1202,23 +1041,14 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
         memcpy(&term, &filt_info[1], sizeof(float));
         set_filter_window(m, term, filt_info[2] == 0);
     }
-    if (collapsed) {
-        depth4 = 0;
-        while (depth4 <= kMaxLevels4 && level_hist[depth4] > 0) depth4++;
-        nnodes4 = level_hist[kMaxLevels4 + 1];
-    }
     m->depth = depth_leaves[0];
     m->nleaves = depth_leaves[1];
     m->nodes32 = nodes32;
     m->obb = obb;
-    m->nodes4_32 = nodes4_32;
-    m->nodes4_64 = nodes4_64;
-    m->nnodes4 = nnodes4;
-    m->depth4 = depth4;
     m->tris32 = t32;
     m->tris64 = t64;
     m->filt32 = filt;
-    if (m->depth >= kStackSize || 3 * m->depth4 >= kStackSize)
+    if (m->depth >= kStackSize)
         return fail(SSDF_ERR_NOT_SUPPORTED,
                     "BVH depth " + std::to_string(m->depth) + " exceeds the traversal stack (" +
                         std::to_string(kStackSize) + ")");
