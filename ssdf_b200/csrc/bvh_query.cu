@@ -943,148 +943,284 @@ __global__ void __launch_bounds__(kThreads, PREC == SSDF_PREC_F64 ? kF64MinBlock
 // same value as the sequential walk, since each triangle's double distance does not depend on the
 // order. The boxes and the float test are the first stage's: the double winner
 // lies inside the window by the margin tau, so its boxes pass.
-constexpr int kWinStack = 1024;  // node slots of a warp's shared stack
-// Blocks per SM of the second stage's grid. Its kernel keeps its registers (116: capping them at 64 or
-// 40 spilled the double evaluation and lost 10-100 %), so 4 blocks are resident per SM; a grid of 12
-// per SM queues the rest behind them, so a warp takes one query where 4 per SM had each take two or
-// three, and blocks that finish early make room. Measured: 64^3 icosphere step 0.487 -> 0.447 ms,
-// 20,480-triangle sphere 96^3 1.58 -> 1.44 ms, the serving leg's heaviest grid 8.22 -> 8.03 ms, the
-// torus knot unchanged.
+constexpr int kWinStack = 512;  // node slots of a warp's shared stack
+// Blocks per SM of the second stage's grid. Its kernel keeps its registers (capping them for 5, 6 or 8
+// resident blocks: 64^3 icosphere grid 233 -> 234 / 238 / 255 us); a grid of 12 per SM queues the rest
+// behind the resident blocks, so a warp takes one query where a smaller grid had each take two or three,
+// and blocks that finish early make room.
 #ifndef SSDF_B200_WINDOW_BLOCKS_PER_SM
 #define SSDF_B200_WINDOW_BLOCKS_PER_SM 12
 #endif
 constexpr int kWindowBlocksPerSm = SSDF_B200_WINDOW_BLOCKS_PER_SM;
 
-struct WindowBest {
-    double d2;
-    int id, pos;
-};
-
 // A window of +inf takes every node and triangle, whatever its float key (a query point beyond the
 // float filter's range, whose keys may have overflowed, is answered this way: exactly, in double).
 __device__ __forceinline__ bool in_window(float key, float thr) { return key < thr || thr == finf(); }
 
-// kbest: the smallest key of a non-proxy triangle the lane has met (the window may shrink to it, as in
-// the first stage: any such key bounds the window from below, so the double winner stays inside).
-__device__ __forceinline__ void window_leaf(const DeviceMesh &m, int ref, float px, float py, float pz, float thr,
-                                            double qx, double qy, double qz, WindowBest &b, Counters &cnt,
-                                            bool count, float &kbest) {
-    const int first = leaf_first(ref), n = leaf_count(ref);
-    for (int k = 0; k < n; k++) {
-        const FiltRec r = load_filt(m.filt32, first + k);
-        const float f = tri_dist_sq_filter(px, py, pz, r);  // the first stage's key
-        if (r.pen == 0.f && f < kbest) kbest = f;
-        if (count) cnt.tri++;
-        if (in_window(f, thr)) {
-            const Tri64 u = load_tri64(m.tris64, first + k);
-            const double e2 =
-                tri_dist_sq_exact<double>(qx, qy, qz, u.ax, u.ay, u.az, u.bx, u.by, u.bz, u.cx, u.cy, u.cz);
-            if (count) cnt.fix++;
-            if (e2 < b.d2 || (e2 == b.d2 && u.id < b.id)) b = WindowBest{e2, u.id, first + k};
+// What a lane of a warp-per-query walk knows: the query in the arithmetic's own terms, the lexicographic
+// minimum of the triangles the lane evaluated, and the box threshold its finds allow. PREC as the query
+// kernels'.
+template <int PREC>
+struct LaneWalk {
+    using T = typename std::conditional<PREC == SSDF_PREC_F32, float, double>::type;
+    const DeviceMesh &m;
+    T qx, qy, qz;
+    float2 bx, by, bz;  // the point in the box frame, each coordinate twice
+    T d2;               // the minimum, its triangle and leaf position (-1: the incoming bound)
+    int id = -1, pos = -1;
+    float kbest = finf();  // fix-up: the smallest key of a non-proxy triangle met
+    float tau_rel;
+    T margin;
+    __device__ LaneWalk(const QueryArgs &a, double x, double y, double z, T init)
+        : m(a.m), qx(T(x)), qy(T(y)), qz(T(z)), d2(init), tau_rel(a.tau_rel), margin(ExactData<T>::margin(a.m)) {
+        if constexpr (PREC == SSDF_PREC_F32_FIXUP) {
+            bx = twice(filter_coord(x, 0, m)), by = twice(filter_coord(y, 1, m)), bz = twice(filter_coord(z, 2, m));
+        } else {
+            bx = twice(ExactData<T>::box_coord(qx, 0, m));
+            by = twice(ExactData<T>::box_coord(qy, 1, m));
+            bz = twice(ExactData<T>::box_coord(qz, 2, m));
         }
     }
-}
+    __device__ __forceinline__ bool finite() const { return isfinite(qx) && isfinite(qy) && isfinite(qz); }
+    // the threshold the incoming bound allows
+    __device__ __forceinline__ float start_thr() const {
+        if constexpr (PREC == SSDF_PREC_F32_FIXUP)
+            return window_thr(d2 < T(dinf()) ? __double2float_ru(d2) : finf(), tau_rel, m.coord_scale);
+        else
+            return ExactData<T>::box_thr(d2, margin, m);
+    }
+    // the threshold the whole warp's finds allow (warp-wide)
+    __device__ __forceinline__ float found_thr() const {
+        if constexpr (PREC == SSDF_PREC_F32_FIXUP)
+            return window_thr(warp_min(kbest), tau_rel, m.coord_scale);
+        else
+            return warp_min(ExactData<T>::box_thr(d2, margin, m));
+    }
+    // the threshold a squared distance (in the box frame) that some triangle does not exceed allows, and
+    // whether the minimum found bears it out
+    __device__ __forceinline__ float cut_thr(float cut) const {
+        if constexpr (PREC == SSDF_PREC_F32_FIXUP) return window_thr(cut, tau_rel, m.coord_scale);
+        return cut;
+    }
+    __device__ __forceinline__ bool confirms(float cut) const {
+        if constexpr (PREC == SSDF_PREC_F32_FIXUP) return d2 <= double(cut);
+        return ExactData<T>::box_thr(d2, margin, m) <= cut;
+    }
+    __device__ __forceinline__ bool wants(float key, float thr) const {
+        if constexpr (PREC == SSDF_PREC_F32_FIXUP) return in_window(key, thr);
+        return ExactData<T>::box_key(key) < thr;
+    }
+    __device__ __forceinline__ void take(T e2, int t, int p) {
+        if (e2 < d2 || (e2 == d2 && t < id)) d2 = e2, id = t, pos = p;
+    }
+    // tests the triangle at leaf position k
+    __device__ __forceinline__ void triangle(int k, float thr, bool count, Counters &cnt) {
+        if (count) cnt.tri++;
+        if constexpr (PREC == SSDF_PREC_F32_FIXUP) {
+            const FiltRec r = load_filt(m.filt32, k);
+            const float f = tri_dist_sq_filter(bx.x, by.x, bz.x, r);  // the packets' key
+            if (r.pen == 0.f && f < kbest) kbest = f;
+            if (!in_window(f, thr)) return;
+            if (count) cnt.fix++;
+        }
+        const auto u = ExactData<T>::tri(m, k);
+        take(tri_dist_sq_exact<T>(qx, qy, qz, u.ax, u.ay, u.az, u.bx, u.by, u.bz, u.cx, u.cy, u.cz), u.id, k);
+    }
+};
 
 // A lane's own depth-first walk of the subtree under `root` (when the warp's stack is full). Depth
 // below kStackSize is checked when the mesh is built, and a depth-first walk that pushes both
 // children holds at most depth + 1 entries.
-__device__ __noinline__ void window_subtree(const DeviceMesh &m, int root, float px, float py, float pz, float thr,
-                                            double qx, double qy, double qz, WindowBest &b, Counters &cnt,
-                                            bool count, float &kbest) {
+template <int PREC>
+__device__ __noinline__ void lane_subtree(LaneWalk<PREC> &w, int root, float thr, bool count, Counters &cnt) {
     int st[kStackSize];
     int sp = 0;
     st[sp++] = root;
     while (sp > 0) {
-        int r0, r1;
-        const float2 d = obb_dist_sq_pair(twice(px), twice(py), twice(pz), m.obb + 8 * st[--sp], r0, r1);
+        int r[2];
+        const float2 d = obb_dist_sq_pair(w.bx, w.by, w.bz, w.m.obb + 8 * st[--sp], r[0], r[1]);
         if (count) cnt.box += 2;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            const int c = h ? r1 : r0;
-            if (c == kEmptyRef || !in_window(h ? d.y : d.x, thr)) continue;
-            if (c < 0)
-                window_leaf(m, c, px, py, pz, thr, qx, qy, qz, b, cnt, count, kbest);
+            if (r[h] == kEmptyRef || !w.wants(h ? d.y : d.x, thr)) continue;
+            if (r[h] < 0)
+                for (int k = 0; k < leaf_count(r[h]); k++) w.triangle(leaf_first(r[h]) + k, thr, count, cnt);
             else if (sp < kStackSize)
-                st[sp++] = c;
+                st[sp++] = r[h];
         }
     }
 }
 
-// The whole warp answers overflowed query `idx` of job `a`; lane 0 writes the result.
-template <bool COUNT>
-__device__ void window_warp(const QueryArgs &a, int idx, int *__restrict__ stack, int cap, Counters &cnt) {
+// A warp's shared memory: its node stack, the nodes of a step, and the leaves they found.
+struct WarpShared {
+    int stack[kWinStack];
+    float4 node[32][9];  // 8 per node, rows of 144 bytes: a lane reads its own without bank conflicts
+    int leaf[64];
+};
+
+// The whole warp walks the tree for one query from threshold thr; w then holds the minimum in every lane.
+// Each step takes up to 32 nodes from the warp's stack, a lane each. The loads are the bound (a lane
+// reading its own 128-byte node touches a line per lane and load): eight lanes fetch a node together
+// and each lane reads its node back from shared memory, and the leaves' triangles go four lanes to a leaf,
+// neighbours reading neighbouring records. 130,000 points near the 131,072-triangle knot, a warp each:
+// 1,862 -> 1,604 us, from the root; with the copy below 1,460.
+// shrink: the threshold follows the finds (false: it stays +inf, everything is evaluated). upper: no close
+// bound is known yet, so the boxes' own upper bounds (the farthest a triangle inside can be) cut the walk
+// before the first triangle is met. Such a cut assumes that a triangle's computed distance is not above
+// its box's bound (with 5 % to spare), which a needle's rounding can break: the walk returns false when
+// the minimum found does not confirm the smallest cut it used, and is then repeated without them.
+template <int PREC, bool COUNT>
+__device__ bool warp_walk(LaneWalk<PREC> &w, float thr, bool shrink, bool upper, WarpShared &sh, int cap,
+                          Counters &cnt) {
     const unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const long long q = a.fallback_ids[idx];
-    long long i = 0, j = 0, k = 0;
-    if (a.is_grid) grid_ijk(a, q, i, j, k);
-    double qx, qy, qz;
-    query_point(a, q, i, j, k, qx, qy, qz);
-    const float px = filter_coord(qx, 0, a.m), py = filter_coord(qy, 1, a.m), pz = filter_coord(qz, 2, a.m);
-    float thr = a.fallback_thr[idx];
-    const bool shrink = thr < finf();  // an infinite window (a point beyond the float range) stays
-    float kbest = finf();
-    const DeviceMesh &m = a.m;
-    WindowBest b{initial_bound(a, q), -1, -1};
-    if (lane == 0) stack[0] = 0;
+    const unsigned below = (1u << lane) - 1u;
+    using T = typename LaneWalk<PREC>::T;
+    float cut = finf();  // the smallest box upper bound used
+    int *const stack = sh.stack;
+    // the walk starts from the tree's first nodes with internal children only, at most 32 (k_box_frame)
     int sp = 1;  // warp-uniform
+    if (cap >= 32) {
+        sp = __ldg(w.m.entry);
+        if (lane < sp) stack[lane] = __ldg(w.m.entry + 1 + lane);
+    } else if (lane == 0) {
+        stack[0] = 0;
+    }
     __syncwarp();
     while (sp > 0) {
-        const int take = sp < 32 ? sp : 32;
-        const int node = lane < take ? stack[sp - take + lane] : -1;
-        sp -= take;
-        __syncwarp();  // the slots just read are free for the pushes below
+        const int take = sp < 32 ? sp : 32, base = sp - take;
+        sp = base;
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            const int row = 4 * r + (lane >> 3);
+            if (row < take) sh.node[row][lane & 7] = __ldg(w.m.obb + 8 * stack[base + row] + (lane & 7));
+        }
+        __syncwarp();
         int c0 = kEmptyRef, c1 = kEmptyRef;
-        bool w0 = false, w1 = false;
-        if (node >= 0) {
-            const float2 d = obb_dist_sq_pair(twice(px), twice(py), twice(pz), m.obb + 8 * node, c0, c1);
+        float2 d = make_float2(0.f, 0.f), far = make_float2(finf(), finf());
+        if (lane < take) {
+            d = obb_dist_sq_bounds(w.bx, w.by, w.bz, sh.node[lane], c0, c1, far);
             if (COUNT) cnt.box += 2;
-            w0 = c0 != kEmptyRef && in_window(d.x, thr);
-            w1 = c1 != kEmptyRef && in_window(d.y, thr);
-            if (w0 && c0 < 0) {
-                window_leaf(m, c0, px, py, pz, thr, qx, qy, qz, b, cnt, COUNT, kbest);
-                w0 = false;
-            }
-            if (w1 && c1 < 0) {
-                window_leaf(m, c1, px, py, pz, thr, qx, qy, qz, b, cnt, COUNT, kbest);
-                w1 = false;
+        }
+        if (upper) {
+            const float u = warp_min(fminf(c0 == kEmptyRef ? finf() : far.x, c1 == kEmptyRef ? finf() : far.y));
+            cut = fminf(cut, fmaxf(u * 1.05f, FLT_MIN));  // an overflow or a NaN cuts nothing
+            thr = fminf(thr, w.cut_thr(cut));
+        }
+        const bool w0 = c0 != kEmptyRef && w.wants(d.x, thr), w1 = c1 != kEmptyRef && w.wants(d.y, thr);
+        // leaves: listed, then tested eight at a time, four lanes to each
+        const unsigned l0 = __ballot_sync(kAll, w0 && c0 < 0), l1 = __ballot_sync(kAll, w1 && c1 < 0);
+        const int nl0 = __popc(l0), nl = nl0 + __popc(l1);
+        if (nl > 0) {
+            if (w0 && c0 < 0) sh.leaf[__popc(l0 & below)] = c0;
+            if (w1 && c1 < 0) sh.leaf[nl0 + __popc(l1 & below)] = c1;
+            __syncwarp();
+            for (int f = 0; f < nl; f += 8) {
+                const int at = f + (lane >> 2);
+                if (at < nl) {
+                    const int ref = sh.leaf[at], first = leaf_first(ref), n = leaf_count(ref);
+                    for (int k = lane & 3; k < n; k += 4) w.triangle(first + k, thr, COUNT, cnt);
+                }
+                __syncwarp();
+                if (shrink) thr = fminf(thr, w.found_thr());
             }
         }
-        if (shrink) {  // the window the warp's smallest key allows, as the first stage computes it
-            const float wb = __uint_as_float(__reduce_min_sync(kAll, __float_as_uint(kbest)));
-            thr = fminf(thr, window_thr(wb, a.tau_rel, m.coord_scale));
-        }
-        const unsigned m0 = __ballot_sync(kAll, w0), m1 = __ballot_sync(kAll, w1);
+        const bool p0 = w0 && c0 >= 0, p1 = w1 && c1 >= 0;
+        const unsigned m0 = __ballot_sync(kAll, p0), m1 = __ballot_sync(kAll, p1);
         const int n0 = __popc(m0), total = n0 + __popc(m1);
         if (sp + total <= cap) {
-            const unsigned below = (1u << lane) - 1u;
-            if (w0) stack[sp + __popc(m0 & below)] = c0;
-            if (w1) stack[sp + n0 + __popc(m1 & below)] = c1;
+            if (p0) stack[sp + __popc(m0 & below)] = c0;
+            if (p1) stack[sp + n0 + __popc(m1 & below)] = c1;
             sp += total;
         } else {
-            if (w0) window_subtree(m, c0, px, py, pz, thr, qx, qy, qz, b, cnt, COUNT, kbest);
-            if (w1) window_subtree(m, c1, px, py, pz, thr, qx, qy, qz, b, cnt, COUNT, kbest);
+            LaneWalk<PREC> own = w;  // a copy goes by reference, so that w stays in registers
+            if (p0) lane_subtree(own, c0, thr, COUNT, cnt);
+            if (p1) lane_subtree(own, c1, thr, COUNT, cnt);
+            w.d2 = own.d2, w.id = own.id, w.pos = own.pos, w.kbest = own.kbest;
         }
         __syncwarp();
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        const double od = __shfl_xor_sync(kAll, b.d2, o);
-        const int oid = __shfl_xor_sync(kAll, b.id, o), opos = __shfl_xor_sync(kAll, b.pos, o);
-        if (od < b.d2 || (od == b.d2 && oid < b.id)) b = WindowBest{od, oid, opos};
+        const T od = __shfl_xor_sync(kAll, w.d2, o);
+        const int oid = __shfl_xor_sync(kAll, w.id, o), opos = __shfl_xor_sync(kAll, w.pos, o);
+        if (od < w.d2 || (od == w.d2 && oid < w.id)) w.d2 = od, w.id = oid, w.pos = opos;
     }
-    if (lane == 0) write_result(a, q, qx, qy, qz, b.d2, b.id, b.pos);
+    return !(cut < finf()) || w.confirms(cut);  // whatever the cuts left out lies above the minimum
+}
+
+// The whole warp answers overflowed query `idx` of job `a`; lane 0 writes the result.
+template <bool COUNT>
+__device__ void window_warp(const QueryArgs &a, int idx, WarpShared &sh, int cap, Counters &cnt) {
+    const long long q = a.fallback_ids[idx];
+    long long i = 0, j = 0, k = 0;
+    if (a.is_grid) grid_ijk(a, q, i, j, k);
+    double qx, qy, qz;
+    query_point(a, q, i, j, k, qx, qy, qz);
+    const float thr = a.fallback_thr[idx];
+    LaneWalk<SSDF_PREC_F32_FIXUP> w(a, qx, qy, qz, initial_bound(a, q));
+    // an infinite window (a point beyond the float range) stays
+    warp_walk<SSDF_PREC_F32_FIXUP, COUNT>(w, thr, thr < finf(), false, sh, cap, cnt);
+    if ((threadIdx.x & 31) == 0) write_result(a, q, qx, qy, qz, w.d2, w.id, w.pos);
 }
 
 // Overflowed queries of one launch, a warp each. `cap` (<= kWinStack) is the shared stack's usable
 // depth: kWinStack, lowered only to test the per-lane subtree walk.
 template <bool COUNT>
 __global__ void __launch_bounds__(kThreads) k_window(const QueryArgs a, int cap) {
-    __shared__ int s_stack[kThreads / 32][kWinStack];
+    __shared__ WarpShared s_warp[kThreads / 32];
     const int n = *a.fallback_count;
     const int w = (blockIdx.x * kThreads + threadIdx.x) >> 5, nw = (gridDim.x * kThreads) >> 5;
     Counters cnt;
-    for (int idx = w; idx < n; idx += nw) window_warp<COUNT>(a, idx, s_stack[threadIdx.x >> 5], cap, cnt);
+    for (int idx = w; idx < n; idx += nw) window_warp<COUNT>(a, idx, s_warp[threadIdx.x >> 5], cap, cnt);
+    if (COUNT) flush_counters(a, cnt);
+}
+
+// ---- small point lists: one warp per query ------------------------------------------------------------
+//
+// A list too short to fill the GPU with 32-query packets is bound by one walk's serial chain. Here the 32
+// lanes share it: up to 32 nodes a step, so a walk takes about as many steps as the tree is deep, in one
+// launch without ordering the points, an overflow list or a second stage. It is bound by the latency of its
+// dependent loads (4,165 instructions a query, 30 % of issue slots busy). us against packets (fix-up, points
+// near the surface; 131,072-triangle knot, 1,280-triangle sphere): 100 points 57 / 244 and 44 / 106; 1,000
+// 59 / 320 and 46 / 98; 16,000 242 / 577 and 162 / 215; 65,536 836 / 620 and 508 / 214.
+template <int PREC, bool COUNT>
+__global__ void __launch_bounds__(kThreads, 6) k_query_warp(const QueryArgs a, int cap) {
+    __shared__ WarpShared s_warp[kThreads / 32];
+    const long long q = (blockIdx.x * (long long)kThreads + threadIdx.x) >> 5;
+    if (q >= a.npoints) return;  // a whole warp
+    WarpShared &sh = s_warp[threadIdx.x >> 5];
+    using T = typename LaneWalk<PREC>::T;
+    Counters cnt;
+    double x, y, z;
+    query_point(a, q, 0, 0, 0, x, y, z);
+    T init;
+    if constexpr (PREC == SSDF_PREC_F32) {
+        const float o = a.out_f64 ? float(((const double *)a.out)[q]) : ((const float *)a.out)[q];
+        init = a.output == SSDF_OUT_SQEDF ? o : o * o;
+    } else {
+        init = initial_bound(a, q);
+    }
+    LaneWalk<PREC> w(a, x, y, z, init);
+    if (w.finite()) {
+        // a finite point beyond the filter's range: everything, exactly, in double
+        const bool beyond = PREC == SSDF_PREC_F32_FIXUP &&
+                            fmax(fmax(fabs(x), fabs(y)), fabs(z)) > double(kFilterMaxCoord);
+        bool upper = !beyond;
+        while (!warp_walk<PREC, COUNT>(w, beyond ? finf() : w.start_thr(), !beyond, upper, sh, cap, cnt)) upper = false;
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if constexpr (PREC == SSDF_PREC_F32) {
+            if (a.output == SSDF_OUT_SQEDF) {
+                store_out(a, q, double(w.d2));
+            } else {
+                store_out(a, q, double(sqrtf(w.d2)));
+                if (a.outtri && w.id >= 0) a.outtri[q] = w.id;
+            }
+        } else {
+            write_result(a, q, x, y, z, w.d2, w.id, w.pos);
+        }
+    }
     if (COUNT) flush_counters(a, cnt);
 }
 
@@ -1124,7 +1260,7 @@ __global__ void __launch_bounds__(kThreads, PREC == SSDF_PREC_F64 ? kF64MinBlock
 template <bool COUNT>
 __global__ void __launch_bounds__(kThreads) k_window_batch(const BatchHeader *__restrict__ hdr,
                                                            const QueryArgs *__restrict__ jobs, int cap) {
-    __shared__ int s_stack[kThreads / 32][kWinStack];
+    __shared__ WarpShared s_warp[kThreads / 32];
     const int njobs = hdr->njobs;
     const long long w = (blockIdx.x * kThreads + threadIdx.x) >> 5, nw = (gridDim.x * kThreads) >> 5;
     Counters cnt;
@@ -1134,7 +1270,7 @@ __global__ void __launch_bounds__(kThreads) k_window_batch(const BatchHeader *__
         if (!a.fallback_count) continue;
         const int n = *a.fallback_count;
         for (long long idx = ((w - base) % nw + nw) % nw; idx < n; idx += nw)
-            window_warp<COUNT>(a, int(idx), s_stack[threadIdx.x >> 5], cap, cnt);
+            window_warp<COUNT>(a, int(idx), s_warp[threadIdx.x >> 5], cap, cnt);
         base += n;
     }
     if (COUNT && njobs > 0) flush_counters(jobs[0], cnt);
@@ -1175,6 +1311,15 @@ int batch_occupancy() {
 }
 
 thread_local unsigned long long t_last_counts[4] = {0, 0, 0, 0};
+
+template <int PREC>
+cudaError_t launch_query_warp(const QueryArgs &a, bool count, cudaStream_t stream) {
+    const unsigned blocks = unsigned((a.npoints * 32 + kThreads - 1) / kThreads);
+    const int cap = window_stack_cap();
+    count ? k_query_warp<PREC, true><<<blocks, kThreads, 0, stream>>>(a, cap)
+          : k_query_warp<PREC, false><<<blocks, kThreads, 0, stream>>>(a, cap);
+    return cudaGetLastError();
+}
 
 template <int PREC, bool WARP>
 cudaError_t launch_main(const QueryArgs &a, bool count, unsigned nblocks, cudaStream_t stream) {
@@ -1366,7 +1511,9 @@ int launch_query_keep(const QueryArgs &args_in, int precision, cudaStream_t stre
             if (p) cudaFreeAsync(p, s);
         }
     } sorted{nullptr, stream};
-    if (!a.is_grid && !a.force_traversal && n >= kSortMinPoints && n < 0x7fffffffll &&
+    const bool short_list = !a.is_grid && !a.force_traversal && !env_str("SSDF_B200_TRAVERSAL") &&
+                            n <= env_int("SSDF_B200_WARP_POINTS", kWarpPoints);
+    if (!a.is_grid && !short_list && !a.force_traversal && n >= kSortMinPoints && n < 0x7fffffffll &&
         env_int("SSDF_B200_SORT_POINTS", 1) != 0) {
         SSDF_CHECK(morton_point_order(n, a.x, a.y, a.z, a.coord_f64, a.m.nodes32, &sorted.p, stream));
         a.order = sorted.p;
@@ -1383,7 +1530,11 @@ int launch_query_keep(const QueryArgs &args_in, int precision, cudaStream_t stre
     }
     a.counters = counters;
     cudaError_t e = cudaSuccess;
-    if (precision == SSDF_PREC_F32_FIXUP) {
+    if (short_list) {
+        e = precision == SSDF_PREC_F64   ? launch_query_warp<SSDF_PREC_F64>(a, count, stream)
+            : precision == SSDF_PREC_F32 ? launch_query_warp<SSDF_PREC_F32>(a, count, stream)
+                                         : launch_query_warp<SSDF_PREC_F32_FIXUP>(a, count, stream);
+    } else if (precision == SSDF_PREC_F32_FIXUP) {
         if (n >= 0x7fffffffll) {
             st = fail(SSDF_ERR_NOT_SUPPORTED, "more than 2^31 - 1 queries in one fix-up launch");
         } else if (cudaMallocAsync(&fb, sizeof(int) * size_t(2 * n + 1), stream) != cudaSuccess) {

@@ -205,23 +205,40 @@ __device__ __forceinline__ float box_dist_sq_fast(const float px, const float py
 // instructions: per axis the point's coordinate along it less the centre's (three FFMA2), its excess
 // over the half extent, and the squared norm. 24 floating-point instructions for the two boxes, against
 // 18 for two axis-aligned ones. A NaN coordinate gives an excess of 0 (a bound that culls nothing).
-__device__ __forceinline__ float2 obb_dist_sq_pair(const float2 x2, const float2 y2, const float2 z2,
-                                                   const float4 *__restrict__ n, int &r0, int &r1) {
-    const float4 h0 = __ldg(n + 6), h1 = __ldg(n + 7);
+// FAR: also the squared distances to the boxes' farthest points (in the stored, slightly shrunk frame: up to
+// 3.2 % below the true ones, see kObbMaxAlpha), the node read from shared memory.
+template <bool FAR>
+__device__ __forceinline__ float2 obb_pair(const float2 x2, const float2 y2, const float2 z2,
+                                           const float4 *__restrict__ n, int &r0, int &r1, float2 &far) {
+    auto ld = [&](int k) { return FAR ? n[k] : __ldg(n + k); };
+    const float4 h0 = ld(6), h1 = ld(7);
     float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        const float4 a = __ldg(n + 2 * k), b = __ldg(n + 2 * k + 1);
+        const float4 a = ld(2 * k), b = ld(2 * k + 1);
         const float2 t = __ffma2_rn(make_float2(a.x, a.y), x2,
                                     __ffma2_rn(make_float2(a.z, a.w), y2,
                                                __ffma2_rn(make_float2(b.x, b.y), z2, make_float2(b.z, b.w))));
         const float hx = k == 0 ? h0.x : (k == 1 ? h0.z : h1.x), hy = k == 0 ? h0.y : (k == 1 ? h0.w : h1.y);
         const float2 e = make_float2(fmaxf(fabsf(t.x) - hx, 0.f), fmaxf(fabsf(t.y) - hy, 0.f));
         acc = k == 0 ? __fmul2_rn(e, e) : __ffma2_rn(e, e, acc);
+        if (FAR) {
+            const float2 g = make_float2(fabsf(t.x) + hx, fabsf(t.y) + hy);
+            far = k == 0 ? __fmul2_rn(g, g) : __ffma2_rn(g, g, far);
+        }
     }
     r0 = __float_as_int(h1.z);
     r1 = __float_as_int(h1.w);
     return acc;
+}
+__device__ __forceinline__ float2 obb_dist_sq_pair(const float2 x2, const float2 y2, const float2 z2,
+                                                   const float4 *__restrict__ n, int &r0, int &r1) {
+    float2 far;
+    return obb_pair<false>(x2, y2, z2, n, r0, r1, far);
+}
+__device__ __forceinline__ float2 obb_dist_sq_bounds(const float2 x2, const float2 y2, const float2 z2,
+                                                     const float4 *__restrict__ n, int &r0, int &r1, float2 &far) {
+    return obb_pair<true>(x2, y2, z2, n, r0, r1, far);
 }
 
 // Node-grid coordinate in G precision (serial/bvh/bvh.cpp:1665-1667, 1744): lo + i * h, one

@@ -70,6 +70,8 @@ struct DeviceMesh {
     // lower bound of any contained triangle's distance, exact or as the float arithmetic evaluates it
     // (mesh_build.cu, k_obb).
     const float4 *obb = nullptr;
+    // where a walk shared by a warp starts: entry[0] nodes (at most 32), entry[1 ..]
+    const int *entry = nullptr;
     float box_c[3] = {0.f, 0.f, 0.f};
     float box_scale = 1.f;
     const float4 *tris32 = nullptr;    // [3 * nt], leaf order
@@ -337,6 +339,10 @@ inline int resolve_warp_budget(int b, long long n, int ntri, bool grid) {
 // Point lists of at least this many queries are visited in Morton order (SSDF_B200_SORT_POINTS=0
 // keeps input order).
 constexpr long long kSortMinPoints = 4096;
+// Point lists of at most this many queries are answered a warp per query (k_query_warp), whose time grows
+// with the list (about 12 us per 1,000) where packets' does not until they fill the GPU; the lines cross
+// between 16,000 and 40,000 points in every mesh and arithmetic measured (SSDF_B200_WARP_POINTS overrides).
+constexpr int kWarpPoints = 24576;
 // Morton order of n (< 2^31) points over the mesh's root box: *order (n ints, stream-ordered
 // allocation the caller frees with cudaFreeAsync) lists the point indices in key order (bvh_query.cu).
 int morton_point_order(long long n, const void *x, const void *y, const void *z, int f64, const float4 *nodes32,

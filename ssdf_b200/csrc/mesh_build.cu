@@ -441,28 +441,56 @@ namespace {
 
 // Middle and scale of the mesh's box (the union of the root's children), and M in that frame: w[0..2],
 // w[3], w[4] as floats. A mesh outside [2^-60, 2^100], or with a coordinate that is not finite, gets M < 0:
-// its boxes cull nothing.
-__global__ void k_box_frame(const float4 *__restrict__ nodes, int *__restrict__ w) {
+// its boxes cull nothing. And the nodes a warp-wide walk starts from (DeviceMesh::entry): the root, each
+// node whose children are both nodes replaced by them, five times over. One warp.
+__global__ void k_box_frame(const float4 *__restrict__ nodes, int *__restrict__ w, int *__restrict__ entry) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x;
     const float4 a = nodes[0], b = nodes[1], c = nodes[2];
-    const float lo[3] = {fminf(a.x, b.x), fminf(a.z, b.z), fminf(c.x, c.z)};
-    const float hi[3] = {fmaxf(a.y, b.y), fmaxf(a.w, b.w), fmaxf(c.y, c.w)};
-    float mid[3], m = 0.f;
-    for (int d = 0; d < 3; d++) {
-        mid[d] = 0.5f * lo[d] + 0.5f * hi[d];
-        m = fmaxf(m, fmaxf(hi[d] - mid[d], mid[d] - lo[d]));
+    if (lane == 0) {
+        const float lo[3] = {fminf(a.x, b.x), fminf(a.z, b.z), fminf(c.x, c.z)};
+        const float hi[3] = {fmaxf(a.y, b.y), fmaxf(a.w, b.w), fmaxf(c.y, c.w)};
+        float mid[3], m = 0.f;
+        for (int d = 0; d < 3; d++) {
+            mid[d] = 0.5f * lo[d] + 0.5f * hi[d];
+            m = fmaxf(m, fmaxf(hi[d] - mid[d], mid[d] - lo[d]));
+        }
+        float scale = 1.f;
+        if (!(m >= 0x1p-60f && m <= 0x1p100f)) {
+            m = -1.f;
+            for (int d = 0; d < 3; d++) mid[d] = 0.f;
+        } else if (m > 0x1p60f) {
+            int e;
+            m = frexpf(m, &e);  // M in [0.5, 1)
+            scale = ldexpf(1.f, -e);
+        }
+        for (int d = 0; d < 3; d++) w[d] = __float_as_int(mid[d]);
+        w[3] = __float_as_int(scale);
+        w[4] = __float_as_int(m);
     }
-    float scale = 1.f;
-    if (!(m >= 0x1p-60f && m <= 0x1p100f)) {
-        m = -1.f;
-        for (int d = 0; d < 3; d++) mid[d] = 0.f;
-    } else if (m > 0x1p60f) {
-        int e;
-        m = frexpf(m, &e);  // M in [0.5, 1)
-        scale = ldexpf(1.f, -e);
+    int n = 1, node = 0;  // lanes 0 .. n - 1 hold a node each
+    for (int round = 0; round < 5; round++) {
+        int r0 = -1, r1 = -1;
+        if (lane < n) {
+            const float4 r = nodes[4 * size_t(node) + 3];
+            r0 = __float_as_int(r.x), r1 = __float_as_int(r.y);
+        }
+        const bool open = r0 >= 0 && r1 >= 0;
+        const unsigned m = __ballot_sync(kAll, open);
+        const int at = lane < n ? lane + __popc(m & ((1u << lane) - 1u)) : 0;  // at most 2 n <= 32 of them
+        if (lane < n) {
+            entry[1 + at] = open ? r0 : node;
+            if (open) entry[2 + at] = r1;
+        }
+        n += __popc(m);
+        __syncwarp();
+        node = lane < n ? entry[1 + lane] : 0;
+        __syncwarp();
     }
-    for (int d = 0; d < 3; d++) w[d] = __float_as_int(mid[d]);
-    w[3] = __float_as_int(scale);
-    w[4] = __float_as_int(m);
+    if (lane == 0) {
+        entry[0] = n;
+        if (n == 1) entry[1] = node;
+    }
 }
 
 __global__ void k_tri_records(int nt, const int *__restrict__ sorted_ids, const int *__restrict__ s0,
@@ -586,7 +614,8 @@ __global__ void __launch_bounds__(128) k_obb(int nnodes, int L, const int *__res
     const float scale = __int_as_float(frame[3]), M = __int_as_float(frame[4]);
     // child's axes, -centre coordinates and half extents (a box that culls nothing)
     Vec3 ax[3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
-    float off[3] = {0.f, 0.f, 0.f}, half[3] = {0.f, 0.f, 0.f};
+    const float inf = __int_as_float(0x7f800000);
+    float off[3] = {0.f, 0.f, 0.f}, half[3] = {inf, inf, inf};
     int writer = 0;
     if (ref != kEmptyRef && M >= 0.f) {
         const bool leaf = ref < 0;
@@ -678,7 +707,7 @@ __global__ void __launch_bounds__(128) k_obb(int nnodes, int L, const int *__res
                 ax[a] = {ax[a].x * s, ax[a].y * s, ax[a].z * s};
                 off[a] *= s;
                 // an extent the margins cannot bound (an overflow) culls nothing
-                half[a] = half[a] < FLT_MAX ? half[a] * s : __int_as_float(0x7f800000);
+                half[a] = half[a] < FLT_MAX ? half[a] * s : inf;
             }
         } else {
             // the axis-aligned box of the double corners
@@ -704,7 +733,10 @@ __global__ void __launch_bounds__(128) k_obb(int nnodes, int L, const int *__res
             }
         }
     }
-    if (ref == kEmptyRef) off[0] = 0x1p60f;  // never entered, and the farther child
+    if (ref == kEmptyRef) {  // never entered, and the farther child
+        off[0] = 0x1p60f;
+        half[0] = half[1] = half[2] = 0.f;
+    }
     if (lane != writer) return;
     float *o = obb + 32 * size_t(i) + h;
 #pragma unroll
@@ -1014,7 +1046,9 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
     SSDF_CHECK(dalloc(s, &t32, 3 * size_t(nt), stream));
     if (keep64) SSDF_CHECK(dalloc(s, &t64, 5 * size_t(nt), stream));
     if (keep64) SSDF_CHECK(dalloc(s, &filt, 3 * size_t(nt), stream));  // the fix-up path's filter records
-    k_box_frame<<<1, 1, 0, stream>>>(nodes32, flags + 16);
+    int *entry;
+    SSDF_CHECK(dalloc(s, &entry, 33, stream));
+    k_box_frame<<<1, 32, 0, stream>>>(nodes32, flags + 16, entry);
     LAUNCH_CHECK("k_box_frame");
     k_tri_records<<<grid_blocks(nt, 256), 256, 0, stream>>>(nt, ids, s0, s1, s2, vx, vy, vz, t32, t64, filt,
                                                             flags + 16, flags + 10);
@@ -1045,6 +1079,7 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
     m->nleaves = depth_leaves[1];
     m->nodes32 = nodes32;
     m->obb = obb;
+    m->entry = entry;
     m->tris32 = t32;
     m->tris64 = t64;
     m->filt32 = filt;

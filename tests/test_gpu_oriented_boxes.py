@@ -88,8 +88,17 @@ def run(dm, pts, precision, dtype):
     return out.cpu().numpy(), tri.cpu().numpy()
 
 
+# a warp per query (short lists' default, and with a stack that sends lanes into their own subtrees), a
+# thread per query, 32-query packets
+WALKS = {"warp": {}, "warp, short stack": {"SSDF_B200_WINDOW_STACK": "3"}, "thread": {"SSDF_B200_WARP_POINTS": "0"},
+         "packet": {"SSDF_B200_TRAVERSAL": "warp"}}
+
+
+@pytest.mark.parametrize("walk", list(WALKS))
 @pytest.mark.parametrize("name", list(MESHES))
-def test_every_arithmetic_equals_brute_force(name):
+def test_every_arithmetic_equals_brute_force(name, walk, monkeypatch):
+    for k, v in WALKS[walk].items():
+        monkeypatch.setenv(k, v)
     mesh = MESHES[name]
     pts = queries(mesh)
     want, wtri = oracle.edf(pts, mesh, with_index=True)
@@ -104,6 +113,23 @@ def test_every_arithmetic_equals_brute_force(name):
     got, tri = run(single, p32, S.PREC_F32, torch.float32)
     single.close()
     assert np.array_equal(got, want) and np.array_equal(tri, wtri)
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 24576, 24577])
+def test_list_lengths_at_the_warp_walk_limit(n):
+    """Both sides of the length up to which a warp answers each query, and partial blocks: equal to the
+    oracle on a sample, and to the plain double kernel at every point."""
+    mesh = W.torus(nu=30, nv=15, jitter=0.02)
+    lo, hi = mesh.bbox()
+    pts = np.random.default_rng(n).uniform(lo - 0.2, hi + 0.2, (n, 3)).T.copy()
+    dm = S.DeviceMesh(mesh)
+    got, tri = run(dm, pts, S.PREC_F32_FIXUP, torch.float64)
+    d64, t64 = run(dm, pts, S.PREC_F64, torch.float64)
+    dm.close()
+    ids = np.arange(0, n, max(1, n // 500))
+    want, wtri = oracle.edf(pts[:, ids].copy(), mesh, with_index=True)
+    assert np.array_equal(got, d64) and np.array_equal(tri, t64)
+    assert np.array_equal(got[ids], want) and np.array_equal(tri[ids], wtri)
 
 
 def test_points_that_are_not_finite_keep_their_bound():
