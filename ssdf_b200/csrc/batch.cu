@@ -231,17 +231,21 @@ int ssdf_batch_add_points(ssdf_batch *b, ssdf_mesh *mesh, ptrdiff_t npoints, con
     return batch_add(b, a, opts);
 }
 
-// Sizes the fix-up overflow lists for runs of up to max_queries queries, so that such runs never
+// Sizes the hand-over lists for runs of up to max_queries queries, so that such runs never
 // reallocate them (a reallocation synchronises the device).
 int ssdf_batch_reserve(ssdf_batch *b, long long max_queries, void *stream_) {
     if (!b || max_queries < 0) return fail(SSDF_ERR_INVALID_ARGUMENT, "ssdf_batch_reserve: bad arguments");
-    const size_t need = b->precision == SSDF_PREC_F32_FIXUP ? 2 * size_t(max_queries) : 0;
+    const size_t need = 2 * size_t(max_queries);
     if (need <= b->fb_cap) return SSDF_OK;
     SSDF_CUDA(cudaStreamSynchronize((cudaStream_t)stream_));
     cudaFree(b->d_fb);
     b->d_fb = nullptr;
     b->fb_cap = 0;
-    SSDF_CUDA(cudaMalloc(&b->d_fb, sizeof(int) * need));
+    if (cudaMalloc(&b->d_fb, sizeof(int) * need) != cudaSuccess) {
+        cudaGetLastError();
+        b->d_fb = nullptr;
+        return fail(SSDF_ERR_OUT_OF_MEMORY, "hand-over lists of " + std::to_string(max_queries) + " queries");
+    }
     b->fb_cap = need;
     return SSDF_OK;
 }
@@ -270,12 +274,15 @@ int ssdf_batch_run(ssdf_batch *b, int use_graph, void *stream_) {
     for (int i = 0; i < njobs; i++) order[i] = i;
     auto cost = [&](const QueryArgs &a) { return double(query_blocks(a)) * std::log2(2.0 + a.m.nt); };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost(b->jobs[x]) > cost(b->jobs[y]); });
-    // fix-up overflow lists: one slice of (ids, thresholds) per job of the first table
+    // hand-over lists: one slice of (ids, thresholds) per job
     size_t need = 0;
-    if (fixup)
-        for (const auto &j : b->jobs)
-            if (!to_f64(j)) need += 2 * size_t(j.is_grid ? j.nx * j.ny * j.nz : j.npoints);
-    if (need > b->fb_cap) SSDF_CHECK(ssdf_batch_reserve(b, (long long)(need / 2), stream));
+    for (const auto &j : b->jobs) need += 2 * size_t(j.is_grid ? j.nx * j.ny * j.nz : j.npoints);
+    bool lists = true;
+    if (need > b->fb_cap) {
+        const int st = ssdf_batch_reserve(b, (long long)(need / 2), stream);
+        if (fixup) SSDF_CHECK(st);
+        lists = st == SSDF_OK;  // the plain arithmetics only walk on without a budget
+    }
     // the staging buffers may still feed the previous run's copies
     SSDF_CUDA(cudaStreamSynchronize(stream));
     struct Orders {  // the runs' visiting orders, freed in stream order when the call returns
@@ -307,26 +314,21 @@ int ssdf_batch_run(ssdf_batch *b, int use_graph, void *stream_) {
             a.order = ord;
         }
         a.counters = nullptr;
-        if (to_f64(a)) {
-            a.fallback_count = nullptr;
-            a.fallback_ids = nullptr;
-            a.fallback_thr = nullptr;
-            a.warp_budget = 0;
-            b->h_jobs64[k64] = a;
-            b->h_first64[k64++] = total64;
-            total64 += query_blocks(a);
-            continue;
-        }
-        if (fixup) {
-            const size_t n = size_t(a.is_grid ? a.nx * a.ny * a.nz : a.npoints);
-            a.fallback_count = b->d_fbcount + k;
+        const size_t n = size_t(a.is_grid ? a.nx * a.ny * a.nz : a.npoints);
+        if (lists) {
+            a.fallback_count = b->d_fbcount + r;
             a.fallback_ids = b->d_fb + off;
             a.fallback_thr = reinterpret_cast<float *>(b->d_fb + off + n);
             off += 2 * n;
         } else {
             a.fallback_count = nullptr;
-            a.fallback_ids = nullptr;
-            a.fallback_thr = nullptr;
+            a.warp_budget = 0;
+        }
+        if (to_f64(a)) {
+            b->h_jobs64[k64] = a;
+            b->h_first64[k64++] = total64;
+            total64 += query_blocks(a);
+            continue;
         }
         b->h_jobs[k] = a;
         b->h_first[k++] = total;

@@ -235,6 +235,7 @@ struct ExactPolicy {
     float2 bx[Q], by[Q], bz[Q];  // the point in the box frame, each coordinate twice (two-wide FP32)
     float thr[Q];
     int bid[Q], bpos[Q];
+    bool gone = false;  // the packet handed its queries to the second stage
     T margin;
     __device__ explicit ExactPolicy(const DeviceMesh &mesh) : m(mesh) { margin = ExactData<T>::margin(m); }
     __device__ __forceinline__ void set(int q, T x, T y, T z, T init) {
@@ -250,6 +251,7 @@ struct ExactPolicy {
         bx[q] = by[q] = bz[q] = twice(kNowhere);
         thr[q] = -1.f;
     }
+    __device__ __forceinline__ void abandon() { gone = true; }
     // Starts query q from the triangle at leaf position pos, as if the walk had tested it first (it
     // replaces the incoming bound only when strictly closer; the walk meets it again without effect).
     __device__ __forceinline__ void seed(int q, int pos) {
@@ -329,7 +331,6 @@ template <int Q>
 struct FastPolicy {
     using R = float;
     static constexpr int kQn = Q;
-    static constexpr bool kBudgeted = true;
     const DeviceMesh &m;
     float2 bx[Q], by[Q], bz[Q];  // the point in the box frame (the filter records' too), each coordinate twice
     float best[Q], thr[Q], evicted[Q];
@@ -451,17 +452,6 @@ __device__ __forceinline__ R min_of(const R (&d)[Q]) {
     return v;
 }
 
-// Policies that can hand their queries to a second stage (P::kBudgeted) stop a packet's walk after a
-// work budget; the others always finish it.
-template <class P, class = void>
-struct HasBudget : std::false_type {};
-template <class P>
-struct HasBudget<P, std::void_t<decltype(P::kBudgeted)>> : std::bool_constant<P::kBudgeted> {};
-template <class P>
-constexpr bool budgeted() {
-    return HasBudget<P>::value;
-}
-
 constexpr int kRepLane = 21;  // (1, 1, 1) of the 4 x 4 x 2 brick
 
 // Warp minimum / maximum of a float (sm_100's redux on floats).
@@ -496,7 +486,7 @@ __device__ __forceinline__ void traverse_packet(P &p, Counters &cnt, int budget)
     int node = 0;
     auto test_leaf = [&](int ref, unsigned m) {
         p.template leaf<COUNT>(leaf_first(ref), leaf_count(ref), m, cnt);
-        if constexpr (budgeted<P>()) work += leaf_count(ref);
+        work += leaf_count(ref);
     };
     while (true) {
         float d0[Q], d1[Q];
@@ -536,11 +526,9 @@ __device__ __forceinline__ void traverse_packet(P &p, Counters &cnt, int budget)
             else next = r;
         }
         if (next < 0) {
-            if constexpr (budgeted<P>()) {
-                if (work > budget) {  // warp-uniform; checked where a path ends
-                    p.abandon();
-                    break;
-                }
+            if (work > budget) {  // warp-uniform; checked where a path ends
+                p.abandon();
+                break;
             }
             const float tmax = warp_max(p.max_thr());
             while (sp > 0) {
@@ -767,6 +755,13 @@ __device__ __forceinline__ void signal_chunk(const QueryArgs &a) {
     }
 }
 
+// Lists query q for the second stage, with its threshold (q < 2^31 is checked on the host).
+__device__ __forceinline__ void hand_over(const QueryArgs &a, long long q, float thr) {
+    const int slot = atomicAdd(a.fallback_count, 1);
+    a.fallback_ids[slot] = int(q);
+    a.fallback_thr[slot] = thr;
+}
+
 // One block of 128 lanes x kQ queries: a point-list block, or one step of a grid block's column.
 // Lanes without a query (the edge of a grid brick, the tail of a point list) take part in warp-mode
 // traversal with a negative threshold, so they never ask for a node. seed[s] is the leaf position of
@@ -791,10 +786,14 @@ __device__ __forceinline__ void query_step(const QueryArgs &a, int step, const b
                 p.disable(s);
             }
         }
-        if (WARP || any) traverse<WARP, COUNT>(p, cnt, 0);
+        if (WARP || any) traverse<WARP, COUNT>(p, cnt, a.warp_budget);
 #pragma unroll
         for (int s = 0; s < Q; s++) {
             if (!valid[s]) continue;
+            if (WARP && p.gone && p.thr[s] > 0.f) {
+                hand_over(a, qid[s], p.thr[s]);
+                continue;
+            }
             write_result(a, qid[s], p.px[s], p.py[s], p.pz[s], p.best[s], p.bid[s], p.bpos[s]);
             if (p.bpos[s] >= 0) seed[s] = p.bpos[s];
         }
@@ -814,11 +813,15 @@ __device__ __forceinline__ void query_step(const QueryArgs &a, int step, const b
                 p.disable(s);
             }
         }
-        if (WARP || any) traverse<WARP, COUNT>(p, cnt, 0);
+        if (WARP || any) traverse<WARP, COUNT>(p, cnt, a.warp_budget);
 #pragma unroll
         for (int s = 0; s < Q; s++) {
             if (!valid[s]) continue;
             const long long q = qid[s];
+            if (WARP && p.gone && p.thr[s] > 0.f) {
+                hand_over(a, q, p.thr[s]);
+                continue;
+            }
             if (a.output == SSDF_OUT_SQEDF) {
                 store_out(a, q, double(p.best[s]));
             } else {
@@ -860,9 +863,7 @@ __device__ __forceinline__ void query_step(const QueryArgs &a, int step, const b
             if (!valid[s]) continue;
             const long long q = qid[s];
             if (exact[s] || p.evicted[s] < p.thr[s]) {
-                const int slot = atomicAdd(a.fallback_count, 1);
-                a.fallback_ids[slot] = int(q);  // q < 2^31 is checked on the host
-                a.fallback_thr[slot] = exact[s] ? finf() : p.thr[s];
+                hand_over(a, q, exact[s] ? finf() : p.thr[s]);
                 continue;
             }
             // the double point and bound are recomputed here rather than kept live through the walk
@@ -1149,8 +1150,33 @@ __device__ bool warp_walk(LaneWalk<PREC> &w, float thr, bool shrink, bool upper,
     return !(cut < finf()) || w.confirms(cut);  // whatever the cuts left out lies above the minimum
 }
 
-// The whole warp answers overflowed query `idx` of job `a`; lane 0 writes the result.
-template <bool COUNT>
+// The incoming bound of a query in the arithmetic's own terms, and its result.
+template <int PREC>
+__device__ __forceinline__ typename LaneWalk<PREC>::T lane_bound(const QueryArgs &a, long long q) {
+    if constexpr (PREC == SSDF_PREC_F32) {
+        const float o = a.out_f64 ? float(((const double *)a.out)[q]) : ((const float *)a.out)[q];
+        return a.output == SSDF_OUT_SQEDF ? o : o * o;
+    } else {
+        return initial_bound(a, q);
+    }
+}
+template <int PREC>
+__device__ __forceinline__ void lane_result(const QueryArgs &a, long long q, double x, double y, double z,
+                                            const LaneWalk<PREC> &w) {
+    if constexpr (PREC == SSDF_PREC_F32) {
+        if (a.output == SSDF_OUT_SQEDF) {
+            store_out(a, q, double(w.d2));
+        } else {
+            store_out(a, q, double(sqrtf(w.d2)));
+            if (a.outtri && w.id >= 0) a.outtri[q] = w.id;
+        }
+    } else {
+        write_result(a, q, x, y, z, w.d2, w.id, w.pos);
+    }
+}
+
+// The whole warp answers handed-over query `idx` of job `a`; lane 0 writes the result.
+template <int PREC, bool COUNT>
 __device__ void window_warp(const QueryArgs &a, int idx, WarpShared &sh, int cap, Counters &cnt) {
     const long long q = a.fallback_ids[idx];
     long long i = 0, j = 0, k = 0;
@@ -1158,21 +1184,22 @@ __device__ void window_warp(const QueryArgs &a, int idx, WarpShared &sh, int cap
     double qx, qy, qz;
     query_point(a, q, i, j, k, qx, qy, qz);
     const float thr = a.fallback_thr[idx];
-    LaneWalk<SSDF_PREC_F32_FIXUP> w(a, qx, qy, qz, initial_bound(a, q));
-    // an infinite window (a point beyond the float range) stays
-    warp_walk<SSDF_PREC_F32_FIXUP, COUNT>(w, thr, thr < finf(), false, sh, cap, cnt);
-    if ((threadIdx.x & 31) == 0) write_result(a, q, qx, qy, qz, w.d2, w.id, w.pos);
+    LaneWalk<PREC> w(a, qx, qy, qz, lane_bound<PREC>(a, q));
+    // fix-up: an infinite window (a point beyond the float range) stays
+    const bool shrink = PREC != SSDF_PREC_F32_FIXUP || thr < finf();
+    warp_walk<PREC, COUNT>(w, thr, shrink, false, sh, cap, cnt);
+    if ((threadIdx.x & 31) == 0) lane_result(a, q, qx, qy, qz, w);
 }
 
-// Overflowed queries of one launch, a warp each. `cap` (<= kWinStack) is the shared stack's usable
+// Handed-over queries of one launch, a warp each. `cap` (<= kWinStack) is the shared stack's usable
 // depth: kWinStack, lowered only to test the per-lane subtree walk.
-template <bool COUNT>
+template <int PREC, bool COUNT>
 __global__ void __launch_bounds__(kThreads) k_window(const QueryArgs a, int cap) {
     __shared__ WarpShared s_warp[kThreads / 32];
     const int n = *a.fallback_count;
     const int w = (blockIdx.x * kThreads + threadIdx.x) >> 5, nw = (gridDim.x * kThreads) >> 5;
     Counters cnt;
-    for (int idx = w; idx < n; idx += nw) window_warp<COUNT>(a, idx, s_warp[threadIdx.x >> 5], cap, cnt);
+    for (int idx = w; idx < n; idx += nw) window_warp<PREC, COUNT>(a, idx, s_warp[threadIdx.x >> 5], cap, cnt);
     if (COUNT) flush_counters(a, cnt);
 }
 
@@ -1190,18 +1217,10 @@ __global__ void __launch_bounds__(kThreads, 6) k_query_warp(const QueryArgs a, i
     const long long q = (blockIdx.x * (long long)kThreads + threadIdx.x) >> 5;
     if (q >= a.npoints) return;  // a whole warp
     WarpShared &sh = s_warp[threadIdx.x >> 5];
-    using T = typename LaneWalk<PREC>::T;
     Counters cnt;
     double x, y, z;
     query_point(a, q, 0, 0, 0, x, y, z);
-    T init;
-    if constexpr (PREC == SSDF_PREC_F32) {
-        const float o = a.out_f64 ? float(((const double *)a.out)[q]) : ((const float *)a.out)[q];
-        init = a.output == SSDF_OUT_SQEDF ? o : o * o;
-    } else {
-        init = initial_bound(a, q);
-    }
-    LaneWalk<PREC> w(a, x, y, z, init);
+    LaneWalk<PREC> w(a, x, y, z, lane_bound<PREC>(a, q));
     if (w.finite()) {
         // a finite point beyond the filter's range: everything, exactly, in double
         const bool beyond = PREC == SSDF_PREC_F32_FIXUP &&
@@ -1209,18 +1228,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_query_warp(const QueryArgs a, i
         bool upper = !beyond;
         while (!warp_walk<PREC, COUNT>(w, beyond ? finf() : w.start_thr(), !beyond, upper, sh, cap, cnt)) upper = false;
     }
-    if ((threadIdx.x & 31) == 0) {
-        if constexpr (PREC == SSDF_PREC_F32) {
-            if (a.output == SSDF_OUT_SQEDF) {
-                store_out(a, q, double(w.d2));
-            } else {
-                store_out(a, q, double(sqrtf(w.d2)));
-                if (a.outtri && w.id >= 0) a.outtri[q] = w.id;
-            }
-        } else {
-            write_result(a, q, x, y, z, w.d2, w.id, w.pos);
-        }
-    }
+    if ((threadIdx.x & 31) == 0) lane_result(a, q, x, y, z, w);
     if (COUNT) flush_counters(a, cnt);
 }
 
@@ -1257,7 +1265,7 @@ __global__ void __launch_bounds__(kThreads, PREC == SSDF_PREC_F64 ? kF64MinBlock
 
 // Overflowed queries of every job: the jobs' lists laid end to end and dealt to the warps in turn,
 // so no warp takes the same position of every list.
-template <bool COUNT>
+template <int PREC, bool COUNT>
 __global__ void __launch_bounds__(kThreads) k_window_batch(const BatchHeader *__restrict__ hdr,
                                                            const QueryArgs *__restrict__ jobs, int cap) {
     __shared__ WarpShared s_warp[kThreads / 32];
@@ -1270,7 +1278,7 @@ __global__ void __launch_bounds__(kThreads) k_window_batch(const BatchHeader *__
         if (!a.fallback_count) continue;
         const int n = *a.fallback_count;
         for (long long idx = ((w - base) % nw + nw) % nw; idx < n; idx += nw)
-            window_warp<COUNT>(a, int(idx), s_warp[threadIdx.x >> 5], cap, cnt);
+            window_warp<PREC, COUNT>(a, int(idx), s_warp[threadIdx.x >> 5], cap, cnt);
         base += n;
     }
     if (COUNT && njobs > 0) flush_counters(jobs[0], cnt);
@@ -1283,6 +1291,21 @@ int window_stack_cap() {
     return v < 1 ? 1 : (v > kWinStack ? kWinStack : v);
 }
 
+// Blocks of the second fix-up stage (kWindowBlocksPerSm per SM, four warps each; more than fit at
+// once). The warps stride over the overflow count, which is only known on the device.
+unsigned window_grid() {
+    static int cached[64] = {0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int &g = cached[dev & 63];
+    if (g == 0) {
+        int sms = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        g = kWindowBlocksPerSm * std::max(1, sms);
+    }
+    return unsigned(g);
+}
+
 template <int PREC, bool WARP>
 cudaError_t launch_batch_main(const BatchLaunch &b, bool count, cudaStream_t stream) {
     if (count)
@@ -1290,11 +1313,11 @@ cudaError_t launch_batch_main(const BatchLaunch &b, bool count, cudaStream_t str
     else
         k_query_batch<PREC, WARP, false><<<b.grid, kThreads, 0, stream>>>(b.hdr, b.jobs, b.first_block, b.next_item);
     cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || PREC != SSDF_PREC_F32_FIXUP) return e;
+    if (e != cudaSuccess) return e;
     if (count)
-        k_window_batch<true><<<kWindowBlocksPerSm * b.sms, kThreads, 0, stream>>>(b.hdr, b.jobs, window_stack_cap());
+        k_window_batch<PREC, true><<<kWindowBlocksPerSm * b.sms, kThreads, 0, stream>>>(b.hdr, b.jobs, window_stack_cap());
     else
-        k_window_batch<false><<<kWindowBlocksPerSm * b.sms, kThreads, 0, stream>>>(b.hdr, b.jobs, window_stack_cap());
+        k_window_batch<PREC, false><<<kWindowBlocksPerSm * b.sms, kThreads, 0, stream>>>(b.hdr, b.jobs, window_stack_cap());
     return cudaGetLastError();
 }
 
@@ -1337,6 +1360,18 @@ cudaError_t launch_main(const QueryArgs &a, bool count, unsigned nblocks, cudaSt
 template <int PREC>
 cudaError_t launch_prec(const QueryArgs &a, bool warp, bool count, unsigned nblocks, cudaStream_t stream) {
     return warp ? launch_main<PREC, true>(a, count, nblocks, stream) : launch_main<PREC, false>(a, count, nblocks, stream);
+}
+
+// The query kernel and, with a hand-over list, the second stage.
+template <int PREC>
+cudaError_t launch_two_stages(const QueryArgs &a, bool warp, bool count, unsigned nblocks, cudaStream_t stream,
+                              int cap = 0) {
+    const cudaError_t e = launch_prec<PREC>(a, warp, count, nblocks, stream);
+    if (e != cudaSuccess || !a.fallback_count) return e;
+    if (cap == 0) cap = window_stack_cap();
+    count ? k_window<PREC, true><<<window_grid(), kThreads, 0, stream>>>(a, cap)
+          : k_window<PREC, false><<<window_grid(), kThreads, 0, stream>>>(a, cap);
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -1459,21 +1494,6 @@ int morton_point_order(long long n, const void *x, const void *y, const void *z,
     return st;
 }
 
-// Blocks of the second fix-up stage (kWindowBlocksPerSm per SM, four warps each; more than fit at
-// once). The warps stride over the overflow count, which is only known on the device.
-unsigned window_grid() {
-    static int cached[64] = {0};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    int &g = cached[dev & 63];
-    if (g == 0) {
-        int sms = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        g = kWindowBlocksPerSm * std::max(1, sms);
-    }
-    return unsigned(g);
-}
-
 int launch_query(const QueryArgs &args_in, int precision, cudaStream_t stream) {
     return launch_query_keep(args_in, precision, stream, nullptr);
 }
@@ -1534,29 +1554,29 @@ int launch_query_keep(const QueryArgs &args_in, int precision, cudaStream_t stre
         e = precision == SSDF_PREC_F64   ? launch_query_warp<SSDF_PREC_F64>(a, count, stream)
             : precision == SSDF_PREC_F32 ? launch_query_warp<SSDF_PREC_F32>(a, count, stream)
                                          : launch_query_warp<SSDF_PREC_F32_FIXUP>(a, count, stream);
-    } else if (precision == SSDF_PREC_F32_FIXUP) {
-        if (n >= 0x7fffffffll) {
+    } else {
+        const bool fixup = precision == SSDF_PREC_F32_FIXUP;
+        if (fixup && n >= 0x7fffffffll) {
             st = fail(SSDF_ERR_NOT_SUPPORTED, "more than 2^31 - 1 queries in one fix-up launch");
-        } else if (cudaMallocAsync(&fb, sizeof(int) * size_t(2 * n + 1), stream) != cudaSuccess) {
-            st = fail(SSDF_ERR_OUT_OF_MEMORY, "fix-up overflow list");
-        } else {
+        } else if (fixup || (warp && a.warp_budget > 0 && n <= kHandOverMaxQueries)) {
+            if (cudaMallocAsync(&fb, sizeof(int) * size_t(2 * n + 1), stream) != cudaSuccess) {
+                fb = nullptr;
+                if (fixup) st = fail(SSDF_ERR_OUT_OF_MEMORY, "fix-up overflow list");
+                else cudaGetLastError();  // the plain arithmetics only walk on without a budget
+            }
+        }
+        if (fb) {
             a.fallback_count = fb;
             a.fallback_ids = fb + 1;
             a.fallback_thr = reinterpret_cast<float *>(fb + 1 + n);
             e = cudaMemsetAsync(fb, 0, sizeof(int), stream);
-            if (e == cudaSuccess) e = launch_prec<SSDF_PREC_F32_FIXUP>(a, warp, count, unsigned(nblocks), stream);
-            if (e == cudaSuccess) {
-                const unsigned wg = window_grid();
-                const int cap = window_stack_cap();
-                count ? k_window<true><<<wg, kThreads, 0, stream>>>(a, cap)
-                      : k_window<false><<<wg, kThreads, 0, stream>>>(a, cap);
-                e = cudaGetLastError();
-            }
+        } else {
+            a.warp_budget = 0;
         }
-    } else if (precision == SSDF_PREC_F64) {
-        e = launch_prec<SSDF_PREC_F64>(a, warp, count, unsigned(nblocks), stream);
-    } else {
-        e = launch_prec<SSDF_PREC_F32>(a, warp, count, unsigned(nblocks), stream);
+        if (st == SSDF_OK && e == cudaSuccess)
+            e = precision == SSDF_PREC_F64   ? launch_two_stages<SSDF_PREC_F64>(a, warp, count, unsigned(nblocks), stream)
+                : precision == SSDF_PREC_F32 ? launch_two_stages<SSDF_PREC_F32>(a, warp, count, unsigned(nblocks), stream)
+                                             : launch_two_stages<SSDF_PREC_F32_FIXUP>(a, warp, count, unsigned(nblocks), stream);
     }
     if (e != cudaSuccess && st == SSDF_OK) st = cuda_fail(e, "query launch", __FILE__, __LINE__);
     if (count && st == SSDF_OK) {
@@ -1663,11 +1683,6 @@ int launch_query_noalloc(const QueryArgs &args_in, cudaStream_t stream) {
     a.counters = nullptr;
     const bool warp = use_warp(a);
     const long long nblocks = query_blocks(a);
-    if (fixup_runs_f64(a.m)) {  // the same bits from the FP64 kernel, which has no overflow list
-        const cudaError_t e = launch_prec<SSDF_PREC_F64>(a, warp, false, unsigned(nblocks), stream);
-        if (e != cudaSuccess) return cuda_fail(e, "allocation-free query launch", __FILE__, __LINE__);
-        return SSDF_OK;
-    }
     a.warp_budget = resolve_warp_budget(a.warp_budget, n, a.m.nt, a.is_grid != 0);
     int *scratch = nullptr;
     SSDF_CHECK(noalloc_scratch(&scratch));
@@ -1675,11 +1690,9 @@ int launch_query_noalloc(const QueryArgs &args_in, cudaStream_t stream) {
     a.fallback_ids = scratch + 1;
     a.fallback_thr = reinterpret_cast<float *>(scratch + 1 + n);
     cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(int), stream);  // the count starts at zero
-    if (e == cudaSuccess) e = launch_prec<SSDF_PREC_F32_FIXUP>(a, warp, false, unsigned(nblocks), stream);
-    if (e == cudaSuccess) {
-        k_window<false><<<window_grid(), kThreads, 0, stream>>>(a, kWinStack);
-        e = cudaGetLastError();
-    }
+    if (e == cudaSuccess)
+        e = fixup_runs_f64(a.m) ? launch_two_stages<SSDF_PREC_F64>(a, warp, false, unsigned(nblocks), stream, kWinStack)
+                                : launch_two_stages<SSDF_PREC_F32_FIXUP>(a, warp, false, unsigned(nblocks), stream, kWinStack);
     if (e != cudaSuccess) return cuda_fail(e, "allocation-free query launch", __FILE__, __LINE__);
     return SSDF_OK;
 }

@@ -126,11 +126,11 @@ struct QueryArgs {
     void *outx, *outy, *outz;
     // fix-up window: tau = tau_rel * (coord_scale + d)
     float tau_rel;
-    // fix-up path, warp packets: a packet that has tested more than this many triangle records hands
+    // warp packets: a packet that has tested more than this many triangle records hands
     // its queries to the second stage (a warp per query) with their current windows; 0: no limit;
     // < 0: the default for the launch's size (resolve_warp_budget)
     int warp_budget;
-    // overflow list of the FP32 fix-up kernel (query, final window), finished by k_window
+    // hand-over list (query, threshold), finished by k_window; null without a budget
     int *fallback_ids;
     float *fallback_thr;
     int *fallback_count;
@@ -194,9 +194,8 @@ int exclusive_scan_i32(const int *in, int *out, int n, cudaStream_t stream);
 
 // ---- queries (bvh_query.cu) ----------------------------------------------------------------------
 int launch_query(const QueryArgs &args, int precision, cudaStream_t stream);
-// launch_query that, on success with the fix-up arithmetic, hands back the second stage's query list
-// (device ints: count, then the query indices) instead of freeing it; *fallback_list stays null for
-// the other arithmetics. The caller frees it with cudaFreeAsync on `stream`.
+// launch_query that, on success, hands back the second stage's query list (device ints: count, then the
+// query indices) instead of freeing it; *fallback_list stays null where there is none. The caller frees it with cudaFreeAsync on `stream`.
 int launch_query_keep(const QueryArgs &args, int precision, cudaStream_t stream, int **fallback_list);
 // A grid query whose results go to host arrays: args.out / args.outtri are device buffers of the
 // grid's size, and each slab chunk is copied to host_out / host_tri as soon as the kernel has
@@ -265,7 +264,7 @@ __device__ __forceinline__ void flush_pair_counts(unsigned long long *c, unsigne
     }
 }
 
-// ---- brute force and cell list (brute_force.cu, celllist.cu) -------------------------------------
+// ---- plain methods (brute_force.cu, celllist.cu) -------------------------------------
 // With SSDF_B200_COUNT set, both run a counting instantiation and leave their triangle (Ericson)
 // and box tests in ssdf_last_query_counts.
 int brute_force_edf(int f64, ptrdiff_t npoints, const void *x, const void *y, const void *z, ptrdiff_t nt,
@@ -329,6 +328,8 @@ inline int grid_blocks(long long n, int threads) { return int((n + threads - 1) 
 // SSDF_B200_WARP_BUDGET sets it for every launch (0 = no limit).
 constexpr int kWarpBudgetMin = 64, kWarpBudgetMax = 700;
 constexpr long long kBudgetSmallLaunch = 1ll << 21;
+// Largest launch of the plain arithmetics (F64, F32) that keeps a hand-over list, 8 bytes a query.
+constexpr long long kHandOverMaxQueries = 1ll << 24;
 inline int resolve_warp_budget(int b, long long n, int ntri, bool grid) {
     if (b >= 0) return b;
     const double t = ntri > 0 ? ntri : 0;

@@ -89,9 +89,10 @@ def run(dm, pts, precision, dtype):
 
 
 # a warp per query (short lists' default, and with a stack that sends lanes into their own subtrees), a
-# thread per query, 32-query packets
+# thread per query, 32-query packets, packets that hand their queries to the second stage
 WALKS = {"warp": {}, "warp, short stack": {"SSDF_B200_WINDOW_STACK": "3"}, "thread": {"SSDF_B200_WARP_POINTS": "0"},
-         "packet": {"SSDF_B200_TRAVERSAL": "warp"}}
+         "packet": {"SSDF_B200_TRAVERSAL": "warp"},
+         "packet, handed over": {"SSDF_B200_TRAVERSAL": "warp", "SSDF_B200_WARP_BUDGET": "2"}}
 
 
 @pytest.mark.parametrize("walk", list(WALKS))
