@@ -25,6 +25,7 @@ namespace {
 
 constexpr int kRec = 16;  // ax ay az bx by bz cx cy cz lox hix loy hiy loz hiz -
 constexpr int kBruteThreads = 256;
+constexpr int kNoBadTriangle = 0x7f7f7f7f;  // above any triangle index; one byte, so that a memset sets it
 
 template <typename T>
 __device__ __forceinline__ T rel_margin() {
@@ -230,9 +231,8 @@ int brute_impl(ptrdiff_t npoints, const T *x, const T *y, const T *z, ptrdiff_t 
         return cuda_fail(e, "brute force flags", __FILE__, __LINE__);
     }
     int st = SSDF_OK;
-    const int h0[4] = {0x7fffffff, 0, 0, 0};
-    e = cudaMemcpyAsync(flags, h0, sizeof(h0), cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    e = cudaMemsetAsync(flags, 0x7f, sizeof(int), stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(flags + 1, 0, 3 * sizeof(int), stream);
     if (e == cudaSuccess) {
         k_brute_records<T><<<grid_blocks(nt, 256), 256, 0, stream>>>(int(nt), int(nv), s0, s1, s2, sx, sy, sz, rec,
                                                                      flags, flags + 2);
@@ -263,7 +263,7 @@ int brute_impl(ptrdiff_t npoints, const T *x, const T *y, const T *z, ptrdiff_t 
         }
         if (e == cudaSuccess) e = cudaGetLastError();
     }
-    int h[4] = {0x7fffffff, 0, 0, 0};
+    int h[4] = {kNoBadTriangle, 0, 0, 0};
     if (e == cudaSuccess) e = cudaMemcpyAsync(h, flags, sizeof(h), cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess && counters) e = cudaMemcpyAsync(hc, counters, sizeof(hc), cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
@@ -272,7 +272,7 @@ int brute_impl(ptrdiff_t npoints, const T *x, const T *y, const T *z, ptrdiff_t 
         if (e == cudaSuccess) set_last_counts(hc[0], hc[1], 0, 0);
     }
     if (e != cudaSuccess) st = cuda_fail(e, "brute-force edf", __FILE__, __LINE__);
-    else if (h[0] != 0x7fffffff)
+    else if (h[0] != kNoBadTriangle)
         st = fail(SSDF_ERR_INVALID_ARGUMENT, "triangle " + std::to_string(h[0]) + " has a vertex index out of range");
     else if (h[1])
         st = fail(SSDF_ERR_INTERNAL, "brute-force edf: a tile copy did not complete (bounded wait gave up)");
