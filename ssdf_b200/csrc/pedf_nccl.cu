@@ -143,7 +143,8 @@ int edf_inout(long long np, const G *x, const G *y, const G *z, T *out, long lon
     const int prec = out_precision(sizeof(T) == 8);
     const int ct = sizeof(G) == 8 ? SSDF_F64 : SSDF_F32;
     ssdf_build_opts bo;
-    bo.leaf_size = 0, bo.keep_fp64 = prec != SSDF_PREC_F32, bo.normals = 0, bo.treelet_opt = 1;
+    bo.leaf_size = 0, bo.keep_fp64 = prec != SSDF_PREC_F32, bo.normals = 0;
+    bo.treelet_opt = call_treelet_rounds(np);
     ssdf_mesh *m = nullptr;
     SSDF_CHECK(ssdf_mesh_create(&m, ptrdiff_t(nt), s0, s1, s2, ptrdiff_t(nv), sx, sy, sz, ct, 1, &bo, s));
     ssdf_query_opts qo;

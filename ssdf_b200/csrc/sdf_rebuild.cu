@@ -368,7 +368,7 @@ int rebuild_device(const GridDesc &gd, const T *d_f, T level, T band, long long 
         ssdf_mesh *mesh = nullptr;
         if (st == SSDF_OK) {
             ssdf_build_opts bo;
-            bo.leaf_size = 0, bo.keep_fp64 = 1, bo.normals = 0, bo.treelet_opt = 1;
+            bo.leaf_size = 0, bo.keep_fp64 = 1, bo.normals = 0, bo.treelet_opt = call_treelet_rounds(nout);
             st = ssdf_mesh_create(&mesh, ptrdiff_t(ntri), idx, idx + ntri, idx + 2 * ntri, ptrdiff_t(3 * ntri), x, y, z,
                                   g64 ? SSDF_F64 : SSDF_F32, 1, &bo, stream);
         }
