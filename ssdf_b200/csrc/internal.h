@@ -305,8 +305,8 @@ int round_device(const GridDesc &gd, const T *d_f, T radius, T band, bool open, 
 // Treelet refinement rounds of a resident mesh's BVH (built once, queried many times). Measured on the
 // current kernels, queries against 1 round: beam lattice (8e6 points + 512^3 grid, float) 335.6 ->
 // 313.1 / 308.7 / 304.8 ms for 2 / 3 / 4 rounds; torus knot 256^3 16.70 -> 16.63 ms (3); 64^3
-// icosphere 0.470 -> 0.465 ms; the serving leg's heaviest grid 3.74 -> 3.67 ms. Each round adds about
-// 1.5 ms to the torus knot's build, which calls that build per query do not repay
+// icosphere 0.470 -> 0.465 ms; the serving leg's heaviest grid 3.74 -> 3.67 ms. Each round adds
+// 0.45 ms to the torus knot's build, which calls that build per query do not repay
 // (call_treelet_rounds).
 constexpr int kResidentTreeletRounds = 3;
 
@@ -351,8 +351,8 @@ int morton_point_order(long long n, const void *x, const void *y, const void *z,
 int env_int(const char *name, int dflt);
 const char *env_str(const char *name);
 // Treelet refinement rounds for a mesh that one call builds and queries once (host-array calls, rebuilds,
-// pedf): none below 2^21 queries (SSDF_B200_TREELET overrides). The refinement is latency bound (about 1.1
-// ms whatever the mesh size) and, with oriented boxes, saves 0-10 % of a query on closed surfaces and 30 %
+// pedf): none below 2^21 queries (SSDF_B200_TREELET overrides). The refinement is latency bound (0.3 to 0.5
+// ms a round whatever the mesh size) and, with oriented boxes, saves 0-10 % of a query on closed surfaces and 30 %
 // on the beam lattice. us without it and with one round: 110^3 grid on 81,920 triangles 2,296 / 2,157, 128^3
 // around the knot 2,373 / 2,330, 256^3 10,672 / 10,222, 100,000 points near a torus 425 / 427, 4,000,000 on
 // the beam lattice 8,472 / 5,986; a 72^3 field rounded (four rebuilds) 9,588 with it, 4,683 without.

@@ -22,8 +22,8 @@
 namespace ssdf_b200 {
 
 // SAH treelet refinement (treelet_opt.cu): restructures the topology in place, refits the boxes and
-// re-derives the leaf order (ids, leaf references, first_of) so subtrees stay contiguous ranges.
-int treelet_optimize(int n, int *child_l, int *child_r, int *parent_int, int *parent_leaf, int *first_of,
+// re-derives the leaf order (ids, leaf references, first_of) and the counts, so subtrees stay contiguous ranges.
+int treelet_optimize(int n, int *child_l, int *child_r, int *parent_int, int *parent_leaf, int *first_of, int *count,
                      float *nbox32, double *nbox64, const float *pbox32, const double *pbox64, int *sorted_ids,
                      cudaStream_t stream);
 
@@ -148,9 +148,9 @@ __device__ __forceinline__ int karras_delta(const uint32_t *__restrict__ k, int 
     return __clz(a ^ b);
 }
 
-// Internal node i of the n-1: children (>= 0 internal, < 0 leaf -(pos + 1)), range, parents.
+// Internal node i of the n-1: children (>= 0 internal, < 0 leaf -(pos + 1)), range (first leaf, count), parents.
 __global__ void k_karras(int n, const uint32_t *__restrict__ k, int *__restrict__ child_l, int *__restrict__ child_r,
-                         int *__restrict__ first_of, int *__restrict__ last_of, int *__restrict__ parent_int,
+                         int *__restrict__ first_of, int *__restrict__ count, int *__restrict__ parent_int,
                          int *__restrict__ parent_leaf) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n - 1) return;
@@ -175,7 +175,7 @@ __global__ void k_karras(int n, const uint32_t *__restrict__ k, int *__restrict_
     child_l[i] = left;
     child_r[i] = right;
     first_of[i] = first;
-    last_of[i] = last;
+    count[i] = last - first + 1;
     if (left < 0) parent_leaf[gamma] = i; else parent_int[gamma] = i;
     if (right < 0) parent_leaf[gamma + 1] = i; else parent_int[gamma + 1] = i;
     if (i == 0) parent_int[0] = -1;
@@ -219,25 +219,6 @@ __global__ void k_refit(int n, const int *__restrict__ sorted_ids, const int *__
             __stcg(nbox32 + 6 * node + k, b32[k]);
             __stcg(nbox64 + 6 * node + k, b64[k]);
         }
-        node = parent_int[node];
-    }
-}
-
-// Subtree sizes after treelet restructuring: recomputed bottom-up the same way.
-__global__ void k_counts(int n, const int *__restrict__ child_l, const int *__restrict__ child_r,
-                         const int *__restrict__ parent_int, const int *__restrict__ parent_leaf, int *count,
-                         int *arrivals) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    int node = parent_leaf[p];
-    while (node >= 0) {
-        __threadfence();
-        if (atomicAdd(&arrivals[node], 1) == 0) return;
-        __threadfence();
-        const int l = child_l[node], r = child_r[node];
-        const int cl = l < 0 ? 1 : __ldcg(count + l);
-        const int cr = r < 0 ? 1 : __ldcg(count + r);
-        __stcg(count + node, cl + cr);
         node = parent_int[node];
     }
 }
@@ -1004,20 +985,19 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
         k_write_small_root<<<1, 1, 0, stream>>>(nt, box32, nodes32);
         LAUNCH_CHECK("k_write_small_root");
     } else {
-        int *child_l, *child_r, *first_of, *last_of, *parent_int, *parent_leaf, *arrivals, *count;
+        int *child_l, *child_r, *first_of, *parent_int, *parent_leaf, *arrivals, *count;
         float *nbox32;
         double *nbox64;
         SSDF_CHECK(dalloc(tmp, &child_l, nint, stream));
         SSDF_CHECK(dalloc(tmp, &child_r, nint, stream));
         SSDF_CHECK(dalloc(tmp, &first_of, nint, stream));
-        SSDF_CHECK(dalloc(tmp, &last_of, nint, stream));
         SSDF_CHECK(dalloc(tmp, &parent_int, nint, stream));
         SSDF_CHECK(dalloc(tmp, &parent_leaf, nt, stream));
         SSDF_CHECK(dalloc(tmp, &arrivals, nint, stream));
         SSDF_CHECK(dalloc(tmp, &count, nint, stream));
         SSDF_CHECK(dalloc(tmp, &nbox32, 6 * size_t(nint), stream));
         SSDF_CHECK(dalloc(tmp, &nbox64, 6 * size_t(nint), stream));
-        k_karras<<<grid_blocks(nint, 256), 256, 0, stream>>>(nt, keys, child_l, child_r, first_of, last_of,
+        k_karras<<<grid_blocks(nint, 256), 256, 0, stream>>>(nt, keys, child_l, child_r, first_of, count,
                                                              parent_int, parent_leaf);
         LAUNCH_CHECK("k_karras");
         SSDF_CUDA(cudaMemsetAsync(arrivals, 0, sizeof(int) * nint, stream));
@@ -1025,13 +1005,9 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
                                                           box64, nbox32, nbox64, arrivals);
         LAUNCH_CHECK("k_refit");
         for (int round = 0; round < opts.treelet_opt && round < 8; round++) {  // treelet_opt: rounds (0 = none)
-            SSDF_CHECK(treelet_optimize(nt, child_l, child_r, parent_int, parent_leaf, first_of, nbox32, nbox64,
+            SSDF_CHECK(treelet_optimize(nt, child_l, child_r, parent_int, parent_leaf, first_of, count, nbox32, nbox64,
                                         box32, box64, ids, stream));
         }
-        SSDF_CUDA(cudaMemsetAsync(arrivals, 0, sizeof(int) * nint, stream));
-        k_counts<<<grid_blocks(nt, 256), 256, 0, stream>>>(nt, child_l, child_r, parent_int, parent_leaf, count,
-                                                           arrivals);
-        LAUNCH_CHECK("k_counts");
         k_write_nodes<<<grid_blocks(nint, 256), 256, 0, stream>>>(nt, L, child_l, child_r, first_of, count, ids,
                                                                   box32, nbox32, nodes32);
         LAUNCH_CHECK("k_write_nodes");

@@ -67,134 +67,157 @@ __device__ __forceinline__ void set_parent(const TreeArrays &t, int ref, int par
         __stcg(t.parent_leaf + (-ref - 1), parent);
 }
 
-// A treelet in the making, in shared memory (one per warp): its members and their boxes and costs,
-// the internal nodes it reuses, and the dynamic programme's cost and best split of every subset.
+// A treelet in the making, in shared memory (one per warp): its members and their boxes, the internal nodes
+// it reuses, and the dynamic programme's area, cost and best split of every subset.
 struct TreeletWork {
     double mb64[kTreeletLeaves][6];
     float mb[kTreeletLeaves][6];
-    float mcost[kTreeletLeaves];
     int mcount[kTreeletLeaves];
     int member[kTreeletLeaves];
     int inner[kTreeletLeaves - 1];
-    int m, ni;  // members, internal nodes (m < 3: nothing to optimise)
+    int m;
     float old_cost;
+    float area[kSubsets];
     float c[kSubsets];
     unsigned char split[kSubsets];
-    unsigned char subs[40];  // a round's subsets, in increasing order (at most C(7, 3) = 35)
     // the rebuilt arrangement: internal node onode[k] now covers the members of subset oset[k]
     int onode[kTreeletLeaves - 1], oset[kTreeletLeaves - 1];
     int norder;
 };
 
-// One lane: grows the treelet rooted at internal node x (its subtree is final) from its two children
-// by opening the largest-area internal member until it has seven members. A treelet of fewer than
-// three members gets its cost stored here and w.m < 3.
-__device__ void form_treelet(const TreeArrays &t, int x, TreeletWork &w) {
-    int m = 2, ni = 1;
-    w.member[0] = __ldcg(t.child_l + x);
-    w.member[1] = __ldcg(t.child_r + x);
-    w.inner[0] = x;
-    ref_box32(t, w.member[0], w.mb[0]);
-    ref_box32(t, w.member[1], w.mb[1]);
-    while (m < kTreeletLeaves) {
-        int pick = -1;
-        float best = -1.f;
-        for (int k = 0; k < m; k++) {
-            if (w.member[k] >= 0) {
-                const float a = area6(w.mb[k]);
-                if (a > best) best = a, pick = k;
-            }
+// The subsets of seven members by size, each size in increasing order (so those of the first m members come
+// first), and where each size starts.
+struct SubsetTable {
+    unsigned char set[kSubsets];
+    int start[kTreeletLeaves + 2];
+};
+constexpr SubsetTable make_subsets() {
+    SubsetTable t{};
+    int n = 0;
+    for (int size = 0; size <= kTreeletLeaves; size++) {
+        t.start[size] = n;
+        for (int s = 0; s < kSubsets; s++) {
+            int bits = 0;
+            for (int b = 0; b < kTreeletLeaves; b++) bits += (s >> b) & 1;
+            if (bits == size) t.set[n++] = (unsigned char)s;
         }
-        if (pick < 0) break;
-        const int y = w.member[pick];
-        w.inner[ni++] = y;
-        w.member[pick] = __ldcg(t.child_l + y);
-        w.member[m] = __ldcg(t.child_r + y);
-        ref_box32(t, w.member[pick], w.mb[pick]);
-        ref_box32(t, w.member[m], w.mb[m]);
+    }
+    t.start[kTreeletLeaves + 1] = n;
+    return t;
+}
+__constant__ SubsetTable kSubsetTable = make_subsets();
+
+// The whole warp: the treelet rooted at internal node x (its subtree is final), grown from its two children by
+// opening the largest-area internal member until it has seven members, a lane to each; then the best
+// binary tree over them, by dynamic programming over the member subsets. One lane growing the treelet
+// waited 22,000 cycles, a programme searching every second submask in vain 46,000 more: a round on a 65,536-
+// triangle torus takes 416 us with a lane per member and per subset, 1,111 before, for the same tree. A treelet of fewer than three members only gets its cost stored (w.m < 3).
+__device__ void treelet_best(const TreeArrays &t, int x, TreeletWork &w, const unsigned char *__restrict__ sets,
+                             int lane) {
+    constexpr unsigned kAll = 0xffffffffu;
+    float bx[6], b[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int q = 0; q < 6; q++) bx[q] = __ldcg(t.nbox32 + 6 * x + q);
+    int ref = -1;
+    if (lane < 2) {
+        ref = __ldcg((lane ? t.child_r : t.child_l) + x);
+        ref_box32(t, ref, b);
+    }
+    float old_cost = area6(bx);  // the old internal nodes' areas, then the members' costs
+    if (lane == 0) w.inner[0] = x;
+    int m = 2;
+    while (m < kTreeletLeaves) {
+        const int key = lane < m && ref >= 0 ? __float_as_int(area6(b)) : -1;  // areas are not negative
+        const int best = __reduce_max_sync(kAll, key);
+        if (best < 0) break;
+        const int pick = __ffs(__ballot_sync(kAll, key == best)) - 1;
+        const int y = __shfl_sync(kAll, ref, pick);
+        old_cost += __int_as_float(best);
+        if (lane == 0) w.inner[m - 1] = y;
+        if (lane == pick || lane == m) {
+            ref = __ldcg((lane == pick ? t.child_l : t.child_r) + y);
+            ref_box32(t, ref, b);
+        }
         m++;
     }
-    w.m = m, w.ni = ni;
+    float mcost = 0.f;
+    if (lane < m) {
+        mcost = ref_cost(t, ref);
+        w.member[lane] = ref;
+        w.mcount[lane] = ref_count(t, ref);
+        for (int q = 0; q < 6; q++) w.mb[lane][q] = b[q];
+        double d[6];
+        ref_box64(t, ref, d);
+        for (int q = 0; q < 6; q++) w.mb64[lane][q] = d[q];
+    }
+    for (int k = 0; k < m; k++) old_cost += __shfl_sync(kAll, mcost, k);
+    if (lane == 0) {
+        w.m = m;
+        w.old_cost = old_cost;
+        if (m < 3) __stcg(t.cost + x, old_cost);
+    }
     if (m < 3) {
-        float b[6];
-        for (int q = 0; q < 6; q++) b[q] = __ldcg(t.nbox32 + 6 * x + q);
-        __stcg(t.cost + x, area6(b) + ref_cost(t, w.member[0]) + ref_cost(t, w.member[1]));
+        __syncwarp();
         return;
     }
-    for (int k = 0; k < m; k++) {
-        w.mcost[k] = ref_cost(t, w.member[k]);
-        w.mcount[k] = ref_count(t, w.member[k]);
-        ref_box64(t, w.member[k], w.mb64[k]);
-    }
-    // current cost of the treelet: the old internal nodes' areas + members' costs
-    float old_cost = 0.f;
-    for (int k = 0; k < ni; k++) {
-        float b[6];
-        for (int q = 0; q < 6; q++) b[q] = __ldcg(t.nbox32 + 6 * w.inner[k] + q);
-        old_cost += area6(b);
-    }
-    for (int k = 0; k < m; k++) old_cost += w.mcost[k];
-    w.old_cost = old_cost;
-}
-
-// The whole warp: the best binary tree over the members, by dynamic programming over the member
-// subsets in rounds of growing size (a round reads only smaller subsets). A round's subsets are listed
-// in increasing order and dealt to groups of g lanes (g as large as the count allows: one lane per
-// subset in the crowded rounds, 4 per subset for the 7 subsets of 6 members, all 32 for the full set);
-// the lanes of a group search every g-th split of their subset in the sequential order, and the group
-// keeps the cheapest split, the first in that order among equals -- the sequential search's choice.
-__device__ void treelet_dp(TreeletWork &w, int lane) {
-    constexpr unsigned kAll = 0xffffffffu;
-    const int m = w.m, full = (1 << m) - 1;
-    for (int s = 1 + lane; s <= full; s += 32)
-        if ((s & (s - 1)) == 0) w.c[s] = w.mcost[__ffs(s) - 1], w.split[s] = 0;
-    __syncwarp();
-    for (int size = 2; size <= m; size++) {
-        int nsub = 0;
-        for (int base = 1; base <= full; base += 32) {
-            const int s = base + lane;
-            const bool in = s <= full && __popc(s) == size;
-            const unsigned bal = __ballot_sync(kAll, in);
-            if (in) w.subs[nsub + __popc(bal & ((1u << lane) - 1u))] = (unsigned char)s;
-            nsub += __popc(bal);
+    // areas of all subsets: lane l those of members 2 .. 6 in the bits of l, with and without members 0 and 1
+    {
+        float u[6] = {FLT_MAX, -FLT_MAX, FLT_MAX, -FLT_MAX, FLT_MAX, -FLT_MAX}, e[2][6];
+        for (int k = 0; k < kTreeletLeaves; k++)
+            for (int q = 0; q < 6; q++) {
+                const float v = __shfl_sync(kAll, b[q], k);
+                if (k < 2) e[k][q] = v;
+                else if ((lane >> (k - 2)) & 1) u[q] = (q & 1) ? fmaxf(u[q], v) : fminf(u[q], v);
+            }
+        for (int v = 0; v < 4; v++) {
+            float r[6];
+            for (int q = 0; q < 6; q++) {
+                r[q] = u[q];
+                if (v & 1) r[q] = (q & 1) ? fmaxf(r[q], e[0][q]) : fminf(r[q], e[0][q]);
+                if (v & 2) r[q] = (q & 1) ? fmaxf(r[q], e[1][q]) : fminf(r[q], e[1][q]);
+            }
+            w.area[4 * lane + v] = area6(r);
         }
-        __syncwarp();
-        int g = 1;
-        while (g * 2 * nsub <= 32) g *= 2;
-        const int r = lane & (g - 1);
-        for (int first = 0; first < nsub; first += 32 / g) {
-            const int j = first + lane / g;
-            const int s = j < nsub ? int(w.subs[j]) : 0;
+    }
+    if (lane < m) w.c[1 << lane] = mcost, w.split[1 << lane] = 0;
+    __syncwarp();
+    // sizes in turn (a size reads only smaller subsets): g lanes to a subset, each the splits that agree with its
+    // number in the lowest bits of the subset without its lowest member (each split is met once, by the half
+    // that holds that member); the cheapest wins, the larger half among equals
+    int before = 1, nsub = m;  // C(m, size) from C(m, size - 1)
+    for (int size = 2; size <= m; size++) {
+        nsub = nsub * (m - size + 1) / size;
+        before = kSubsetTable.start[size];
+        int lg = 0;
+        while (lg < size - 1 && (2 << lg) * nsub <= 32) lg++;
+        const int g = 1 << lg, r = lane & (g - 1);
+        for (int first = 0; first < nsub; first += 32 >> lg) {
+            const int j = first + (lane >> lg);
+            const int s = j < nsub ? int(sets[before + j]) : 0;
             float best = FLT_MAX;
-            int bp = 0, bk = 0x7fffffff;
+            int bp = 0;
             if (s) {
-                // partitions (p, s \ p) with p holding the lowest member of s: each split once
                 const int low = s & -s;
-                int k = 0;
-                for (int p = (s - 1) & s; p > 0; p = (p - 1) & s) {
-                    if (!(p & low)) continue;
-                    if ((k & (g - 1)) == r) {
+                int rest = s ^ low, half = low;
+                for (int k = 0; k < lg; k++) {
+                    const int bit = rest & -rest;
+                    rest ^= bit;
+                    if ((r >> k) & 1) half |= bit;
+                }
+                for (int q = rest;; q = (q - 1) & rest) {
+                    const int p = half | q;
+                    if (p != s) {
                         const float v = w.c[p] + w.c[s ^ p];
-                        if (v < best) best = v, bp = p, bk = k;
+                        if (v < best || (v == best && p > bp)) best = v, bp = p;
                     }
-                    k++;
+                    if (q == 0) break;
                 }
             }
             for (int o = 1; o < g; o <<= 1) {
                 const float ob = __shfl_xor_sync(kAll, best, o);
-                const int obp = __shfl_xor_sync(kAll, bp, o), obk = __shfl_xor_sync(kAll, bk, o);
-                if (ob < best || (ob == best && obk < bk)) best = ob, bp = obp, bk = obk;
+                const int obp = __shfl_xor_sync(kAll, bp, o);
+                if (ob < best || (ob == best && obp > bp)) best = ob, bp = obp;
             }
-            if (s && r == 0) {
-                float b[6] = {FLT_MAX, -FLT_MAX, FLT_MAX, -FLT_MAX, FLT_MAX, -FLT_MAX};
-                for (int k = 0; k < m; k++) {
-                    if (!((s >> k) & 1)) continue;
-                    for (int q = 0; q < 6; q += 2)
-                        b[q] = fminf(b[q], w.mb[k][q]), b[q + 1] = fmaxf(b[q + 1], w.mb[k][q + 1]);
-                }
-                w.c[s] = area6(b) + best;
-                w.split[s] = (unsigned char)bp;
-            }
+            if (s && r == 0) w.c[s] = w.area[s] + best, w.split[s] = (unsigned char)bp;
         }
         __syncwarp();
     }
@@ -275,6 +298,9 @@ constexpr int kTreeletThreads = 128;
 // warp-wide votes need every lane) until the whole warp has climbed out.
 __global__ void __launch_bounds__(kTreeletThreads) k_treelets(int n, TreeArrays t, int *arrivals) {
     __shared__ TreeletWork s_work[kTreeletThreads / 32];
+    __shared__ unsigned char s_sets[kSubsets];
+    for (int k = threadIdx.x; k < kSubsets; k += kTreeletThreads) s_sets[k] = kSubsetTable.set[k];
+    __syncthreads();
     TreeletWork &w = s_work[threadIdx.x >> 5];
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -305,10 +331,8 @@ __global__ void __launch_bounds__(kTreeletThreads) k_treelets(int n, TreeArrays 
             const int owner = __ffs(todo) - 1;
             todo &= todo - 1;
             const int x = __shfl_sync(kAll, node, owner);
-            if (lane == owner) form_treelet(t, x, w);
-            __syncwarp();
+            treelet_best(t, x, w, s_sets, lane);
             if (w.m >= 3) {
-                treelet_dp(w, lane);
                 if (lane == owner) rebuild_plan(t, x, w);
                 __syncwarp();
                 rebuild_write(t, w, lane);
@@ -369,20 +393,19 @@ __global__ void k_first_of(int nint, const int *__restrict__ child_l, int *__res
 
 }  // namespace
 
-int treelet_optimize(int n, int *child_l, int *child_r, int *parent_int, int *parent_leaf, int *first_of,
+int treelet_optimize(int n, int *child_l, int *child_r, int *parent_int, int *parent_leaf, int *first_of, int *count,
                      float *nbox32, double *nbox64, const float *pbox32, const double *pbox64, int *sorted_ids,
                      cudaStream_t stream) {
     const int nint = n - 1;
     if (nint < kTreeletLeaves) return SSDF_OK;
     float *cost = nullptr;
-    int *count = nullptr, *arrivals = nullptr, *newpos = nullptr, *ids2 = nullptr, *pl2 = nullptr, *cl2 = nullptr,
+    int *arrivals = nullptr, *newpos = nullptr, *ids2 = nullptr, *pl2 = nullptr, *cl2 = nullptr,
         *cr2 = nullptr;
     int st = SSDF_OK;
     auto alloc = [&](void **p, size_t b) {
         if (st == SSDF_OK && cudaMallocAsync(p, b, stream) != cudaSuccess) st = fail(SSDF_ERR_OUT_OF_MEMORY, "treelet scratch");
     };
     alloc((void **)&cost, sizeof(float) * nint);
-    alloc((void **)&count, sizeof(int) * nint);
     alloc((void **)&arrivals, sizeof(int) * nint);
     alloc((void **)&newpos, sizeof(int) * n);
     alloc((void **)&ids2, sizeof(int) * n);
@@ -418,7 +441,7 @@ int treelet_optimize(int n, int *child_l, int *child_r, int *parent_int, int *pa
         }
         if (e != cudaSuccess) st = cuda_fail(e, "treelet refinement", __FILE__, __LINE__);
     }
-    for (void *p : {(void *)cost, (void *)count, (void *)arrivals, (void *)newpos, (void *)ids2, (void *)pl2,
+    for (void *p : {(void *)cost, (void *)arrivals, (void *)newpos, (void *)ids2, (void *)pl2,
                     (void *)cl2, (void *)cr2})
         if (p) cudaFreeAsync(p, stream);
     return st;
