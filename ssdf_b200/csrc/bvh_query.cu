@@ -920,10 +920,12 @@ __device__ __forceinline__ void query_block(const QueryArgs &a, long long block,
 
 // SIGNAL: the streamed grid download's instantiation, whose blocks count themselves done per chunk
 // (a separate instantiation: the dormant signal code cost the fix-up kernel 3 % where it was merely
-// compiled in).
+// compiled in). The arguments are __grid_constant__: their address is passed on (to query_step,
+// map_query, write_result), and without it each thread first copies them to its local memory (64^3 grid on
+// 5,120 triangles 239 -> 224 us, 262,144 points near the knot 915 -> 889, 1,000 points 48 -> 43).
 template <int PREC, bool WARP, bool COUNT, bool SIGNAL = false>
 __global__ void __launch_bounds__(kThreads, PREC == SSDF_PREC_F64 ? kF64MinBlocks : SSDF_B200_QUERY_MIN_BLOCKS)
-    k_query(const QueryArgs a) {
+    k_query(const __grid_constant__ QueryArgs a) {
     Counters cnt;
     query_block<PREC, WARP, COUNT>(a, blockIdx.x, cnt);
     if (COUNT) flush_counters(a, cnt);
@@ -1194,7 +1196,7 @@ __device__ void window_warp(const QueryArgs &a, int idx, WarpShared &sh, int cap
 // Handed-over queries of one launch, a warp each. `cap` (<= kWinStack) is the shared stack's usable
 // depth: kWinStack, lowered only to test the per-lane subtree walk.
 template <int PREC, bool COUNT>
-__global__ void __launch_bounds__(kThreads) k_window(const QueryArgs a, int cap) {
+__global__ void __launch_bounds__(kThreads) k_window(const __grid_constant__ QueryArgs a, int cap) {
     __shared__ WarpShared s_warp[kThreads / 32];
     const int n = *a.fallback_count;
     const int w = (blockIdx.x * kThreads + threadIdx.x) >> 5, nw = (gridDim.x * kThreads) >> 5;
@@ -1212,7 +1214,7 @@ __global__ void __launch_bounds__(kThreads) k_window(const QueryArgs a, int cap)
 // near the surface; 131,072-triangle knot, 1,280-triangle sphere): 100 points 57 / 244 and 44 / 106; 1,000
 // 59 / 320 and 46 / 98; 16,000 242 / 577 and 162 / 215; 65,536 836 / 620 and 508 / 214.
 template <int PREC, bool COUNT>
-__global__ void __launch_bounds__(kThreads, 6) k_query_warp(const QueryArgs a, int cap) {
+__global__ void __launch_bounds__(kThreads, 6) k_query_warp(const __grid_constant__ QueryArgs a, int cap) {
     __shared__ WarpShared s_warp[kThreads / 32];
     const long long q = (blockIdx.x * (long long)kThreads + threadIdx.x) >> 5;
     if (q >= a.npoints) return;  // a whole warp
