@@ -295,18 +295,23 @@ int ssdf_batch_run(ssdf_batch *b, int use_graph, void *stream_) {
     long long total = 0, total64 = 0, nq = 0, one_step = 0;
     for (auto &j : b->jobs) {
         nq += j.is_grid ? j.nx * j.ny * j.nz : j.npoints;
-        if (j.is_grid) j.grid_steps = 1;
+        if (!j.is_grid) continue;
+        j.grid_steps = 1;
         one_step += query_blocks(j);
     }
-    // the batch fills the GPU as a whole: its grid jobs walk columns of as many steps as its total
-    // work leaves four waves of blocks for
-    const int steps = grid_steps_for(one_step);
+    // A fix-up grid job walks as many steps as it would by itself: the items of a batch are uneven and a
+    // longer column only adds to the last ones' length. Double jobs take two once the batch's grids fill the
+    // GPU. us at 1 / 2 / 4 steps, uneven meshes, their grids' sizes together: 3.1M nodes 2,340 / 2,663 /
+    // 3,459, 10M 4,895 / 5,050 / 5,250, 52M 33,698 / 33,983 / 34,624; double 10M 4,731 / 4,532 / 4,584, 25M
+    // 12,086 / 11,758 / 12,482, 52M 34,647 / 32,825 / 33,032.
+    const int steps64 = std::min(2, grid_steps_for(one_step));
     size_t off = 0;
     int k = 0, k64 = 0;
     for (int r = 0; r < njobs; r++) {
         QueryArgs a = b->jobs[order[r]];
         a.warp_budget = resolve_warp_budget(a.warp_budget, nq, a.m.nt, a.is_grid != 0);
-        if (a.is_grid) a.grid_steps = steps;
+        set_grid_steps(&a);
+        if (a.is_grid && (!fixup || to_f64(a))) a.grid_steps = std::max(a.grid_steps, steps64);
         if (sort_points && !a.is_grid && a.npoints >= kSortMinPoints) {
             int *ord = nullptr;
             SSDF_CHECK(morton_point_order(a.npoints, a.x, a.y, a.z, a.coord_f64, a.m.nodes32, &ord, stream));

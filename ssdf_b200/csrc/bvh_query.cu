@@ -1446,6 +1446,15 @@ __global__ void k_point_keys(long long n, const void *__restrict__ x, const void
     vals[i] = int(i);
 }
 
+// Seeded steps save box and triangle tests, but a column is one serial chain, and its last wave is as long
+// as its steps. Ten waves of resident blocks is where one pays for the other. us at 1 / 2 / 4 / 8 steps,
+// fix-up: 110^3 on 81,920 triangles (10 waves at one step) 1,824 / 2,113 / 2,823 / 3,567; 145^3 (23 waves)
+// 4,109 / 4,013 / 4,947; 200^3 (60) 6,476 / 6,128 / 6,195 / 7,214; torus knot 115^3 (11) 1,982 / 1,924 /
+// 2,329, 145^3 (23) 3,192 / 2,922 / 2,954, 180^3 (44) 5,160 / 4,699 / 4,481, 200^3 (60) 6,574 / 5,945 /
+// 5,563 / 5,575, 256^3 (127) 12,111 / 10,864 / 10,190 / 9,910, 400^3 (483) 38,789 / 34,249 / 31,691 / 30,203;
+// 41,006-triangle torus 150^3 (25) 2,417 / 2,625 / 2,994, 256^3 7,658 / 7,461 / 7,430 / 7,618.
+constexpr long long kGridWaves = 10;
+
 int grid_steps_for(long long one_step_blocks) {
     const int forced = env_int("SSDF_B200_GRID_STEPS", 0);
     if (forced > 0) return forced < kMaxGridSteps ? forced : kMaxGridSteps;
@@ -1458,8 +1467,8 @@ int grid_steps_for(long long one_step_blocks) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         r = std::max(1, sms) * SSDF_B200_QUERY_MIN_BLOCKS;
     }
-    int steps = kDefaultGridSteps;
-    while (steps > 1 && one_step_blocks / steps < 4ll * r) steps >>= 1;
+    int steps = kMaxGridSteps;
+    while (steps > 1 && one_step_blocks / steps < kGridWaves * r) steps >>= 1;
     return steps;
 }
 

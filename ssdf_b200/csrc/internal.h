@@ -224,10 +224,9 @@ constexpr int kQ = SSDF_B200_QUERIES_PER_LANE;
 // QueryArgs::grid_steps steps (1 .. kMaxGridSteps) of 4 kQ z-planes, each step an 8 x 4 x 4kQ brick
 // of nodes (each warp a 4 x 4 x 2kQ part of it). A lane starts each step from the closest triangle it
 // found one step below, 4 kQ nodes away: a tight upper bound (SSDF_B200_SEED=0 starts from the
-// incoming bound alone). Large grids take kDefaultGridSteps; a grid too small to fill the GPU with
-// such columns takes fewer (grid_steps_for).
-constexpr int kMaxGridSteps = 8;      // the most SSDF_B200_GRID_STEPS may ask for
-constexpr int kDefaultGridSteps = 4;   // the most the launch rule picks
+// incoming bound alone). Large grids take kMaxGridSteps; a grid too small to fill the GPU many times
+// over with such columns takes fewer (grid_steps_for).
+constexpr int kMaxGridSteps = 8;
 __host__ __device__ inline long long grid_blocks_x(long long nx) { return (nx + 7) / 8; }
 __host__ __device__ inline long long grid_blocks_y(long long ny) { return (ny + 3) / 4; }
 __host__ __device__ inline long long grid_block_planes(int steps) { return 4ll * kQ * steps; }
@@ -241,7 +240,7 @@ inline long long query_blocks(const QueryArgs &a) {
     return (a.npoints + 128 * kQ - 1) / (128 * kQ);
 }
 // Steps per grid block for a launch whose work, at one step per block, is `one_step_blocks` blocks:
-// the most steps (up to kMaxGridSteps) that still leave four waves of resident blocks on this
+// the most steps (1, 2, 4 or kMaxGridSteps) that still leave ten waves of resident blocks on this
 // device (SSDF_B200_GRID_STEPS overrides). bvh_query.cu.
 int grid_steps_for(long long one_step_blocks);
 // Sets QueryArgs::grid_steps of a grid job from its own size (no-op for point lists).
