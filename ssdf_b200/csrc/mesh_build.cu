@@ -576,7 +576,9 @@ __device__ __forceinline__ void frame_corners(const float4 *__restrict__ t32, co
 // up to seven of the child's triangles with one of its edges, or the sum of the triangles' normals with an
 // edge -- and projects every corner on it; the frame of least half surface area wins (the summed normal
 // often does: with triangle normals alone the torus knot keeps 75 triangle iterations a packet, not 52).
-// Bound by the triangle records' loads, read once per level of up to kObbMaxTris triangles.
+// Bound by issue: 45 operations a triangle and candidate. The corners are taken into the box frame once, a
+// triangle a lane, and shared from there: with every lane converting every triangle's doubles the FP64
+// conversions bound it (41,006 / 131,072 triangles: 68 -> 43 us, 186 -> 126).
 __global__ void __launch_bounds__(128) k_obb(int nnodes, int L, const int *__restrict__ count,
                                              const int *__restrict__ first_of, const double *__restrict__ pbox64,
                                              const double *__restrict__ nbox64, const int *__restrict__ sorted_ids,
@@ -584,6 +586,12 @@ __global__ void __launch_bounds__(128) k_obb(int nnodes, int L, const int *__res
                                              const double2 *__restrict__ t64, const int *__restrict__ frame,
                                              float *__restrict__ obb) {
     constexpr unsigned kAll = 0xffffffffu;
+    __shared__ float4 s_corners[4][3 * kObbMaxTris];  // a warp's child: v0 v1.x, v1.yz v2.xy, v2.z
+    float4 *const corners = s_corners[threadIdx.x >> 5];
+    auto shared_corners = [&](int t, Vec3(&v)[3]) {
+        const float4 a = corners[3 * t], b = corners[3 * t + 1];
+        v[0] = {a.x, a.y, a.z}, v[1] = {a.w, b.x, b.y}, v[2] = {b.z, b.w, corners[3 * t + 2].x};
+    };
     const long long w = (blockIdx.x * 128ll + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const int i = int(w >> 1), h = int(w & 1);
@@ -610,6 +618,9 @@ __global__ void __launch_bounds__(128) k_obb(int nnodes, int L, const int *__res
             for (int t = lane; t < n; t += 32) {
                 Vec3 v[3];
                 frame_corners(t32, t64, first + t, mid, scale, v);
+                corners[3 * t] = make_float4(v[0].x, v[0].y, v[0].z, v[1].x);
+                corners[3 * t + 1] = make_float4(v[1].y, v[1].z, v[2].x, v[2].y);
+                corners[3 * t + 2].x = v[2].z;
                 const Vec3 e1 = vsub(v[1], v[0]), e2 = vsub(v[2], v[0]), e3 = vsub(v[2], v[1]);
                 const Vec3 c = vcross(e1, e2);
                 const float l2 = fmaxf(vdot(e1, e1), fmaxf(vdot(e2, e2), vdot(e3, e3)));
@@ -626,6 +637,7 @@ __global__ void __launch_bounds__(128) k_obb(int nnodes, int L, const int *__res
                 ns.y += __shfl_xor_sync(kAll, ns.y, o);
                 ns.z += __shfl_xor_sync(kAll, ns.z, o);
             }
+            __syncwarp();
         }
         if (small && alpha <= kObbMaxAlpha) {
             // this lane's frame
@@ -636,7 +648,7 @@ __global__ void __launch_bounds__(128) k_obb(int nnodes, int L, const int *__res
             ax[0] = {1.f, 0.f, 0.f}, ax[1] = {0.f, 1.f, 0.f}, ax[2] = {0.f, 0.f, 1.f};
             if (lane > 0 && lane < 31 && j < nsample) {
                 Vec3 v[3];
-                frame_corners(t32, t64, first + (j * n) / nsample, mid, scale, v);
+                shared_corners((j * n) / nsample, v);
                 const Vec3 edge = e == 0 ? vsub(v[1], v[0]) : (e == 1 ? vsub(v[2], v[0]) : vsub(v[2], v[1]));
                 Vec3 c = summed ? ns : vcross(vsub(v[1], v[0]), vsub(v[2], v[0]));
                 const float rc = rsqrtf(vdot(c, c));
@@ -656,11 +668,11 @@ __global__ void __launch_bounds__(128) k_obb(int nnodes, int L, const int *__res
                 if (ok) ax[0] = d, ax[1] = f, ax[2] = c;
             }
             Vec3 o[3];
-            frame_corners(t32, t64, first, mid, scale, o);
+            shared_corners(0, o);
             float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
             for (int t = 0; t < n; t++) {
                 Vec3 v[3];
-                frame_corners(t32, t64, first + t, mid, scale, v);
+                shared_corners(t, v);
 #pragma unroll
                 for (int k = 0; k < 3; k++) {
                     const Vec3 q = vsub(v[k], o[0]);
