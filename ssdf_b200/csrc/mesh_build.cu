@@ -181,45 +181,140 @@ __global__ void k_karras(int n, const uint32_t *__restrict__ k, int *__restrict_
     if (i == 0) parent_int[0] = -1;
 }
 
-// Bottom-up refit: the second thread to reach a node unions its two children's boxes.
-__global__ void k_refit(int n, const int *__restrict__ sorted_ids, const int *__restrict__ child_l,
-                        const int *__restrict__ child_r, const int *__restrict__ parent_int,
-                        const int *__restrict__ parent_leaf, const float *__restrict__ pbox32,
-                        const double *__restrict__ pbox64, float *nbox32, double *nbox64, int *arrivals) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    int node = parent_leaf[p];
+// Node boxes. Every box is a union of leaves' boxes, and minima and maxima come out the same in any order, so
+// nothing has to climb the tree through L2 (with one thread a leaf that did, an arrival counter and a box
+// load a level, the deepest path took 40 to 75 us). A block of k_boxes_inside has the subtrees inside its
+// kRefitBlock leaves to itself and climbs them in shared memory (a node's index lies in its range of
+// leaves); it also unites its leaves by 32 and all together. k_boxes_across gives each of the remaining nodes,
+// whose leaves lie in several blocks, a warp: the leaves at the range's ends one by one, then by 32, the
+// blocks between them whole. Bound by latency: three dependent loads and a union over the warp, a node at a
+// time; a warp looks through kAcrossNodes nodes (131,072 triangles: 27 us with 32, 14 with 8, 19 with 2).
+// Together 16 / 20 / 27 / 33 us instead of 40 / 55 / 63 / 75 at 5,120 / 41,006 / 81,920 / 131,072 triangles.
+constexpr int kRefitBlock = 256, kRuns = kRefitBlock / 32, kAcrossNodes = 8;
+
+// A box as three (min, max) pairs, 24 and 48 bytes: aligned for two-element loads.
+struct Boxes {
+    float2 f[3];
+    double2 d[3];
+};
+__device__ __forceinline__ void clear_box(Boxes &b) {
+#pragma unroll
+    for (int k = 0; k < 3; k++) b.f[k] = make_float2(FLT_MAX, -FLT_MAX), b.d[k] = make_double2(DBL_MAX, -DBL_MAX);
+}
+__device__ __forceinline__ void add_pair(Boxes &b, int k, float2 x, double2 y) {
+    b.f[k] = make_float2(fminf(b.f[k].x, x.x), fmaxf(b.f[k].y, x.y));
+    b.d[k] = make_double2(fmin(b.d[k].x, y.x), fmax(b.d[k].y, y.y));
+}
+__device__ __forceinline__ void add_box(Boxes &b, const Boxes &o) {
+#pragma unroll
+    for (int k = 0; k < 3; k++) add_pair(b, k, o.f[k], o.d[k]);
+}
+__device__ __forceinline__ void add_box(Boxes &b, const float *f, const double *d, size_t i) {
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        add_pair(b, k, __ldg(reinterpret_cast<const float2 *>(f + 6 * i) + k),
+                 __ldg(reinterpret_cast<const double2 *>(d + 6 * i) + k));
+}
+__device__ __forceinline__ void store_box(const Boxes &b, float *f, double *d, size_t i) {
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        reinterpret_cast<float2 *>(f + 6 * i)[k] = b.f[k];
+        reinterpret_cast<double2 *>(d + 6 * i)[k] = b.d[k];
+    }
+}
+// Union over the warp, in every lane.
+__device__ __forceinline__ void warp_union(Boxes &b) {
+    constexpr unsigned kAll = 0xffffffffu;
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const float2 x = make_float2(__shfl_xor_sync(kAll, b.f[k].x, o), __shfl_xor_sync(kAll, b.f[k].y, o));
+            const double2 y = make_double2(__shfl_xor_sync(kAll, b.d[k].x, o), __shfl_xor_sync(kAll, b.d[k].y, o));
+            add_pair(b, k, x, y);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kRefitBlock)
+    k_boxes_inside(int n, const int *__restrict__ sorted_ids, const int *__restrict__ child_l,
+                   const int *__restrict__ child_r, const int *__restrict__ parent_int,
+                   const int *__restrict__ parent_leaf, const int *__restrict__ first_of,
+                   const int *__restrict__ count, const float *__restrict__ pbox32,
+                   const double *__restrict__ pbox64, float *__restrict__ nbox32, double *__restrict__ nbox64,
+                   float *__restrict__ run32, double *__restrict__ run64, float *__restrict__ block32,
+                   double *__restrict__ block64) {
+    __shared__ int s_arrivals[kRefitBlock], s_left[kRefitBlock], s_right[kRefitBlock], s_parent[kRefitBlock];
+    __shared__ Boxes s_leaf[kRefitBlock], s_box[kRefitBlock];
+    constexpr int kElsewhere = 1 << 30;  // arrivals of a node with leaves in other blocks
+    const int base = blockIdx.x * kRefitBlock, tid = threadIdx.x, p = base + tid;
+    bool mine = false;  // node p has all its leaves in this block
+    if (p < n - 1) {
+        s_left[tid] = child_l[p], s_right[tid] = child_r[p], s_parent[tid] = parent_int[p];
+        const int first = first_of[p] - base;
+        mine = first >= 0 && first + count[p] <= kRefitBlock;
+    }
+    s_arrivals[tid] = mine ? 0 : kElsewhere;
+    Boxes own, all;
+    clear_box(own);
+    if (p < n) add_box(own, pbox32, pbox64, sorted_ids[p]);
+    s_leaf[tid] = own;
+    all = own;
+    warp_union(all);
+    if ((tid & 31) == 0 && p < n) store_box(all, run32, run64, p >> 5);
+    __syncthreads();
+    int node = p < n ? parent_leaf[p] : -1, self = -p - 1;
     while (node >= 0) {
-        __threadfence();
-        if (atomicAdd(&arrivals[node], 1) == 0) return;
-        __threadfence();
-        const int c[2] = {child_l[node], child_r[node]};
-        float b32[6];
-        double b64[6];
-        for (int k = 0; k < 6; k++) b32[k] = (k & 1) ? -FLT_MAX : FLT_MAX, b64[k] = (k & 1) ? -DBL_MAX : DBL_MAX;
-        for (int h = 0; h < 2; h++) {
-            const float *s32;
-            const double *s64;
-            if (c[h] < 0) {
-                const int prim = sorted_ids[-c[h] - 1];
-                s32 = pbox32 + 6 * prim;
-                s64 = pbox64 + 6 * prim;
-            } else {
-                s32 = nbox32 + 6 * c[h];
-                s64 = nbox64 + 6 * c[h];
-            }
-            for (int k = 0; k < 6; k += 2) {
-                b32[k] = fminf(b32[k], __ldcg(s32 + k));
-                b32[k + 1] = fmaxf(b32[k + 1], __ldcg(s32 + k + 1));
-                b64[k] = fmin(b64[k], __ldcg(s64 + k));
-                b64[k + 1] = fmax(b64[k + 1], __ldcg(s64 + k + 1));
-            }
-        }
-        for (int k = 0; k < 6; k++) {
-            __stcg(nbox32 + 6 * node + k, b32[k]);
-            __stcg(nbox64 + 6 * node + k, b64[k]);
-        }
-        node = parent_int[node];
+        const int at = node - base;
+        if (at < 0 || at >= kRefitBlock || s_arrivals[at] >= kElsewhere) break;
+        const int l = s_left[at], r = s_right[at], other = l == self ? r : l;
+        __threadfence_block();
+        if (atomicAdd(&s_arrivals[at], 1) == 0) break;  // the second child to arrive goes on
+        __threadfence_block();
+        add_box(own, other < 0 ? s_leaf[-other - 1 - base] : s_box[other - base]);
+        s_box[at] = own;
+        self = node;
+        node = s_parent[at];
+    }
+    __syncthreads();
+    if (mine) store_box(s_box[tid], nbox32, nbox64, p);
+    __syncthreads();
+    if ((tid & 31) == 0) s_box[tid >> 5] = all;
+    __syncthreads();
+    if (tid < 32) {
+        clear_box(all);
+        if (tid < kRefitBlock / 32) add_box(all, s_box[tid]);
+        warp_union(all);
+        if (tid == 0) store_box(all, block32, block64, blockIdx.x);
+    }
+}
+
+__global__ void __launch_bounds__(128)
+    k_boxes_across(int n, const int *__restrict__ sorted_ids, const int *__restrict__ first_of,
+                   const int *__restrict__ count, const float *__restrict__ pbox32,
+                   const double *__restrict__ pbox64, const float *__restrict__ run32,
+                   const double *__restrict__ run64, const float *__restrict__ block32,
+                   const double *__restrict__ block64, float *__restrict__ nbox32, double *__restrict__ nbox64) {
+    // nodes a warp count apart: such nodes' indices cluster at the blocks' edges
+    const int lane = threadIdx.x & 31, warps = int(gridDim.x * 4);
+    const int i = lane < kAcrossNodes ? lane * warps + int(blockIdx.x * 4 + (threadIdx.x >> 5)) : n;
+    int first = 0, end = 0;
+    if (i < n - 1) first = first_of[i], end = first + count[i];
+    unsigned todo = __ballot_sync(0xffffffffu, i < n - 1 && first / kRefitBlock != (end - 1) / kRefitBlock);
+    for (; todo; todo &= todo - 1) {  // warp-uniform
+        const int from = __ffs(int(todo)) - 1;
+        const int f = __shfl_sync(0xffffffffu, first, from), e = __shfl_sync(0xffffffffu, end, from);
+        const int b0 = (f + kRefitBlock - 1) / kRefitBlock, b1 = e / kRefitBlock;  // whole blocks [b0, b1)
+        Boxes b;
+        clear_box(b);
+        const int r0 = (f + 31) / 32, r1 = e / 32;  // whole runs of 32 leaves [r0, r1)
+        if (f + lane < r0 * 32) add_box(b, pbox32, pbox64, sorted_ids[f + lane]);
+        if (r1 * 32 + lane < e) add_box(b, pbox32, pbox64, sorted_ids[r1 * 32 + lane]);
+        if (r0 + lane < b0 * kRuns) add_box(b, run32, run64, r0 + lane);
+        if (b1 * kRuns + lane < r1) add_box(b, run32, run64, b1 * kRuns + lane);
+#pragma unroll 4
+        for (int q = b0 + lane; q < b1; q += 32) add_box(b, block32, block64, q);
+        warp_union(b);
+        if (lane == from) store_box(b, nbox32, nbox64, i);
     }
 }
 
@@ -997,7 +1092,7 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
         k_write_small_root<<<1, 1, 0, stream>>>(nt, box32, nodes32);
         LAUNCH_CHECK("k_write_small_root");
     } else {
-        int *child_l, *child_r, *first_of, *parent_int, *parent_leaf, *arrivals, *count;
+        int *child_l, *child_r, *first_of, *parent_int, *parent_leaf, *count;
         float *nbox32;
         double *nbox64;
         SSDF_CHECK(dalloc(tmp, &child_l, nint, stream));
@@ -1005,17 +1100,26 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
         SSDF_CHECK(dalloc(tmp, &first_of, nint, stream));
         SSDF_CHECK(dalloc(tmp, &parent_int, nint, stream));
         SSDF_CHECK(dalloc(tmp, &parent_leaf, nt, stream));
-        SSDF_CHECK(dalloc(tmp, &arrivals, nint, stream));
         SSDF_CHECK(dalloc(tmp, &count, nint, stream));
         SSDF_CHECK(dalloc(tmp, &nbox32, 6 * size_t(nint), stream));
         SSDF_CHECK(dalloc(tmp, &nbox64, 6 * size_t(nint), stream));
         k_karras<<<grid_blocks(nint, 256), 256, 0, stream>>>(nt, keys, child_l, child_r, first_of, count,
                                                              parent_int, parent_leaf);
         LAUNCH_CHECK("k_karras");
-        SSDF_CUDA(cudaMemsetAsync(arrivals, 0, sizeof(int) * nint, stream));
-        k_refit<<<grid_blocks(nt, 256), 256, 0, stream>>>(nt, ids, child_l, child_r, parent_int, parent_leaf, box32,
-                                                          box64, nbox32, nbox64, arrivals);
-        LAUNCH_CHECK("k_refit");
+        const unsigned blocks = grid_blocks(nt, kRefitBlock);
+        float *run32, *block32;
+        double *run64, *block64;
+        SSDF_CHECK(dalloc(tmp, &run32, 6 * size_t(kRuns) * blocks, stream));
+        SSDF_CHECK(dalloc(tmp, &run64, 6 * size_t(kRuns) * blocks, stream));
+        SSDF_CHECK(dalloc(tmp, &block32, 6 * size_t(blocks), stream));
+        SSDF_CHECK(dalloc(tmp, &block64, 6 * size_t(blocks), stream));
+        k_boxes_inside<<<blocks, kRefitBlock, 0, stream>>>(nt, ids, child_l, child_r, parent_int, parent_leaf, first_of,
+                                                           count, box32, box64, nbox32, nbox64, run32, run64, block32,
+                                                           block64);
+        LAUNCH_CHECK("k_boxes_inside");
+        k_boxes_across<<<grid_blocks(nint, 4 * kAcrossNodes), 128, 0, stream>>>(nt, ids, first_of, count, box32, box64, run32,
+                                                                   run64, block32, block64, nbox32, nbox64);
+        LAUNCH_CHECK("k_boxes_across");
         for (int round = 0; round < opts.treelet_opt && round < 8; round++) {  // treelet_opt: rounds (0 = none)
             SSDF_CHECK(treelet_optimize(nt, child_l, child_r, parent_int, parent_leaf, first_of, count, nbox32, nbox64,
                                         box32, box64, ids, stream));
