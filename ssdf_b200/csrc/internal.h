@@ -305,7 +305,7 @@ int round_device(const GridDesc &gd, const T *d_f, T radius, T band, bool open, 
 // current kernels, queries against 1 round: beam lattice (8e6 points + 512^3 grid, float) 335.6 ->
 // 313.1 / 308.7 / 304.8 ms for 2 / 3 / 4 rounds; torus knot 256^3 16.70 -> 16.63 ms (3); 64^3
 // icosphere 0.470 -> 0.465 ms; the serving leg's heaviest grid 3.74 -> 3.67 ms. Each round adds
-// 0.45 ms to the torus knot's build, which calls that build per query do not repay
+// 0.3 ms to the torus knot's build, which calls that build per query do not repay
 // (call_treelet_rounds).
 constexpr int kResidentTreeletRounds = 3;
 

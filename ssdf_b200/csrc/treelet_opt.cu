@@ -58,7 +58,6 @@ __device__ __forceinline__ float ref_cost(const TreeArrays &t, int ref) {
     ref_box32(t, ref, b);
     return area6(b);
 }
-__device__ __forceinline__ int ref_count(const TreeArrays &t, int ref) { return ref >= 0 ? __ldcg(t.count + ref) : 1; }
 
 __device__ __forceinline__ void set_parent(const TreeArrays &t, int ref, int parent) {
     if (ref >= 0)
@@ -75,18 +74,17 @@ struct TreeletWork {
     int mcount[kTreeletLeaves];
     int member[kTreeletLeaves];
     int inner[kTreeletLeaves - 1];
-    int m;
     float old_cost;
     float area[kSubsets];
     float c[kSubsets];
     unsigned char split[kSubsets];
     // the rebuilt arrangement: internal node onode[k] now covers the members of subset oset[k]
     int onode[kTreeletLeaves - 1], oset[kTreeletLeaves - 1];
+    int2 oref[kTreeletLeaves - 1], stack[kTreeletLeaves];
     int norder;
 };
 
-// The subsets of seven members by size, each size in increasing order (so those of the first m members come
-// first), and where each size starts.
+// The subsets of seven members by size, each size in increasing order, and where each size starts.
 struct SubsetTable {
     unsigned char set[kSubsets];
     int start[kTreeletLeaves + 2];
@@ -107,58 +105,105 @@ constexpr SubsetTable make_subsets() {
 }
 __constant__ SubsetTable kSubsetTable = make_subsets();
 
-// The whole warp: the treelet rooted at internal node x (its subtree is final), grown from its two children by
-// opening the largest-area internal member until it has seven members, a lane to each; then the best
-// binary tree over them, by dynamic programming over the member subsets. One lane growing the treelet
-// waited 22,000 cycles, a programme searching every second submask in vain 46,000 more: a round on a 65,536-
-// triangle torus takes 416 us with a lane per member and per subset, 1,111 before, for the same tree. A treelet of fewer than three members only gets its cost stored (w.m < 3).
+// The best split of every subset of SIZE members, from the smaller subsets' costs: 2^LG lanes to
+// a subset, each the splits that agree with its number in the lowest bits of the subset without its lowest
+// member (each split is met once, by the half that holds that member); the cheapest wins, the larger half
+// among equals. Sizes and counts are constants, so a lane's costs are all asked for at once.
+constexpr int choose(int n, int k) { return k == 0 ? 1 : choose(n - 1, k - 1) * n / k; }
+constexpr int lanes_log(int size, int nsub) {
+    int lg = 0;
+    while (lg < size - 1 && (2 << lg) * nsub <= 32) lg++;
+    return lg;
+}
+template <int SIZE>
+__device__ __forceinline__ void best_splits(TreeletWork &w, const unsigned char *__restrict__ sets, int lane) {
+    constexpr int kSub = choose(kTreeletLeaves, SIZE), kLg = lanes_log(SIZE, kSub), kTrips = 1 << (SIZE - 1 - kLg);
+    const int before = kSubsetTable.start[SIZE], r = lane & ((1 << kLg) - 1);
+#pragma unroll
+    for (int first = 0; first < kSub; first += 32 >> kLg) {
+        const int j = first + (lane >> kLg);
+        const int s = j < kSub ? int(sets[before + j]) : 0;
+        float best = FLT_MAX;
+        int bp = 0;
+        if (s) {
+            const int low = s & -s;
+            int rest = s ^ low, half = low;
+#pragma unroll
+            for (int k = 0; k < kLg; k++) {
+                const int bit = rest & -rest;
+                rest ^= bit;
+                if ((r >> k) & 1) half |= bit;
+            }
+            int q = rest;
+#pragma unroll
+            for (int k = 0; k < kTrips; k++) {
+                const int p = half | q;
+                if (p != s) {
+                    const float v = w.c[p] + w.c[s ^ p];
+                    if (v < best || (v == best && p > bp)) best = v, bp = p;
+                }
+                q = (q - 1) & rest;
+            }
+        }
+#pragma unroll
+        for (int o = 1; o < (1 << kLg); o <<= 1) {
+            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+            const int obp = __shfl_xor_sync(0xffffffffu, bp, o);
+            if (ob < best || (ob == best && obp > bp)) best = ob, bp = obp;
+        }
+        if (s && r == 0) w.c[s] = w.area[s] + best, w.split[s] = (unsigned char)bp;
+    }
+    __syncwarp();
+}
+
+// The whole warp: the treelet rooted at internal node x (its subtree is final, of kTreeletLeaves triangles or
+// more), grown from its two children by opening the largest-area internal member until it has seven members,
+// a lane to each; then the best binary tree over them, by dynamic programming over the member subsets. Bound by
+// latency, one treelet after the other up the tree's deepest path: a member's lane asks for its children's
+// links together with its box, so an opening waits once, and the programme's sizes are unrolled (11,100 cycles
+// as loops, two reads at a time). A round on 5,120 / 41,006 / 81,920 / 131,072 triangles takes 154 / 230 /
+// 277 / 331 us, 283 / 394 / 455 / 500 with the loops, two waits an opening and 32 climbers a warp.
 __device__ void treelet_best(const TreeArrays &t, int x, TreeletWork &w, const unsigned char *__restrict__ sets,
                              int lane) {
     constexpr unsigned kAll = 0xffffffffu;
-    float bx[6], b[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    float bx[6], b[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, mcost = 0.f;
+    double d[6];
+    int ref = -1, cl = 0, cr = 0, mcount = 1;
+    // everything an internal member will be asked for, its children for the case that it is opened among it
+    auto take = [&](int r) {
+        ref = r;
+        if (r < 0) return;
+        cl = __ldcg(t.child_l + r), cr = __ldcg(t.child_r + r);
+        ref_box32(t, r, b);
+        ref_box64(t, r, d);
+        mcost = __ldcg(t.cost + r), mcount = __ldcg(t.count + r);
+    };
     for (int q = 0; q < 6; q++) bx[q] = __ldcg(t.nbox32 + 6 * x + q);
-    int ref = -1;
-    if (lane < 2) {
-        ref = __ldcg((lane ? t.child_r : t.child_l) + x);
-        ref_box32(t, ref, b);
-    }
+    if (lane < 2) take(__ldcg((lane ? t.child_r : t.child_l) + x));
     float old_cost = area6(bx);  // the old internal nodes' areas, then the members' costs
     if (lane == 0) w.inner[0] = x;
-    int m = 2;
-    while (m < kTreeletLeaves) {
+    for (int m = 2; m < kTreeletLeaves; m++) {  // with kTreeletLeaves triangles below x, one is internal
         const int key = lane < m && ref >= 0 ? __float_as_int(area6(b)) : -1;  // areas are not negative
         const int best = __reduce_max_sync(kAll, key);
-        if (best < 0) break;
         const int pick = __ffs(__ballot_sync(kAll, key == best)) - 1;
-        const int y = __shfl_sync(kAll, ref, pick);
+        const int y = __shfl_sync(kAll, ref, pick), l = __shfl_sync(kAll, cl, pick), r = __shfl_sync(kAll, cr, pick);
         old_cost += __int_as_float(best);
         if (lane == 0) w.inner[m - 1] = y;
-        if (lane == pick || lane == m) {
-            ref = __ldcg((lane == pick ? t.child_l : t.child_r) + y);
-            ref_box32(t, ref, b);
-        }
-        m++;
+        if (lane == pick || lane == m) take(lane == pick ? l : r);
     }
-    float mcost = 0.f;
-    if (lane < m) {
-        mcost = ref_cost(t, ref);
+    if (lane < kTreeletLeaves) {
+        if (ref < 0) {  // triangles: only now, so that no opening waited for them
+            ref_box32(t, ref, b);
+            ref_box64(t, ref, d);
+            mcost = area6(b), mcount = 1;
+        }
         w.member[lane] = ref;
-        w.mcount[lane] = ref_count(t, ref);
+        w.mcount[lane] = mcount;
         for (int q = 0; q < 6; q++) w.mb[lane][q] = b[q];
-        double d[6];
-        ref_box64(t, ref, d);
         for (int q = 0; q < 6; q++) w.mb64[lane][q] = d[q];
     }
-    for (int k = 0; k < m; k++) old_cost += __shfl_sync(kAll, mcost, k);
-    if (lane == 0) {
-        w.m = m;
-        w.old_cost = old_cost;
-        if (m < 3) __stcg(t.cost + x, old_cost);
-    }
-    if (m < 3) {
-        __syncwarp();
-        return;
-    }
+    for (int k = 0; k < kTreeletLeaves; k++) old_cost += __shfl_sync(kAll, mcost, k);
+    if (lane == 0) w.old_cost = old_cost;
     // areas of all subsets: lane l those of members 2 .. 6 in the bits of l, with and without members 0 and 1
     {
         float u[6] = {FLT_MAX, -FLT_MAX, FLT_MAX, -FLT_MAX, FLT_MAX, -FLT_MAX}, e[2][6];
@@ -178,99 +223,63 @@ __device__ void treelet_best(const TreeArrays &t, int x, TreeletWork &w, const u
             w.area[4 * lane + v] = area6(r);
         }
     }
-    if (lane < m) w.c[1 << lane] = mcost, w.split[1 << lane] = 0;
+    if (lane < kTreeletLeaves) w.c[1 << lane] = mcost, w.split[1 << lane] = 0;
     __syncwarp();
-    // sizes in turn (a size reads only smaller subsets): g lanes to a subset, each the splits that agree with its
-    // number in the lowest bits of the subset without its lowest member (each split is met once, by the half
-    // that holds that member); the cheapest wins, the larger half among equals
-    int before = 1, nsub = m;  // C(m, size) from C(m, size - 1)
-    for (int size = 2; size <= m; size++) {
-        nsub = nsub * (m - size + 1) / size;
-        before = kSubsetTable.start[size];
-        int lg = 0;
-        while (lg < size - 1 && (2 << lg) * nsub <= 32) lg++;
-        const int g = 1 << lg, r = lane & (g - 1);
-        for (int first = 0; first < nsub; first += 32 >> lg) {
-            const int j = first + (lane >> lg);
-            const int s = j < nsub ? int(sets[before + j]) : 0;
-            float best = FLT_MAX;
-            int bp = 0;
-            if (s) {
-                const int low = s & -s;
-                int rest = s ^ low, half = low;
-                for (int k = 0; k < lg; k++) {
-                    const int bit = rest & -rest;
-                    rest ^= bit;
-                    if ((r >> k) & 1) half |= bit;
-                }
-                for (int q = rest;; q = (q - 1) & rest) {
-                    const int p = half | q;
-                    if (p != s) {
-                        const float v = w.c[p] + w.c[s ^ p];
-                        if (v < best || (v == best && p > bp)) best = v, bp = p;
-                    }
-                    if (q == 0) break;
-                }
-            }
-            for (int o = 1; o < g; o <<= 1) {
-                const float ob = __shfl_xor_sync(kAll, best, o);
-                const int obp = __shfl_xor_sync(kAll, bp, o);
-                if (ob < best || (ob == best && obp > bp)) best = ob, bp = obp;
-            }
-            if (s && r == 0) w.c[s] = w.area[s] + best, w.split[s] = (unsigned char)bp;
-        }
-        __syncwarp();
-    }
+    best_splits<2>(w, sets, lane);
+    best_splits<3>(w, sets, lane);
+    best_splits<4>(w, sets, lane);
+    best_splits<5>(w, sets, lane);
+    best_splits<6>(w, sets, lane);
+    best_splits<7>(w, sets, lane);
 }
 
-// One lane: replaces the treelet's arrangement by the programme's when it is cheaper, reusing the
-// treelet's internal nodes (the root keeps x): child and parent links top-down, and in w.onode /
-// w.oset which members each reused node now covers (w.norder of them; 0 when the old arrangement
-// stays, whose cost is stored here).
+// One lane: the arrangement by the programme's splits when it is cheaper, reusing the treelet's internal nodes
+// (the root keeps x): in w.onode / w.oset / w.oref the reused nodes, the members each now covers and its two
+// children (w.norder of them; 0 when the old arrangement stays, whose cost is stored here).
 __device__ void rebuild_plan(const TreeArrays &t, int x, TreeletWork &w) {
-    const int m = w.m, full = (1 << m) - 1;
+    constexpr int full = kSubsets - 1;
     w.norder = 0;
     if (!(w.c[full] < w.old_cost * (1.f - 1e-6f))) {
         __stcg(t.cost + x, w.old_cost);
         return;
     }
-    int stack_set[kTreeletLeaves], stack_node[kTreeletLeaves];
     int sp = 0, used = 1, norder = 0;
-    stack_set[sp] = full, stack_node[sp] = x, sp++;
+    w.stack[sp++] = make_int2(full, x);
     while (sp > 0) {
-        sp--;
-        const int s = stack_set[sp], node = stack_node[sp];
-        w.onode[norder] = node, w.oset[norder] = s, norder++;
-        const int halves[2] = {w.split[s], s ^ w.split[s]};
+        const int2 top = w.stack[--sp];
+        const int split = w.split[top.x];
+        const int halves[2] = {split, top.x ^ split};
         int refs[2];
+#pragma unroll
         for (int h = 0; h < 2; h++) {
             const int hs = halves[h];
-            if ((hs & (hs - 1)) == 0) {
-                refs[h] = w.member[__ffs(hs) - 1];
-            } else {
-                refs[h] = w.inner[used++];
-                stack_set[sp] = hs, stack_node[sp] = refs[h], sp++;
-            }
+            const bool single = (hs & (hs - 1)) == 0;
+            refs[h] = single ? w.member[__ffs(hs) - 1] : w.inner[used];
+            if (!single) w.stack[sp++] = make_int2(hs, refs[h]), used++;
         }
-        __stcg(t.child_l + node, refs[0]);
-        __stcg(t.child_r + node, refs[1]);
-        set_parent(t, refs[0], node);
-        set_parent(t, refs[1], node);
+        w.onode[norder] = top.y, w.oset[norder] = top.x;
+        w.oref[norder++] = make_int2(refs[0], refs[1]);
     }
     w.norder = norder;
 }
 
-// The whole warp, after rebuild_plan: lane k writes reused node w.onode[k]'s boxes (float and double),
-// triangle count and cost. A node's box is the union of its members' boxes -- the same values the
-// union of its two children's boxes gives, min and max being exact -- so no lane waits for another.
+// The whole warp, after rebuild_plan: lane k writes reused node w.onode[k]'s child and parent links, boxes
+// (float and double), triangle count and cost. A node's box is the union of its members' boxes -- the same
+// values the union of its two children's boxes gives, min and max being exact -- so no lane waits for
+// another. The owner's fence before its next arrival, after the warp's barrier, publishes every lane's stores.
 __device__ void rebuild_write(const TreeArrays &t, const TreeletWork &w, int lane) {
     if (lane >= w.norder) return;
     const int node = w.onode[lane], s = w.oset[lane];
+    const int2 refs = w.oref[lane];
+    __stcg(t.child_l + node, refs.x);
+    __stcg(t.child_r + node, refs.y);
+    set_parent(t, refs.x, node);
+    set_parent(t, refs.y, node);
     float b[6];
     double d[6];
     int cnt = 0;
     bool first = true;
-    for (int j = 0; j < w.m; j++) {
+    for (int j = 0; j < kTreeletLeaves; j++) {
         if (!((s >> j) & 1)) continue;
         for (int q = 0; q < 6; q += 2) {
             b[q] = first ? w.mb[j][q] : fminf(b[q], w.mb[j][q]);
@@ -287,16 +296,20 @@ __device__ void rebuild_write(const TreeArrays &t, const TreeletWork &w, int lan
     }
     __stcg(t.count + node, cnt);
     __stcg(t.cost + node, w.c[s]);
-    __threadfence();
 }
 
 constexpr int kTreeletThreads = 128;
+// Lanes of a warp that start from a triangle. With fewer, more warps share the treelets close to the triangles,
+// where one warp has several at once; with many triangles the GPU is full of warps anyway. us at 16 and 32:
+// 5,120 triangles 169 / 196, 41,006 255 / 271, 81,920 305 / 328, 131,072 387 / 357.
+constexpr int treelet_climbers(int n) { return n <= 100000 ? 16 : 32; }
 
-// One thread per triangle climbs from its leaf; the second thread to reach a node owns it (its
+// One lane per triangle climbs from its leaf; the second thread to reach a node owns it (its
 // subtree is then final). Each round, the warp optimises its lanes' owned treelets one after the
 // other, all 32 lanes sharing each one's dynamic programme. Lanes without work stay in the loop (the
 // warp-wide votes need every lane) until the whole warp has climbed out.
-__global__ void __launch_bounds__(kTreeletThreads) k_treelets(int n, TreeArrays t, int *arrivals) {
+__global__ void __launch_bounds__(kTreeletThreads) k_treelets(int n, int climbers, TreeArrays t,
+                                                             int *arrivals) {
     __shared__ TreeletWork s_work[kTreeletThreads / 32];
     __shared__ unsigned char s_sets[kSubsets];
     for (int k = threadIdx.x; k < kSubsets; k += kTreeletThreads) s_sets[k] = kSubsetTable.set[k];
@@ -304,19 +317,20 @@ __global__ void __launch_bounds__(kTreeletThreads) k_treelets(int n, TreeArrays 
     TreeletWork &w = s_work[threadIdx.x >> 5];
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    int node = p < n ? __ldcg(t.parent_leaf + p) : -1;
+    const int p = int((blockIdx.x * kTreeletThreads + threadIdx.x) >> 5) * climbers + lane;
+    int node = lane < climbers && p < n ? __ldcg(t.parent_leaf + p) : -1;
     while (__any_sync(kAll, node >= 0)) {
         bool own = false;
+        int parent = -1;
         if (node >= 0) {
+            // a node's links and count stay as they are until it is owned, so they don't wait for the arrival
+            parent = __ldcg(t.parent_int + node);
+            const int cnt = __ldcg(t.count + node), l = __ldcg(t.child_l + node), r = __ldcg(t.child_r + node);
             __threadfence();
             if (atomicAdd(&arrivals[node], 1) == 0) {
                 node = -1;  // the first arrival: the other child's thread continues
             } else {
                 __threadfence();
-                const int l = __ldcg(t.child_l + node), r = __ldcg(t.child_r + node);
-                const int cnt = ref_count(t, l) + ref_count(t, r);
-                __stcg(t.count + node, cnt);
                 if (cnt >= kTreeletLeaves) {
                     own = true;
                 } else {
@@ -332,17 +346,12 @@ __global__ void __launch_bounds__(kTreeletThreads) k_treelets(int n, TreeArrays 
             todo &= todo - 1;
             const int x = __shfl_sync(kAll, node, owner);
             treelet_best(t, x, w, s_sets, lane);
-            if (w.m >= 3) {
-                if (lane == owner) rebuild_plan(t, x, w);
-                __syncwarp();
-                rebuild_write(t, w, lane);
-            }
+            if (lane == owner) rebuild_plan(t, x, w);
+            __syncwarp();
+            rebuild_write(t, w, lane);
             __syncwarp();
         }
-        if (node >= 0) {
-            __threadfence();
-            node = __ldcg(t.parent_int + node);
-        }
+        if (node >= 0) node = parent;
     }
 }
 
@@ -417,7 +426,9 @@ int treelet_optimize(int n, int *child_l, int *child_r, int *parent_int, int *pa
         TreeArrays t{child_l, child_r, parent_int, parent_leaf, nbox32, nbox64, pbox32, pbox64, sorted_ids, cost, count};
         e = cudaMemsetAsync(arrivals, 0, sizeof(int) * nint, stream);
         if (e == cudaSuccess) {
-            k_treelets<<<grid_blocks(n, kTreeletThreads), kTreeletThreads, 0, stream>>>(n, t, arrivals);
+            const int climbers = treelet_climbers(n);
+            k_treelets<<<grid_blocks(n, kTreeletThreads / 32 * climbers), kTreeletThreads, 0, stream>>>(n, climbers, t,
+                                                                                                        arrivals);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) {
