@@ -230,6 +230,7 @@ template <typename T, int Q>
 struct ExactPolicy {
     using R = float;
     static constexpr int kQn = Q;
+    static constexpr bool kVote = sizeof(T) == sizeof(float);
     const DeviceMesh &m;
     T px[Q], py[Q], pz[Q], best[Q];
     float2 bx[Q], by[Q], bz[Q];  // the point in the box frame, each coordinate twice (two-wide FP32)
@@ -331,6 +332,7 @@ template <int Q>
 struct FastPolicy {
     using R = float;
     static constexpr int kQn = Q;
+    static constexpr bool kVote = true;
     const DeviceMesh &m;
     float2 bx[Q], by[Q], bz[Q];  // the point in the box frame (the filter records' too), each coordinate twice
     float best[Q], thr[Q], evicted[Q];
@@ -452,11 +454,15 @@ __device__ __forceinline__ R min_of(const R (&d)[Q]) {
     return v;
 }
 
-// Lane whose ranking of two children the packet follows: (1, 1, 1) of its 4 x 4 x 2 brick, or, at the
-// grid's edges, the same clamped to the lanes that hold a query (of a list's last packet: its last one).
-// A lane without one sits far outside, where the children's order says nothing: with it a 145^3 grid of
-// the torus knot, whose last bricks have one column each, took 5,900 us against 2,900 for 144^3.
-__device__ __forceinline__ unsigned packet_rank_bit(unsigned active) {
+// Lanes that rank two children for their packet, of those that hold a query: a lane without one sits far
+// outside, where the children's order says nothing (asked all the same, at (1, 1, 1) of the 4 x 4 x 2 brick, a
+// 145^3 grid of the torus knot, whose last bricks have one column each, took 5,900 us against 2,900 for 144^3).
+// All of them vote: 262,144 points near the knot 862 -> 829 us, the beams' points 5,280 -> 5,235, 64^3 grid on
+// 5,120 triangles 226 -> 221. The double kernel follows one lane, (1, 1, 1) clamped to the brick's part inside
+// the grid (of a list's last packet: its last lane); counting the votes cost it 2 % (1,167 -> 1,195).
+template <class P>
+__device__ __forceinline__ unsigned packet_rankers(unsigned active) {
+    if (P::kVote) return active;
     int lane = 21;
     if (!(active & 0xeeeeeeeeu)) lane -= 1;   // one column of x
     if (!(active & 0xfff0fff0u)) lane -= 4;   // one row of y
@@ -482,7 +488,7 @@ __device__ __forceinline__ float warp_max(float v) {
 // the smallest box distance over the warp's lanes and is entered on pop while that is below the
 // largest lane threshold: a superset of "some lane's distance below its own threshold", so never a
 // miss. Lanes without a query sit far from the mesh (P::disable), so they take no part in the keys.
-// Of two wanted children the one the brick's centre lane (packet_rank_bit) ranks first is the nearer; a
+// Of two wanted children the one the packet's lanes (packet_rankers) rank first is the nearer; a
 // wanted leaf is tested at once, and when it was the nearer one the other child is asked for again, its lanes'
 // thresholds having shrunk.
 template <bool COUNT, class P>
@@ -493,7 +499,8 @@ __device__ __forceinline__ void traverse_packet(P &p, Counters &cnt, int budget)
     if (budget <= 0) budget = 0x7fffffff;
     __shared__ int2 s_entry[kThreads / 32][kStackSize];  // node, key bits
     int2 *const entry = s_entry[threadIdx.x >> 5];
-    const unsigned rank_bit = packet_rank_bit(__ballot_sync(kAll, p.max_thr() > 0.f));
+    const unsigned rankers = packet_rankers<P>(__ballot_sync(kAll, p.max_thr() > 0.f));
+    const int half = __popc(rankers) / 2;
     int sp = 0;
     int node = 0;
     auto test_leaf = [&](int ref, unsigned m) {
@@ -510,7 +517,8 @@ __device__ __forceinline__ void traverse_packet(P &p, Counters &cnt, int budget)
         int next = -1;
         if (any0 && any1) {
             const float k0 = min_of<float, Q>(d0), k1 = min_of<float, Q>(d1);
-            const bool swap = __ballot_sync(kAll, k1 < k0) & rank_bit;
+            const unsigned votes = __ballot_sync(kAll, k1 < k0) & rankers;
+            const bool swap = P::kVote ? __popc(votes) > half : votes != 0;
             const int rn = swap ? r1 : r0, rf = swap ? r0 : r1;
             if (rf >= 0 && rn >= 0) {
                 if (sp < kStackSize) {
