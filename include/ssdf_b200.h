@@ -72,8 +72,8 @@ int ssdf_b200_edf_dd(ptrdiff_t npoints, const double *x, const double *y, const 
                      const int *s0, const int *s1, const int *s2, ptrdiff_t nspoints, const double *sx,
                      const double *sy, const double *sz, double *out);
 
-/* ssdf::edf_celllist (serial/ssdf.hpp:642-963): 2-D cell list over the two widest axes on the
- * GPU. Result bitwise equal to the reference's in T's precision. */
+/* ssdf::edf_celllist (serial/ssdf.hpp:642-963): the BVH walk, over a tree built in the call. Result
+ * bitwise equal to the reference's in T's precision. */
 int ssdf_b200_edf_celllist_ff(ptrdiff_t npoints, const float *x, const float *y, const float *z,
                               ptrdiff_t nselements, const int *s0, const int *s1, const int *s2, ptrdiff_t nspoints,
                               const float *sx, const float *sy, const float *sz, float *out);
@@ -425,7 +425,7 @@ int ssdf_mesh_filter_info(const ssdf_mesh *mesh, float *tau_rel, int *float_filt
 int ssdf_query_points(ssdf_mesh *mesh, ptrdiff_t npoints, const void *x, const void *y, const void *z, void *out,
                       int *outtri, void *outx, void *outy, void *outz, const ssdf_query_opts *opts, void *stream);
 /* ssdf::edf / ssdf::edf_celllist (serial/ssdf.hpp:447-619, 642-963) on device arrays: method 0 the
- * brute force (edf), 1 the cell list (edf_celllist); points, vertices and out all of coord_type
+ * brute force (edf), 1 a BVH built in the call (edf_celllist); points, vertices and out all of coord_type
  * (G == T, as the reference instantiates them), out in/out; outtri (the closest triangle) may be
  * NULL. Enqueued on `stream`; returns when the query has finished (it reads back a validation flag). */
 int ssdf_edf_device(int method, ptrdiff_t npoints, const void *x, const void *y, const void *z, ptrdiff_t nselements,

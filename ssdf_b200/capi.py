@@ -279,7 +279,7 @@ def edf(points, mesh, out=None, dtype=np.float64):
 
 
 def edf_celllist(points, mesh, out=None, dtype=np.float64):
-    """ssdf::edf_celllist<G, G, int>: GPU cell list, bitwise the reference's value."""
+    """ssdf::edf_celllist<G, G, int>: a BVH per call on the GPU, bitwise the reference's value."""
     s = _suffix(dtype)
     return _edf_call(f"ssdf_b200_edf_celllist_{s}{s}", points, mesh, out, dtype, dtype)
 

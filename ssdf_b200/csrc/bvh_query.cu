@@ -1485,8 +1485,8 @@ void set_grid_steps(QueryArgs *a) {
     a->grid_steps = grid_steps_for(grid_blocks_x(a->nx) * grid_blocks_y(a->ny) * grid_blocks_z(a->nz, 1));
 }
 
-// Measured on B200: the torus knot with 29 % of its triangles slivers still runs 1.4x faster on the
-// fix-up path than on FP64; the beam lattice (64 % slivers, in parallel bundles) runs 5x slower.
+// Measured on B200 over axis-aligned boxes: the torus knot with 29 % of its triangles slivers still ran 1.4x
+// faster on the fix-up path than on FP64; the beam lattice (64 % slivers, in parallel bundles) ran 5x slower.
 constexpr double kIllMaxFraction = 0.5;
 
 // The fix-up path hands a mesh to the FP64 kernel when more than this fraction of its triangles are
