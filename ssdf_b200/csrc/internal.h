@@ -177,9 +177,10 @@ struct BatchLaunch {
 struct MeshStorage;  // owns the device allocations behind a DeviceMesh
 int mesh_build(MeshStorage **storage, DeviceMesh *mesh, ptrdiff_t nt, const int *s0, const int *s1, const int *s2,
                ptrdiff_t nv, const void *sx, const void *sy, const void *sz, int coord_f64, int device_ptrs,
-               const ssdf_build_opts &opts, cudaStream_t stream, bool query_boxes = true);
+               const ssdf_build_opts &opts, cudaStream_t stream, bool query_boxes = true,
+               bool check_indices = true);
 // query_boxes false: without the oriented boxes (DeviceMesh::obb null), for walks of the axis-aligned nodes
-// only (contact.cu).
+// only (contact.cu). check_indices false: device index arrays that this library wrote (sdf_rebuild.cu).
 void mesh_free(MeshStorage *storage);                            // after the work using it completed
 void mesh_free_async(MeshStorage *storage, cudaStream_t stream);  // in stream order
 size_t mesh_bytes(const MeshStorage *storage);

@@ -995,7 +995,7 @@ static int readback_words(int **out) {
 static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int nt, const int *s0_in,
                            const int *s1_in, const int *s2_in, int nv, const void *sx, const void *sy, const void *sz,
                            int coord_f64, int device_ptrs, const ssdf_build_opts &opts, bool query_boxes,
-                           cudaStream_t stream) {
+                           bool check_indices, cudaStream_t stream) {
     const int L = opts.leaf_size > 0 ? opts.leaf_size : 4;
     m->nt = nt;
     m->nv = nv;
@@ -1041,7 +1041,7 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
     SSDF_CHECK(dalloc(tmp, &flags, 24, stream));
     k_init_flags<<<1, 32, 0, stream>>>(flags);
     LAUNCH_CHECK("k_init_flags");
-    if (device_ptrs) {
+    if (device_ptrs && check_indices) {
         // host arrays were checked on the host (check_mesh_host); device arrays are checked here,
         // before any kernel indexes the vertices with them
         k_validate<<<grid_blocks(nt, 256), 256, 0, stream>>>(nt, nv, s0, s1, s2, flags);
@@ -1184,7 +1184,7 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
 
 int mesh_build(MeshStorage **storage, DeviceMesh *mesh, ptrdiff_t nt, const int *s0, const int *s1, const int *s2,
                ptrdiff_t nv, const void *sx, const void *sy, const void *sz, int coord_f64, int device_ptrs,
-               const ssdf_build_opts &opts, cudaStream_t stream, bool query_boxes) {
+               const ssdf_build_opts &opts, cudaStream_t stream, bool query_boxes, bool check_indices) {
     if (nt <= 0 || nv <= 0) return fail(SSDF_ERR_INVALID_ARGUMENT, "empty mesh");
     if (nt >= kMaxTriangles) return fail(SSDF_ERR_NOT_SUPPORTED, "more than 2^26 triangles in one mesh");
     if (nv >= (1ll << 31)) return fail(SSDF_ERR_NOT_SUPPORTED, "more than 2^31 vertices");
@@ -1196,7 +1196,7 @@ int mesh_build(MeshStorage **storage, DeviceMesh *mesh, ptrdiff_t nt, const int 
     MeshStorage tmp;
     *mesh = DeviceMesh();
     int st = mesh_build_impl(s, &tmp, mesh, int(nt), s0, s1, s2, int(nv), sx, sy, sz, coord_f64, device_ptrs, opts,
-                             query_boxes, stream);
+                             query_boxes, check_indices, stream);
     for (void *p : tmp.blocks) cudaFreeAsync(p, stream);
     if (st == SSDF_OK) {
         cudaError_t e = cudaStreamSynchronize(stream);

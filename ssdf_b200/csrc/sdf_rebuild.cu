@@ -310,19 +310,20 @@ int level_set_device(const GridDesc &gd, const T *d_f, T level, long long *ntri,
     if (ncells >= 0x7fffffffll) return fail(SSDF_ERR_NOT_SUPPORTED, "more than 2^31 - 1 cells");
     int *count = nullptr, *offset = *d_offsets;
     if (!offset) {
-        SSDF_CUDA(cudaMallocAsync(&count, sizeof(int) * size_t(ncells), stream));
-        SSDF_CUDA(cudaMallocAsync(&offset, sizeof(int) * size_t(ncells), stream));
+        // one entry more than cells: its offset is the number of triangles
+        SSDF_CUDA(cudaMallocAsync(&count, sizeof(int) * (size_t(ncells) + 1), stream));
+        SSDF_CUDA(cudaMallocAsync(&offset, sizeof(int) * (size_t(ncells) + 1), stream));
+        SSDF_CUDA(cudaMemsetAsync(count + ncells, 0, sizeof(int), stream));
         k_marching<G, T, false><<<blocks_for(ncells, kThreadsR), kThreadsR, 0, stream>>>(
             gd, d_f, double(level), ncells, count, nullptr, nullptr, nullptr, nullptr);
         SSDF_CUDA(cudaGetLastError());
-        SSDF_CHECK(exclusive_scan_i32(count, offset, int(ncells), stream));
-        int last[2] = {0, 0};
-        SSDF_CUDA(cudaMemcpyAsync(&last[0], offset + ncells - 1, sizeof(int), cudaMemcpyDeviceToHost, stream));
-        SSDF_CUDA(cudaMemcpyAsync(&last[1], count + ncells - 1, sizeof(int), cudaMemcpyDeviceToHost, stream));
+        SSDF_CHECK(exclusive_scan_i32(count, offset, int(ncells) + 1, stream));
+        int total = 0;
+        SSDF_CUDA(cudaMemcpyAsync(&total, offset + ncells, sizeof(int), cudaMemcpyDeviceToHost, stream));
         SSDF_CUDA(cudaStreamSynchronize(stream));
         cudaFreeAsync(count, stream);
         *d_offsets = offset;
-        *ntri = (long long)last[0] + last[1];
+        *ntri = (long long)(unsigned)total;
     }
     if (x) {
         k_marching<G, T, true><<<blocks_for(ncells, kThreadsR), kThreadsR, 0, stream>>>(
@@ -369,8 +370,16 @@ int rebuild_device(const GridDesc &gd, const T *d_f, T level, T band, long long 
         if (st == SSDF_OK) {
             ssdf_build_opts bo;
             bo.leaf_size = 0, bo.keep_fp64 = 1, bo.normals = 0, bo.treelet_opt = call_treelet_rounds(nout);
-            st = ssdf_mesh_create(&mesh, ptrdiff_t(ntri), idx, idx + ntri, idx + 2 * ntri, ptrdiff_t(3 * ntri), x, y, z,
-                                  g64 ? SSDF_F64 : SSDF_F32, 1, &bo, stream);
+            mesh = new ssdf_mesh();
+            cudaGetDevice(&mesh->device);
+            // k_soup_indices wrote the indices: checking them would only make the host wait
+            st = mesh_build(&mesh->storage, &mesh->m, ptrdiff_t(ntri), idx, idx + ntri, idx + 2 * ntri,
+                            ptrdiff_t(3 * ntri), x, y, z, g64, 1, bo, stream, /*query_boxes=*/true,
+                            /*check_indices=*/false);
+            if (st != SSDF_OK) {
+                delete mesh;
+                mesh = nullptr;
+            }
         }
         if (st == SSDF_OK) {
             // the strided samples o + i h (in double from G's o and h), in/out from the band
