@@ -1077,14 +1077,14 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
     float4 *obb = nullptr;
     SSDF_CHECK(dalloc(s, &nodes32, 4 * size_t(m->nnodes), stream));
     if (query_boxes) SSDF_CHECK(dalloc(s, &obb, 8 * size_t(m->nnodes), stream));
-    // read-backs: depth and leaves, the coordinate scale, the three filter words and the box frame's four
-    static_assert(10 <= kReadbackWords, "read-back words");
+    // read back in one copy: flag words 7 to 19, the coordinate scale, depth and leaves, the three filter words
+    // and (from word 16) the box frame's four
+    constexpr int kFirstWord = 7, kWords = 13;
+    static_assert(kWords <= kReadbackWords, "read-back words");
     int *rb = nullptr;
     SSDF_CHECK(readback_words(&rb));
-    int *const depth_leaves = rb;
-    int *const scale_word = rb + 2, *const filt_info = scale_word + 1;
-    int *const frame_words = filt_info + 3;
-    depth_leaves[0] = depth_leaves[1] = 1;
+    const int *const scale_word = rb, *const depth_leaves = rb + 8 - kFirstWord;
+    const int *const filt_info = rb + 10 - kFirstWord, *const frame_words = rb + 16 - kFirstWord;
     const int *obb_first = nullptr, *obb_count = nullptr;  // subtree ranges (null: the small root)
     const double *obb_nbox = nullptr;
     if (nt <= L) {
@@ -1117,8 +1117,9 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
                                                            count, box32, box64, nbox32, nbox64, run32, run64, block32,
                                                            block64);
         LAUNCH_CHECK("k_boxes_inside");
-        k_boxes_across<<<grid_blocks(nint, 4 * kAcrossNodes), 128, 0, stream>>>(nt, ids, first_of, count, box32, box64, run32,
-                                                                   run64, block32, block64, nbox32, nbox64);
+        k_boxes_across<<<grid_blocks(nint, 4 * kAcrossNodes), 128, 0, stream>>>(nt, ids, first_of, count, box32, box64,
+                                                                                run32, run64, block32, block64, nbox32,
+                                                                                nbox64);
         LAUNCH_CHECK("k_boxes_across");
         for (int round = 0; round < opts.treelet_opt && round < 8; round++) {  // treelet_opt: rounds (0 = none)
             SSDF_CHECK(treelet_optimize(nt, child_l, child_r, parent_int, parent_leaf, first_of, count, nbox32, nbox64,
@@ -1129,7 +1130,6 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
         LAUNCH_CHECK("k_write_nodes");
         k_depth<<<grid_blocks(nint, 256), 256, 0, stream>>>(nt, L, count, parent_int, child_l, child_r, flags + 8);
         LAUNCH_CHECK("k_depth");
-        SSDF_CUDA(cudaMemcpyAsync(depth_leaves, flags + 8, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream));
         obb_first = first_of, obb_count = count, obb_nbox = nbox64;
     }
     // triangle records in leaf order
@@ -1151,9 +1151,7 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
             m->nnodes, L, obb_count, obb_first, box64, obb_nbox, ids, nodes32, t32, t64, flags + 16, (float *)obb);
         LAUNCH_CHECK("k_obb");
     }
-    SSDF_CUDA(cudaMemcpyAsync(frame_words, flags + 16, 4 * sizeof(int), cudaMemcpyDeviceToHost, stream));
-    SSDF_CUDA(cudaMemcpyAsync(scale_word, flags + 7, sizeof(int), cudaMemcpyDeviceToHost, stream));
-    SSDF_CUDA(cudaMemcpyAsync(filt_info, flags + 10, 3 * sizeof(int), cudaMemcpyDeviceToHost, stream));
+    SSDF_CUDA(cudaMemcpyAsync(rb, flags + kFirstWord, kWords * sizeof(int), cudaMemcpyDeviceToHost, stream));
     if (opts.normals) SSDF_CHECK(build_normals(s, m, s0, s1, s2, vx, vy, vz, stream));
     SSDF_CUDA(cudaStreamSynchronize(stream));  // the build's one wait: every read-back has landed
     float scale;
@@ -1167,8 +1165,8 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
         memcpy(&term, &filt_info[1], sizeof(float));
         set_filter_window(m, term, filt_info[2] == 0);
     }
-    m->depth = depth_leaves[0];
-    m->nleaves = depth_leaves[1];
+    m->depth = nt <= L ? 1 : depth_leaves[0];
+    m->nleaves = nt <= L ? 1 : depth_leaves[1];
     m->nodes32 = nodes32;
     m->obb = obb;
     m->entry = entry;
