@@ -1,13 +1,13 @@
 // radix_sort.cu -- stable LSD radix sort of (key, value) pairs and an exclusive scan, on the device.
 //
-// One kernel counts every pass' 8-bit digits, one turns the counts into offsets, and each pass is then a
-// single kernel after Adinets and Merrill's "Onesweep" (2022): a tile ranks its keys by digit (inside a
-// warp with __match_any_sync, across the tile's warps through shared memory), learns how many equal digits
-// the tiles before it hold by looking back over their published counts, and writes its keys in runs. Keys
-// and values cross memory twice a pass, in two launches and one per pass: a pass of histogram, table scan
-// (three launches) and scatter read the keys twice and moved a 256-entry table per 256 keys. 30-bit keys,
-// us before -> after: 4,000,000 450 -> 256, 500,003 92 -> 45. Used by the BVH builder (30-bit Morton keys), the pseudo-normal pass (vertex ids,
-// 64-bit edge keys) and point lists (Morton order).
+// One kernel counts every pass' 8-bit digits, and each pass is then a single kernel after Adinets and
+// Merrill's "Onesweep" (2022): a tile ranks its keys by digit (inside a warp with __match_any_sync, across the
+// tile's warps through shared memory), learns how many equal digits the tiles before it hold by looking back
+// over their published counts, scans the digit counts for itself (a kernel of its own for that cost 4 us a
+// sort) and writes its keys in runs. Keys and values cross memory twice a pass, in one launch and one per
+// pass: a pass of histogram, table scan (three launches) and scatter read the keys twice and moved a 256-entry
+// table per 256 keys. 30-bit keys, us before -> after: 4,000,000 450 -> 256, 500,003 92 -> 45. Used by the BVH
+// builder (30-bit Morton keys), the pseudo-normal pass (vertex ids, 64-bit edge keys) and point lists.
 #include <cuda_runtime.h>
 
 #include "internal.h"
@@ -58,13 +58,6 @@ __device__ __forceinline__ unsigned block_exclusive(unsigned v, unsigned *warp_t
     return before + incl - v;
 }
 
-// Offsets of the digits from their counts, in place: a block per pass.
-__global__ void __launch_bounds__(kSortThreads) k_digit_offsets(unsigned *__restrict__ counts) {
-    __shared__ unsigned warp_tot[kSortWarps];
-    unsigned *const c = counts + blockIdx.x * 256;
-    c[threadIdx.x] = block_exclusive(c[threadIdx.x], warp_tot);
-}
-
 // A tile's published word for a digit: state in the low two bits (0: nothing yet), count above.
 constexpr unsigned long long kTileOwn = 1;   // the tile's own count
 constexpr unsigned long long kTileUpTo = 2;  // the count of all tiles up to this one
@@ -76,16 +69,17 @@ constexpr int kMaxPolls = 1 << 16;
 template <typename K>
 __global__ void __launch_bounds__(kSortThreads) k_sort_pass(const K *__restrict__ kin, const int *__restrict__ vin,
                                                             K *__restrict__ kout, int *__restrict__ vout, int n,
-                                                            int shift, const unsigned *__restrict__ offsets,
+                                                            int shift, const unsigned *__restrict__ counts,
                                                             unsigned long long *tile_words, int *next_tile) {
     __shared__ unsigned cnt[kSortWarps][256];
     __shared__ unsigned tile_start[256], to_global[256];
-    __shared__ unsigned warp_tot[kSortWarps];
+    __shared__ unsigned warp_tot[kSortWarps], digit_tot[kSortWarps];
     __shared__ int s_tile;
     __shared__ K s_key[kSortTile];
     __shared__ int s_val[kSortTile];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, digit = threadIdx.x;
     if (threadIdx.x == 0) s_tile = atomicAdd(next_tile, 1);
+    const unsigned digit_count = counts[digit];
     for (int w = 0; w < kSortWarps; w++) cnt[w][digit] = 0;
     __syncthreads();
     const int tile = s_tile;
@@ -122,6 +116,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_pass(const K *__restrict_
     volatile unsigned long long *const mine = tile_words + (long long)tile * 256 + digit;
     *mine = (unsigned long long)total << 2 | (tile == 0 ? kTileUpTo : kTileOwn);
     tile_start[digit] = block_exclusive(total, warp_tot);
+    const unsigned digit_start = block_exclusive(digit_count, digit_tot);
     __syncthreads();
     // the tile's keys in digit order, while the words travel
 #pragma unroll
@@ -148,7 +143,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_pass(const K *__restrict_
         if ((w & 3) == kTileUpTo) break;
     }
     if (tile > 0) *mine = (prev + total) << 2 | kTileUpTo;
-    to_global[digit] = offsets[digit] + unsigned(prev) - tile_start[digit];
+    to_global[digit] = digit_start + unsigned(prev) - tile_start[digit];
     __syncthreads();
     const int m = int(n - base < kSortTile ? n - base : kSortTile);
     for (int i = threadIdx.x; i < m; i += kSortThreads) {
@@ -251,7 +246,6 @@ static int radix_sort_pairs(K *keys, int *vals, int n, int key_bits, cudaStream_
     if (e == cudaSuccess) {
         const int blocks = ntiles < 148 * 4 ? ntiles : 148 * 4;
         k_digit_counts<K><<<blocks, kSortThreads, 0, stream>>>(keys, n, passes, counts);
-        k_digit_offsets<<<passes, kSortThreads, 0, stream>>>(counts);
         e = cudaGetLastError();
     }
     K *kin = keys, *kout = k2;
