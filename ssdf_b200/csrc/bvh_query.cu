@@ -1525,6 +1525,15 @@ int morton_point_order(long long n, const void *x, const void *y, const void *z,
     return st;
 }
 
+// A captured double or float launch stays a single kernel node: a list would put an allocation into the
+// caller's graph, which then cannot be a child graph or run twice at once.
+static bool capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
 int launch_query(const QueryArgs &args_in, int precision, cudaStream_t stream) {
     return launch_query_keep(args_in, precision, stream, nullptr);
 }
@@ -1589,7 +1598,7 @@ int launch_query_keep(const QueryArgs &args_in, int precision, cudaStream_t stre
         const bool fixup = precision == SSDF_PREC_F32_FIXUP;
         if (fixup && n >= 0x7fffffffll) {
             st = fail(SSDF_ERR_NOT_SUPPORTED, "more than 2^31 - 1 queries in one fix-up launch");
-        } else if (fixup || (warp && a.warp_budget > 0 && n <= kHandOverMaxQueries)) {
+        } else if (fixup || (warp && a.warp_budget > 0 && n <= kHandOverMaxQueries && !capturing(stream))) {
             if (cudaMallocAsync(&fb, sizeof(int) * size_t(2 * n + 1), stream) != cudaSuccess) {
                 fb = nullptr;
                 if (fixup) st = fail(SSDF_ERR_OUT_OF_MEMORY, "fix-up overflow list");

@@ -40,3 +40,23 @@ def test_grids_with_partly_filled_bricks(n, steps, monkeypatch):
             torch.cuda.synchronize()
             assert np.array_equal(out.cpu().numpy(), want) and np.array_equal(tri.cpu().numpy(), wtri), (prec, budget)
     dm.close()
+
+
+@pytest.mark.parametrize("prec", [S.PREC_F64, S.PREC_F32_FIXUP])
+def test_captured_grid_equals_the_plain_call(prec):
+    mesh = W.torus(nu=30, nv=15, jitter=0.02)
+    grid = W.Grid.padded_nodes(mesh, 21, 0.2)
+    dm = S.DeviceMesh(mesh)
+    plain, replayed = (torch.zeros(grid.size, dtype=torch.float64, device="cuda") for _ in range(2))
+    dm.query_grid(grid, plain, precision=prec)
+    torch.cuda.synchronize()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        dm.query_grid(grid, replayed, precision=prec, stream=stream)
+    for _ in range(2):
+        replayed.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(plain, replayed)
+    del graph
+    dm.close()
