@@ -34,6 +34,7 @@
 #include <string>
 #include <type_traits>
 
+#include "box_margin.h"
 #include "device_geom.cuh"
 #include "internal.h"
 
@@ -200,13 +201,10 @@ struct ExactData<double> {
 template <>
 struct ExactData<float> {
     using Tri = Tri32;
-    // distance margin of the prune threshold: the float vertices against the (perhaps double) ones the
-    // boxes hold, and the float squared distances' absolute error
-    static __device__ __forceinline__ float margin(const DeviceMesh &m) { return m.coord_scale * 0x1p-16f; }
+    // the prune threshold's margins (box_margin.h)
+    static __device__ __forceinline__ float margin(const DeviceMesh &m) { return float_box_margin(m.coord_scale); }
     static __device__ __forceinline__ float box_thr(float best, float margin, const DeviceMesh &m) {
-        const float d = sqrtf(best) + 0x1p-7f * margin;  // 2^-23 of the coordinates' magnitude
-        const float t = fmaxf(d * d, best + margin * margin) * (1.0f + 1.0f / 65536.0f);
-        return fmaxf(t * m.box_scale * m.box_scale, FLT_MIN);
+        return fmaxf(float_box_reach(best, margin) * m.box_scale * m.box_scale, FLT_MIN);
     }
     static __device__ __forceinline__ float box_coord(float p, int d, const DeviceMesh &m) {
         return (p - m.box_c[d]) * m.box_scale;

@@ -633,7 +633,8 @@ __global__ void k_tri_records(int nt, const int *__restrict__ sorted_ids, const 
 //   region tests, on dot products within 11 u of their lengths, put the closest point at most D = 90 u
 //   alpha R off the triangle (alpha = longest edge / smallest altitude, R <= d + L the distance to the
 //   farthest corner, L the longest edge), in its plane. So half extents are also stored 128 u alpha L
-//   larger and everything scaled by 1 / (1 + 128 u alpha), alpha and L over the child's triangles. A child
+//   larger and everything scaled by 1 / (1 + 128 u alpha), alpha and L over the child's triangles. (The closest
+//   point's own rounding and the float corners' are of the mesh's place, not of M: box_margin.h.) A child
 //   with alpha above kObbMaxAlpha keeps its axis-aligned box, as does one of more than kObbMaxTris
 //   triangles (its patch is no longer flat; building it would read every triangle at every level).
 constexpr int kObbMaxTris = 64;
