@@ -341,6 +341,9 @@ __global__ void __launch_bounds__(kTreeletThreads) k_treelets(int n, int climber
             }
         }
         unsigned todo = __ballot_sync(kAll, own);
+        // every lane reads the owned subtrees, but only their owners met the other arrivals and fenced: a vote or
+        // a shuffle orders no memory, this barrier does
+        __syncwarp();
         while (todo) {
             const int owner = __ffs(todo) - 1;
             todo &= todo - 1;
