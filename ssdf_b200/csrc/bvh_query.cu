@@ -469,16 +469,14 @@ __device__ __forceinline__ unsigned packet_rankers(unsigned active) {
     return 1u << lane;
 }
 
-// Warp minimum / maximum of a float (sm_100's redux on floats).
+// Warp minimum / maximum of floats that order like their bits: distances (not negative) and thresholds (not
+// negative, or -1). Through the intrinsics, which the compiler keeps where the whole warp is: the results
+// feed divergent code, and an inline redux on floats could be sunk into it.
 __device__ __forceinline__ float warp_min(float v) {
-    float r;
-    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-    return r;
+    return __int_as_float(__reduce_min_sync(0xffffffffu, __float_as_int(v)));
 }
 __device__ __forceinline__ float warp_max(float v) {
-    float r;
-    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-    return r;
+    return __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(v)));
 }
 
 // Packet walk (a grid warp as one packet): the node ids on the stack are the same in every lane, so
