@@ -976,6 +976,12 @@ constexpr int kWindowBlocksPerSm = SSDF_B200_WINDOW_BLOCKS_PER_SM;
 // float filter's range, whose keys may have overflowed, is answered this way: exactly, in double).
 __device__ __forceinline__ bool in_window(float key, float thr) { return key < thr || thr == finf(); }
 
+// A finite point beyond the fix-up filter's range: everything is evaluated, exactly, in double.
+template <int PREC>
+__device__ __forceinline__ bool beyond_filter(double x, double y, double z) {
+    return PREC == SSDF_PREC_F32_FIXUP && fmax(fmax(fabs(x), fabs(y)), fabs(z)) > double(kFilterMaxCoord);
+}
+
 // What a lane of a warp-per-query walk knows: the query in the arithmetic's own terms, the lexicographic
 // minimum of the triangles the lane evaluated, and the box threshold its finds allow. PREC as the query
 // kernels'.
@@ -1011,7 +1017,7 @@ struct LaneWalk {
     // the threshold the whole warp's finds allow (warp-wide)
     __device__ __forceinline__ float found_thr() const {
         if constexpr (PREC == SSDF_PREC_F32_FIXUP)
-            return window_thr(warp_min(kbest), tau_rel, m.coord_scale);
+            return window_thr(warp_min(fminf(kbest, __double2float_ru(d2))), tau_rel, m.coord_scale);
         else
             return warp_min(ExactData<T>::box_thr(d2, margin, m));
     }
@@ -1203,9 +1209,9 @@ __device__ void window_warp(const QueryArgs &a, int idx, WarpShared &sh, int cap
     query_point(a, q, i, j, k, qx, qy, qz);
     const float thr = a.fallback_thr[idx];
     LaneWalk<PREC> w(a, qx, qy, qz, lane_bound<PREC>(a, q));
-    // fix-up: an infinite window (a point beyond the float range) stays
-    const bool shrink = PREC != SSDF_PREC_F32_FIXUP || thr < finf();
-    warp_walk<PREC, COUNT>(w, thr, shrink, false, sh, cap, cnt);
+    // The infinite window of a point beyond the filter's range stays; a packet that met only proxies before
+    // its budget ran out hands over an infinite one too, which shrinks like any other.
+    warp_walk<PREC, COUNT>(w, thr, !beyond_filter<PREC>(qx, qy, qz), false, sh, cap, cnt);
     if ((threadIdx.x & 31) == 0) lane_result(a, q, qx, qy, qz, w);
 }
 
@@ -1240,9 +1246,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_query_warp(const __grid_constan
     query_point(a, q, 0, 0, 0, x, y, z);
     LaneWalk<PREC> w(a, x, y, z, lane_bound<PREC>(a, q));
     if (w.finite()) {
-        // a finite point beyond the filter's range: everything, exactly, in double
-        const bool beyond = PREC == SSDF_PREC_F32_FIXUP &&
-                            fmax(fmax(fabs(x), fabs(y)), fabs(z)) > double(kFilterMaxCoord);
+        const bool beyond = beyond_filter<PREC>(x, y, z);
         bool upper = !beyond;
         while (!warp_walk<PREC, COUNT>(w, beyond ? finf() : w.start_thr(), !beyond, upper, sh, cap, cnt)) upper = false;
     }
