@@ -589,7 +589,7 @@ int ssdf_server_reset_stats(ssdf_server *server);
  * beforehand with ssdf_mesh_create. The first call on a device looks up the array's device address
  * (once per device): make that first call before any stream capture. All calls share the array and
  * each one resets it, so calls whose kernels overlap on the GPU (concurrent streams) race: order
- * them on one stream. */
+ * them on one stream. (Calls on meshes that the double kernel answers, see ssdf_mesh_filter_info, use no array.) */
 int ssdf_query_grid_noalloc(ssdf_mesh *mesh, ptrdiff_t nx, ptrdiff_t ny, ptrdiff_t nz, const double lo[3],
                             const double hi[3], void *out, int *outtri, const ssdf_query_opts *opts, void *stream);
 long long ssdf_query_grid_noalloc_max(void);

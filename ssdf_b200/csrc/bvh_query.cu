@@ -1723,16 +1723,23 @@ int launch_query_noalloc(const QueryArgs &args_in, cudaStream_t stream) {
     a.counters = nullptr;
     const bool warp = use_warp(a);
     const long long nblocks = query_blocks(a);
-    a.warp_budget = resolve_warp_budget(a.warp_budget, n, a.m.nt, a.is_grid != 0);
-    int *scratch = nullptr;
-    SSDF_CHECK(noalloc_scratch(&scratch));
-    a.fallback_count = scratch;
-    a.fallback_ids = scratch + 1;
-    a.fallback_thr = reinterpret_cast<float *>(scratch + 1 + n);
-    cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(int), stream);  // the count starts at zero
-    if (e == cudaSuccess)
-        e = fixup_runs_f64(a.m) ? launch_two_stages<SSDF_PREC_F64>(a, warp, false, unsigned(nblocks), stream, kWinStack)
-                                : launch_two_stages<SSDF_PREC_F32_FIXUP>(a, warp, false, unsigned(nblocks), stream, kWinStack);
+    cudaError_t e;
+    if (fixup_runs_f64(a.m)) {
+        // the same bits from the double kernel, without a budget: it hands nothing over, so these calls share
+        // nothing and may overlap
+        a.warp_budget = 0;
+        e = launch_prec<SSDF_PREC_F64>(a, warp, false, unsigned(nblocks), stream);
+    } else {
+        a.warp_budget = resolve_warp_budget(a.warp_budget, n, a.m.nt, a.is_grid != 0);
+        int *scratch = nullptr;
+        SSDF_CHECK(noalloc_scratch(&scratch));
+        a.fallback_count = scratch;
+        a.fallback_ids = scratch + 1;
+        a.fallback_thr = reinterpret_cast<float *>(scratch + 1 + n);
+        e = cudaMemsetAsync(scratch, 0, sizeof(int), stream);  // the count starts at zero
+        if (e == cudaSuccess)
+            e = launch_two_stages<SSDF_PREC_F32_FIXUP>(a, warp, false, unsigned(nblocks), stream, kWinStack);
+    }
     if (e != cudaSuccess) return cuda_fail(e, "allocation-free query launch", __FILE__, __LINE__);
     return SSDF_OK;
 }
