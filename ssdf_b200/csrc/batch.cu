@@ -231,23 +231,36 @@ int ssdf_batch_add_points(ssdf_batch *b, ssdf_mesh *mesh, ptrdiff_t npoints, con
     return batch_add(b, a, opts);
 }
 
-// Sizes the hand-over lists for runs of up to max_queries queries, so that such runs never
-// reallocate them (a reallocation synchronises the device).
-int ssdf_batch_reserve(ssdf_batch *b, long long max_queries, void *stream_) {
-    if (!b || max_queries < 0) return fail(SSDF_ERR_INVALID_ARGUMENT, "ssdf_batch_reserve: bad arguments");
-    const size_t need = 2 * size_t(max_queries);
+// The hand-over lists hold 8 bytes a query. A fix-up job must have its list (windows that overflow their slots are
+// finished from it); a plain job only walks without a budget where it has none. So plain lists are kept for jobs of
+// the size that a launch of their own would keep one for, and up to this many queries a batch (2 GiB), and a
+// batch runs all the same when there is no memory for them.
+static constexpr long long kPlainListQueries = 1ll << 28;
+
+// Lists of `need` words (after the work on `stream`; a reallocation synchronises the device).
+static int reserve_lists(ssdf_batch *b, size_t need, cudaStream_t stream) {
     if (need <= b->fb_cap) return SSDF_OK;
-    SSDF_CUDA(cudaStreamSynchronize((cudaStream_t)stream_));
+    SSDF_CUDA(cudaStreamSynchronize(stream));
     cudaFree(b->d_fb);
     b->d_fb = nullptr;
     b->fb_cap = 0;
     if (cudaMalloc(&b->d_fb, sizeof(int) * need) != cudaSuccess) {
         cudaGetLastError();
         b->d_fb = nullptr;
-        return fail(SSDF_ERR_OUT_OF_MEMORY, "hand-over lists of " + std::to_string(max_queries) + " queries");
+        return fail(SSDF_ERR_OUT_OF_MEMORY, "hand-over lists of " + std::to_string(need / 2) + " queries");
     }
     b->fb_cap = need;
     return SSDF_OK;
+}
+
+// Sizes the hand-over lists for runs of up to max_queries queries, so that such runs never
+// reallocate them.
+int ssdf_batch_reserve(ssdf_batch *b, long long max_queries, void *stream_) {
+    if (!b || max_queries < 0) return fail(SSDF_ERR_INVALID_ARGUMENT, "ssdf_batch_reserve: bad arguments");
+    const bool fixup = b->precision == SSDF_PREC_F32_FIXUP;
+    const long long n = fixup ? max_queries : std::min(max_queries, kPlainListQueries);
+    const int st = reserve_lists(b, 2 * size_t(n), (cudaStream_t)stream_);
+    return fixup ? st : SSDF_OK;
 }
 
 // One persistent launch over every job (+ the fix-up window stage). use_graph: capture the launch
@@ -274,14 +287,24 @@ int ssdf_batch_run(ssdf_batch *b, int use_graph, void *stream_) {
     for (int i = 0; i < njobs; i++) order[i] = i;
     auto cost = [&](const QueryArgs &a) { return double(query_blocks(a)) * std::log2(2.0 + a.m.nt); };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost(b->jobs[x]) > cost(b->jobs[y]); });
-    // hand-over lists: one slice of (ids, thresholds) per job
-    size_t need = 0;
-    for (const auto &j : b->jobs) need += 2 * size_t(j.is_grid ? j.nx * j.ny * j.nz : j.npoints);
-    bool lists = true;
-    if (need > b->fb_cap) {
-        const int st = ssdf_batch_reserve(b, (long long)(need / 2), stream);
-        if (fixup) SSDF_CHECK(st);
-        lists = st == SSDF_OK;  // the plain arithmetics only walk on without a budget
+    // hand-over lists: one slice of (ids, thresholds) per job that has one
+    auto queries = [](const QueryArgs &a) { return size_t(a.is_grid ? a.nx * a.ny * a.nz : a.npoints); };
+    size_t need = 0, plain = 0;
+    std::vector<char> listed(njobs, 0);  // by the job's place in `order`
+    for (int r = 0; r < njobs; r++) {
+        const QueryArgs &j = b->jobs[order[r]];
+        const size_t n = queries(j);
+        if (fixup && !to_f64(j)) {
+            listed[r] = 1;
+            need += 2 * n;
+        } else if (warp && n <= size_t(kHandOverMaxQueries) && plain + n <= size_t(kPlainListQueries)) {
+            listed[r] = 2;
+            plain += n;
+        }
+    }
+    if (reserve_lists(b, need + 2 * plain, stream) != SSDF_OK) {
+        SSDF_CHECK(reserve_lists(b, need, stream));
+        for (char &l : listed) l &= 1;
     }
     // the staging buffers may still feed the previous run's copies
     SSDF_CUDA(cudaStreamSynchronize(stream));
@@ -319,8 +342,8 @@ int ssdf_batch_run(ssdf_batch *b, int use_graph, void *stream_) {
             a.order = ord;
         }
         a.counters = nullptr;
-        const size_t n = size_t(a.is_grid ? a.nx * a.ny * a.nz : a.npoints);
-        if (lists) {
+        const size_t n = queries(a);
+        if (listed[r]) {
             a.fallback_count = b->d_fbcount + r;
             a.fallback_ids = b->d_fb + off;
             a.fallback_thr = reinterpret_cast<float *>(b->d_fb + off + n);
