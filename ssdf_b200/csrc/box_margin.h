@@ -16,6 +16,7 @@
 // tests/box_margin_check.c looks for the largest need. Plain C, for that check.
 #pragma once
 
+#include <float.h>
 #include <math.h>
 
 #ifdef __CUDACC__
@@ -24,11 +25,14 @@
 #define SSDF_BOX_MARGIN_FN static inline
 #endif
 
-// c as float_box_reach takes it.
-SSDF_BOX_MARGIN_FN float float_box_margin(float c) { return c * 0x1p-16f; }
+// c as float_box_reach takes it. Squares below the smallest normal float are not relative: at least 2^-63, the root
+// of that number, which is as near as the float arithmetic tells distances apart.
+SSDF_BOX_MARGIN_FN float float_box_margin(float c) { return fmaxf(c * 0x1p-16f, 0x1p-63f); }
 
-// The squared distance below which a box is entered: (sqrt(best) + 8 u c)^2, and at least best + (2^-16 c)^2.
-SSDF_BOX_MARGIN_FN float float_box_reach(float best, float margin) {
-    const float d = sqrtf(best) + 0x1p-5f * margin;
-    return fmaxf(d * d, best + margin * margin) * (1.0f + 1.0f / 65536.0f);
+// The squared distance in the box frame (scale s) below which a box is entered: (sqrt(best) + 8 u c)^2, and at least
+// best + (2^-16 c)^2. A best of +inf is taken as the largest finite one: a box farther than that holds no
+// triangle with a finite float distance.
+SSDF_BOX_MARGIN_FN float float_box_reach(float best, float margin, float s) {
+    const float b = fminf(best, FLT_MAX), d = (sqrtf(b) + 0x1p-5f * margin) * s, near = margin * s;
+    return fmaxf(d * d, b * s * s + near * near) * (1.0f + 1.0f / 65536.0f);
 }

@@ -188,11 +188,15 @@ struct ExactData<double> {
     }
     // the float threshold of the boxes (in the box frame's scale), rounded up
     static __device__ __forceinline__ float box_thr(double best, double margin, const DeviceMesh &m) {
-        const double t = (best * (1.0 + 1.0 / 65536.0) + margin) * (double(m.box_scale) * double(m.box_scale));
+        const double t = (best * (1.0 + 1.0 / 65536.0) + margin) * (m.box_scale * m.box_scale);
         return fmaxf(__double2float_ru(t), FLT_MIN);  // a box at distance 0 is always wanted
     }
     static __device__ __forceinline__ float box_coord(double p, int d, const DeviceMesh &m) {
-        return float((p - double(m.box_c[d])) * double(m.box_scale));
+        return float((p - double(m.box_c[d])) * m.box_scale);
+    }
+    // a coordinate from here on has no finite squared distance to the mesh (in a mesh within float's range)
+    static __device__ __forceinline__ double beyond(const DeviceMesh &m) {
+        return m.coord_scale < __int_as_float(0x7f800000) ? 0x1p520 : dinf();
     }
     // a threshold beyond float's range is +inf: a box distance that overflowed still counts as inside
     static __device__ __forceinline__ float box_key(float d) { return fminf(d, FLT_MAX); }
@@ -204,11 +208,13 @@ struct ExactData<float> {
     // the prune threshold's margins (box_margin.h)
     static __device__ __forceinline__ float margin(const DeviceMesh &m) { return float_box_margin(m.coord_scale); }
     static __device__ __forceinline__ float box_thr(float best, float margin, const DeviceMesh &m) {
-        return fmaxf(float_box_reach(best, margin) * m.box_scale * m.box_scale, FLT_MIN);
+        return fmaxf(float_box_reach(best, margin, m.box_scale_f), FLT_MIN);
     }
     static __device__ __forceinline__ float box_coord(float p, int d, const DeviceMesh &m) {
-        return (p - m.box_c[d]) * m.box_scale;
+        return (p - m.box_c[d]) * m.box_scale_f;
     }
+    // a coordinate from here on has no finite squared distance to the mesh
+    static __device__ __forceinline__ float beyond(const DeviceMesh &) { return __int_as_float(0x7f800000); }
     static __device__ __forceinline__ float box_key(float d) { return d; }
     static __device__ __forceinline__ Tri tri(const DeviceMesh &m, int pos) { return load_tri32(m.tris32, pos); }
 };
@@ -242,7 +248,8 @@ struct ExactPolicy {
         bx[q] = twice(ExactData<T>::box_coord(x, 0, m));
         by[q] = twice(ExactData<T>::box_coord(y, 1, m));
         bz[q] = twice(ExactData<T>::box_coord(z, 2, m));
-        const bool finite = isfinite(x) && isfinite(y) && isfinite(z);
+        const T lim = ExactData<T>::beyond(m);
+        const bool finite = fabs(x) < lim && fabs(y) < lim && fabs(z) < lim;
         thr[q] = finite ? ExactData<T>::box_thr(init, margin, m) : -1.f;
     }
     __device__ __forceinline__ void disable(int q) {
@@ -1006,7 +1013,10 @@ struct LaneWalk {
             bz = twice(ExactData<T>::box_coord(qz, 2, m));
         }
     }
-    __device__ __forceinline__ bool finite() const { return isfinite(qx) && isfinite(qy) && isfinite(qz); }
+    __device__ __forceinline__ bool finite() const {
+        const T lim = ExactData<T>::beyond(m);
+        return fabs(qx) < lim && fabs(qy) < lim && fabs(qz) < lim;
+    }
     // the threshold the incoming bound allows
     __device__ __forceinline__ float start_thr() const {
         if constexpr (PREC == SSDF_PREC_F32_FIXUP)
@@ -1129,7 +1139,7 @@ __device__ bool warp_walk(LaneWalk<PREC> &w, float thr, bool shrink, bool upper,
         }
         if (upper) {
             const float u = warp_min(fminf(c0 == kEmptyRef ? finf() : far.x, c1 == kEmptyRef ? finf() : far.y));
-            cut = fminf(cut, fmaxf(u * 1.05f, FLT_MIN));  // an overflow or a NaN cuts nothing
+            cut = fminf(cut, u < finf() ? fmaxf(u * 1.05f, FLT_MIN) : finf());  // an overflow or a NaN cuts nothing
             thr = fminf(thr, w.cut_thr(cut));
         }
         const bool w0 = c0 != kEmptyRef && w.wants(d.x, thr), w1 = c1 != kEmptyRef && w.wants(d.y, thr);

@@ -73,7 +73,8 @@ struct DeviceMesh {
     // where a walk shared by a warp starts: entry[0] nodes (at most 32), entry[1 ..]
     const int *entry = nullptr;
     float box_c[3] = {0.f, 0.f, 0.f};
-    float box_scale = 1.f;
+    double box_scale = 1.0;    // a power of two, 1 for a mesh of half size 2^-26 to 2^28
+    float box_scale_f = 1.f;   // the same for the float walk; NaN (every box at distance 0) beyond float's range
     const float4 *tris32 = nullptr;    // [3 * nt], leaf order
     const double2 *tris64 = nullptr;   // [5 * nt], leaf order, or null
     // the fix-up path's FP32 filter records, [3 * nt], leaf order, with the double data or null:

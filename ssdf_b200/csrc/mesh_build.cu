@@ -515,34 +515,40 @@ void set_filter_window(DeviceMesh *m, float largest_term, bool records_safe) {
 
 namespace {
 
-// Middle and scale of the mesh's box (the union of the root's children), and M in that frame: w[0..2],
-// w[3], w[4] as floats. A mesh outside [2^-60, 2^100], or with a coordinate that is not finite, gets M < 0:
-// its boxes cull nothing. And the nodes a warp-wide walk starts from (DeviceMesh::entry): the root, each
-// node whose children are both nodes replaced by them, five times over. One warp.
-__global__ void k_box_frame(const float4 *__restrict__ nodes, int *__restrict__ w, int *__restrict__ entry) {
+// Middle and scale of the mesh's box (the union of the nbox boxes box64), and M in that frame: w[0..2] the
+// middle and w[6] M as floats, w[4..5] the scale as a double. The scale is 1 for a half size of 2^-26 to 2^28, which
+// holds every mesh that the float filter takes (its records have the frame's middle but no scale), and else
+// brings the half size into [8, 16): k_obb's fourth powers of lengths and the walks' squared distances then stay
+// in float's range. A mesh with a coordinate that is not finite in float gets M < 0: its boxes cull nothing. And the
+// nodes a warp-wide walk starts from (DeviceMesh::entry): the root, each node whose children are both nodes
+// replaced by them, five times over. One warp.
+__global__ void k_box_frame(const float4 *__restrict__ nodes, const double *__restrict__ box64, int nbox,
+                            int *__restrict__ w, int *__restrict__ entry) {
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x;
-    const float4 a = nodes[0], b = nodes[1], c = nodes[2];
     if (lane == 0) {
-        const float lo[3] = {fminf(a.x, b.x), fminf(a.z, b.z), fminf(c.x, c.z)};
-        const float hi[3] = {fmaxf(a.y, b.y), fmaxf(a.w, b.w), fmaxf(c.y, c.w)};
-        float mid[3], m = 0.f;
+        double lo[3] = {DBL_MAX, DBL_MAX, DBL_MAX}, hi[3] = {-DBL_MAX, -DBL_MAX, -DBL_MAX};
+        for (int i = 0; i < nbox; i++)
+            for (int d = 0; d < 3; d++)
+                lo[d] = fmin(lo[d], box64[6 * i + 2 * d]), hi[d] = fmax(hi[d], box64[6 * i + 2 * d + 1]);
+        float mid[3];
+        double m = 0.0;
+        bool ok = true;
         for (int d = 0; d < 3; d++) {
-            mid[d] = 0.5f * lo[d] + 0.5f * hi[d];
-            m = fmaxf(m, fmaxf(hi[d] - mid[d], mid[d] - lo[d]));
+            ok = ok && lo[d] <= hi[d] && lo[d] >= -double(FLT_MAX) && hi[d] <= double(FLT_MAX);
+            mid[d] = ok ? float(0.5 * lo[d] + 0.5 * hi[d]) : 0.f;
+            m = fmax(m, fmax(hi[d] - mid[d], mid[d] - lo[d]));
         }
-        float scale = 1.f;
-        if (!(m >= 0x1p-60f && m <= 0x1p100f)) {
-            m = -1.f;
-            for (int d = 0; d < 3; d++) mid[d] = 0.f;
-        } else if (m > 0x1p60f) {
-            int e;
-            m = frexpf(m, &e);  // M in [0.5, 1)
-            scale = ldexpf(1.f, -e);
+        double scale = 1.0;
+        if (ok && m > 0.0 && !(m >= 0x1p-26 && m <= 0x1p28)) {
+            int e = ilogb(m) - 3;
+            e = e < -450 ? -450 : e;
+            scale = ldexp(1.0, -e);
         }
-        for (int d = 0; d < 3; d++) w[d] = __float_as_int(mid[d]);
-        w[3] = __float_as_int(scale);
-        w[4] = __float_as_int(m);
+        for (int d = 0; d < 3; d++) w[d] = ok ? __float_as_int(mid[d]) : 0;
+        w[4] = __double2loint(scale);
+        w[5] = __double2hiint(scale);
+        w[6] = __float_as_int(ok ? __double2float_ru(m * scale) : -1.f);
     }
     int n = 1, node = 0;  // lanes 0 .. n - 1 hold a node each
     for (int round = 0; round < 5; round++) {
@@ -619,7 +625,7 @@ __global__ void k_tri_records(int nt, const int *__restrict__ sorted_ids, const 
 // lattice of thin beams 23 and 164 instead of 166 and 225.
 //
 // Box frame: points are taken as (p - box_c) * box_scale, box_c the middle of the mesh's box (a float,
-// so p - box_c has one rounding) and box_scale 1 unless the mesh is larger than 2^60. M below is the
+// so p - box_c has one rounding) and box_scale a power of two (k_box_frame). M below is the
 // largest coordinate in that frame, u = 2^-24, d the distance from a query to a point q of the child.
 // Why the float box distance is a lower bound of d:
 // - With R the matrix of the three float axes, each axis' excess |axis.(p - centre)| - h is at most
@@ -651,17 +657,17 @@ __device__ __forceinline__ Vec3 vcross(Vec3 a, Vec3 b) {
 
 // Corners of the triangle at leaf position p in the box frame.
 __device__ __forceinline__ void frame_corners(const float4 *__restrict__ t32, const double2 *__restrict__ t64, int p,
-                                              const float (&mid)[3], float scale, Vec3 (&v)[3]) {
+                                              const float (&mid)[3], double s, Vec3 (&v)[3]) {
     if (t64) {
         const double2 *r = t64 + 5 * size_t(p);
         const double2 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2), d = __ldg(r + 3);
-        const double e = __ldg(&r[4].x), mx = mid[0], my = mid[1], mz = mid[2], s = scale;
+        const double e = __ldg(&r[4].x), mx = mid[0], my = mid[1], mz = mid[2];
         v[0] = {float((a.x - mx) * s), float((a.y - my) * s), float((b.x - mz) * s)};
         v[1] = {float((b.y - mx) * s), float((c.x - my) * s), float((c.y - mz) * s)};
         v[2] = {float((d.x - mx) * s), float((d.y - my) * s), float((e - mz) * s)};
     } else {
         const float4 a = __ldg(t32 + 3 * p), b = __ldg(t32 + 3 * p + 1);
-        const float e = __ldg(&t32[3 * p + 2].x);
+        const float e = __ldg(&t32[3 * p + 2].x), scale = float(s);  // beyond float's range: no query walks the boxes
         v[0] = {(a.x - mid[0]) * scale, (a.y - mid[1]) * scale, (a.z - mid[2]) * scale};
         v[1] = {(a.w - mid[0]) * scale, (b.x - mid[1]) * scale, (b.y - mid[2]) * scale};
         v[2] = {(b.z - mid[0]) * scale, (b.w - mid[1]) * scale, (e - mid[2]) * scale};
@@ -696,7 +702,8 @@ __global__ void __launch_bounds__(128) k_obb(int nnodes, int L, const int *__res
     const float4 r4 = nodes[4 * size_t(i) + 3];
     const int ref = __float_as_int(h ? r4.y : r4.x);
     const float mid[3] = {__int_as_float(frame[0]), __int_as_float(frame[1]), __int_as_float(frame[2])};
-    const float scale = __int_as_float(frame[3]), M = __int_as_float(frame[4]);
+    const double scale = __hiloint2double(frame[5], frame[4]);
+    const float M = __int_as_float(frame[6]);
     // child's axes, -centre coordinates and half extents (a box that culls nothing)
     Vec3 ax[3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
     const float inf = __int_as_float(0x7f800000);
@@ -721,7 +728,7 @@ __global__ void __launch_bounds__(128) k_obb(int nnodes, int L, const int *__res
                 const Vec3 c = vcross(e1, e2);
                 const float l2 = fmaxf(vdot(e1, e1), fmaxf(vdot(e2, e2), vdot(e3, e3)));
                 // all corners equal: no region test can err
-                const float al = l2 > 0.f ? l2 / sqrtf(vdot(c, c)) : 0.f;
+                const float al = l2 == 0.f ? 0.f : l2 / sqrtf(vdot(c, c));
                 alpha = al <= kObbMaxAlpha ? fmaxf(alpha, al) : FLT_MAX;  // a NaN or an overflow: too thin
                 grow = fmaxf(grow, al * sqrtf(l2));
                 ns = {ns.x + c.x, ns.y + c.y, ns.z + c.z};
@@ -815,8 +822,8 @@ __global__ void __launch_bounds__(128) k_obb(int nnodes, int L, const int *__res
             const float s = 1.f - 0x1p-18f;
             ax[0] = {s, 0.f, 0.f}, ax[1] = {0.f, s, 0.f}, ax[2] = {0.f, 0.f, s};
             for (int a = 0; a < 3; a++) {
-                const float lo = float((e[2 * a] - double(mid[a])) * double(scale));
-                const float hi = float((e[2 * a + 1] - double(mid[a])) * double(scale));
+                const float lo = float((e[2 * a] - double(mid[a])) * scale);
+                const float hi = float((e[2 * a + 1] - double(mid[a])) * scale);
                 half[a] = (0.5f * (hi - lo) + margin) * s;
                 off[a] = -0.5f * (lo + hi) * s;
             }
@@ -1037,7 +1044,7 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
     LAUNCH_CHECK("k_widen");
     // validation + per-triangle boxes
     // [0] first bad triangle, [1..6] scene, [7] scale, [8..9] depth / leaves, [10] ill, [11] largest
-    // filter bound term (float bits), [12] records unsafe for the float filter, [16..20] the box frame
+    // filter bound term (float bits), [12] records unsafe for the float filter, [16..22] the box frame
     int *flags;
     SSDF_CHECK(dalloc(tmp, &flags, 24, stream));
     k_init_flags<<<1, 32, 0, stream>>>(flags);
@@ -1078,9 +1085,9 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
     float4 *obb = nullptr;
     SSDF_CHECK(dalloc(s, &nodes32, 4 * size_t(m->nnodes), stream));
     if (query_boxes) SSDF_CHECK(dalloc(s, &obb, 8 * size_t(m->nnodes), stream));
-    // read back in one copy: flag words 7 to 19, the coordinate scale, depth and leaves, the three filter words
-    // and (from word 16) the box frame's four
-    constexpr int kFirstWord = 7, kWords = 13;
+    // read back in one copy: flag words 7 to 21, the coordinate scale, depth and leaves, the three filter words
+    // and (from word 16) the box frame's middle and scale
+    constexpr int kFirstWord = 7, kWords = 15;
     static_assert(kWords <= kReadbackWords, "read-back words");
     int *rb = nullptr;
     SSDF_CHECK(readback_words(&rb));
@@ -1141,7 +1148,7 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
     if (keep64) SSDF_CHECK(dalloc(s, &filt, 3 * size_t(nt), stream));  // the fix-up path's filter records
     int *entry;
     SSDF_CHECK(dalloc(s, &entry, 33, stream));
-    k_box_frame<<<1, 32, 0, stream>>>(nodes32, flags + 16, entry);
+    k_box_frame<<<1, 32, 0, stream>>>(nodes32, obb_nbox ? obb_nbox : box64, obb_nbox ? 1 : nt, flags + 16, entry);
     LAUNCH_CHECK("k_box_frame");
     k_tri_records<<<grid_blocks(nt, 256), 256, 0, stream>>>(nt, ids, s0, s1, s2, vx, vy, vz, t32, t64, filt,
                                                             flags + 16, flags + 10);
@@ -1159,12 +1166,13 @@ static int mesh_build_impl(MeshStorage *s, MeshStorage *tmp, DeviceMesh *m, int 
     memcpy(&scale, scale_word, sizeof(float));
     m->coord_scale = scale;
     memcpy(m->box_c, frame_words, 3 * sizeof(float));
-    memcpy(&m->box_scale, frame_words + 3, sizeof(float));
+    memcpy(&m->box_scale, frame_words + 4, sizeof(double));
+    m->box_scale_f = m->box_scale >= 0x1p-126 && m->box_scale <= 0x1p126 ? float(m->box_scale) : NAN;
     m->nill = filt_info[0];
     if (keep64) {
         float term;
         memcpy(&term, &filt_info[1], sizeof(float));
-        set_filter_window(m, term, filt_info[2] == 0);
+        set_filter_window(m, term, filt_info[2] == 0 && m->box_scale == 1.0);
     }
     m->depth = nt <= L ? 1 : depth_leaves[0];
     m->nleaves = nt <= L ? 1 : depth_leaves[1];
