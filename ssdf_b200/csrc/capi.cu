@@ -627,6 +627,7 @@ int ssdf_mesh_create(ssdf_mesh **mesh, ptrdiff_t nselements, const int *s0, cons
         o.leaf_size = 0, o.keep_fp64 = 1, o.normals = 1, o.treelet_opt = kResidentTreeletRounds;
     }
     if (!device_ptrs) SSDF_CHECK(check_mesh_host(nselements, s0, s1, s2, nspoints, sx, sy, sz));
+    if (nselements >= kMaxTriangles) return fail(SSDF_ERR_NOT_SUPPORTED, "2^26 triangles or more in one mesh");
     cudaStream_t s = (cudaStream_t)stream;
     ssdf_mesh *h = new ssdf_mesh();
     cudaGetDevice(&h->device);

@@ -46,7 +46,8 @@ int celllist_edf(int f64, ptrdiff_t npoints, const void *x, const void *y, const
     SSDF_CHECK(mesh_build(&h.mesh.storage, &h.mesh.m, nt, s0, s1, s2, nv, sx, sy, sz, f64, /*device_ptrs=*/1, bo,
                           stream));
     ssdf_query_opts qo{};
-    qo.precision = f64 ? SSDF_PREC_F32_FIXUP : SSDF_PREC_F32;
+    // (a fix-up launch takes one query less than this call)
+    qo.precision = !f64 ? SSDF_PREC_F32 : (npoints < 0x7fffffff ? SSDF_PREC_F32_FIXUP : SSDF_PREC_F64);
     qo.output = SSDF_OUT_EDF;
     qo.coord_type = qo.out_type = f64 ? SSDF_F64 : SSDF_F32;
     QueryArgs a;

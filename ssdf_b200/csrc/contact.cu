@@ -387,6 +387,7 @@ struct MeshHold {
 // A mesh for the contact walks: the axis-aligned tree and the float records alone.
 int contact_mesh(MeshHold *mh, ptrdiff_t nt, const int *s0, const int *s1, const int *s2, ptrdiff_t nv, const void *sx,
                  const void *sy, const void *sz, int coord_f64, int device_ptrs, long long nqueries) {
+    if (nt >= kMaxTriangles) return fail(SSDF_ERR_NOT_SUPPORTED, "2^26 triangles or more in one mesh");
     ssdf_build_opts bo;
     bo.leaf_size = env_int("SSDF_B200_LEAF", 0), bo.keep_fp64 = 0, bo.normals = 0;
     bo.treelet_opt = call_treelet_rounds(nqueries);

@@ -1193,7 +1193,7 @@ int mesh_build(MeshStorage **storage, DeviceMesh *mesh, ptrdiff_t nt, const int 
                ptrdiff_t nv, const void *sx, const void *sy, const void *sz, int coord_f64, int device_ptrs,
                const ssdf_build_opts &opts, cudaStream_t stream, bool query_boxes, bool check_indices) {
     if (nt <= 0 || nv <= 0) return fail(SSDF_ERR_INVALID_ARGUMENT, "empty mesh");
-    if (nt >= kMaxTriangles) return fail(SSDF_ERR_NOT_SUPPORTED, "more than 2^26 triangles in one mesh");
+    if (nt > kMaxTriangles) return fail(SSDF_ERR_NOT_SUPPORTED, "more than 2^26 triangles in one mesh");
     if (nv >= (1ll << 31)) return fail(SSDF_ERR_NOT_SUPPORTED, "more than 2^31 vertices");
     if (opts.leaf_size < 0 || opts.leaf_size > kMaxLeafSize)
         return fail(SSDF_ERR_INVALID_ARGUMENT, "leaf_size must be 0 (default) or 1.." + std::to_string(kMaxLeafSize));
