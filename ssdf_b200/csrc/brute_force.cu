@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(kBruteThreads) k_brute_tile(int npoints, const
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw);
     T *buf = reinterpret_cast<T *>(smem_raw + 128);
+    if (*err != kNoBadTriangle) return;  // the call is refused: out stays as it is
     const int p = blockIdx.x * kBruteThreads + threadIdx.x;
     const bool valid = p < npoints;
     const T margin = abs_margin<T>(__int_as_float(*scale_bits));
@@ -174,7 +175,9 @@ __global__ void __launch_bounds__(kBruteThreads) k_brute_warp(int npoints, const
                                                               int nt, const T *__restrict__ rec, T *__restrict__ out,
                                                               int *__restrict__ outtri,
                                                               const int *__restrict__ scale_bits,
+                                                              const int *__restrict__ err,
                                                               unsigned long long *__restrict__ counters) {
+    if (*err != kNoBadTriangle) return;  // the call is refused: out stays as it is
     unsigned long long n_tri = 0, n_box = 0;
     const int warp = (blockIdx.x * kBruteThreads + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -249,10 +252,10 @@ int brute_impl(ptrdiff_t npoints, const T *x, const T *y, const T *z, ptrdiff_t 
             const long long threads = (long long)npoints * 32;
             if (count)
                 k_brute_warp<T, true><<<grid_blocks(threads, kBruteThreads), kBruteThreads, 0, stream>>>(
-                    int(npoints), x, y, z, int(nt), rec, out, outtri, flags + 2, counters);
+                    int(npoints), x, y, z, int(nt), rec, out, outtri, flags + 2, flags, counters);
             else
                 k_brute_warp<T, false><<<grid_blocks(threads, kBruteThreads), kBruteThreads, 0, stream>>>(
-                    int(npoints), x, y, z, int(nt), rec, out, outtri, flags + 2, counters);
+                    int(npoints), x, y, z, int(nt), rec, out, outtri, flags + 2, flags, counters);
         } else {
             const size_t smem = 128 + 2 * size_t(TILE) * kRec * sizeof(T);
             auto kern = count ? k_brute_tile<T, TILE, true> : k_brute_tile<T, TILE, false>;
