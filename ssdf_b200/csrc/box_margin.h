@@ -33,6 +33,6 @@ SSDF_BOX_MARGIN_FN float float_box_margin(float c) { return fmaxf(c * 0x1p-16f, 
 // best + (2^-16 c)^2. A best of +inf is taken as the largest finite one: a box farther than that holds no
 // triangle with a finite float distance.
 SSDF_BOX_MARGIN_FN float float_box_reach(float best, float margin, float s) {
-    const float b = fminf(best, FLT_MAX), d = (sqrtf(b) + 0x1p-5f * margin) * s, near = margin * s;
+    const float b = best > FLT_MAX ? FLT_MAX : best, d = (sqrtf(b) + 0x1p-5f * margin) * s, near = margin * s;
     return fmaxf(d * d, b * s * s + near * near) * (1.0f + 1.0f / 65536.0f);
 }

@@ -352,7 +352,7 @@ struct FastPolicy {
         bx[q] = twice(x), by[q] = twice(y), bz[q] = twice(z), best[q] = init, evicted[q] = finf(), used[q] = 0;
         // a NaN or infinite coordinate: no finite distance, nothing to walk for
         const bool finite = isfinite(x) && isfinite(y) && isfinite(z);
-        thr[q] = finite ? window_thr(init, tau_rel, m.coord_scale) : -1.f;
+        thr[q] = finite && !(init < 0.f) ? window_thr(init, tau_rel, m.coord_scale) : -1.f;  // no distance is below 0
     }
     __device__ __forceinline__ void disable(int q) {
         set(q, kNowhere, kNowhere, kNowhere, finf());
@@ -1020,7 +1020,7 @@ struct LaneWalk {
     // the threshold the incoming bound allows
     __device__ __forceinline__ float start_thr() const {
         if constexpr (PREC == SSDF_PREC_F32_FIXUP)
-            return window_thr(d2 < T(dinf()) ? __double2float_ru(d2) : finf(), tau_rel, m.coord_scale);
+            return d2 < T(0) ? -1.f : window_thr(d2 < T(dinf()) ? __double2float_ru(d2) : finf(), tau_rel, m.coord_scale);
         else
             return ExactData<T>::box_thr(d2, margin, m);
     }
