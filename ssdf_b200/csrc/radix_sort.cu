@@ -63,16 +63,16 @@ constexpr unsigned long long kTileOwn = 1;   // the tile's own count
 constexpr unsigned long long kTileUpTo = 2;  // the count of all tiles up to this one
 // Polls of a word before the tile counts its predecessors' keys itself. Tiles are numbered in the order they
 // start, so a predecessor is always running and the wait is short; the bound only makes that unconditional.
-// SSDF_B200_SORT_POLLS lowers it, to 0 for tiles that look at no word and count for themselves (tests).
 constexpr int kMaxPolls = 1 << 16;
 
-// One pass. tile_words: [tile * 256 + digit], zeroed before; next_tile: zeroed before.
-template <typename K>
+// One pass. tile_words: [tile * 256 + digit], zeroed before; next_tile: zeroed before. ALONE: tiles look at no word
+// and count for themselves (SSDF_B200_SORT_ALONE=1, for tests; an instantiation of its own, since polls given as
+// an argument cost 15 us of 5,285 on 4,000,000 points).
+template <typename K, bool ALONE>
 __global__ void __launch_bounds__(kSortThreads) k_sort_pass(const K *__restrict__ kin, const int *__restrict__ vin,
                                                             K *__restrict__ kout, int *__restrict__ vout, int n,
                                                             int shift, const unsigned *__restrict__ counts,
-                                                            unsigned long long *tile_words, int *next_tile,
-                                                            int max_polls) {
+                                                            unsigned long long *tile_words, int *next_tile) {
     __shared__ unsigned cnt[kSortWarps][256];
     __shared__ unsigned tile_start[256], to_global[256];
     __shared__ unsigned warp_tot[kSortWarps], digit_tot[kSortWarps];
@@ -134,8 +134,9 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_pass(const K *__restrict_
     unsigned long long prev = 0;
     for (int t = tile - 1; t >= 0; t--) {
         volatile const unsigned long long *const word = tile_words + (long long)t * 256 + digit;
-        unsigned long long w = 0;
-        for (int poll = 0; (w & 3) == 0 && poll < max_polls; poll++) w = *word;
+        unsigned long long w = ALONE ? 0 : *word;
+        if (!ALONE)
+            for (int poll = 0; (w & 3) == 0 && poll < kMaxPolls; poll++) w = *word;
         if ((w & 3) == 0) {  // count tile t's keys
             const long long end = (long long)(t + 1) * kSortTile;
             for (long long i = (long long)t * kSortTile; i < end; i++) prev += int((kin[i] >> shift) & 0xff) == digit;
@@ -232,7 +233,7 @@ static int radix_sort_pairs(K *keys, int *vals, int n, int key_bits, cudaStream_
     if (n <= 1) return SSDF_OK;
     const int ntiles = int(((long long)n + kSortTile - 1) / kSortTile);
     const int passes = (key_bits + 7) / 8;
-    const int polls = env_int("SSDF_B200_SORT_POLLS", kMaxPolls), max_polls = polls < 0 ? 0 : (polls < kMaxPolls ? polls : kMaxPolls);
+    const bool alone = env_int("SSDF_B200_SORT_ALONE", 0) != 0;
     // scratch: the second keys and values, then (zeroed) the tile words, the digit counts and the tile tickets
     const size_t words = size_t(passes) * ntiles * 256 * sizeof(unsigned long long);
     const size_t zeroed = words + size_t(passes) * 256 * sizeof(unsigned) + size_t(passes) * sizeof(int);
@@ -247,15 +248,20 @@ static int radix_sort_pairs(K *keys, int *vals, int n, int key_bits, cudaStream_
     int *tickets = reinterpret_cast<int *>(counts + passes * 256);
     cudaError_t e = cudaMemsetAsync(tile_words, 0, zeroed, stream);
     if (e == cudaSuccess) {
-        const int blocks = ntiles < 148 * 4 ? ntiles : 148 * 4;
+        const int blocks = ntiles < 148 * 4 ? ntiles : 148 * 4;  // at most four an SM
         k_digit_counts<K><<<blocks, kSortThreads, 0, stream>>>(keys, n, passes, counts);
         e = cudaGetLastError();
     }
     K *kin = keys, *kout = k2;
     int *vin = vals, *vout = v2;
     for (int p = 0; p < passes && e == cudaSuccess; p++) {
-        k_sort_pass<K><<<ntiles, kSortThreads, 0, stream>>>(kin, vin, kout, vout, n, 8 * p, counts + p * 256,
-                                                           tile_words + size_t(p) * ntiles * 256, tickets + p, max_polls);
+        unsigned long long *const pass_words = tile_words + size_t(p) * ntiles * 256;
+        if (alone)
+            k_sort_pass<K, true><<<ntiles, kSortThreads, 0, stream>>>(kin, vin, kout, vout, n, 8 * p, counts + p * 256,
+                                                                      pass_words, tickets + p);
+        else
+            k_sort_pass<K, false><<<ntiles, kSortThreads, 0, stream>>>(kin, vin, kout, vout, n, 8 * p, counts + p * 256,
+                                                                       pass_words, tickets + p);
         e = cudaGetLastError();
         K *tk = kin;
         kin = kout;

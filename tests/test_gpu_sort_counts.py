@@ -1,6 +1,6 @@
 """GPU: a sort tile that gives up on its predecessors' published counts counts their keys itself. Tiles wait
-tens of thousands of polls, so that never happens by itself; with no polls every tile counts for itself, with
-one some do. Builds (30-bit keys, 64-bit edge keys for the pseudo-normals) and point orders are the same."""
+tens of thousands of polls, so that never happens by itself; here every tile counts for itself. Builds (30-bit
+keys, 64-bit edge keys for the pseudo-normals) and point orders are the same."""
 
 import numpy as np
 import pytest
@@ -24,15 +24,14 @@ def answers(mesh, pts):
     return out.cpu().numpy(), tri.cpu().numpy(), stats
 
 
-@pytest.mark.parametrize("polls", ["0", "1"])
 @pytest.mark.parametrize("n", [2048, 2049, 4097, 26625, 100003])
-def test_tiles_that_count_for_themselves(n, polls, monkeypatch):
+def test_tiles_that_count_for_themselves(n, monkeypatch):
     nu = max(24, int(np.sqrt(n)))
     mesh = W.torus(nu=nu, nv=nu // 2, jitter=0.01)
     pts = np.random.default_rng(n).uniform(-1.5, 1.5, (n, 3)).T.copy()
     monkeypatch.setenv("SSDF_B200_WARP_POINTS", "0")
     want = answers(mesh, pts)
-    monkeypatch.setenv("SSDF_B200_SORT_POLLS", polls)
+    monkeypatch.setenv("SSDF_B200_SORT_ALONE", "1")
     got = answers(mesh, pts)
     assert got[2] == want[2]
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
