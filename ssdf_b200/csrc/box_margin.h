@@ -16,7 +16,6 @@
 // tests/box_margin_check.c looks for the largest need. Plain C, for that check.
 #pragma once
 
-#include <float.h>
 #include <math.h>
 
 #ifdef __CUDACC__
@@ -29,10 +28,15 @@
 // of that number, which is as near as the float arithmetic tells distances apart.
 SSDF_BOX_MARGIN_FN float float_box_margin(float c) { return fmaxf(c * 0x1p-16f, 0x1p-63f); }
 
-// The squared distance in the box frame (scale s) below which a box is entered: (sqrt(best) + 8 u c)^2, and at least
-// best + (2^-16 c)^2. A best of +inf is taken as the largest finite one: a box farther than that holds no
-// triangle with a finite float distance.
-SSDF_BOX_MARGIN_FN float float_box_reach(float best, float margin, float s) {
-    const float b = best > FLT_MAX ? FLT_MAX : best, d = (sqrtf(b) + 0x1p-5f * margin) * s, near = margin * s;
-    return fmaxf(d * d, b * s * s + near * near) * (1.0f + 1.0f / 65536.0f);
+// The squared distance below which a box is entered: (sqrt(best) + 8 u c)^2, and at least best + (2^-16 c)^2.
+SSDF_BOX_MARGIN_FN float float_box_reach(float best, float margin) {
+    const float d = sqrtf(best) + 0x1p-5f * margin;
+    return fmaxf(d * d, best + margin * margin) * (1.0f + 1.0f / 65536.0f);
+}
+
+// The same, in a box frame of scale s, where no distance is known: a box farther than this holds no triangle
+// whose float squared distance is finite (below 2^128).
+SSDF_BOX_MARGIN_FN float float_box_limit(float margin, float s) {
+    const float d = (0x1p64f + 0x1p-5f * margin) * s;
+    return d * d * (1.0f + 1.0f / 65536.0f);
 }

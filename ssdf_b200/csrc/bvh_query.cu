@@ -191,6 +191,9 @@ struct ExactData<double> {
         const double t = (best * (1.0 + 1.0 / 65536.0) + margin) * (m.box_scale * m.box_scale);
         return fmaxf(__double2float_ru(t), FLT_MIN);  // a box at distance 0 is always wanted
     }
+    static __device__ __forceinline__ float start_thr(double init, double margin, const DeviceMesh &m) {
+        return box_thr(init, margin, m);
+    }
     static __device__ __forceinline__ float box_coord(double p, int d, const DeviceMesh &m) {
         return float((p - double(m.box_c[d])) * m.box_scale);
     }
@@ -208,7 +211,11 @@ struct ExactData<float> {
     // the prune threshold's margins (box_margin.h)
     static __device__ __forceinline__ float margin(const DeviceMesh &m) { return float_box_margin(m.coord_scale); }
     static __device__ __forceinline__ float box_thr(float best, float margin, const DeviceMesh &m) {
-        return fmaxf(float_box_reach(best, margin, m.box_scale_f), FLT_MIN);
+        return fmaxf(float_box_reach(best, margin) * m.box_scale_f * m.box_scale_f, FLT_MIN);
+    }
+    // the threshold a walk starts with, from an incoming bound that may be infinite
+    static __device__ __forceinline__ float start_thr(float init, float margin, const DeviceMesh &m) {
+        return init > FLT_MAX ? fmaxf(float_box_limit(margin, m.box_scale_f), FLT_MIN) : box_thr(init, margin, m);
     }
     static __device__ __forceinline__ float box_coord(float p, int d, const DeviceMesh &m) {
         return (p - m.box_c[d]) * m.box_scale_f;
@@ -250,7 +257,7 @@ struct ExactPolicy {
         bz[q] = twice(ExactData<T>::box_coord(z, 2, m));
         const T lim = ExactData<T>::beyond(m);
         const bool finite = fabs(x) < lim && fabs(y) < lim && fabs(z) < lim;
-        thr[q] = finite ? ExactData<T>::box_thr(init, margin, m) : -1.f;
+        thr[q] = finite ? ExactData<T>::start_thr(init, margin, m) : -1.f;
     }
     __device__ __forceinline__ void disable(int q) {
         px[q] = py[q] = pz[q] = T(0), best[q] = T(0), bid[q] = -1, bpos[q] = -1;
@@ -1022,7 +1029,7 @@ struct LaneWalk {
         if constexpr (PREC == SSDF_PREC_F32_FIXUP)
             return d2 < T(0) ? -1.f : window_thr(d2 < T(dinf()) ? __double2float_ru(d2) : finf(), tau_rel, m.coord_scale);
         else
-            return ExactData<T>::box_thr(d2, margin, m);
+            return ExactData<T>::start_thr(d2, margin, m);
     }
     // the threshold the whole warp's finds allow (warp-wide)
     __device__ __forceinline__ float found_thr() const {

@@ -3,7 +3,7 @@
  * needs. A triangle's oriented box, built as mesh_build.cu's k_obb builds it in the frame of a mesh of half
  * size 1, is restated here with the reference's float distance (device_geom.cuh, tri_dist_sq_exact) and
  * the box distance (obb_pair). The box must be entered while the triangle's own float distance is the best:
- *     box distance < float_box_reach(distance, float_box_margin(c), 1),   c the mesh's largest coordinate.
+ *     box distance < float_box_reach(distance, float_box_margin(c)),   c the mesh's largest coordinate.
  * Triangles lie 1 to 3e5 mesh sizes from the origin, most across the direction to it (where the closest
  * point's rounding adds up), given in floats or doubles; points lie 1e-5 c to 0.06 c off them. Prints the number
  * of cases, of boxes that were not entered, and the largest need: k of (sqrt(distance) + k u c)^2, u = 2^-24.
@@ -141,7 +141,7 @@ int main(int argc, char **argv) {
         }
         const float margin = float_box_margin(c);
         done++;
-        left_out += !(box < float_box_reach(d2, margin, 1.f));
+        left_out += !(box < float_box_reach(d2, margin));
         if (box >= (d2 + margin * margin) * (1.f + 0x1p-16f))  // else the near margin alone admits it
             worst = fmax(worst, (sqrt(box / (1.0 + 0x1p-16)) - sqrt((double)d2)) / (0x1p-24 * c));
     }
