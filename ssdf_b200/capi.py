@@ -642,7 +642,7 @@ class DeviceMesh:
     def from_device(cls, s0, s1, s2, sx, sy, sz, keep_fp64=True, normals=False, leaf_size=0, treelet=True,
                     stream=None):
         """A mesh from device arrays (torch CUDA tensors: int32 indices, one float dtype for the
-        vertices), built without a host round trip."""
+        vertices); no array passes through the host. treelet: rounds of refinement (True: one)."""
         self = cls.__new__(cls)
         self._h = C.c_void_p()
         opts = BuildOpts(int(leaf_size), int(keep_fp64), int(normals), int(treelet))
@@ -718,7 +718,7 @@ class Batch:
             pass
 
     def reserve(self, max_queries, stream=None):
-        """Pre-size the fix-up overflow lists for runs of up to max_queries queries."""
+        """Pre-size the hand-over lists for runs of up to max_queries queries."""
         _check(lib.ssdf_batch_reserve(self._h, int(max_queries), _stream_handle(stream)), "ssdf_batch_reserve")
 
     def clear(self):

@@ -44,8 +44,9 @@ namespace {
 
 constexpr int kThreads = 128;
 // F32X window slots: candidates kept per query in shared memory. A window that overflows them sends
-// its query to the second stage (k_window). On the torus-knot 256^3 grid: 8 slots overflow 0.72% of
-// the queries (22.9 ms), 12 slots 0.01% (21.6 ms), 16 slots none (23.2 ms: the longer insertion).
+// its query to the second stage (k_window). Torus-knot 256^3 grid: 11.1 ms with 8 slots, 10.8 with 10, 10.0 with
+// 12, which overflow on 0.01 % of the queries. (16, with none there and a longer insertion, were slower on an
+// earlier kernel and not measured again.)
 #ifndef SSDF_B200_WINDOW_SLOTS
 #define SSDF_B200_WINDOW_SLOTS 12
 #endif
@@ -60,8 +61,8 @@ constexpr int kCand = SSDF_B200_WINDOW_SLOTS;
 #define SSDF_B200_QUERY_MIN_BLOCKS 7
 #endif
 
-// The double kernel keeps 5 resident blocks per SM (at most 102 registers), its occupancy before the
-// seeded column walk added a few live values.
+// The double kernel keeps 5 resident blocks per SM (at most 102 registers), chosen when it walked double boxes and
+// not measured again since.
 constexpr int kF64MinBlocks = 5;
 
 struct Counters {
@@ -575,18 +576,10 @@ __device__ __forceinline__ void traverse_packet(P &p, Counters &cnt, int budget)
     }
 }
 
-// Nearest-child-first traversal with a per-lane stack of (node, smallest box distance), culled on
-// pop. WARP = false: every thread walks its own queries. WARP = true (packet): the 32 lanes of a
-// warp walk one path together -- a child is entered if any lane wants it, the nearer child is the
-// one the brick's centre lane ranks first (traverse_packet) -- so node and triangle loads are
-// warp-uniform (broadcast) and leaf work does not diverge. Every lane must call it
-// (warp-synchronous when WARP).
-template <bool WARP, bool COUNT, class P>
-__device__ __forceinline__ void traverse(P &p, Counters &cnt, int budget) {
-    if constexpr (WARP) {
-        traverse_packet<COUNT>(p, cnt, budget);
-        return;
-    }
+// Nearest-child-first traversal of every thread for its own queries, with a stack of (node, smallest box
+// distance) culled on pop.
+template <bool COUNT, class P>
+__device__ __forceinline__ void traverse_thread(P &p, Counters &cnt) {
     using R = typename P::R;
     constexpr int Q = P::kQn;
     int snode[kStackSize];
@@ -599,8 +592,7 @@ __device__ __forceinline__ void traverse(P &p, Counters &cnt, int budget) {
         p.boxes(node, d0, d1, r0, r1);
         if (COUNT) cnt.box += 2 * Q;
         R k0 = min_of<R, Q>(d0), k1 = min_of<R, Q>(d1);
-        const bool swap = WARP ? (__popc(__ballot_sync(0xffffffffu, k1 < k0)) > 16) : (k1 < k0);
-        if (swap) {
+        if (k1 < k0) {
 #pragma unroll
             for (int q = 0; q < Q; q++) {
                 const R t = d0[q];
@@ -619,7 +611,7 @@ __device__ __forceinline__ void traverse(P &p, Counters &cnt, int budget) {
         for (int h = 0; h < 2; h++) {
             const int rc = h ? r1 : r0;
             const unsigned m = rc == kEmptyRef ? 0u : (h ? want_mask(p, d1) : want_mask(p, d0));
-            if (WARP ? !__any_sync(0xffffffffu, m != 0u) : m == 0u) continue;
+            if (m == 0u) continue;
             if (rc < 0) {
                 p.template leaf<COUNT>(leaf_first(rc), leaf_count(rc), m, cnt);
             } else if (next < 0) {
@@ -634,8 +626,7 @@ __device__ __forceinline__ void traverse(P &p, Counters &cnt, int budget) {
             const R tmax = p.max_thr();
             while (sp > 0) {
                 sp--;
-                const bool w = sdist[sp] < tmax;
-                if (WARP ? __any_sync(0xffffffffu, w) : w) {
+                if (sdist[sp] < tmax) {
                     next = snode[sp];
                     break;
                 }
@@ -644,6 +635,16 @@ __device__ __forceinline__ void traverse(P &p, Counters &cnt, int budget) {
         }
         node = next;
     }
+}
+
+// WARP: the 32 lanes of a warp walk one path together (every lane must call it), so node and triangle loads are
+// broadcasts and leaf work does not diverge; else every thread walks by itself.
+template <bool WARP, bool COUNT, class P>
+__device__ __forceinline__ void traverse(P &p, Counters &cnt, int budget) {
+    if constexpr (WARP)
+        traverse_packet<COUNT>(p, cnt, budget);
+    else
+        traverse_thread<COUNT>(p, cnt);
 }
 
 // ---- outputs ----------------------------------------------------------------------------------------
@@ -966,9 +967,11 @@ __global__ void __launch_bounds__(kThreads, PREC == SSDF_PREC_F64 ? kF64MinBlock
 //
 // A query whose window overflowed its slots is walked again from its final window, and a query whose
 // packet ran out of budget from the window it had then: every triangle whose float distance is
-// inside the window is re-evaluated in double. The window only shrinks (after each step, to what the
-// warp's smallest non-proxy key allows, by the first stage's rule), so the visiting order is free,
-// and the warp walks the tree breadth-parallel: each step
+// inside the window is re-evaluated in double. The window only shrinks: after each step, by the first stage's
+// rule, to what the warp's smallest non-proxy key allows, or the smallest double distance found where that is
+// nearer (it bounds the winner's distance as a key does, without a key's error; beside needles, whose proxies'
+// keys count for nothing, it is all there is: 24^3 nodes at 2,000 needles 3,251 -> 303 us). So the visiting
+// order is free, and the warp walks the tree breadth-parallel: each step
 // the 32 lanes take up to 32 nodes from the warp's shared stack, test their children, run the
 // wanted leaves, and push the wanted internal children (ballot-compacted). A lane keeps the
 // lexicographic (d^2, index) minimum of the triangles it evaluated (the incoming bound ranks -1, so
@@ -1478,6 +1481,8 @@ __global__ void k_point_keys(long long n, const void *__restrict__ x, const void
 // 2,329, 145^3 (23) 3,192 / 2,922 / 2,954, 180^3 (44) 5,160 / 4,699 / 4,481, 200^3 (60) 6,574 / 5,945 /
 // 5,563 / 5,575, 256^3 (127) 12,111 / 10,864 / 10,190 / 9,910, 400^3 (483) 38,789 / 34,249 / 31,691 / 30,203;
 // 41,006-triangle torus 150^3 (25) 2,417 / 2,625 / 2,994, 256^3 7,658 / 7,461 / 7,430 / 7,618.
+// The double kernel takes the same steps, by the float kernels' blocks per SM, without sweeps of its own; the knot's
+// 128^3 grid in double loses by it (2,582 us with the rule of four waves, 2,753 with this one).
 constexpr long long kGridWaves = 10;
 
 int grid_steps_for(long long one_step_blocks) {
@@ -1503,7 +1508,8 @@ void set_grid_steps(QueryArgs *a) {
 }
 
 // Measured on B200 over axis-aligned boxes: the torus knot with 29 % of its triangles slivers still ran 1.4x
-// faster on the fix-up path than on FP64; the beam lattice (64 % slivers, in parallel bundles) ran 5x slower.
+// faster on the fix-up path than on FP64; the beam lattice (64 % slivers, in parallel bundles) ran 5x slower. Not
+// measured again over oriented boxes, with which the two kernels are closer.
 constexpr double kIllMaxFraction = 0.5;
 
 // The fix-up path hands a mesh to the FP64 kernel when more than this fraction of its triangles are

@@ -34,7 +34,7 @@ int cuda_fail(cudaError_t err, const char *what, const char *file, int line);
 // ---- device layouts ------------------------------------------------------------------------------
 //
 // BVH: binary, child-box layout. Every internal node holds both children's boxes and references,
-// so one visit tests two boxes from one 64-byte (FP32) or 128-byte (FP64) record:
+// so one visit tests two boxes from one record, 64 bytes (axis-aligned) or 128 (oriented):
 //   FP32 node (4 x float4): (c0.lox, c0.hix, c0.loy, c0.hiy), (c1.lox, c1.hix, c1.loy, c1.hiy),
 //                           (c0.loz, c0.hiz, c1.loz, c1.hiz), (ref0, ref1, -, -) as int bits
 //   oriented node (8 x float4): the same children's oriented boxes in the mesh's box frame (see

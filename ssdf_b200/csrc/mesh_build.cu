@@ -5,10 +5,11 @@
 //   1. validate indices, gather vertices, triangle boxes (FP32 and FP64), scene box of centroids;
 //   2. 30-bit Morton codes of the centroids, stable radix sort (radix_sort.cu);
 //   3. Karras LBVH topology over the sorted primitives (index tie-break for equal codes);
-//   4. bottom-up refit with per-node arrival counters;
+//   4. node boxes as unions of leaf ranges (k_boxes_inside, k_boxes_across);
 //   5. optional SAH treelet refinement (treelet_opt.cu);
 //   6. node records in the child-box layout, subtrees of <= leaf_size triangles collapsed into
-//      leaves, triangle records in leaf order (internal.h documents both layouts);
+//      leaves, triangle records in leaf order, oriented boxes of the same children (internal.h documents the
+//      layouts);
 //   7. optional angle-weighted pseudo-normals (serial/bvh/bvh.cpp:1669-1721), summed in the
 //      reference's order so they are bitwise its values up to the last bit of acos.
 #include <cuda_runtime.h>
