@@ -332,7 +332,7 @@ int ssdf_batch_run(ssdf_batch *b, int use_graph, void *stream_) {
     int k = 0, k64 = 0;
     for (int r = 0; r < njobs; r++) {
         QueryArgs a = b->jobs[order[r]];
-        a.warp_budget = resolve_warp_budget(a.warp_budget, nq, a.m.nt, a.is_grid != 0);
+        resolve_hand_over(&a, fixup && !to_f64(a), nq);
         set_grid_steps(&a);
         if (a.is_grid && (!fixup || to_f64(a))) a.grid_steps = std::max(a.grid_steps, steps64);
         if (sort_points && !a.is_grid && a.npoints >= kSortMinPoints) {

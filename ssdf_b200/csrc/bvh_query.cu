@@ -242,7 +242,7 @@ template <typename T, int Q>
 struct ExactPolicy {
     using R = float;
     static constexpr int kQn = Q;
-    static constexpr bool kVote = sizeof(T) == sizeof(float);
+    static constexpr bool kVote = sizeof(T) == sizeof(float), kRestarts = false;
     const DeviceMesh &m;
     T px[Q], py[Q], pz[Q], best[Q];
     float2 bx[Q], by[Q], bz[Q];  // the point in the box frame, each coordinate twice (two-wide FP32)
@@ -345,7 +345,7 @@ template <int Q>
 struct FastPolicy {
     using R = float;
     static constexpr int kQn = Q;
-    static constexpr bool kVote = true;
+    static constexpr bool kVote = true, kRestarts = true;
     const DeviceMesh &m;
     float2 bx[Q], by[Q], bz[Q];  // the point in the box frame (the filter records' too), each coordinate twice
     float best[Q], thr[Q], evicted[Q];
@@ -376,6 +376,11 @@ struct FastPolicy {
             best[q] = d2;
             thr[q] = window_thr(best[q], tau_rel, m.coord_scale);
         }
+    }
+    // the walk starts over with the windows it has
+    __device__ __forceinline__ void restart() {
+#pragma unroll
+        for (int q = 0; q < Q; q++) used[q] = 0, evicted[q] = finf();
     }
     // the walk stops early: every live query goes to the second stage with its current window
     __device__ __forceinline__ void abandon() {
@@ -494,6 +499,18 @@ __device__ __forceinline__ float warp_max(float v) {
     return __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(v)));
 }
 
+// The next node of the packet's stack that some lane still wants (-1: none). An entry: node, key bits.
+template <class P>
+__device__ __forceinline__ int next_entry(const P &p, const int2 *const entry, int &sp) {
+    const float tmax = warp_max(p.max_thr());
+    while (sp > 0) {
+        sp--;
+        const int2 e = entry[sp];
+        if (__int_as_float(e.y) < tmax) return e.x;
+    }
+    return -1;
+}
+
 // Packet walk (a grid warp as one packet): the node ids on the stack are the same in every lane, so
 // the warp keeps one stack in shared memory instead of 32 copies in local memory. An entry keeps
 // the smallest box distance over the warp's lanes and is entered on pop while that is below the
@@ -502,18 +519,17 @@ __device__ __forceinline__ float warp_max(float v) {
 // Of two wanted children the one the packet's lanes (packet_rankers) rank first is the nearer; a
 // wanted leaf is tested at once, and when it was the nearer one the other child is asked for again, its lanes'
 // thresholds having shrunk.
+//
+// Walks from `node` with sp nodes on the stack. Past its budget (checked where a path ends) the walk stops and returns
+// how many nodes the stack still holds, else -1.
 template <bool COUNT, class P>
-__device__ __forceinline__ void traverse_packet(P &p, Counters &cnt, int budget) {
+__device__ __forceinline__ int traverse_packet(P &p, Counters &cnt, int budget, int2 *const entry, int node, int sp) {
     constexpr int Q = P::kQn;
     constexpr unsigned kAll = 0xffffffffu;
     int work = 0;  // triangle records the packet has tested (the same in every lane)
     if (budget <= 0) budget = 0x7fffffff;
-    __shared__ int2 s_entry[kThreads / 32][kStackSize];  // node, key bits
-    int2 *const entry = s_entry[threadIdx.x >> 5];
     const unsigned rankers = packet_rankers<P>(__ballot_sync(kAll, p.max_thr() > 0.f));
     const int half = __popc(rankers) / 2;
-    int sp = 0;
-    int node = 0;
     auto test_leaf = [&](int ref, unsigned m) {
         p.template leaf<COUNT>(leaf_first(ref), leaf_count(ref), m, cnt);
         work += leaf_count(ref);
@@ -557,20 +573,9 @@ __device__ __forceinline__ void traverse_packet(P &p, Counters &cnt, int budget)
             else next = r;
         }
         if (next < 0) {
-            if (work > budget) {  // warp-uniform; checked where a path ends
-                p.abandon();
-                break;
-            }
-            const float tmax = warp_max(p.max_thr());
-            while (sp > 0) {
-                sp--;
-                const int2 e = entry[sp];
-                if (__int_as_float(e.y) < tmax) {
-                    next = e.x;
-                    break;
-                }
-            }
-            if (next < 0) break;
+            if (work > budget) return sp;  // warp-uniform
+            next = next_entry(p, entry, sp);
+            if (next < 0) return -1;
         }
         node = next;
     }
@@ -638,13 +643,32 @@ __device__ __forceinline__ void traverse_thread(P &p, Counters &cnt) {
 }
 
 // WARP: the 32 lanes of a warp walk one path together (every lane must call it), so node and triangle loads are
-// broadcasts and leaf work does not diverge; else every thread walks by itself.
+// broadcasts and leaf work does not diverge; else every thread walks by itself. A packet past its budget hands
+// over while the list is short (QueryArgs::hand_most). Else it walks on without one; the fix-up's packets
+// from the root again, with the windows they have: they seldom do, and a walk that can be entered anywhere cost
+// every packet 2.5 % (knot 256^3 9,887 -> 10,143 us, spheres' 160^3 7 %).
 template <bool WARP, bool COUNT, class P>
-__device__ __forceinline__ void traverse(P &p, Counters &cnt, int budget) {
-    if constexpr (WARP)
-        traverse_packet<COUNT>(p, cnt, budget);
-    else
+__device__ __forceinline__ void traverse(P &p, Counters &cnt, const QueryArgs &a) {
+    if constexpr (WARP) {
+        __shared__ int2 s_entry[kThreads / 32][kStackSize];
+        int2 *const entry = s_entry[threadIdx.x >> 5];
+        int node = 0, sp = 0, budget = a.warp_budget;
+        while ((sp = traverse_packet<COUNT>(p, cnt, budget, entry, node, P::kRestarts ? 0 : sp)) >= 0) {
+            if (__any_sync(0xffffffffu, *(volatile int *)a.fallback_count < a.hand_most)) {
+                p.abandon();
+                break;
+            }
+            budget = 0;
+            if constexpr (P::kRestarts) {
+                p.restart();
+            } else {
+                node = next_entry(p, entry, sp);
+                if (node < 0) break;
+            }
+        }
+    } else {
         traverse_thread<COUNT>(p, cnt);
+    }
 }
 
 // ---- outputs ----------------------------------------------------------------------------------------
@@ -817,7 +841,7 @@ __device__ __forceinline__ void query_step(const QueryArgs &a, int step, const b
                 p.disable(s);
             }
         }
-        if (WARP || any) traverse<WARP, COUNT>(p, cnt, a.warp_budget);
+        if (WARP || any) traverse<WARP, COUNT>(p, cnt, a);
 #pragma unroll
         for (int s = 0; s < Q; s++) {
             if (!valid[s]) continue;
@@ -844,7 +868,7 @@ __device__ __forceinline__ void query_step(const QueryArgs &a, int step, const b
                 p.disable(s);
             }
         }
-        if (WARP || any) traverse<WARP, COUNT>(p, cnt, a.warp_budget);
+        if (WARP || any) traverse<WARP, COUNT>(p, cnt, a);
 #pragma unroll
         for (int s = 0; s < Q; s++) {
             if (!valid[s]) continue;
@@ -888,7 +912,7 @@ __device__ __forceinline__ void query_step(const QueryArgs &a, int step, const b
                 p.disable(s);
             }
         }
-        if (WARP || any) traverse<WARP, COUNT>(p, cnt, a.warp_budget);
+        if (WARP || any) traverse<WARP, COUNT>(p, cnt, a);
 #pragma unroll
         for (int s = 0; s < Q; s++) {
             if (!valid[s]) continue;
@@ -1579,7 +1603,8 @@ int launch_query_keep(const QueryArgs &args_in, int precision, cudaStream_t stre
     // plain FP64 kernel: the fix-up filter sees each such triangle through a wide proxy, whose keys
     // crowd the window. Both give the same bits.
     if (precision == SSDF_PREC_F32_FIXUP && fixup_runs_f64(a.m)) precision = SSDF_PREC_F64;
-    a.warp_budget = resolve_warp_budget(a.warp_budget, n, a.m.nt, a.is_grid != 0);
+    const bool forced_budget = a.warp_budget >= 0;
+    resolve_hand_over(&a, precision == SSDF_PREC_F32_FIXUP, n);
     if (a.output == SSDF_OUT_CLOSEST && (!a.m.tris64 || !a.outx || !a.outy || !a.outz || !a.outtri))
         return fail(SSDF_ERR_INVALID_ARGUMENT, "closest-point queries need outx/outy/outz/outtri and double data");
     if (precision == SSDF_PREC_F32 && (a.output == SSDF_OUT_SDF || a.output == SSDF_OUT_CLOSEST))
@@ -1621,7 +1646,8 @@ int launch_query_keep(const QueryArgs &args_in, int precision, cudaStream_t stre
         const bool fixup = precision == SSDF_PREC_F32_FIXUP;
         if (fixup && n >= 0x7fffffffll) {
             st = fail(SSDF_ERR_NOT_SUPPORTED, "more than 2^31 - 1 queries in one fix-up launch");
-        } else if (fixup || (warp && a.warp_budget > 0 && n <= kHandOverMaxQueries && !capturing(stream))) {
+        } else if (fixup || (warp && a.warp_budget > 0 && (forced_budget || budget_reachable(a)) &&
+                             n <= kHandOverMaxQueries && !capturing(stream))) {
             if (cudaMallocAsync(&fb, sizeof(int) * size_t(2 * n + 1), stream) != cudaSuccess) {
                 fb = nullptr;
                 if (fixup) st = fail(SSDF_ERR_OUT_OF_MEMORY, "fix-up overflow list");
@@ -1753,7 +1779,7 @@ int launch_query_noalloc(const QueryArgs &args_in, cudaStream_t stream) {
         a.warp_budget = 0;
         e = launch_prec<SSDF_PREC_F64>(a, warp, false, unsigned(nblocks), stream);
     } else {
-        a.warp_budget = resolve_warp_budget(a.warp_budget, n, a.m.nt, a.is_grid != 0);
+        resolve_hand_over(&a, true, n);
         int *scratch = nullptr;
         SSDF_CHECK(noalloc_scratch(&scratch));
         a.fallback_count = scratch;

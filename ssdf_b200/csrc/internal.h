@@ -1,6 +1,7 @@
 // internal.h -- shared declarations of the library's host runtime and kernels.
 #pragma once
 
+#include <algorithm>
 #include <cmath>
 
 #include <cuda_runtime.h>
@@ -129,8 +130,10 @@ struct QueryArgs {
     float tau_rel;
     // warp packets: a packet that has tested more than this many triangle records hands
     // its queries to the second stage (a warp per query) with their current windows; 0: no limit;
-    // < 0: the default for the launch's size (resolve_warp_budget)
+    // < 0: the default for the launch's size (resolve_hand_over)
     int warp_budget;
+    // they may while fewer queries than this are on the list (resolve_hand_over)
+    int hand_most;
     // hand-over list (query, threshold), finished by k_window; null without a budget
     int *fallback_ids;
     float *fallback_thr;
@@ -326,18 +329,40 @@ inline int grid_blocks(long long n, int threads) { return int((n + threads - 1) 
 // 748; 1,000,000 in its box 2,653: 10,229 / 6,473 / 2,882 / 2,102 / 2,054. Above 2^21 queries: 200^3 on 81,920
 // triangles 12,950 without, 7,040 / 6,518 / 6,641 / 7,572 at 500 / 700 / 1,000 / 1,500; 48 uneven meshes,
 // 42M queries in one batch, 44.2 ms without, 26.4 at 700; the knot's 256^3 unchanged.
-// SSDF_B200_WARP_BUDGET sets it for every launch (0 = no limit).
+// SSDF_B200_WARP_BUDGET sets it for every launch (0 = no limit), and then nothing below holds packets back.
 constexpr int kWarpBudgetMin = 64, kWarpBudgetMax = 700;
 constexpr long long kBudgetSmallLaunch = 1ll << 21;
 // Largest launch of the plain arithmetics (F64, F32) that keeps a hand-over list, 8 bytes a query.
 constexpr long long kHandOverMaxQueries = 1ll << 24;
-inline int resolve_warp_budget(int b, long long n, int ntri, bool grid) {
-    if (b >= 0) return b;
-    const double t = ntri > 0 ? ntri : 0;
+// How many queries of a launch (of a batch's job) may be handed over (QueryArgs::hand_most). The second stage shares
+// no triangle between queries: it is worth its 2 to 5 times a packet's work a query where the GPU would else wait
+// for a few packets, and not where most packets run out of budget, as among random overlapping triangles, or far from a
+// small mesh, whose packets a warp walk's fixed cost exceeds. Where it pays, few are handed over: up to 12,200 on
+// grids of up to 160^3 around spheres, tori and the knot; of points in their boxes 33,000 of 200,000, 82,000 of
+// 1,000,000. So 8,192 and a 64th of the launch on meshes below 2,048 triangles, 16,384 and a 64th on other grids,
+// 32,768 and a 16th (an 8th from 20,000 triangles on) of other point lists. Without a limit: launches too small to fill the
+// GPU either way, and fix-up launches up to 2^21 queries or on larger meshes, whose windows' double evaluations share
+// out well (64^3 nodes, 5,120 triangles at 1e4: 7,913 us without a budget, 3,437 with).
+// us without a budget, handing over without a limit, and by this rule: 127^3 nodes among 500 random triangles, float
+// 1,310 / 6,745 / 1,443; 160^3 among 20,000, fix-up 52,898 / 293,992 / 63,100; 1,000,000 points 30 sizes away from 320
+// triangles, float 562 / 1,870 / 609; from 131,072, double 26,689 / 17,321 / 26,421, the one that loses by it.
+inline void resolve_hand_over(QueryArgs *a, bool fixup, long long n_launch) {
+    a->hand_most = 0x7fffffff;
+    if (a->warp_budget >= 0) return;
+    const long long n = a->is_grid ? a->nx * a->ny * a->nz : a->npoints;
+    const double t = a->m.nt > 0 ? a->m.nt : 0;
     auto within = [](double v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : int(v)); };
-    if (n > kBudgetSmallLaunch) return within(3.0 * std::sqrt(t), 2 * kWarpBudgetMin, 1000);
-    return within(grid ? t / 40 : 1.2 * std::sqrt(t), kWarpBudgetMin, kWarpBudgetMax);
+    const bool grid = a->is_grid != 0, small = n_launch <= kBudgetSmallLaunch;
+    a->warp_budget = small ? within(grid ? t / 40 : 1.2 * std::sqrt(t), kWarpBudgetMin, kWarpBudgetMax)
+                           : within(3.0 * std::sqrt(t), 2 * kWarpBudgetMin, 1000);
+    const bool few = a->m.nt < 2048;
+    if (few ? n_launch <= 1 << 15 : (fixup ? small || a->m.nt > 24576 : n_launch <= (grid ? 1 << 17 : 1 << 16))) return;
+    const double base = few ? 8192 : (grid ? 16384 : 32768);
+    a->hand_most = int(std::max(1024.0, base * double(n) / double(n_launch)) +
+                       double(n / (few || grid ? 64 : (a->m.nt < 20000 ? 16 : 8))));
 }
+// Whether a budget can matter on a mesh: a packet tests a triangle at most once.
+inline bool budget_reachable(const QueryArgs &a) { return a.warp_budget > 0 && a.m.nt > 4ll * a.warp_budget; }
 // Point lists of at least this many queries are visited in Morton order (SSDF_B200_SORT_POINTS=0
 // keeps input order).
 constexpr long long kSortMinPoints = 4096;
