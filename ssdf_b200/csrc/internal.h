@@ -358,7 +358,9 @@ inline void resolve_hand_over(QueryArgs *a, bool fixup, long long n_launch) {
     const bool few = a->m.nt < 2048;
     if (few ? n_launch <= 1 << 15 : (fixup ? small || a->m.nt > 24576 : n_launch <= (grid ? 1 << 17 : 1 << 16))) return;
     const double base = few ? 8192 : (grid ? 16384 : 32768);
-    a->hand_most = int(std::max(1024.0, base * double(n) / double(n_launch)) +
+    // a batch's small jobs have their share of the launch's
+    const double part = std::max(double(n) / double(n_launch), std::min(1.0, double(n) / 262144.0));
+    a->hand_most = int(std::max(1024.0, base * part) +
                        double(n / (few || grid ? 64 : (a->m.nt < 20000 ? 16 : 8))));
 }
 // Whether a budget can matter on a mesh: a packet tests a triangle at most once.
