@@ -475,7 +475,7 @@ __device__ __forceinline__ R min_of(const R (&d)[Q]) {
 // Lanes that rank two children for their packet, of those that hold a query: a lane without one sits far
 // outside, where the children's order says nothing (asked all the same, at (1, 1, 1) of the 4 x 4 x 2 brick, a
 // 145^3 grid of the torus knot, whose last bricks have one column each, took 5,900 us against 2,900 for 144^3).
-// All of them vote: 262,144 points near the knot 862 -> 829 us, the beams' points 5,280 -> 5,235, 64^3 grid on
+// All of them vote: 500,003 points near the knot 862 -> 829 us, the beams' points 5,280 -> 5,235, 64^3 grid on
 // 5,120 triangles 226 -> 221. The double kernel follows one lane, (1, 1, 1) clamped to the brick's part inside
 // the grid (of a list's last packet: its last lane); counting the votes cost it 2 % (1,167 -> 1,195).
 template <class P>
@@ -977,7 +977,7 @@ __device__ __forceinline__ void query_block(const QueryArgs &a, long long block,
 // (a separate instantiation: the dormant signal code cost the fix-up kernel 3 % where it was merely
 // compiled in). The arguments are __grid_constant__: their address is passed on (to query_step,
 // map_query, write_result), and without it each thread first copies them to its local memory (64^3 grid on
-// 5,120 triangles 239 -> 224 us, 262,144 points near the knot 915 -> 889, 1,000 points 48 -> 43).
+// 5,120 triangles 239 -> 224 us, 500,003 points near the knot 915 -> 889, 1,000 points 48 -> 43).
 template <int PREC, bool WARP, bool COUNT, bool SIGNAL = false>
 __global__ void __launch_bounds__(kThreads, PREC == SSDF_PREC_F64 ? kF64MinBlocks : SSDF_B200_QUERY_MIN_BLOCKS)
     k_query(const __grid_constant__ QueryArgs a) {
