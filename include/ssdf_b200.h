@@ -415,7 +415,7 @@ int ssdf_mesh_stats(const ssdf_mesh *mesh, int64_t *nodes, int64_t *leaves, int6
 /* The fix-up path's view of a mesh (no counterpart in the reference): tau_rel, the relative width of
  * its FP32 window (tau = tau_rel (M + d), M the largest coordinate magnitude, d the distance; at least
  * 2^-16, wider for meshes of a few large triangles); float_filter, 1 when fix-up requests on it run the
- * FP32 filter, 0 when they run the FP64 kernel (coordinates beyond 2^28, triangles that rounding to
+ * FP32 filter, 0 when they run the FP64 kernel (coordinates beyond 2^28 or all below 2^-26, triangles that rounding to
  * float collapses or makes smaller than 2^-23, or more than half of its triangles slivers); slivers,
  * the triangles the filter sees through a proxy. Any pointer may be null. */
 int ssdf_mesh_filter_info(const ssdf_mesh *mesh, float *tau_rel, int *float_filter, int64_t *slivers);

@@ -511,7 +511,9 @@ void set_filter_window(DeviceMesh *m, float largest_term, bool records_safe) {
         tau = fmax(tau, u * (6.93 + 2.0 * double(largest_term) / M) * (1.0 + 0x1p-9));
     }
     m->tau_rel_min = float(tau) < tau ? nextafterf(float(tau), INFINITY) : float(tau);
-    m->filter_ok = records_safe && M <= double(kFilterMaxCoord) && tau <= 0x1p-8 ? 1 : 0;
+    // (a safe record that is not one point has M >= 2^-25; a mesh of points nearer the origin, or at it, would have a
+    // window whose square is 0, which holds nothing)
+    m->filter_ok = records_safe && M >= 0x1p-26 && M <= double(kFilterMaxCoord) && tau <= 0x1p-8 ? 1 : 0;
 }
 
 namespace {
