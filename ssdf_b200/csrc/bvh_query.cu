@@ -1276,7 +1276,7 @@ __global__ void __launch_bounds__(kThreads) k_window(const __grid_constant__ Que
 // A list too short to fill the GPU with 32-query packets is bound by one walk's serial chain. Here the 32
 // lanes share it: up to 32 nodes a step, so a walk takes about as many steps as the tree is deep, in one
 // launch without ordering the points, an overflow list or a second stage. It is bound by the latency of its
-// dependent loads (4,165 instructions a query, 30 % of issue slots busy). us against packets (fix-up, points
+// dependent loads (1,000 points on the sphere: 2,419 instructions a query, 13 % of issue slots busy). us against packets (fix-up, points
 // near the surface; 131,072-triangle knot, 1,280-triangle sphere): 100 points 57 / 244 and 44 / 106; 1,000
 // 59 / 320 and 46 / 98; 16,000 242 / 577 and 162 / 215; 65,536 836 / 620 and 508 / 214.
 template <int PREC, bool COUNT>
